@@ -116,6 +116,28 @@ def layer_gemv_call():
     return _layer_gemv_call
 
 
+_torch_call = None
+
+
+def torch_call():
+    """The ``_q4torch`` module (built in-tree on first use), bound to the loaded library: products on torch tensors as
+    one native call each.  Its functions return ``None`` for operands they do not take."""
+    global _torch_call
+    if _torch_call is not None:
+        return _torch_call
+    handle = lib()
+    with _lock:
+        if _torch_call is None:
+            if not os.path.exists(os.path.join(_PKG, "_q4torch.so")):
+                from . import build as _build
+                _build.build_torch_call()
+            from . import _q4torch
+            _q4torch.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
+                "q4_gemv", "q4_gemm_fwd_residual", "q4_gemm_bwd_table", "q4_gemm_bwd", "q4_swiglu_fwd", "q4_last_error_string")))
+            _torch_call = _q4torch
+    return _torch_call
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         msg = lib().q4_last_error_string().decode("utf-8", "replace")

@@ -157,25 +157,27 @@ class Autograd4bitQuantLinear(nn.Module):
         self.__dict__["_q4_residual"] = residual
 
     def forward(self, x):
-        residual = self.take_residual()
-        out = self._forward(x, residual)
-        return out
+        return self._forward(x, self.__dict__.pop("_q4_residual", None))
 
     def _forward(self, x, residual=None):
+        if self.bits == 4 and not torch.is_grad_enabled():
+            if backend != 'cuda':
+                raise ValueError('Backend not supported.')
+            b, v1 = self._buffers, self.is_v1_model            # (a buffer looked up as an attribute costs the host a microsecond a call)
+            if 'qweight' not in b or 'bias' not in b:          # registered as something else by whoever wrapped the module
+                b = {n: getattr(self, n, None) for n in ('qweight', 'scales', 'zeros', 'qzeros', 'g_idx', 'bias')}
+            return mm4b.linear(x, b['qweight'], b['scales'], b['zeros' if v1 else 'qzeros'], None if v1 else b['g_idx'],
+                               self.groupsize, None if self.disable_bias else b['bias'], residual)
         zeros = self.zeros if self.is_v1_model else self.qzeros
         if self.bits == 4:
-            if torch.is_grad_enabled():
-                if AutogradMatmul4bit is AutogradMatmul4bitCuda:
-                    # bias and residual ride in the product's epilogue instead of further passes over the output
-                    bias = None if (self.disable_bias or self.bias is None) else self.bias
-                    if residual is not None and residual.dtype != torch.float16:
-                        out = AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, bias)
-                        return out + residual.to(out.dtype)
-                    return AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, bias, residual)
-                out = AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq)
-            else:
-                out = matmul4bit_with_backend(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq,
-                                              self.groupsize)
+            if AutogradMatmul4bit is AutogradMatmul4bitCuda:
+                # bias and residual ride in the product's epilogue instead of further passes over the output
+                bias = None if (self.disable_bias or self.bias is None) else self.bias
+                if residual is not None and residual.dtype != torch.float16:
+                    out = AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, bias)
+                    return out + residual.to(out.dtype)
+                return AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, bias, residual)
+            out = AutogradMatmul4bit.apply(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq)
         elif self.bits == 2:
             out = AutogradMatmul2bit.apply(x, self.qweight, self.scales, self.qzeros, self.g_idx, self.bits, self.maxq)
         else:

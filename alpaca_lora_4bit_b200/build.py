@@ -86,6 +86,33 @@ def build_call(force: bool = False) -> str:
     return CALL_LIB
 
 
+TORCH_SRC = os.path.join(CSRC, "host", "q4torch.cpp")
+TORCH_LIB = os.path.join(PKG, "_q4torch.so")
+
+
+def build_torch_call(force: bool = False) -> str:
+    """Builds ``_q4torch.so`` (the CPython module that takes torch tensors through the library) with the C++ compiler,
+    against the headers and libraries of the installed torch."""
+    deps = [TORCH_SRC, os.path.join(ROOT, "include", "q4b200.h")]
+    if not force and os.path.exists(TORCH_LIB) and all(os.path.getmtime(TORCH_LIB) >= os.path.getmtime(d) for d in deps):
+        return TORCH_LIB
+    import sysconfig
+    import torch
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        raise RuntimeError("no C++ compiler; _q4torch.so cannot be built")
+    base = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    tmp = TORCH_LIB + ".tmp"
+    subprocess.check_call([cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           "-I", os.path.join(base, "include"), "-I", os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                           "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], TORCH_SRC, "-o", tmp,
+                           "-L", os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    os.replace(tmp, TORCH_LIB)
+    return TORCH_LIB
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
     print(build_call(force="--force" in sys.argv))
+    print(build_torch_call(force="--force" in sys.argv))

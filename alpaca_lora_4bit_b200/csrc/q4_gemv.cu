@@ -60,8 +60,14 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void store_y(const GemvParams& p, int b, int n, float v) {
-  if (p.bias) v += __half2float(p.bias[n]);
+// The bias of output column n, for callers that fetch it before they wait for the sums it is added to.  (A plain load:
+// cuda_fp16.h's __ldg of a __half is inline assembly without side effects, which the compiler may move out of the branch
+// that keeps it from a null pointer.)
+__device__ __forceinline__ float bias_of(const GemvParams& p, int n) {
+  if (p.bias == nullptr) return 0.f;
+  return __half2float(p.bias[n]);
+}
+__device__ __forceinline__ void store_y_biased(const GemvParams& p, int b, int n, float v) {
   const size_t o = (size_t)b * p.N + n;
   if (p.y_f32) {
     float* y = reinterpret_cast<float*>(p.y);
@@ -71,6 +77,7 @@ __device__ __forceinline__ void store_y(const GemvParams& p, int b, int n, float
     y[o] = __float2half_rn(p.accumulate ? __half2float(y[o]) + v : v);
   }
 }
+__device__ __forceinline__ void store_y(const GemvParams& p, int b, int n, float v) { store_y_biased(p, b, n, v + bias_of(p, n)); }
 
 // Cross-warp (shared memory) and cross-split (workspace) reduction; `red` is [8][MT*8][32].
 template <int MT>
@@ -1276,14 +1283,15 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
       named_bar_arrive(1, CT);
       return;
     }
-    named_bar_sync(1, CT);
     const int tc0 = tile * GEMV_TN, col = lane;
+    const float bv = bias_of(p, tc0 + col);        // on its way while the other warps finish
+    named_bar_sync(1, CT);
     const bool whole = seg_first == 0 && seg_last == upt - 1;
     float v = 0.f;
 #pragma unroll
     for (int w = 0; w < W; ++w) v += red[w * GEMV_TN + col];
     named_bar_arrive(2, CT);
-    if (whole) { store_y(p, 0, tc0 + col, v); return; }
+    if (whole) { store_y_biased(p, 0, tc0 + col, v + bv); return; }
     if (seg_first > 0) {
       // a later part of a tile another CTA owns: sum and flag in one 8-byte store (one store is atomic, so
       // the owner never sees a flag without its sum, and nothing has to be fenced)
@@ -1292,7 +1300,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
     }
     // the first part of a tile that later CTAs continue: their sums, collected by the helper warp
     if (!mbar_spin_bounded(rfull, 0, flags[0] ? 64u : 20000000u)) { flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED); }
-    store_y(p, 0, tc0 + col, v + remote[col]);
+    store_y_biased(p, 0, tc0 + col, v + remote[col] + bv);
   };
 
   int n = 0;
@@ -1665,12 +1673,13 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       __threadfence_block();
       named_bar_arrive(1, CT);
     } else {
+      const float bv = bias_of(p, tile * GEMV_TN + lane);
       named_bar_sync(1, CT);
       for (int r = 0; r < p.M; ++r) {
-        float v = 0.f;
+        float v = bv;
 #pragma unroll
         for (int w = 0; w < W; ++w) v += red[(w * MR + r) * GEMV_TN + lane];
-        store_y(p, r, tile * GEMV_TN + lane, v);
+        store_y_biased(p, r, tile * GEMV_TN + lane, v);
       }
       named_bar_arrive(2, CT);
     }

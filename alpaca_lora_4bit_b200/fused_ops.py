@@ -123,6 +123,10 @@ class _SwiGLUFused(torch.autograd.Function):
 def swiglu_fused(gu: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for ``gu = [gate | up]`` along the last dimension (the output of a fused gate_up
     projection); falls back to ``swiglu`` on the two halves where the kernel does not apply."""
+    if gu.is_cuda and not (torch.is_grad_enabled() and gu.requires_grad):      # nothing to differentiate: one native call
+        out = _lib.torch_call().swiglu(gu)
+        if out is not None:
+            return out
     I = gu.shape[-1] // 2
     if _fusable(gu) and gu.shape[-1] == 2 * I and I % 8 == 0 and gu.numel() > 0 and gu.is_contiguous() and gu.data_ptr() % 16 == 0:
         return _SwiGLUFused.apply(gu)

@@ -234,6 +234,18 @@ def decode_v2(x, qweight, scales, zeros, groupsize, plan_key=None):
     return y
 
 
+def gemv_new(x, qweight, scales, zeros, g_idx, bias, groupsize, flags):
+    """``x @ W (+ bias)`` for 1..16 rows ``x [..., K]`` in a new fp16 tensor through one native call (``_q4torch.gemv``:
+    checks, allocation and launch), or ``None`` for operands it does not take."""
+    idx = x.device.index
+    st = _raw_stream(idx)
+    w = _decode_ws.get((idx, st))
+    if w is None:
+        t = _lib.workspace_for(x.device, st)
+        w = _decode_ws[(idx, st)] = (t.data_ptr(), t.numel(), t)
+    return (_lib._torch_call or _lib.torch_call()).gemv(x, qweight, scales, zeros, g_idx, bias, groupsize, flags, w[2])
+
+
 _gemm_ws_bytes: dict = {}
 
 
@@ -286,6 +298,30 @@ def _zero_terms(scales, zeros, G, N, st):
     return table
 
 
+def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, residual=None, lora_u=None, lora_w=None):
+    """The product of ``gemm`` for ``x [..., K]`` (transpose: ``[..., N]``) through one native call (``_q4torch.gemm``),
+    into ``out`` or, with ``out=None``, a new tensor; ``None`` - and nothing done - for operands it does not take."""
+    dev = x.device
+    idx = dev.index
+    if idx != _current_device() or qweight.dim() != 2 or scales.dim() != 2:
+        return None
+    K, N, G = qweight.shape[0] * 8, qweight.shape[1], scales.shape[0]
+    st = _raw_stream(idx)
+    need = _gemm_ws_bytes.get((K, N, G))
+    if need is None:
+        need = _gemm_ws_bytes[(K, N, G)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, G))
+    ws = _lib._gemm_workspaces.get((idx, st))
+    if ws is None or ws.numel() < need:
+        ws = _lib.gemm_workspace_for(dev, st, need)
+    zt, seq_gs = None, 0
+    if cache_zero_terms and scales.dtype is _F16 and scales.is_cuda and scales.is_contiguous() and zeros.is_contiguous():
+        # forward: see the comment in gemm()
+        if transpose or (N % 256 == 0 and K % G == 0 and groups_are_sequential(g_idx, G)):
+            zt = _zero_terms(scales, zeros, G, N, st)
+            seq_gs = K // G if (zt is not None and not transpose and promise_sequential_groups) else 0
+    return (_lib._torch_call or _lib.torch_call()).gemm(x, qweight, out, scales, zeros, g_idx, bias, residual, lora_u, lora_w, transpose, zt, seq_gs, ws)
+
+
 def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora_u=None, lora_w=None, residual=None) -> None:
     """Fused large-M product on the tensor cores: ``out = x @ W (+ bias)`` or, with ``transpose``,
     ``out = x @ W.T``; ``x``, ``out``, ``scales`` fp16, W never leaves shared memory.
@@ -294,6 +330,10 @@ def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora
     the same kernel: forward ``+ lora_u[:, :r] @ lora_w.T`` with ``lora_w = lora_B [N, r]``; transpose
     ``+ lora_u[:, :r] @ lora_w`` with ``lora_w = lora_A [r, K]``.  ``residual`` fp16 ``[M, N]`` (forward only) is
     added to the rounded product in the epilogue: ``out = half(half(x @ W + bias) + residual)``."""
+    if x.is_cuda and x.dim() == 2 and x.shape[0] > 0 and out.dim() == 2 and out.shape[0] == x.shape[0]:
+        if gemm_new(x, qweight, out, scales, zeros, g_idx, transpose, bias, residual, lora_u, lora_w) is not None:
+            return
+    # operands the native call does not take: say what is wrong, or run them from another current device
     dev = _lib.require_cuda(x, qweight, out, scales, zeros, g_idx, bias, lora_u, lora_w, residual)
     R, N = qweight.shape
     K = R * 8

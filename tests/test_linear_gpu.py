@@ -1,0 +1,68 @@
+"""The no-grad forward of the quant linear module through the native call: bias and residual in the kernels'
+epilogues, every row range and layer format, against the oracle's reconstruct."""
+import pytest
+import torch
+
+from alpaca_lora_4bit_b200 import autograd_4bit as a4, matmul_utils_4bit as mm4b, quant_cuda, synth
+from oracle import q4_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+K, N = 512, 768
+
+
+def build(fmt, groupsize):
+    layer = synth.make_layer(K, N, groupsize, act_order=fmt == "act", seed=3)
+    mod = a4.Autograd4bitQuantLinear(K, N, groupsize=-1 if fmt == "v1" else groupsize, is_v1_model=fmt == "v1")
+    gen = torch.Generator().manual_seed(4)
+    bias = torch.randn(N, generator=gen).half()
+    if fmt == "v1":
+        scales = (torch.rand(N, 1, generator=gen) * 0.018 + 0.002).half()
+        zeros = (scales.float() * torch.randint(1, 16, (N, 1), generator=gen)).half()
+        mod.scales, mod.zeros = scales.to(DEV), zeros.to(DEV)
+        w = orc.recons_v1(layer.qweight, scales.reshape(-1), zeros.reshape(-1))
+    else:
+        mod.scales, mod.qzeros, mod.g_idx = layer.scales.to(DEV), layer.qzeros.to(DEV), layer.g_idx.to(DEV)
+        w = orc.recons_v2(layer.qweight, layer.scales, layer.qzeros, layer.g_idx)
+    mod.qweight, mod.bias = layer.qweight.to(DEV), bias.to(DEV)
+    return mod.eval(), w.float(), bias.float()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8, 9, 16, 17, 33, 129, 300])
+@pytest.mark.parametrize("fmt,groupsize", [("seq", 128), ("seq", 32), ("act", 128), ("v1", 512)])
+def test_module_without_grad_adds_bias_and_residual(fmt, groupsize, rows):
+    mod, w, bias = build(fmt, groupsize)
+    gen = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, K, generator=gen).half()
+    res = torch.randn(rows, N, generator=gen).half()
+    mm4b.act_order = fmt == "act"
+    try:
+        with torch.no_grad():
+            y = mod(x.to(DEV))
+            y3 = mod(x.to(DEV).reshape(1, rows, K))
+            mod.offer_residual(res.to(DEV))
+            yr = mod(x.to(DEV))
+            mod.disable_bias = True
+            yn = mod(x.to(DEV))
+    finally:
+        mm4b.act_order = False
+    torch.cuda.synchronize()
+    want = x.float() @ w
+    for got, ref in ((y, want + bias), (yr, want + bias + res.float()), (yn, want)):
+        # fp16 result of sums in fp32; decode kernels work on the exact weights, the reference on their fp16 rounding
+        assert float((got.float().cpu() - ref).norm() / ref.norm()) <= 2e-3
+    assert y3.shape == (1, rows, N) and torch.equal(y3.reshape(rows, N), y)
+    assert quant_cuda.device_status() == 0
+
+
+def test_native_call_leaves_operands_it_does_not_take():
+    mod, w, bias = build("seq", 128)
+    x = torch.randn(4, K, generator=torch.Generator().manual_seed(1))
+    ref = x @ w + bias
+    with torch.no_grad():
+        for xx in (x.half().to(DEV).t().contiguous().t(), x.to(DEV), x.bfloat16().to(DEV)):     # not contiguous, fp32, bf16
+            y = mod(xx)
+            assert float((y.float().cpu() - ref).norm() / ref.norm()) <= 1e-2 and y.shape == (4, N)
+        assert mod(x[:0].half().to(DEV)).shape == (0, N)
+        with pytest.raises((RuntimeError, AssertionError)):
+            mod(torch.zeros(4, K + 128, dtype=torch.float16, device=DEV))
