@@ -1687,19 +1687,32 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 }
 
 // ---- act-order (group of row k = g_idx[k]) -------------------------------------------------------
-// Scale and (z+1) of the CTA's 32 columns for every group live in shared memory as half2
-// (s, z+1); every element is dequantised as s*(q - (z+1)) in fp16 pairs before the MMA.
-// The four lanes that share the columns 4g..4g+3 (t = 0..3) hold different k-rows, hence different
-// groups: reading one table they would meet on the same bank in different rows.  The table is
-// therefore kept four times, copy t with the columns of every quad rotated by t, so that the 32
-// lanes of a lookup fall on 32 different banks whatever their groups are (copies = 4; layers with so
-// many groups that four copies do not fit keep one, copies = 1).
+// Every element is dequantised as s*(q - (z+1)) in fp16 pairs before the MMA, with scale and zero point of its own
+// row's group from a shared-memory table of the CTA's 32 columns.  What bounds it: with a 4-byte entry looked up
+// per weight, unpacked pair by pair, the launch waited for shared memory and for the integer pipe (27.7 us on
+// average over the seven projections of a 13B block, where HBM needs 3.5).  Here
+//   * a table entry is the four scales and the four 1024 + z + 1 of a quad of columns, 16 bytes: one LDS.128 serves
+//     the four weights a lane has of a row, and a subtraction from the raw 1024 + q leaves q - (z+1) exactly;
+//   * the rows' table offsets are written to shared memory once per CTA instead of being read and scaled per step;
+//   * packed words and x are fetched ACT_AHEAD steps ahead into registers, the tables and the first words before
+//     the wait for the earlier kernel (programmatic launch), and several CTAs share an SM, so that one's tables are
+//     built while the others multiply.
+// The four lanes t = 0..3 of a quad of columns hold different rows, hence different groups.  A quarter-warp (two
+// quads of columns) reads 8 x 16 bytes: the table is kept four times, copy t of a pair of quads in the t-th 32 bytes
+// of a 128-byte line, so that its lanes fall on different banks whatever their groups are.  Layers with so many groups
+// that three CTAs with four copies do not fit an SM keep two copies, or one.
+constexpr int ACT_AHEAD = 3;
+constexpr size_t ACT_SMEM_TARGET = 74 * 1024;              // three CTAs per SM
+constexpr int ACT_MAX_STEPS = 192;
+constexpr size_t ACT_PART_BYTES = 3584 * 1024;
+constexpr size_t ACT_SMEM_LIMIT = 226 * 1024;              // the reduction has a word of static shared memory
+
 template <int MT>
-__global__ void __launch_bounds__(GEMV_THREADS)
-gemv_act_kernel(const GemvParams p, int G, int copies) {
+__global__ void __launch_bounds__(GEMV_THREADS, MT == 1 ? 3 : 2)
+gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* red = reinterpret_cast<float*>(smem_raw);                              // [8][MT*8][32]
-  __half2* tab = reinterpret_cast<__half2*>(smem_raw + sizeof(float) * GEMV_WARPS * MT * 8 * GEMV_TN);  // [G][4 copies][32]
+  unsigned char* tab = smem_raw + sizeof(float) * GEMV_WARPS * MT * 8 * GEMV_TN;   // [G][4 pairs of quads][copies][32 bytes]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int c0 = blockIdx.x * GEMV_TN;
@@ -1707,17 +1720,30 @@ gemv_act_kernel(const GemvParams p, int G, int copies) {
   const int sb = split * p.steps_per_split;
   const int se = min(sb + p.steps_per_split, p.steps_total);
   const int N = p.N, K = p.K;
+  const int pitch = copies * 128;                                               // bytes of the table per group
+  int* offs = reinterpret_cast<int*>(tab + (size_t)G * pitch);                  // table offset of every row of the split (if staged)
+  auto offset_of = [&](int grp) { return (int)min((unsigned)grp, (unsigned)(G - 1)) * pitch; };
 
-  for (int i = threadIdx.x; i < G * GEMV_TN; i += GEMV_THREADS) {
-    const int grp = i >> 5, col = i & 31;
-    const uint32_t zw = p.qzeros[(size_t)grp * (N >> 3) + ((c0 + col) >> 3)];
-    const unsigned z1 = ((zw >> (4 * (col & 7))) & 0xF) + 1;
-    const __half2 e = __halves2half2(p.scales[(size_t)grp * N + c0 + col], __ushort2half_rn((unsigned short)z1));
+  pdl_launch_dependents();
+  const uint32_t* wp = p.qw + (size_t)t * N + c0 + 4 * g;
+  uint4 wv[ACT_AHEAD];
 #pragma unroll
-    for (int tt = 0; tt < 4; ++tt)
-      if (tt < copies) tab[(grp * copies + tt) * GEMV_TN + (col & ~3) + ((col + tt) & 3)] = e;
+  for (int i = 0; i < ACT_AHEAD; ++i) {
+    const int step = sb + warp + i * GEMV_WARPS;
+    wv[i] = step < se ? ldg_stream(wp + (size_t)(4 * step) * N) : make_uint4(0, 0, 0, 0);
   }
-  __syncthreads();
+  for (int i = threadIdx.x; i < G * 8; i += GEMV_THREADS) {
+    const int grp = i >> 3, quad = i & 7;
+    const uint2 s4 = __ldg(reinterpret_cast<const uint2*>(p.scales + (size_t)grp * N + c0 + 4 * quad));
+    const uint32_t zw = __ldg(p.qzeros + (size_t)grp * (N >> 3) + ((c0 + 4 * quad) >> 3)) >> (16 * (quad & 1));
+    // 1024 + z + 1: the mantissa of 0x6400 plus one
+    const uint32_t z01 = ((zw & 0xFu) | ((zw & 0xF0u) << 12)) + 0x64016401u, z23 = (((zw >> 8) & 0xFu) | ((zw & 0xF000u) << 4)) + 0x64016401u;
+    const uint4 e = make_uint4(s4.x, s4.y, z01, z23);
+    unsigned char* at = tab + (size_t)grp * pitch + (quad >> 1) * copies * 32 + (quad & 1) * 16;
+    for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + c * 32) = e;
+  }
+  if (staged)
+    for (int i = threadIdx.x; i < (se - sb) * 32; i += GEMV_THREADS) offs[i] = offset_of(__ldg(p.g_idx + sb * 32 + i));
 
   float yacc[MT][2][4];
 #pragma unroll
@@ -1727,59 +1753,93 @@ gemv_act_kernel(const GemvParams p, int G, int copies) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) yacc[mt][j][i] = 0.f;
 
-  const uint32_t* wp = p.qw + (size_t)t * N + c0 + 4 * g;
+  pdl_wait();                                    // x, y and the workspace belong to the stream order
   const __half* xp0 = p.x + (size_t)g * K + 8 * t;
-  const bool xok0 = g < p.M, xok1 = (g + 8) < p.M;
-  const int tc = copies == 4 ? t : 0, tstride = copies * GEMV_TN;
-  const __half2* tabt = tab + tc * GEMV_TN + 4 * g;               // this lane's copy, its quad of columns
-  const int qpos[4] = {tc & 3, (tc + 1) & 3, (tc + 2) & 3, (tc + 3) & 3};   // where column 4g + q sits in that copy
+  auto load_x = [&](int step, uint4 (&xv)[MT]) __attribute__((always_inline)) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+      xv[mt] = step < se && g + 8 * mt < p.M ? __ldg(reinterpret_cast<const uint4*>(xp0 + (size_t)(8 * mt) * K + 32 * step)) : make_uint4(0, 0, 0, 0);
+  };
+  uint4 xv[ACT_AHEAD][MT];
+#pragma unroll
+  for (int i = 0; i < ACT_AHEAD; ++i) load_x(sb + warp + i * GEMV_WARPS, xv[i]);
+  __syncthreads();
+  // this lane's quad of columns in its copy (copies = 2 or 1: several t share one)
+  const unsigned char* tabt = tab + (g >> 1) * copies * 32 + (t & (copies - 1)) * 32 + (g & 1) * 16;
 
-  for (int step = sb + warp; step < se; step += GEMV_WARPS) {
-    const uint4 wv = ldg_stream(wp + (size_t)(4 * step) * N);
-    const int k0 = 32 * step + 8 * t;
-    const int4 ga = __ldg(reinterpret_cast<const int4*>(p.g_idx + k0));
-    const int4 gb = __ldg(reinterpret_cast<const int4*>(p.g_idx + k0 + 4));
-    const int gi[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
-    const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
-    uint32_t pr[4][4];                        // pr[word][m] = (w_m, w_m+4) dequantised
+  auto one_step = [&](int step, const uint4& w4, const uint4 (&xq)[MT]) __attribute__((always_inline)) {
+    int4 oa, ob;
+    if (staged) {
+      oa = *reinterpret_cast<const int4*>(offs + (step - sb) * 32 + 8 * t);
+      ob = *reinterpret_cast<const int4*>(offs + (step - sb) * 32 + 8 * t + 4);
+    } else {
+      oa = __ldg(reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t));
+      ob = __ldg(reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t + 4));
+      oa = make_int4(offset_of(oa.x), offset_of(oa.y), offset_of(oa.z), offset_of(oa.w));
+      ob = make_int4(offset_of(ob.x), offset_of(ob.y), offset_of(ob.z), offset_of(ob.w));
+    }
+    const int o[8] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
+    const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int ks = 0; ks < 2; ++ks) {
+      uint32_t pr[4][2];                        // pr[word][i] = rows m and m + 4 of the word, dequantised, m = 2 ks + i
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const uint32_t raw = and_or(w[q] >> (4 * m), 0x000F000Fu, 0x64006400u);
-        const __half2 qq = __hsub2(as_h2(raw), as_h2(0x64006400u));              // (q_m, q_m+4)
-        const __half2 ta = tabt[gi[m] * tstride + qpos[q]], tb = tabt[gi[m + 4] * tstride + qpos[q]];
-        const __half2 sv = __lows2half2(ta, tb), zv = __highs2half2(ta, tb);
-        pr[q][m] = as_u32(__hmul2(sv, __hsub2(qq, zv)));
+      for (int i = 0; i < 2; ++i) {
+        const uint4 ea = *reinterpret_cast<const uint4*>(tabt + o[2 * ks + i]), eb = *reinterpret_cast<const uint4*>(tabt + o[2 * ks + i + 4]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t sel = (q & 1) ? 0x7632 : 0x5410;
+          const uint32_t s2 = q < 2 ? prmt(ea.x, eb.x, sel) : prmt(ea.y, eb.y, sel);
+          const uint32_t z2 = q < 2 ? prmt(ea.z, eb.z, sel) : prmt(ea.w, eb.w, sel);
+          const uint32_t ww = ks ? w[q] >> 8 : w[q];
+          // even m: the low nibbles as 1024 + q; odd m: the high nibbles where they sit as 64 + q, and 960 less to take off
+          const uint32_t v = i ? and_or(ww, 0x00F000F0u, 0x54005400u) : and_or(ww, 0x000F000Fu, 0x64006400u);
+          const __half2 zz = i ? __hsub2(as_h2(z2), as_h2(0x63806380u) /* 960 */) : as_h2(z2);
+          pr[q][i] = as_u32(__hmul2(as_h2(s2), __hsub2(as_h2(v), zz)));
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const uint32_t sel0 = 0x5410, sel1 = 0x7632;
+        const uint32_t b0 = ks ? prmt(xq[mt].y, xq[mt].w, sel0) : prmt(xq[mt].x, xq[mt].z, sel0);
+        const uint32_t b1 = ks ? prmt(xq[mt].y, xq[mt].w, sel1) : prmt(xq[mt].x, xq[mt].z, sel1);
+        mma16816(yacc[mt][0], pr[0][0], pr[1][0], pr[0][1], pr[1][1], b0, b1);
+        mma16816(yacc[mt][1], pr[2][0], pr[3][0], pr[2][1], pr[3][1], b0, b1);
       }
     }
+  };
+  for (int step = sb + warp; step < se;) {
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const bool ok = mt ? xok1 : xok0;
-      const uint4 xq = ok ? __ldg(reinterpret_cast<const uint4*>(xp0 + (size_t)(8 * mt) * K + 32 * step))
-                          : make_uint4(0, 0, 0, 0);
-      const uint32_t xb[4] = {prmt(xq.x, xq.z, 0x5410), prmt(xq.x, xq.z, 0x7632),
-                              prmt(xq.y, xq.w, 0x5410), prmt(xq.y, xq.w, 0x7632)};
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        const uint32_t b0 = xb[2 * ks], b1 = xb[2 * ks + 1];
-        mma16816(yacc[mt][0], pr[0][2 * ks], pr[1][2 * ks], pr[0][2 * ks + 1], pr[1][2 * ks + 1], b0, b1);
-        mma16816(yacc[mt][1], pr[2][2 * ks], pr[3][2 * ks], pr[2][2 * ks + 1], pr[3][2 * ks + 1], b0, b1);
+    for (int i = 0; i < ACT_AHEAD; ++i) {
+      if (step < se) {                           // warp-uniform
+        const int ahead = step + ACT_AHEAD * GEMV_WARPS;
+        one_step(step, wv[i], xv[i]);
+        wv[i] = ahead < se ? ldg_stream(wp + (size_t)(4 * ahead) * N) : make_uint4(0, 0, 0, 0);
+        load_x(ahead, xv[i]);
       }
+      step += GEMV_WARPS;
     }
   }
   gemv_reduce_store<MT>(p, red, yacc, c0, split);
 }
 
+// Splits of the contraction for the act-order kernel: CTAs per SM times what one of them costs in steps (its own and
+// about ten for its tables, its reduction and the exchange), with no fewer than three CTAs' worth on an SM counted: fewer
+// leave it waiting for latency.  A CTA keeps the table offsets of its rows, so a split has at most ACT_MAX_STEPS steps -
+// as long as the partial sums of 16 rows stay within ACT_PART_BYTES.
 static void gemv_plan(int K, int N, int& S, int& steps_per_split) {
-  const int tiles = N / GEMV_TN, steps = K / 32;
-  int want = (592 + tiles - 1) / tiles;                 // about four CTAs per SM
-  int cap = steps / 32; if (cap < 1) cap = 1;           // keep >= 1024 rows per split
-  S = want < cap ? want : cap;
-  if (S < 1) S = 1;
-  steps_per_split = (steps + S - 1) / S;
-  steps_per_split = (steps_per_split + 3) / 4 * 4;
-  S = (steps + steps_per_split - 1) / steps_per_split;
+  const int tiles = N / GEMV_TN, steps = K / 32, sms = 148;      // (a constant: the workspace is sized without a device)
+  long long best = -1;
+  S = 1; steps_per_split = (steps + GEMV_WARPS - 1) / GEMV_WARPS * GEMV_WARPS;
+  for (int want = 1; want <= 64; ++want) {
+    const int per = ((steps + want - 1) / want + GEMV_WARPS - 1) / GEMV_WARPS * GEMV_WARPS;
+    const int s = (steps + per - 1) / per;
+    if (s > 1 && (size_t)s * 16 * N * sizeof(float) > ACT_PART_BYTES) break;
+    const long long ctas = ((long long)tiles * s + sms - 1) / sms;
+    long long cost = (ctas < 3 ? 3 : ctas) * (per + 10);
+    if (per > ACT_MAX_STEPS) cost *= 4;
+    if (best < 0 || cost < best) { best = cost; S = s; steps_per_split = per; }
+  }
 }
 
 // What q4_layer_gemv knows about the layer that follows (set around its call of q4_gemv, on the calling thread)
@@ -1794,6 +1854,27 @@ constexpr size_t GEMV_WS_SLOTS = 65536;                     // 256-byte exchange
 constexpr int GEMV_WS_MAX_CTAS = 255;                       // slots that fit (the last 256 bytes hold the leave signal)
 constexpr int GEMV_MAX_CTAS = 508;                            // upper bound on SMs for workspace sizing (4 slots' worth of
                                                               // room is kept for the 256 bytes ahead of the partial sums)
+
+template <int MT>
+static int launch_act(const GemvParams& p, int G, int copies, int staged, size_t smem, cudaStream_t st) {
+  static std::atomic<bool> attr_done[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
+    if (int e = check_cuda(cudaFuncSetAttribute(gemv_act_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ACT_SMEM_LIMIT), "gemv smem attribute")) return e;
+    if (int e = check_cuda(cudaFuncSetAttribute(gemv_act_kernel<MT>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared),
+                           "gemv carveout attribute")) return e;
+    if (dev >= 0 && dev < 64) attr_done[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.N / GEMV_TN, p.S); cfg.blockDim = dim3(GEMV_THREADS);
+  cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, gemv_act_kernel<MT>, p, G, copies, staged), "gemv launch");
+}
 
 template <int MT, bool FAST, bool XS>
 static int launch_stream(const CUtensorMap& map, const CUtensorMap& smap, const CUtensorMap& zmap,
@@ -2192,19 +2273,15 @@ extern "C" int q4_gemv(const void* x, const int32_t* qweight, void* y, const voi
     return fast ? launch_stream<2, true, false>(map, smap, zmap, sp, grid, st) : launch_stream<2, false, false>(map, smap, zmap, sp, grid, st);
   }
 
-  const dim3 grid(N / GEMV_TN, p.S), block(GEMV_THREADS);
-  const size_t red_bytes = sizeof(float) * GEMV_WARPS * MT * 8 * GEMV_TN;
-  const int copies = red_bytes + (size_t)G * 4 * GEMV_TN * sizeof(__half2) <= 100 * 1024 ? 4 : 1;   // two CTAs per SM at least
-  const size_t smem = red_bytes + (size_t)G * copies * GEMV_TN * sizeof(__half2);
-  if (smem > 200 * 1024) return fail(Q4_E_SHAPE, "gemv: act-order tables for G=%d groups do not fit shared memory", G);
-  if (MT == 1) {
-    if (int e = check_cuda(cudaFuncSetAttribute(gemv_act_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemv smem attr")) return e;
-    gemv_act_kernel<1><<<grid, block, smem, st>>>(p, G, copies);
-  } else {
-    if (int e = check_cuda(cudaFuncSetAttribute(gemv_act_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemv smem attr")) return e;
-    gemv_act_kernel<2><<<grid, block, smem, st>>>(p, G, copies);
-  }
-  return check_cuda(cudaGetLastError(), "gemv launch");
+  // four copies of the table while three CTAs fit an SM, else two, else one; the rows' offsets beside it where they fit at all
+  const size_t red_bytes = sizeof(float) * GEMV_WARPS * MT * 8 * GEMV_TN, offs_bytes = (size_t)p.steps_per_split * 32 * sizeof(int);
+  if (red_bytes + (size_t)G * 128 > 200 * 1024) return fail(Q4_E_SHAPE, "gemv: act-order tables for G=%d groups do not fit shared memory", G);
+  int copies = 4;
+  while (copies > 1 && red_bytes + offs_bytes + (size_t)G * copies * 128 > ACT_SMEM_TARGET) copies >>= 1;
+  size_t smem = red_bytes + (size_t)G * copies * 128;
+  const int staged = smem + offs_bytes <= ACT_SMEM_LIMIT ? 1 : 0;
+  if (staged) smem += offs_bytes;
+  return MT == 1 ? launch_act<1>(p, G, copies, staged, smem, st) : launch_act<2>(p, G, copies, staged, smem, st);
 }
 
 

@@ -173,6 +173,25 @@ def test_gemv_act_order(K, N, g, M):
     assert rel_fro(gemv_gpu(layer, x, torch.float32, _lib.GEMV_ACT_ORDER), want) <= REL_TOL
 
 
+@pytest.mark.parametrize("K,N,g", [(32, 32, 32),            # one step, one group: most warps idle
+                                   (2080, 96, 32),          # steps that neither splits nor warps divide, 65 groups
+                                   (16384, 32, 64),         # 256 groups: two copies of the table
+                                   (16384, 64, 32),         # 512 groups: one copy
+                                   (28672, 4096, 128),      # several splits, 224 groups
+                                   (4096, 65536, 128)])     # partial sums of two splits would not fit: one split
+@pytest.mark.parametrize("M", [1, 3, 9, 16])
+def test_gemv_act_order_table_forms(K, N, g, M):
+    """Every form of the table of the act-order kernel (copies, splits, remainders of warps), against the product with
+    the reconstructed weights in fp32; fp16 dequantised weights on both sides, so only the order of the sums differs."""
+    layer = synth.make_layer(K, N, g, act_order=True, seed=K + N + M).to(DEV)
+    x = synth.make_acts(M, K, seed=M).to(DEV)
+    w = torch.empty((K, N), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v2(layer.qweight, w, layer.scales, layer.qzeros, layer.g_idx)
+    want = torch.cat([x.float() @ w[:, c:c + 8192].float() for c in range(0, N, 8192)], dim=1)
+    y = gemv_gpu(layer, x, torch.float32, _lib.GEMV_ACT_ORDER)
+    assert rel_fro(y, want.cpu()) <= REL_TOL
+
+
 @pytest.mark.parametrize("K,N,g,M", [(32, 32, 32, 1), (64, 32, 32, 5), (4096, 32, 128, 2), (2048, 4096, 64, 7),
                                      (8192, 1024, -1, 16), (1056, 64, 96, 3)])
 def test_gemv_ragged_sizes(K, N, g, M):
