@@ -49,6 +49,8 @@ _SIGNATURES = {
     "q4_zero_term_table": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "q4_gemm_fwd_residual": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "q4_gemm_fwd_v1": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                               c_size_t, c_void_p]),
     "q4_gemm_fwd_table": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "q4_gemm_bwd_table": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -133,7 +135,7 @@ def torch_call():
                 _build.build_torch_call()
             from . import _q4torch
             _q4torch.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
-                "q4_gemv", "q4_gemm_fwd_residual", "q4_gemm_bwd_table", "q4_gemm_bwd", "q4_swiglu_fwd", "q4_last_error_string")))
+                "q4_gemv", "q4_gemm_fwd_residual", "q4_gemm_bwd_table", "q4_gemm_bwd", "q4_swiglu_fwd", "q4_last_error_string", "q4_gemm_fwd_v1")))
             _torch_call = _q4torch
     return _torch_call
 

@@ -50,9 +50,7 @@ class AutogradMatmul4bitCuda(torch.autograd.Function):
         projection): added in the epilogue of the fused product where that runs."""
         ctx.save_for_backward(qweight, scales, zeros, g_idx)
         if g_idx is None:
-            out = mm4b._matmul4bit_v1_recons(x, qweight, scales, zeros)
-            out = out if bias is None else out + bias.to(out.dtype)
-            return out if residual is None else out + residual.to(out.dtype)
+            return mm4b._matmul4bit_v1_recons(x, qweight, scales, zeros, bias=bias, residual=residual)
         return mm4b._matmul4bit_v2_recons(x, qweight, scales, zeros, g_idx, bias=bias, residual=residual)
 
     @staticmethod

@@ -28,6 +28,7 @@ struct Entry {
   decltype(&q4_gemm_bwd) bwd;
   decltype(&q4_swiglu_fwd) swiglu;
   decltype(&q4_last_error_string) error;
+  decltype(&q4_gemm_fwd_v1) v1;
 } g = {};
 
 // A tensor argument, or null for None (and for anything that is no tensor).
@@ -136,6 +137,34 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// gemm_v1(x, qweight, scales, zeros, bias | None, residual | None, workspace) -> y | None: a layer of the first format;
+// x [..., K] fp16
+PyObject* py_gemm_v1(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const at::Tensor *x = nullptr, *qw, *sc, *zr, *ws;
+  if (n != 7 || !(x = tensor(a[0])) || !(qw = tensor(a[1])) || !(sc = tensor(a[2])) || !(zr = tensor(a[3])) || !(ws = tensor(a[6]))) Py_RETURN_NONE;
+  const at::Tensor *bi = tensor(a[4]), *res = tensor(a[5]);
+  if (!x->is_cuda()) Py_RETURN_NONE;
+  const int dev = x->get_device();
+  int64_t K, N, G;
+  if (!plain(*x, at::kHalf, dev) || x->dim() < 1 || !layer_ok(*qw, *sc, *zr, true, dev, &K, &N, &G)) Py_RETURN_NONE;
+  if (K == 0 || N == 0 || K % 128 || N % 256 || x->size(-1) != K) Py_RETURN_NONE;
+  const int64_t M = x->numel() / K;
+  if (M < 1 || M > INT32_MAX) Py_RETURN_NONE;
+  if (bi && (!plain(*bi, at::kHalf, dev) || bi->numel() != N)) Py_RETURN_NONE;
+  if (res && (!plain(*res, at::kHalf, dev) || res->numel() != M * N)) Py_RETURN_NONE;
+  for (const at::Tensor* t : {x, qw, sc, zr, res})                 // (the bias is read by the element)
+    if (t && (uintptr_t)t->data_ptr() % 16) Py_RETURN_NONE;
+  if (!ws->is_cuda() || ws->get_device() != dev) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(dev);
+  at::Tensor out = new_rows(*x, N);
+  const int rc = g.v1(x->data_ptr(), (const int32_t*)qw->data_ptr(), out.data_ptr(), sc->data_ptr(), zr->data_ptr(), ptr(bi), ptr(res),
+                      (int)M, (int)K, (int)N, ws->data_ptr(), (size_t)ws->numel(), c10::cuda::getCurrentCUDAStream(dev).stream());
+  if (rc) return failed("gemm_v1", rc);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
 // swiglu(gu) -> silu(gate) * up | None for gu = [..., gate | up] fp16 (no gradient)
 PyObject* py_swiglu(PyObject*, PyObject* arg) {
   HANDLE_TH_ERRORS
@@ -153,16 +182,16 @@ PyObject* py_swiglu(PyObject*, PyObject* arg) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses of q4_gemv, q4_gemm_fwd_residual, q4_gemm_bwd_table, q4_gemm_bwd, q4_swiglu_fwd, q4_last_error_string)
+// bind(addresses of q4_gemv, q4_gemm_fwd_residual, q4_gemm_bwd_table, q4_gemm_bwd, q4_swiglu_fwd, q4_last_error_string, q4_gemm_fwd_v1)
 PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  void* p[6];
-  if (n != 6) { PyErr_SetString(PyExc_TypeError, "bind takes 6 addresses"); return nullptr; }
-  for (int i = 0; i < 6; ++i) {
+  void* p[7];
+  if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind takes 7 addresses"); return nullptr; }
+  for (int i = 0; i < 7; ++i) {
     p[i] = PyLong_AsVoidPtr(a[i]);
     if (!p[i]) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "bind: null address"); return nullptr; }
   }
   g.gemv = (decltype(g.gemv))p[0]; g.fwd = (decltype(g.fwd))p[1]; g.bwd_table = (decltype(g.bwd_table))p[2];
-  g.bwd = (decltype(g.bwd))p[3]; g.swiglu = (decltype(g.swiglu))p[4]; g.error = (decltype(g.error))p[5];
+  g.bwd = (decltype(g.bwd))p[3]; g.swiglu = (decltype(g.swiglu))p[4]; g.error = (decltype(g.error))p[5]; g.v1 = (decltype(g.v1))p[6];
   Py_RETURN_NONE;
 }
 
@@ -170,6 +199,7 @@ PyMethodDef methods[] = {
     {"bind", (PyCFunction)(void (*)(void))py_bind, METH_FASTCALL, "addresses of the library's entry points"},
     {"gemv", (PyCFunction)(void (*)(void))py_gemv, METH_FASTCALL, "decode product of 1..16 rows"},
     {"gemm", (PyCFunction)(void (*)(void))py_gemm, METH_FASTCALL, "fused large-M product"},
+    {"gemm_v1", (PyCFunction)(void (*)(void))py_gemm_v1, METH_FASTCALL, "fused large-M forward of a layer of the first format"},
     {"swiglu", py_swiglu, METH_O, "silu(gate) * up of a fused gate_up output"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_q4torch", nullptr, -1, methods};

@@ -364,8 +364,9 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
                        const int32_t* qzeros, const int32_t* g_idx, const void* bias, const void* lora_u,
                        const void* lora_w, int lora_r, int M, int K, int N, int G, void* workspace, size_t workspace_bytes,
                        q4_stream_t stream, bool swiglu = false, const void* zp_cached = nullptr, const void* residual = nullptr,
-                       int seq_groupsize = 0) {
-  if (!act || !qweight || !out || !scales || !qzeros || !g_idx) return fail(Q4_E_BADARG, "gemm: null pointer");
+                       int seq_groupsize = 0, bool one_group = false) {
+  // one_group: a layer of the first format - G = 1, the zero-term table given, neither qzeros nor g_idx
+  if (!act || !qweight || !out || !scales || (!one_group && (!qzeros || !g_idx))) return fail(Q4_E_BADARG, "gemm: null pointer");
   const int gv = g_gemm_variant == 5 ? 0 : g_gemm_variant;
   if (M <= 0 || K <= 0 || N <= 0 || G <= 0) return fail(Q4_E_BADARG, "gemm: M=%d K=%d N=%d G=%d", M, K, N, G);
   if (K % 128 || N % 128) return fail(Q4_E_SHAPE, "gemm: K=%d and N=%d must be multiples of 128", K, N);
@@ -397,7 +398,8 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     return fail(Q4_E_SHAPE, "gemm: the CTA-pair kernel needs %d output columns to be a multiple of 256 and G=%d tables to fit", nout, G);
   if (swiglu && (transpose || lora_r > 0 || !pair_ok || N % 256))
     return fail(Q4_E_SHAPE, "gemm: the fused gate_up product needs the CTA-pair kernel (N=%d a multiple of 256, G=%d tables that fit) and no low-rank term", N, G);
-  const bool use_pair = (pair_ok && gv != 1) || gv == 3 || swiglu;
+  if (one_group && !pair_ok) return fail(Q4_E_SHAPE, "gemm: a layer of the first format needs %d output columns to be a multiple of 256", nout);
+  const bool use_pair = (pair_ok && (gv != 1 || one_group)) || gv == 3 || swiglu;
   // weights-in-TMEM kernel: forward, groups of at least the 64 contraction elements of a stage promised sequential
   const bool tm_ok = !transpose && !swiglu && no_tables && seq_shift >= 6 && nout % G2_TILE_N == 0;
   if (gv == 4 && !tm_ok)
@@ -641,6 +643,17 @@ extern "C" int q4_gemm_fwd_residual(const void* x, const int32_t* qweight, void*
   if (zero_terms && !aligned16(zero_terms)) return fail(Q4_E_ALIGN, "gemm_fwd_residual: the zero-term table must be 16-byte aligned");
   return gemm_launch(false, x, qweight, y, scales, qzeros, g_idx, bias, lora_u, lora_b, lora_r, M, K, N, G, workspace, workspace_bytes, stream,
                      false, zero_terms, residual, zero_terms ? sequential_groupsize : 0);
+}
+
+extern "C" int q4_gemm_fwd_v1(const void* x, const int32_t* qweight, void* y, const void* scales, const void* zeros, const void* bias,
+                              const void* residual, int M, int K, int N, void* workspace, size_t workspace_bytes, q4_stream_t stream) {
+  if (!zeros) return fail(Q4_E_BADARG, "gemm_fwd_v1: null pointer");
+  if (!aligned16(zeros)) return fail(Q4_E_ALIGN, "gemm_fwd_v1: zeros must be 16-byte aligned");
+  if (K > (1 << 30)) return fail(Q4_E_SHAPE, "gemm_fwd_v1: K=%d", K);
+  int group = 64;                              // one group of all rows: the next power of two
+  while (group < K) group <<= 1;
+  return gemm_launch(false, x, qweight, y, scales, nullptr, nullptr, bias, nullptr, nullptr, 0, M, K, N, 1, workspace, workspace_bytes, stream,
+                     false, zeros, residual, group, true);
 }
 
 extern "C" int q4_gemm_set_variant(int variant) {

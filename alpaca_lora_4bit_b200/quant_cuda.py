@@ -322,6 +322,25 @@ def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, 
     return (_lib._torch_call or _lib.torch_call()).gemm(x, qweight, out, scales, zeros, g_idx, bias, residual, lora_u, lora_w, transpose, zt, seq_gs, ws)
 
 
+def gemm_v1_new(x, qweight, scales, zeros, bias=None, residual=None):
+    """``x @ W (+ bias) (+ residual)`` for ``x [..., K]`` on a layer of the first format, W never written to memory;
+    ``None`` - and nothing done - for operands the kernels do not take."""
+    dev = x.device
+    if not x.is_cuda or dev.index != _current_device() or qweight.dim() != 2:
+        return None
+    K, N = qweight.shape[0] * 8, qweight.shape[1]
+    if K % 128 or N % 256:
+        return None
+    st = _raw_stream(dev.index)
+    need = _gemm_ws_bytes.get((K, N, 1))
+    if need is None:
+        need = _gemm_ws_bytes[(K, N, 1)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, 1))
+    ws = _lib._gemm_workspaces.get((dev.index, st))
+    if ws is None or ws.numel() < need:
+        ws = _lib.gemm_workspace_for(dev, st, need)
+    return (_lib._torch_call or _lib.torch_call()).gemm_v1(x, qweight, scales, zeros, bias, residual, ws)
+
+
 def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora_u=None, lora_w=None, residual=None) -> None:
     """Fused large-M product on the tensor cores: ``out = x @ W (+ bias)`` or, with ``transpose``,
     ``out = x @ W.T``; ``x``, ``out``, ``scales`` fp16, W never leaves shared memory.

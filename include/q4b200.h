@@ -201,7 +201,13 @@ int q4_gemm_fwd_residual(const void* x, const int32_t* qweight, void* y, const v
                          const void* zero_terms, const int32_t* g_idx, const void* bias, const void* residual,
                          const void* lora_u, const void* lora_b, int lora_r, int M, int K, int N, int G,
                          int sequential_groupsize, void* workspace, size_t workspace_bytes, q4_stream_t stream);
-/* Optional scratch for the two calls above (no reference counterpart: the reference's scratch is
+/* The forward on a layer of the first format (autograd_4bit.py:176-189: one scale and one fp16 zero per column,
+ * W = rn(rn(scale * level) - zero), what q4_recons_v1 writes): a layer of one group whose table of zero terms is `zeros`
+ * itself.  y = half(half(x W + bias) + residual); scales, zeros fp16 [N], 16-byte aligned like the other operands;
+ * N % 256 == 0, K % 128 == 0.  workspace as for q4_gemm_fwd with G = 1. */
+int q4_gemm_fwd_v1(const void* x, const int32_t* qweight, void* y, const void* scales, const void* zeros, const void* bias,
+                   const void* residual, int M, int K, int N, void* workspace, size_t workspace_bytes, q4_stream_t stream);
+/* Optional scratch for the calls above (no reference counterpart: the reference's scratch is
  * the dense fp16 copy of W it reconstructs).  `workspace` may be NULL; with at least
  * q4_gemm_workspace_bytes(K, N, G) bytes of device memory, 16-byte aligned, whose first 64 KiB are
  * zero before the first call (the kernels leave them zero), the CTA-pair kernel

@@ -66,3 +66,35 @@ def test_native_call_leaves_operands_it_does_not_take():
         assert mod(x[:0].half().to(DEV)).shape == (0, N)
         with pytest.raises((RuntimeError, AssertionError)):
             mod(torch.zeros(4, K + 128, dtype=torch.float16, device=DEV))
+
+
+@pytest.mark.parametrize("K2,N2", [(128, 256), (256, 128), (512, 768), (640, 384), (2048, 5120), (11008, 512)])
+@pytest.mark.parametrize("rows", [9, 17, 129, 257, 700])
+def test_first_format_large_products_both_ways(K2, N2, rows):
+    """Layers of the first format above the switch threshold: the fused kernels (output columns a multiple of 256) and
+    the reconstruct path (the rest) against fp32 products of the same fp16 weights, and the gradient the transpose."""
+    gen = torch.Generator().manual_seed(K2 + rows)
+    qweight = torch.randint(-2 ** 31, 2 ** 31 - 1, (K2 // 8, N2), generator=gen).to(torch.int32).to(DEV)
+    scales = (torch.rand(N2, 1, generator=gen) * 0.018 + 0.002).half()
+    scales[::7] = -3.25 * scales[::7]                       # negative scales, and with the next line some above 2
+    scales[3::31] = 2.5
+    zeros = (scales.float() * torch.randint(1, 16, (N2, 1), generator=gen)).half().to(DEV)
+    scales = scales.to(DEV)
+    bias = torch.randn(N2, generator=gen).half().to(DEV)
+    w = torch.empty((K2, N2), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v1(qweight, w, scales.reshape(-1), zeros.reshape(-1))
+    x = torch.randn(2, rows, K2, generator=gen).half().to(DEV)[1:].requires_grad_(True)
+    dy = torch.randn(1, rows, N2, generator=gen).half().to(DEV)
+    res = torch.randn(1, rows, N2, generator=gen).half().to(DEV)
+    y = a4.AutogradMatmul4bitCuda.apply(x, qweight, scales, zeros, None, 4, 15, bias, res)
+    (dx,) = torch.autograd.grad(y, [x], dy)
+    want = (x.detach().double() @ w.double() + bias.double()) + res.double()
+    dwant = dy.double() @ w.double().t()
+    for got, ref in ((y, want), (dx, dwant)):                # fp32 sums rounded to fp16 (twice: product, residual): 2 * 2^-11
+        assert got.shape == ref.shape and float((got.double() - ref).norm() / ref.norm()) <= 1e-3
+    with torch.no_grad():
+        y2 = mm4b.linear(x, qweight, scales, zeros, None, K2, bias, res)
+        yt = torch.func.vmap(lambda v: mm4b.matmul4bit(v, qweight, scales, zeros))(x.detach().expand(2, rows, K2))
+    assert float((y2.double() - want).norm() / want.norm()) <= 1e-3
+    assert float((yt[1].double() - (want - bias.double() - res.double())[0]).norm() / want.norm()) <= 1e-3
+    assert quant_cuda.device_status() == 0
