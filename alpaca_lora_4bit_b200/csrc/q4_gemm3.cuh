@@ -179,10 +179,71 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       }
     }
   };
-  // The pair's last item, when it is a whole tile: nothing follows it, so the dequant warps (three per TMEM lane
-  // quarter) share its epilogue with the epilogue warp of their quarter, blocks of 32 rows dealt round robin.
+  // The pair's last item: nothing follows it, so the dequant warps (three per TMEM lane quarter) share its epilogue
+  // with the epilogue warp of their quarter, blocks of 32 rows dealt round robin - the output of a whole tile, and the
+  // writing or the adding up of the partial sums of a shared one.  (On short prompts, where every item is a piece of a
+  // tile, one warp per quarter did the exchange block by block, a trip to L2 each: 128 rows of 4096 x 4096 23.2 us, now
+  // 18.9, of 11008 x 4096 32.5, now 28.2.)
   const WorkItem w_last = work_item<SPLIT>(p, wr, n_items > 0 ? n_items - 1 : 0, n_pairs, T);
-  const bool share_last = n_items > 0 && !(SPLIT && w_last.split);
+  const bool share_last = n_items > 0;
+
+  // A shared tile of this run: who contributes, its arrival counter (per CTA of the pair and lane quarter) and the
+  // place of a contributor's sums: a warp's 32 columns x 256 rows as [block][j][lane][4 floats] (512 contiguous bytes
+  // per 16-byte access of the warp), indexed [contributing pair][CTA of the pair][lane quarter].
+  struct Shared { bool shared, reducer; int c_first, c_last; unsigned* cnt; };
+  auto shared_of = [&](const WorkItem& wi, int quarter) {
+    Shared s = {SPLIT && wi.split, false, 0, 0, nullptr};
+    if (s.shared) {
+      const long long total = (long long)n_tiles * T;
+      s.reducer = wi.kb == 0;
+      s.c_first = stage_owner((long long)wi.tile * T, n_pairs, total);
+      s.c_last = stage_owner((long long)wi.tile * T + T - 1, n_pairs, total);
+      s.cnt = p.ws_counters + ((size_t)s.c_first * 2 + rank) * 4 + quarter;
+    }
+    return s;
+  };
+  auto part_of = [&](int cpair, int quarter) -> float* { return p.ws_partials + (((size_t)cpair * 2 + rank) * 4 + quarter) * (size_t)(8 * 8 * 32 * 4); };
+  auto await_partials = [&](const Shared& s) {
+    if (lane == 0) {
+      const unsigned want = (unsigned)(s.c_last - s.c_first);
+      bool ok = false;
+      const uint32_t lim = *abort_flag ? 4u : 500000u;                    // x 200 ns
+      for (uint32_t i = 0; i < lim && !ok; ++i) {
+        unsigned have;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(s.cnt) : "memory");
+        ok = have >= want;
+        if (!ok) __nanosleep(200);
+      }
+      if (!ok) { *abort_flag = 1; atomicExch(&g_gemm_status, Q4_STATUS_WAIT_EXPIRED); }
+    }
+    __syncwarp();
+    __threadfence();
+  };
+  // One block of the accumulator: to the workspace, or - with the other contributors' sums added - to shared memory.
+  auto take_block = [&](const Shared& s, int quarter, int cb, uint32_t tsrc, unsigned char* buf, float bv) __attribute__((always_inline)) {
+    uint32_t v[32];
+    tmem_ld32(tsrc + cb * 32, v);
+    tmem_ld_wait();
+    if (s.shared && !s.reducer) {
+      float* part = part_of(pair, quarter);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<uint4*>(part + ((cb * 8 + q) * 32 + lane) * 4) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      return;
+    }
+    if (s.reducer) {
+      for (int c2 = s.c_first + 1; c2 <= s.c_last; ++c2) {
+        const float* src = part_of(c2, quarter);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 a = __ldcg(reinterpret_cast<const float4*>(src + ((cb * 8 + q) * 32 + lane) * 4));
+          v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + a.x); v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + a.y);
+          v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + a.z); v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + a.w);
+        }
+      }
+    }
+    block_to_smem(buf, v, bv);
+  };
 
   if (warp == 0) {
     // ---------------- TMA producer: this CTA's 128 rows of x (or of lora_u) of every stage ----------------
@@ -312,14 +373,20 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       __syncwarp();
       tc_fence_after();
       unsigned char* mine = turn + quarter * 16384;
+      const Shared sh = shared_of(w_last, quarter);
+      if (sh.reducer) {
+        await_partials(sh);
+        named_bar_sync(1 + quarter, 128);                          // all four warps have seen the count: the epilogue warp may clear it
+      }
 #pragma unroll 1
       for (int cb = grp; cb < nb; cb += G3_GROUPS + 1) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + ((uint32_t)(32 * quarter) << 16) + cb * 32, v);
-        tmem_ld_wait();
-        block_to_smem(mine + cb * 2048, v, bv);
+        take_block(sh, quarter, cb, tmem_base + ((uint32_t)(32 * quarter) << 16), mine + cb * 2048, bv);
         __syncwarp();
-        block_to_global(mine + cb * 2048, m_base + cb * 32, n0);
+        if (!sh.shared || sh.reducer) block_to_global(mine + cb * 2048, m_base + cb * 32, n0);
+      }
+      if (sh.shared && !sh.reducer) {
+        __threadfence();
+        named_bar_sync(1 + quarter, 128);                          // this warp's sums are out: the epilogue warp counts for all four
       }
     }
   } else if (warp >= 4 + 4 * G3_GROUPS) {
@@ -342,76 +409,28 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       const int nb = (rows + 31) >> 5;                             // blocks of 32 rows that hold anything
       const bool shared_out = share_last && item == n_items - 1;   // the dequant warps take the blocks cb % 4 = 0, 1, 2
       const int cb0 = shared_out ? G3_GROUPS : 0, cbs = shared_out ? G3_GROUPS + 1 : 1;
-      // Partial sums of a run: this warp's 32 columns x 256 rows as [block][j][lane][4 floats] (512 contiguous bytes
-      // per 16-byte access of the warp), indexed [contributing pair][CTA of the pair][lane quarter].
-      const size_t part_floats = 8 * 8 * 32 * 4;
-      auto part_of = [&](int cpair) -> float* { return p.ws_partials + (((size_t)cpair * 2 + rank) * 4 + quarter) * part_floats; };
-      const bool shared_tile = SPLIT && wi.split;
-      const bool reducer = shared_tile && wi.kb == 0;
-      int c_first = 0, c_last = 0;
-      unsigned* cnt = nullptr;
-      if (shared_tile) {
-        const long long total = (long long)n_tiles * T;
-        c_first = stage_owner((long long)wi.tile * T, n_pairs, total);
-        c_last = stage_owner((long long)wi.tile * T + T - 1, n_pairs, total);
-        cnt = p.ws_counters + ((size_t)c_first * 2 + rank) * 4 + quarter;
-      }
-      if (reducer) {
-        if (lane == 0) {
-          const unsigned want = (unsigned)(c_last - c_first);
-          bool ok = false;
-          const uint32_t lim = *abort_flag ? 4u : 500000u;                    // x 200 ns
-          for (uint32_t i = 0; i < lim && !ok; ++i) {
-            unsigned have;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(cnt) : "memory");
-            ok = have >= want;
-            if (!ok) __nanosleep(200);
-          }
-          if (!ok) { *abort_flag = 1; atomicExch(&g_gemm_status, Q4_STATUS_WAIT_EXPIRED); }
-        }
-        __syncwarp();
-        __threadfence();
+      const Shared sh = shared_of(wi, quarter);
+      if (sh.reducer) {
+        await_partials(sh);
+        if (shared_out) named_bar_sync(1 + quarter, 128);
       }
 #pragma unroll 1
-      for (int cb = cb0; cb < nb; cb += cbs) {
-        uint32_t v[32];
-        tmem_ld32(tsrc + cb * 32, v);
-        tmem_ld_wait();
-        if (shared_tile && !reducer) {
-          float* part = part_of(pair);
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            *reinterpret_cast<uint4*>(part + ((cb * 8 + q) * 32 + lane) * 4) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-          continue;
-        }
-        if (reducer) {
-          for (int c2 = c_first + 1; c2 <= c_last; ++c2) {
-            const float* src = part_of(c2);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const float4 a = __ldcg(reinterpret_cast<const float4*>(src + ((cb * 8 + q) * 32 + lane) * 4));
-              v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + a.x); v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + a.y);
-              v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + a.z); v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + a.w);
-            }
-          }
-        }
-        block_to_smem(mine + cb * 2048, v, bv);
-      }
+      for (int cb = cb0; cb < nb; cb += cbs) take_block(sh, quarter, cb, tsrc, mine + cb * 2048, bv);
       // this warp has read its part of the accumulator: the even CTA may start the next item
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty0);
-      if (!(shared_tile && !reducer)) {
+      if (!sh.shared || sh.reducer) {
 #pragma unroll 1
         for (int cb = cb0; cb < nb; cb += cbs) block_to_global(mine + cb * 2048, m_base + cb * 32, n0);
         __syncwarp();                                      // the rows are read before the next item overwrites them
-      }
-      if (shared_tile && !reducer) {                       // publish: sums, then the count
+      } else {                                             // publish: sums, then the count
         __threadfence();
         __syncwarp();
-        if (lane == 0) atomicAdd(cnt, 1u);
+        if (shared_out) named_bar_sync(1 + quarter, 128);
+        if (lane == 0) atomicAdd(sh.cnt, 1u);
       }
-      if (reducer && lane == 0) *cnt = 0;                  // every contributor has been counted: ready for the next launch
+      if (sh.reducer && lane == 0) *sh.cnt = 0;            // every contributor has been counted: ready for the next launch
     }
   }
   if (threadIdx.x == G3_THREADS - 128) gm_mark_ns(p.trace, 106);
