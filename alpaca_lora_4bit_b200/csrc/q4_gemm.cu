@@ -520,28 +520,46 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       int pairs3 = tiles3 < P ? tiles3 : P;
       bool stream3 = false;
       const long long total3 = (long long)tiles3 * T;
-      // (measured: every further item of a pair's run and the exchange cost about 30 stages together; tiles cut
-      // between several whole pairs - fewer tiles than pairs - never paid)
+      // (measured: every further item of a pair's run and the exchange cost about 30 stages together)
       if (ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 8 && tiles3 > P && tiles3 % P != 0 &&
           total3 * P < (1ll << 32)) {
         const long long whole = (long long)((tiles3 + P - 1) / P) * T, dealt = (total3 + P - 1) / P + 30;
         stream3 = dealt < whole;
       }
-      // Few tiles and a long contraction (short prompts: one row tile, 16 column tiles of a 4096-wide layer on 74
-      // pairs): every tile is cut between a whole number of pairs.  The exchange costs about 12 + 7 nb stages (nb =
-      // blocks of 32 rows a tile really has: the partial sums of the other rows are neither written nor read), so it
-      // pays for short prompts and long contractions (64 rows at 4096 x 4096: 25.7 -> 18.4 us; 32 rows at 11008 x 4096:
-      // 58.2 -> 24.8 us) and not at 256 rows of 4096 x 4096 (27.3 -> 32.8 us).
-      if (!stream3 && ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && tiles3 * 2 <= P && T >= 16) {
-        int per_tile = P / tiles3;
-        if (per_tile > T / 8) per_tile = T / 8;
-        const int nb = ((M < 256 ? M : 256) + 31) / 32;
-        if (per_tile >= 2 && (long long)T * (per_tile - 1) / per_tile > 12 + 7 * nb) { stream3 = true; pairs3 = tiles3 * per_tile; }
+      // Fewer tiles than pairs (short prompts: one row tile, 16 column tiles of a 4096-wide layer on 74 pairs).  With at
+      // least two pairs per tile every tile is cut between a whole number `n` of them.  In stages of the contraction (a
+      // quarter of a microsecond), nb = blocks of 32 rows a tile really has: T / n for the pair's own run, about 9 + 1.2 nb
+      // for writing and announcing the sums and 0.5 + 0.45 nb for every further contributor's sums that are added.  (8192 x
+      // 1024 at 256 rows, n = 2, 4, 6, 8, 16: 33.4, 26.4, 25.4, 25.8, 32.0 us, uncut 46.4; 4096 x 4096 at 32 / 256 rows:
+      // uncut 25.8 / 27.8, n = 4 16.7 / 22.8; 2048 x 2048 at 192 rows is better left uncut: 16.9, n = 2 18.3.  Contractions of
+      // up to 2048 are cut for one block of rows only: 77 rows would gain a microsecond (16.0 / 14.9), and whole tiles add
+      // up in the pair kernel's order.  All of these before the launch became programmatic, which takes another two to
+      // three microseconds off every one of them.)
+      const int nb = ((M < 256 ? M : 256) + 31) / 32;
+      const bool cut_ok = !stream3 && ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 16;
+      if (cut_ok && tiles3 * 2 <= P) {
+        double best = T;
+        for (int n = 2; n <= P / tiles3 && n <= T / 4; ++n) {
+          const double cost = (double)((T + n - 1) / n) + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
+          if (T <= 32 && T * (n - 1) / n <= 12 + 7 * nb) continue;
+          if (cost < best) { best = cost; stream3 = true; pairs3 = tiles3 * n; }
+        }
+      } else if (cut_ok && tiles3 < P && total3 * P < (1ll << 32)) {
+        // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
+        // exchange (4096 x 11008, 43 tiles, uncut / dealt: 26.5 / 23.8 us at 32 rows, 28.1 / 26.8 at 128, 28.7 / 29.1 at 192).
+        const double dealt = (double)total3 / P + 14 + 3 * nb;
+        if (dealt < T) { stream3 = true; pairs3 = P; }
       }
       p.ws_partials = (float*)(ws + ws_off);
       p.ws_counters = (unsigned*)ws;
-      if (stream3) q4_gemm3_kernel<true><<<dim3(2 * pairs3), dim3(G3_THREADS), gemm3_smem_bytes(), st>>>(amap, umap, p);
-      else q4_gemm3_kernel<false><<<dim3(2 * pairs3), dim3(G3_THREADS), gemm3_smem_bytes(), st>>>(amap, umap, p);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2 * pairs3); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = gemm3_smem_bytes(); cfg.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = at; cfg.numAttrs = 1;
+      if (int e = check_cuda(stream3 ? cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<true>, amap, umap, p)
+                                     : cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<false>, amap, umap, p), "gemm launch")) return e;
       return check_cuda(cudaGetLastError(), "gemm launch");
     }
     // Whole tiles per pair, round after round - or, when the last round would leave pairs idle for

@@ -23,6 +23,9 @@
 // first moves its 32 columns x 256 rows into shared memory as fp16 (and hands the accumulator back: the MMAs of the
 // pair's next item start while the stores run), then stores rows of 64 bytes, four lanes each.
 // Every wait is bounded as in the pair kernel.
+// Launched with the programmatic-dependent-launch attribute: set-up and the first packed words, scales and zero terms
+// (weights never depend on an earlier kernel) run before the wait for the earlier kernel; every warp that reads
+// activations, adapters, the skip path or the workspace, or writes, waits first.
 #pragma once
 
 namespace q4 {
@@ -86,6 +89,7 @@ template <bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G3_THREADS, 1)
 q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap umap, const GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
+  pdl_launch_dependents();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   unsigned char* stages = smem;
   constexpr int S = G3_STAGES;
@@ -250,6 +254,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     if (lane == 0) {
       int st = 0, use = 0;
       const uint32_t full0 = mapa_u32(smem_u32(full), 0);
+      pdl_wait();
       for (int item = 0; item < n_items; ++item) {
         const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
         const int m0 = (wi.tile % m_tiles) * 256 + 128 * (int)rank;
@@ -320,6 +325,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
         uint32_t o[32];
         if (j == ncon) {
           // low-rank stage: lane = column n holds lora_B[n][0..r), zero beyond
+          pdl_wait();
           const __half* src = p.lora_w + (size_t)n * p.lora_r;
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
@@ -369,6 +375,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       // the quarter's shared-memory rows are free once its epilogue warp has stored the item before (a meeting of
       // the quarter's four warps: named barrier 1 + quarter)
       named_bar_sync(1 + quarter, 128);
+      pdl_wait();
       if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 100);
       __syncwarp();
       tc_fence_after();
@@ -394,6 +401,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const int quarter = warp & 3;
     const uint32_t acc_empty0 = mapa_u32(smem_u32(acc_empty), 0);
     unsigned char* mine = turn + quarter * 16384;                  // [256 rows][32 columns] fp16
+    pdl_wait();
     for (int item = 0; item < n_items; ++item) {
       const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
       const int n0 = (wi.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter;     // this warp's 32 output columns
