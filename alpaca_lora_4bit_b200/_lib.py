@@ -63,6 +63,7 @@ _SIGNATURES = {
     "q4_swiglu_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "q4_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "q4_lora_project": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, ctypes.c_float, c_void_p]),
+    "q4_cast16": (c_int, [c_void_p, c_void_p, c_size_t, c_int, c_void_p]),
     "q4_lora_grads": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "q4_adamw_flat": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                               ctypes.c_float, ctypes.c_float, ctypes.c_float, c_void_p, ctypes.c_float, ctypes.c_float, c_int, c_void_p, c_void_p]),

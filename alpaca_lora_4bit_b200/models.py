@@ -102,6 +102,17 @@ def _lora_project(x2: torch.Tensor, w: torch.Tensor, scaling: float) -> torch.Te
     return out
 
 
+def _cast16(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``t.to(dtype).contiguous()``; between bf16 and fp16 on the GPU with one pass of the library's own kernel."""
+    if (t.is_cuda and {t.dtype, dtype} == {torch.float16, torch.bfloat16} and t.is_contiguous() and t.numel() > 0
+            and t.data_ptr() % 16 == 0):
+        out = torch.empty(t.shape, dtype=dtype, device=t.device)
+        with _lib.on_device(t.device):
+            _lib.check(_lib.lib().q4_cast16(t.data_ptr(), out.data_ptr(), t.numel(), int(dtype == torch.float16), _lib.stream_of(t)), "cast16")
+        return out
+    return t.to(dtype).contiguous()
+
+
 def _half_of(p: torch.Tensor) -> torch.Tensor:
     """fp16 contiguous copy of a LoRA factor: the copy its optimiser keeps beside it (``_q4_half``, refreshed by the
     flat AdamW kernel) when there is one, else a cast."""
@@ -129,7 +140,7 @@ class LoraMatmul4bit(torch.autograd.Function):
         K, N = qweight.shape[0] * 8, qweight.shape[1]
         x2 = x.reshape(-1, K)
         if x2.dtype != torch.float16 or not x2.is_contiguous():
-            x2 = x2.to(torch.float16).contiguous()
+            x2 = _cast16(x2, torch.float16)
         a_h, b_h = _half_of(lora_a), _half_of(lora_b)                            # [r, K], [N, r]
         u = _lora_project(x2, a_h, scaling)                                      # [M, 64], scaling folded in
         y = torch.empty((x2.shape[0], N), dtype=torch.float16, device=x.device)
@@ -155,7 +166,7 @@ class LoraMatmul4bit(torch.autograd.Function):
         r = lora_a.shape[0]
         dy = grad_output.reshape(-1, N)
         if dy.dtype != torch.float16 or not dy.is_contiguous():
-            dy = dy.to(torch.float16).contiguous()
+            dy = _cast16(dy, torch.float16)
         M = dy.shape[0]
         # v = scaling * dy @ B: the projection kernel wants its small operand as [r, N]
         bt_h = _half_of(lora_b).t().contiguous()
@@ -165,7 +176,8 @@ class LoraMatmul4bit(torch.autograd.Function):
             dx = torch.empty((M, K), dtype=torch.float16, device=dy.device)
             quant_cuda.gemm(dy, qweight, dx, scales.half(), qzeros, g_idx, transpose=True,
                             lora_u=v, lora_w=_half_of(lora_a))
-            dx = dx.reshape(ctx.x_shape).to(ctx.x_dtype)
+            dx = dx.reshape(ctx.x_shape)
+            dx = dx if dx.dtype == ctx.x_dtype else _cast16(dx, ctx.x_dtype)
         want_a, want_b = ctx.needs_input_grad[1], ctx.needs_input_grad[2]
         if want_a or want_b:
             ga = torch.empty((r, K), dtype=torch.float32, device=dy.device) if want_a else None

@@ -251,6 +251,9 @@ int q4_rope(const void* in, const void* cos, const void* sin, void* out, int tok
  *                     (v, u fp16 [M, 64] as produced above; x fp16 [M, K]; dy fp16 [M, N]; K, N % 32 == 0);
  *                     either output may be NULL, its operands are then not read */
 int q4_lora_project(const void* x, const void* w, void* out, int M, int C, int r, float scale, q4_stream_t stream);
+/* dst[i] = src[i] rounded from bf16 to fp16 (to_half != 0) or from fp16 to bf16; n elements, pointers 16-byte aligned:
+ * the activations of a bf16 step on their way into and out of an adapted layer. */
+int q4_cast16(const void* src, void* dst, size_t n, int to_half, q4_stream_t stream);
 int q4_lora_grads(const void* v, const void* x, float* d_a, int K, const void* dy, const void* u, float* d_b, int N,
                   int M, int r, q4_stream_t stream);
 

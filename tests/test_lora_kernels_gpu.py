@@ -21,7 +21,8 @@ def project(x, w, scale):
     return out
 
 
-@pytest.mark.parametrize("M,C,r", [(1024, 4096, 8), (1024, 11008, 16), (37, 256, 3), (2048, 5120, 33), (9, 32, 64), (512, 8192, 1)])
+@pytest.mark.parametrize("M,C,r", [(1024, 4096, 8), (1024, 11008, 16), (37, 256, 3), (2048, 5120, 33), (9, 32, 64), (512, 8192, 1),
+                                   (1185, 4096, 8), (2049, 5120, 16), (4096, 1056, 24), (1201, 96, 64), (3000, 13824, 16)])
 def test_project_matches_fp32_product(M, C, r):
     g = torch.Generator(device=DEV).manual_seed(M + C + r)
     x = torch.randn(M, C, generator=g, device=DEV).half()
@@ -68,3 +69,17 @@ def test_argument_checks():
     assert L.q4_lora_project(x.data_ptr(), w.data_ptr(), out.data_ptr(), 8, 32, 65, 1.0, None) < 0       # r > 64
     assert L.q4_lora_project(None, w.data_ptr(), out.data_ptr(), 8, 32, 4, 1.0, None) < 0
     assert L.q4_lora_grads(None, None, None, 32, None, None, None, 32, 8, 4, None) == 0                  # nothing asked
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2047, 8192, 8193, 3 * 8192 + 5, 2048 * 5120])
+def test_cast16_rounds_as_torch_does(n):
+    for src, dst in ((torch.bfloat16, torch.float16), (torch.float16, torch.bfloat16)):
+        g = torch.Generator(device=DEV).manual_seed(n)
+        bits = torch.randint(-2 ** 15, 2 ** 15, (n,), generator=g, device=DEV, dtype=torch.int32).to(torch.int16)
+        x = bits.view(src)                                   # every kind of value: subnormal, overflowing, infinite, NaN
+        out = torch.full((n + 8,), 7.0, dtype=dst, device=DEV)
+        _lib.check(_lib.lib().q4_cast16(x.data_ptr(), out.data_ptr(), n, int(dst == torch.float16), _lib.stream_of(x)), "cast16")
+        want = x.to(dst)
+        nan = torch.isnan(want)
+        assert torch.equal(torch.isnan(out[:n]), nan) and torch.equal(out[:n][~nan].view(torch.int16), want[~nan].view(torch.int16))
+        assert bool((out[n:] == 7.0).all())
