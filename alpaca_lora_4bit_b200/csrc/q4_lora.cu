@@ -37,21 +37,23 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local, uint32_t rank)
 // 40-60 GB/s); bulk copies, 3.6 us (the two library kernels and the pad it replaces: 9.3 us + 3).
 // A lane takes 16 contiguous bytes of its row of X and of its row of W per block: which four of the MMA's
 // sixteen k-slots those eight elements occupy is the same for both operands, so the order of the sum is the
-// only thing the re-mapping changes.  Rows 8..15 of the MMA tile stay zero.
-constexpr int LP_ROWS = 8, LP_WARPS = 8, LP_THREADS = LP_WARPS * 32;
+// only thing the re-mapping changes.  Rows 8..15 of the MMA tile stay zero, or (RT = 2) hold eight more rows of X: a
+// CTA fills an SM, so from one CTA per SM on sixteen rows each take one round instead of two and read W half as often
+// (2048 rows, r = 16, on average over the projections of a 13B block: 14.0 -> 12.5 us).
+constexpr int LP_WARPS = 8, LP_THREADS = LP_WARPS * 32;
 // chunk length and ring depth per output width: as much of the contraction in flight at once as shared memory holds
 // (a CTA's time is the number of round trips to L2 it has to wait for, one after the other)
-__host__ __device__ constexpr int lp_chunk(int nt) { return nt <= 2 ? 2048 : (nt == 4 ? 1024 : 512); }
-__host__ __device__ constexpr int lp_stages(int nt) { return nt == 1 ? 3 : 2; }
-__host__ __device__ constexpr int lp_pitch(int nt) { return lp_chunk(nt) * 2 + 16; }   // bytes per staged row; + 16 keeps the eight rows a quarter-warp reads on different banks
+__host__ __device__ constexpr int lp_chunk(int nt, int rt) { return rt == 1 ? (nt <= 2 ? 2048 : (nt == 4 ? 1024 : 512)) : (nt <= 2 ? 1024 : 512); }
+__host__ __device__ constexpr int lp_stages(int nt, int rt) { return rt == 1 ? (nt == 1 ? 3 : 2) : (nt == 2 ? 3 : nt == 8 ? 2 : 4); }
+__host__ __device__ constexpr int lp_pitch(int nt, int rt) { return lp_chunk(nt, rt) * 2 + 16; }   // bytes per staged row; + 16 keeps the eight rows a quarter-warp reads on different banks
 
-template <int NT>                                // 8-column tiles of the output that r reaches into
+template <int NT, int RT>                        // 8-column tiles of the output that r reaches into, 8-row tiles of X per CTA
 __global__ void __launch_bounds__(LP_THREADS)
 lora_project_kernel(const __half* __restrict__ X, const __half* __restrict__ W, __half* __restrict__ out, int M, int C, int r, float scale) {
   extern __shared__ __align__(128) unsigned char lp_smem[];
-  constexpr int ROWS = LP_ROWS + 8 * NT;         // staged rows per chunk: 8 of X, then 8 NT of W
-  constexpr int LP_CHUNK = lp_chunk(NT), LP_PITCH = lp_pitch(NT), STAGE = ROWS * LP_PITCH, LP_NS = lp_stages(NT);
-  float* red = reinterpret_cast<float*>(lp_smem + LP_NS * STAGE);          // [warps][8 rows][8 NT + 1]
+  constexpr int LP_ROWS = 8 * RT, ROWS = LP_ROWS + 8 * NT;                 // staged rows per chunk: 8 RT of X, then 8 NT of W
+  constexpr int LP_CHUNK = lp_chunk(NT, RT), LP_PITCH = lp_pitch(NT, RT), STAGE = ROWS * LP_PITCH, LP_NS = lp_stages(NT, RT);
+  float* red = reinterpret_cast<float*>(lp_smem + LP_NS * STAGE);          // [warps][8 RT rows][8 NT + 1]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int n_chunks = (C + LP_CHUNK - 1) / LP_CHUNK;
 
@@ -103,23 +105,29 @@ lora_project_kernel(const __half* __restrict__ X, const __half* __restrict__ W, 
     const int blocks = min(LP_CHUNK, C - c * LP_CHUNK) >> 5;
     for (int b = warp; b < blocks; b += LP_WARPS) {
       const uint4 xv = *reinterpret_cast<const uint4*>(st + g * LP_PITCH + 64 * b + 16 * t);
+      const uint4 xw = RT == 2 ? *reinterpret_cast<const uint4*>(st + (8 * (RT - 1) + g) * LP_PITCH + 64 * b + 16 * t) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const uint4 wv = *reinterpret_cast<const uint4*>(st + (LP_ROWS + 8 * nt + g) * LP_PITCH + 64 * b + 16 * t);
-        mma_f16_16816(acc[nt], xv.x, 0u, xv.y, 0u, wv.x, wv.y);
-        mma_f16_16816(acc[nt], xv.z, 0u, xv.w, 0u, wv.z, wv.w);
+        mma_f16_16816(acc[nt], xv.x, xw.x, xv.y, xw.y, wv.x, wv.y);
+        mma_f16_16816(acc[nt], xv.z, xw.z, xv.w, xw.w, wv.z, wv.w);
       }
     }
   }
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
-    red[(warp * LP_ROWS + g) * (8 * NT + 1) + 8 * nt + 2 * t] = acc[nt][0];
-    red[(warp * LP_ROWS + g) * (8 * NT + 1) + 8 * nt + 2 * t + 1] = acc[nt][1];
+#pragma unroll
+    for (int h = 0; h < RT; ++h) {
+      red[(warp * LP_ROWS + 8 * h + g) * (8 * NT + 1) + 8 * nt + 2 * t] = acc[nt][2 * h];
+      red[(warp * LP_ROWS + 8 * h + g) * (8 * NT + 1) + 8 * nt + 2 * t + 1] = acc[nt][2 * h + 1];
+    }
   }
   __syncthreads();
-  // 8 rows x 32 column pairs: one half2 per thread
-  const int orow = threadIdx.x >> 5, cp = threadIdx.x & 31;
-  if (blockIdx.x * LP_ROWS + orow < M) {
+  // 8 rows x 32 column pairs at a time: one half2 per thread
+  const int cp = threadIdx.x & 31;
+#pragma unroll
+  for (int orow = threadIdx.x >> 5; orow < LP_ROWS; orow += 8) {
+    if (blockIdx.x * LP_ROWS + orow >= M) break;
     float s0 = 0.f, s1 = 0.f;
     if (2 * cp < 8 * NT) {
 #pragma unroll
@@ -134,8 +142,23 @@ lora_project_kernel(const __half* __restrict__ X, const __half* __restrict__ W, 
   }
 }
 
-template <int NT> static size_t lora_project_smem() {
-  return (size_t)lp_stages(NT) * (LP_ROWS + 8 * NT) * lp_pitch(NT) + (size_t)LP_WARPS * LP_ROWS * (8 * NT + 1) * sizeof(float) + 64;
+template <int NT, int RT> static constexpr size_t lora_project_smem() {
+  return (size_t)lp_stages(NT, RT) * (8 * RT + 8 * NT) * lp_pitch(NT, RT) + (size_t)LP_WARPS * 8 * RT * (8 * NT + 1) * sizeof(float) + 64;
+}
+
+template <int NT, int RT>
+static int launch_lora_project(const __half* x, const __half* w, __half* out, int M, int C, int r, float scale, cudaStream_t st) {
+  static std::atomic<bool> attr_done[64];
+  static_assert(lora_project_smem<NT, RT>() <= 226 * 1024, "a CTA's ring and sums fit an SM");
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
+    if (int e = check_cuda(cudaFuncSetAttribute(lora_project_kernel<NT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lora_project_smem<NT, RT>()),
+                           "lora_project smem attribute")) return e;
+    if (dev >= 0 && dev < 64) attr_done[dev].store(true, std::memory_order_release);
+  }
+  lora_project_kernel<NT, RT><<<(M + 8 * RT - 1) / (8 * RT), LP_THREADS, lora_project_smem<NT, RT>(), st>>>(x, w, out, M, C, r, scale);
+  return check_cuda(cudaGetLastError(), "lora_project launch");
 }
 
 // ---- out [j, c] (or out [c, j]) = sum over m of S [m, j] X [m, c], j < r, S of pitch 64 --------------------
@@ -270,27 +293,18 @@ extern "C" int q4_lora_project(const void* x, const void* w, void* out, int M, i
   if (C % 32) return fail(Q4_E_SHAPE, "lora_project: the contraction length %d must be a multiple of 32", C);
   if (!aligned16(x) || !aligned16(w) || !aligned16(out)) return fail(Q4_E_ALIGN, "lora_project: pointers must be 16-byte aligned");
   if (int e = check_device()) return e;
-  const int grid = (M + LP_ROWS - 1) / LP_ROWS;
   const cudaStream_t st = (cudaStream_t)stream;
   const __half *xh = (const __half*)x, *wh = (const __half*)w;
   __half* oh = (__half*)out;
-  static std::atomic<bool> attr_done[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
-    if (int e = check_cuda(cudaFuncSetAttribute(lora_project_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lora_project_smem<4>()), "lora_project smem attribute")) return e;
-    if (int e = check_cuda(cudaFuncSetAttribute(lora_project_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lora_project_smem<8>()), "lora_project smem attribute")) return e;
-    if (int e = check_cuda(cudaFuncSetAttribute(lora_project_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lora_project_smem<2>()), "lora_project smem attribute")) return e;
-    if (int e = check_cuda(cudaFuncSetAttribute(lora_project_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lora_project_smem<1>()), "lora_project smem attribute")) return e;
-    if (dev >= 0 && dev < 64) attr_done[dev].store(true, std::memory_order_release);
-  }
+  const bool tall = (M + 7) / 8 > sm_count();    // eight rows each would take more than one round of CTAs
+#define Q4_LP(NT) return tall ? launch_lora_project<NT, 2>(xh, wh, oh, M, C, r, scale, st) : launch_lora_project<NT, 1>(xh, wh, oh, M, C, r, scale, st)
   switch ((r + 7) / 8) {
-    case 1: lora_project_kernel<1><<<grid, LP_THREADS, lora_project_smem<1>(), st>>>(xh, wh, oh, M, C, r, scale); break;
-    case 2: lora_project_kernel<2><<<grid, LP_THREADS, lora_project_smem<2>(), st>>>(xh, wh, oh, M, C, r, scale); break;
-    case 3: case 4: lora_project_kernel<4><<<grid, LP_THREADS, lora_project_smem<4>(), st>>>(xh, wh, oh, M, C, r, scale); break;
-    default: lora_project_kernel<8><<<grid, LP_THREADS, lora_project_smem<8>(), st>>>(xh, wh, oh, M, C, r, scale); break;
+    case 1: Q4_LP(1);
+    case 2: Q4_LP(2);
+    case 3: case 4: Q4_LP(4);
+    default: Q4_LP(8);
   }
-  return check_cuda(cudaGetLastError(), "lora_project launch");
+#undef Q4_LP
 }
 
 extern "C" int q4_lora_grads(const void* v, const void* x, float* d_a, int K, const void* dy, const void* u, float* d_b, int N,
