@@ -1690,7 +1690,8 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 // Every element is dequantised as s*(q - (z+1)) in fp16 pairs before the MMA, with scale and zero point of its own
 // row's group from a shared-memory table of the CTA's 32 columns.  What bounds it: with a 4-byte entry looked up
 // per weight, unpacked pair by pair, the launch waited for shared memory and for the integer pipe (27.7 us on
-// average over the seven projections of a 13B block, where HBM needs 3.5).  Here
+// average over the seven projections of a 13B block, where HBM needs 3.5; now 19.6, the table's 4 bytes per weight
+// through the shared-memory pipe the largest part).  Here
 //   * a table entry is the four scales and the four 1024 + z + 1 of a quad of columns, 16 bytes: one LDS.128 serves
 //     the four weights a lane has of a row, and a subtraction from the raw 1024 + q leaves q - (z+1) exactly;
 //   * the rows' table offsets are written to shared memory once per CTA instead of being read and scaled per step;
@@ -1740,7 +1741,8 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
     const uint32_t z01 = ((zw & 0xFu) | ((zw & 0xF0u) << 12)) + 0x64016401u, z23 = (((zw >> 8) & 0xFu) | ((zw & 0xF000u) << 4)) + 0x64016401u;
     const uint4 e = make_uint4(s4.x, s4.y, z01, z23);
     unsigned char* at = tab + (size_t)grp * pitch + (quad >> 1) * copies * 32 + (quad & 1) * 16;
-    for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + c * 32) = e;
+    // (copies in turn from quad >> 1 on: the stores of a quarter-warp fall on different banks)
+    for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + ((c + (quad >> 1)) & (copies - 1)) * 32) = e;
   }
   if (staged)
     for (int i = threadIdx.x; i < (se - sb) * 32; i += GEMV_THREADS) offs[i] = offset_of(__ldg(p.g_idx + sb * 32 + i));
