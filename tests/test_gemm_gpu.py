@@ -562,3 +562,68 @@ def test_tensor_memory_kernel_with_runs_dealt_across_pairs(M, K, N):
         assert torch.equal(a, b)                                   # deterministic: partial sums are added in pair order
         assert rel_fro(a, c) <= 1e-3
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,M", [(4096, 11008, 17), (4096, 11008, 77), (4096, 11008, 128),     # 43 tiles dealt to all pairs
+                                   (5120, 13824, 33),                                            # 54 tiles, likewise
+                                   (8192, 256, 1), (8192, 1024, 40), (8192, 1024, 256),          # one and four tiles, many pairs each
+                                   (11008, 4096, 96), (2176, 512, 31), (4096, 4096, 250)])
+def test_short_prompts_cut_between_pairs(K, N, M):
+    """The pieces a tile of the weights-in-TMEM forward is cut into, with bias, skip path and a rank-16 term: against the
+    product with the reconstructed weights in fp64 (fp32 sums rounded to fp16, twice with the skip path: 2 * 2^-11), the
+    same bits on every launch."""
+    layer = synth.make_layer(K, N, 128, act_order=False, seed=K + M).to(DEV)
+    gen = torch.Generator(device=DEV).manual_seed(M)
+    x = torch.randn(M, K, generator=gen, device=DEV).half()
+    bias = torch.randn(N, generator=gen, device=DEV).half()
+    res = torch.randn(M, N, generator=gen, device=DEV).half()
+    u = torch.zeros(M, 64, dtype=torch.float16, device=DEV)
+    u[:, :16] = torch.randn(M, 16, generator=gen, device=DEV).half()
+    b = (torch.randn(N, 16, generator=gen, device=DEV) * 0.05).half()
+    w = torch.empty((K, N), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v2(layer.qweight, w, layer.scales, layer.qzeros, layer.g_idx)
+    want = x.double() @ w.double() + bias.double() + u[:, :16].double() @ b.double().t() + res.double()
+    runs = []
+    for _ in range(3):
+        y = torch.full((M, N), -9.0, dtype=torch.float16, device=DEV)
+        quant_cuda.gemm(x, layer.qweight, y, layer.scales, layer.qzeros, layer.g_idx, bias=bias, lora_u=u, lora_w=b, residual=res)
+        runs.append(y)
+    assert float((runs[0].double() - want).norm() / want.norm()) <= 1e-3
+    assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+    assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 5, 40, 130])
+def test_products_launched_early_wait_for_their_inputs(rows):
+    """A chain of products, each taking the one before as its input and its skip path, launched without waiting: the
+    kernels start before the earlier one has ended and must still see all of it."""
+    from alpaca_lora_4bit_b200 import _lib
+    K = 2048
+    layers = [synth.make_layer(K, K, 128, act_order=False, seed=i).to(DEV) for i in range(4)]
+    x0 = torch.randn(rows, K, generator=torch.Generator(device=DEV).manual_seed(rows), device=DEV).half()
+
+    def step(i, x):
+        L = layers[i % 4]
+        y = torch.empty_like(x)
+        if rows > 16:
+            quant_cuda.gemm(x, L.qweight, y, L.scales, L.qzeros, L.g_idx, residual=x)
+        else:
+            quant_cuda.gemv(x, L.qweight, y, L.scales, L.qzeros, None if i % 2 else L.g_idx, 128, 0 if i % 2 else _lib.GEMV_ACT_ORDER)
+        return (y * (1.0 / 16)).half() if i % 3 == 2 else y
+
+    def chain(wait):
+        x = x0
+        outs = []
+        for i in range(24):
+            x = step(i, x)
+            outs.append(x)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    want = chain(True)
+    for _ in range(5):
+        for a, b in zip(chain(False), want):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert quant_cuda.device_status() == 0
