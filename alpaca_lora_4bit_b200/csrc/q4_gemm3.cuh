@@ -23,9 +23,10 @@
 // first moves its 32 columns x 256 rows into shared memory as fp16 (and hands the accumulator back: the MMAs of the
 // pair's next item start while the stores run), then stores rows of 64 bytes, four lanes each.
 // Every wait is bounded as in the pair kernel.
-// Launched with the programmatic-dependent-launch attribute: set-up and the first packed words, scales and zero terms
-// (weights never depend on an earlier kernel) run before the wait for the earlier kernel; every warp that reads
-// activations, adapters, the skip path or the workspace, or writes, waits first.
+// Launched with the programmatic-dependent-launch attribute: the set-up runs before the wait for the earlier kernel, and
+// every warp waits before its first read or write of global memory.  That holds for the layer's own tensors too: the
+// kernel just ahead may be the one that fills the zero-term table of a layer's first call, or casts its scales or bias.
+// (An L2 prefetch delivers no value, so the first words may be asked for before the wait.)
 #pragma once
 
 namespace q4 {
@@ -57,16 +58,19 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t ldg_pinned_u32(const void* p) {
+// Loads that the compiler may neither move nor take for loads of memory that nobody writes while the kernel lives (an
+// earlier kernel of the stream may still be writing it when this one is launched).
+__device__ __forceinline__ uint32_t ld_pinned_u32(const void* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint32_t ldg_pinned_u16(const void* p) {
+__device__ __forceinline__ uint32_t ld_pinned_u16(const void* p) {
   uint16_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // One packed word = eight consecutive contraction elements of one output column -> four half2 in order.
 // Byte j of the word holds levels 2j (low nibble) and 2j+1 (high nibble): the byte is copied to bytes 0 and 2,
@@ -113,8 +117,6 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   const WorkRange wr = work_range<SPLIT>(pair, n_pairs, n_tiles, T);
   const int n_items = wr.n_items;
 
-  // A dequant warp asks for the words of its first task before the set-up below (barriers, TMEM, the cluster's
-  // meeting: about a microsecond): the loads depend on none of it.
   struct TaskRegs { uint32_t w[8]; uint32_t s, z; };
   const bool is_deq = warp >= 4 && warp < 4 + 4 * G3_GROUPS;
   auto column_of = [&](int tile) { return (tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * (warp & 3) + lane; };
@@ -123,19 +125,27 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const uint32_t* wcol = p.qw + n;
     const uint32_t* src = wcol + (size_t)(j * (GM_TILE_C >> 3)) * N;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) R.w[i] = ldg_pinned_u32(src + (size_t)i * N);
+    for (int i = 0; i < 8; ++i) R.w[i] = ld_pinned_u32(src + (size_t)i * N);
     const size_t at = (size_t)((j * GM_TILE_C) >> p.seq_shift) * N + n;
-    R.s = ldg_pinned_u16(p.scales + at);
-    R.z = ldg_pinned_u16(p.zp_table + at);
+    R.s = ld_pinned_u16(p.scales + at);
+    R.z = ld_pinned_u16(p.zp_table + at);
     // the words of the group's task after the next, asked into L2 (eight rows of 128 bytes per warp)
-    if (j + 2 * G3_GROUPS < T && lane < 8)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(wcol - lane + (size_t)((j + 2 * G3_GROUPS) * (GM_TILE_C >> 3) + lane) * N));
+    if (j + 2 * G3_GROUPS < T && lane < 8) prefetch_l2(wcol - lane + (size_t)((j + 2 * G3_GROUPS) * (GM_TILE_C >> 3) + lane) * N);
   };
-  TaskRegs R0, R1;
+  // A dequant warp asks for its first two tasks before the set-up below (barriers, TMEM, the cluster's meeting: about a
+  // microsecond) and before the wait for the earlier kernel: into L2, where they are read once both are over.
   if (is_deq && n_items > 0) {
     const WorkItem w0 = work_item<SPLIT>(p, wr, 0, n_pairs, T);
-    const int n = column_of(w0.tile), j = w0.kb + ((warp - 4) >> 2);
-    if (j < w0.ke) prefetch(n, j, R0);
+    const int n = column_of(w0.tile) - lane;                       // the warp's 32 columns: 128 bytes of words, 64 of scales
+#pragma unroll
+    for (int ahead = 0; ahead < 2; ++ahead) {
+      const int j = w0.kb + ((warp - 4) >> 2) + ahead * G3_GROUPS;
+      if (j >= w0.ke) break;
+      const size_t at = (size_t)((j * GM_TILE_C) >> p.seq_shift) * N + n;
+      if (lane < 8) prefetch_l2(p.qw + (size_t)(j * (GM_TILE_C >> 3) + lane) * N + n);
+      else if (lane == 8) prefetch_l2(p.scales + at);
+      else if (lane == 9) prefetch_l2(p.zp_table + at);
+    }
   }
 
   if (threadIdx.x == 0) {
@@ -316,6 +326,8 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const uint32_t full0 = mapa_u32(smem_u32(full), 0);
     const uint32_t tdst0 = tmem_base + ((uint32_t)(32 * quarter) << 16) + G3_TMEM_A0;
     int gbase = 0;                                                 // stage uses of all earlier tiles
+    TaskRegs R0, R1;
+    pdl_wait();                                                    // scales, zero terms, adapters, bias, workspace
     for (int item = 0; item < n_items; ++item) {
       const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
       const int n = column_of(wi.tile);
@@ -325,7 +337,6 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
         uint32_t o[32];
         if (j == ncon) {
           // low-rank stage: lane = column n holds lora_B[n][0..r), zero beyond
-          pdl_wait();
           const __half* src = p.lora_w + (size_t)n * p.lora_r;
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
@@ -355,7 +366,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       };
       int j = (grp + G3_GROUPS - gbase % G3_GROUPS) % G3_GROUPS;   // this group's first stage of the tile
       auto ask = [&](int jj, TaskRegs& R) __attribute__((always_inline)) { if (jj < ncon) prefetch(n, wi.kb + jj, R); };
-      if (item > 0) ask(j, R0);                                    // (the first item's came before the set-up)
+      ask(j, R0);
       while (j < nst) {
         ask(j + G3_GROUPS, R1);
         task(j, R0);
@@ -375,7 +386,6 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       // the quarter's shared-memory rows are free once its epilogue warp has stored the item before (a meeting of
       // the quarter's four warps: named barrier 1 + quarter)
       named_bar_sync(1 + quarter, 128);
-      pdl_wait();
       if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 100);
       __syncwarp();
       tc_fence_after();

@@ -627,3 +627,39 @@ def test_products_launched_early_wait_for_their_inputs(rows):
         for a, b in zip(chain(False), want):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [24, 130, 300])
+def test_first_product_of_a_layer_waits_for_its_tables(rows):
+    """The first product of a layer right behind the kernels that make what it reads - packed words copied into place,
+    scales and bias cast to fp16, the zero-term table filled - with nothing waited for, in memory that held NaN a moment
+    ago: the same bits as when everything has been there for long."""
+    K, N = 2048, 1024
+
+    def poison(*likes):                                    # the allocator hands the next tensor of this size the same memory
+        for t in likes:
+            torch.full(t.shape, float("nan"), dtype=torch.float16, device=DEV)
+
+    for seed in range(4):
+        src = synth.make_layer(K, N, 128, act_order=False, seed=seed).to(DEV)
+        gen = torch.Generator(device=DEV).manual_seed(seed)
+        x = torch.randn(rows, K, generator=gen, device=DEV).half()
+        scales32, bias32 = src.scales.float(), torch.randn(N, generator=gen, device=DEV)
+        quant_cuda.groups_are_sequential(src.g_idx, src.scales.shape[0])
+        qweight, qzeros = torch.zeros_like(src.qweight), torch.zeros_like(src.qzeros)
+        cold, warm = (torch.empty(rows, N, dtype=torch.float16, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        poison(scales32, scales32, bias32)
+        qweight.copy_(src.qweight)
+        qzeros.copy_(src.qzeros)
+        scales, bias = scales32.half(), bias32.half()
+        quant_cuda.gemm(x, qweight, cold, scales, qzeros, src.g_idx, bias=bias)
+        torch.cuda.synchronize()
+        quant_cuda.gemm(x, qweight, warm, scales, qzeros, src.g_idx, bias=bias)
+        torch.cuda.synchronize()
+        assert torch.equal(cold.view(torch.int16), warm.view(torch.int16))
+        w = torch.empty((K, N), dtype=torch.float16, device=DEV)
+        quant_cuda.vecquant4recons_v2(src.qweight, w, src.scales, src.qzeros, src.g_idx)
+        want = x.double() @ w.double() + bias.double()
+        assert float((warm.double() - want).norm() / want.norm()) <= 1e-3      # fp32 sums rounded to fp16 once
+    assert quant_cuda.device_status() == 0
