@@ -48,6 +48,23 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   return v;
 }
 
+// Loads for kernels that are launched before the earlier kernel of the stream has ended: behind the wait for that kernel
+// (the compiler may not move them) and coherent - the memory may have been written while this kernel was already there,
+// which the non-coherent loads above promise never happens.
+__device__ __forceinline__ uint4 ld_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_pinned_u4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// Ask for the cache line of `p` in L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // (a & mask) | bits as ONE three-input logic instruction.  Written in C++ with two literal constants
 // the expression compiles to two instructions (the instruction has room for a single immediate);
 // here both constants are register operands, loaded once outside the loops that use them.

@@ -70,7 +70,6 @@ __device__ __forceinline__ uint32_t ld_pinned_u16(const void* p) {
   asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // One packed word = eight consecutive contraction elements of one output column -> four half2 in order.
 // Byte j of the word holds levels 2j (low nibble) and 2j+1 (high nibble): the byte is copied to bytes 0 and 2,

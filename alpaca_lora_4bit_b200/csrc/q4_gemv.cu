@@ -1695,9 +1695,11 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 //   * a table entry is the four scales and the four 1024 + z + 1 of a quad of columns, 16 bytes: one LDS.128 serves
 //     the four weights a lane has of a row, and a subtraction from the raw 1024 + q leaves q - (z+1) exactly;
 //   * the rows' table offsets are written to shared memory once per CTA instead of being read and scaled per step;
-//   * packed words and x are fetched ACT_AHEAD steps ahead into registers, the tables and the first words before
-//     the wait for the earlier kernel (programmatic launch), and several CTAs share an SM, so that one's tables are
-//     built while the others multiply.
+//   * packed words and x are fetched ACT_AHEAD steps ahead into registers, and several CTAs share an SM, so that one's
+//     tables are built while the others multiply;
+//   * the launch is programmatic: before the wait for the earlier kernel a CTA asks for its words, scales, zero points and
+//     group indices, into L2 only (a prefetch delivers no value) - the earlier kernel may be the one that writes them, a
+//     cast of the scales for instance.
 // The four lanes t = 0..3 of a quad of columns hold different rows, hence different groups.  A quarter-warp (two
 // quads of columns) reads 8 x 16 bytes: the table is kept four times, copy t of a pair of quads in the t-th 32 bytes
 // of a 128-byte line, so that its lanes fall on different banks whatever their groups are.  Layers with so many groups
@@ -1727,16 +1729,36 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
 
   pdl_launch_dependents();
   const uint32_t* wp = p.qw + (size_t)t * N + c0 + 4 * g;
+  for (int i = threadIdx.x; i < G; i += GEMV_THREADS) {
+    prefetch_l2(p.scales + (size_t)i * N + c0);
+    prefetch_l2(p.qzeros + (size_t)i * (N >> 3) + (c0 >> 3));
+  }
+  for (int i = threadIdx.x; i < se - sb; i += GEMV_THREADS) prefetch_l2(p.g_idx + (sb + i) * 32);      // 128 bytes a step
+#pragma unroll
+  for (int i = 0; i < ACT_AHEAD; ++i) {
+    const int step = sb + warp + i * GEMV_WARPS;
+    if (step < se && g == 0) prefetch_l2(wp + (size_t)(4 * step) * N);                                   // 128 bytes a packed row
+  }
+  pdl_wait();
   uint4 wv[ACT_AHEAD];
 #pragma unroll
   for (int i = 0; i < ACT_AHEAD; ++i) {
     const int step = sb + warp + i * GEMV_WARPS;
-    wv[i] = step < se ? ldg_stream(wp + (size_t)(4 * step) * N) : make_uint4(0, 0, 0, 0);
+    wv[i] = step < se ? ld_stream(wp + (size_t)(4 * step) * N) : make_uint4(0, 0, 0, 0);
   }
+  const __half* xp0 = p.x + (size_t)g * K + 8 * t;
+  auto load_x = [&](int step, uint4 (&xv)[MT]) __attribute__((always_inline)) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+      xv[mt] = step < se && g + 8 * mt < p.M ? ld_pinned_u4(xp0 + (size_t)(8 * mt) * K + 32 * step) : make_uint4(0, 0, 0, 0);
+  };
+  uint4 xv[ACT_AHEAD][MT];
+#pragma unroll
+  for (int i = 0; i < ACT_AHEAD; ++i) load_x(sb + warp + i * GEMV_WARPS, xv[i]);
   for (int i = threadIdx.x; i < G * 8; i += GEMV_THREADS) {
     const int grp = i >> 3, quad = i & 7;
-    const uint2 s4 = __ldg(reinterpret_cast<const uint2*>(p.scales + (size_t)grp * N + c0 + 4 * quad));
-    const uint32_t zw = __ldg(p.qzeros + (size_t)grp * (N >> 3) + ((c0 + 4 * quad) >> 3)) >> (16 * (quad & 1));
+    const uint2 s4 = *reinterpret_cast<const uint2*>(p.scales + (size_t)grp * N + c0 + 4 * quad);
+    const uint32_t zw = p.qzeros[(size_t)grp * (N >> 3) + ((c0 + 4 * quad) >> 3)] >> (16 * (quad & 1));
     // 1024 + z + 1: the mantissa of 0x6400 plus one
     const uint32_t z01 = ((zw & 0xFu) | ((zw & 0xF0u) << 12)) + 0x64016401u, z23 = (((zw >> 8) & 0xFu) | ((zw & 0xF000u) << 4)) + 0x64016401u;
     const uint4 e = make_uint4(s4.x, s4.y, z01, z23);
@@ -1745,7 +1767,7 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
     for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + ((c + (quad >> 1)) & (copies - 1)) * 32) = e;
   }
   if (staged)
-    for (int i = threadIdx.x; i < (se - sb) * 32; i += GEMV_THREADS) offs[i] = offset_of(__ldg(p.g_idx + sb * 32 + i));
+    for (int i = threadIdx.x; i < (se - sb) * 32; i += GEMV_THREADS) offs[i] = offset_of(p.g_idx[sb * 32 + i]);
 
   float yacc[MT][2][4];
 #pragma unroll
@@ -1755,16 +1777,6 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) yacc[mt][j][i] = 0.f;
 
-  pdl_wait();                                    // x, y and the workspace belong to the stream order
-  const __half* xp0 = p.x + (size_t)g * K + 8 * t;
-  auto load_x = [&](int step, uint4 (&xv)[MT]) __attribute__((always_inline)) {
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-      xv[mt] = step < se && g + 8 * mt < p.M ? __ldg(reinterpret_cast<const uint4*>(xp0 + (size_t)(8 * mt) * K + 32 * step)) : make_uint4(0, 0, 0, 0);
-  };
-  uint4 xv[ACT_AHEAD][MT];
-#pragma unroll
-  for (int i = 0; i < ACT_AHEAD; ++i) load_x(sb + warp + i * GEMV_WARPS, xv[i]);
   __syncthreads();
   // this lane's quad of columns in its copy (copies = 2 or 1: several t share one)
   const unsigned char* tabt = tab + (g >> 1) * copies * 32 + (t & (copies - 1)) * 32 + (g & 1) * 16;
@@ -1775,8 +1787,8 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
       oa = *reinterpret_cast<const int4*>(offs + (step - sb) * 32 + 8 * t);
       ob = *reinterpret_cast<const int4*>(offs + (step - sb) * 32 + 8 * t + 4);
     } else {
-      oa = __ldg(reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t));
-      ob = __ldg(reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t + 4));
+      oa = *reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t);
+      ob = *reinterpret_cast<const int4*>(p.g_idx + step * 32 + 8 * t + 4);
       oa = make_int4(offset_of(oa.x), offset_of(oa.y), offset_of(oa.z), offset_of(oa.w));
       ob = make_int4(offset_of(ob.x), offset_of(ob.y), offset_of(ob.z), offset_of(ob.w));
     }
@@ -1816,7 +1828,7 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
       if (step < se) {                           // warp-uniform
         const int ahead = step + ACT_AHEAD * GEMV_WARPS;
         one_step(step, wv[i], xv[i]);
-        wv[i] = ahead < se ? ldg_stream(wp + (size_t)(4 * ahead) * N) : make_uint4(0, 0, 0, 0);
+        wv[i] = ahead < se ? ld_stream(wp + (size_t)(4 * ahead) * N) : make_uint4(0, 0, 0, 0);
         load_x(ahead, xv[i]);
       }
       step += GEMV_WARPS;

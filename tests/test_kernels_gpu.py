@@ -479,3 +479,32 @@ def test_recorded_layer_plan_serves_repeated_calls_and_expires():
     assert key not in quant_cuda._plans
     torch.cuda.synchronize()
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [1, 9])
+def test_act_order_decode_waits_for_what_it_reads(M):
+    """An act-order decode product right behind the kernels that write what it reads - words, group indices and zero
+    points copied into place, scales cast to fp16, x produced - with nothing waited for, in memory that held something
+    else a moment ago: the same bits as when everything has been there for long."""
+    K, N = 4096, 1024
+    for seed in range(4):
+        src = synth.make_layer(K, N, 128, act_order=True, seed=seed).to(DEV)
+        x32 = torch.randn(M, K, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+        scales32 = src.scales.float()
+        qweight, qzeros, g_idx = torch.zeros_like(src.qweight), torch.zeros_like(src.qzeros), torch.zeros_like(src.g_idx)
+        cold, warm = (torch.empty(M, N, dtype=torch.float32, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        for t in (scales32, x32):                          # the allocator hands the casts below the same memory
+            torch.full(t.shape, float("nan"), dtype=torch.float16, device=DEV)
+        qweight.copy_(src.qweight)
+        qzeros.copy_(src.qzeros)
+        g_idx.copy_(src.g_idx)
+        x, scales = x32.half(), scales32.half()
+        quant_cuda.gemv(x, qweight, cold, scales, qzeros, g_idx, 128, _lib.GEMV_ACT_ORDER)
+        torch.cuda.synchronize()
+        quant_cuda.gemv(x, qweight, warm, scales, qzeros, g_idx, 128, _lib.GEMV_ACT_ORDER)
+        torch.cuda.synchronize()
+        assert torch.equal(cold.view(torch.int32), warm.view(torch.int32))
+        want = orc.matmul4bit_ref(x.cpu(), src.qweight.cpu(), src.scales.cpu(), src.qzeros.cpu(), src.g_idx.cpu())
+        assert rel_fro(warm, want) <= REL_TOL
+    assert quant_cuda.device_status() == 0
