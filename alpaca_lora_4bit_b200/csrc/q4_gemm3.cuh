@@ -179,7 +179,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       if (m < p.M) {
         const size_t at = (size_t)m * N + n0 + 8 * cc;
         if (p.residual) {                                          // rounded first, as the separate add of the decoder layer would see it
-          const uint4 rv = __ldg(reinterpret_cast<const uint4*>(p.residual + at));
+          const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + at);      // (an earlier kernel's output: no read-only load)
           uint32_t* ov = reinterpret_cast<uint32_t*>(&o);
           const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
 #pragma unroll

@@ -413,7 +413,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       const int idx = base + threadIdx.x;
       const bool ok = idx < total;
       const int m = ok ? idx / blocks_per_row : 0, blk = ok ? idx - m * blocks_per_row : 0;
-      const uint4 v = ok ? __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K + 8 * blk)) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 v = ok ? ld_pinned_u4(p.x + (size_t)m * K + 8 * blk) : make_uint4(0u, 0u, 0u, 0u);
       const __half2 h01 = as_h2(v.x), h23 = as_h2(v.y), h45 = as_h2(v.z), h67 = as_h2(v.w);
       const __half2 sixteenth = as_h2(0x2C002C00u);
       const __half2 e04 = __lows2half2(h01, h45), o15 = __hmul2(__highs2half2(h01, h45), sixteenth);
@@ -442,7 +442,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
           xv[mt][u] = ok ? *reinterpret_cast<const uint4*>(xs_buf + (size_t)g * K + 8 * t + 32 * stp)
                          : *reinterpret_cast<const uint4*>(xs_base);
         else
-          xv[mt][u] = ok ? __ldg(reinterpret_cast<const uint4*>(xrow + (size_t)(8 * mt) * K + 32 * stp))
+          xv[mt][u] = ok ? ld_pinned_u4(xrow + (size_t)(8 * mt) * K + 32 * stp)
                          : make_uint4(0, 0, 0, 0);
       }
     }
@@ -717,7 +717,7 @@ gemv_fast_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
     for (int idx = threadIdx.x; idx < MR * blocks; idx += GF_THREADS) {
       const int m = idx / blocks, blk = idx - m * blocks;
       const bool ok = m < p.M && 8 * blk < K;
-      const uint4 v = ok ? __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K + 8 * blk)) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 v = ok ? ld_pinned_u4(p.x + (size_t)m * K + 8 * blk) : make_uint4(0u, 0u, 0u, 0u);
       const __half2 h01 = as_h2(v.x), h23 = as_h2(v.y), h45 = as_h2(v.z), h67 = as_h2(v.w);
       const __half2 sixteenth = as_h2(0x2C002C00u);
       const __half2 e04 = __lows2half2(h01, h45), o15 = __hmul2(__highs2half2(h01, h45), sixteenth);
@@ -1218,7 +1218,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
         int b = idx + rot;
         if (b >= n_blocks) b -= n_blocks;
         blk[i] = idx < n_blocks ? b : n_blocks;
-        if (base + i * CT < n_blocks) v[i] = 8 * blk[i] < K ? __ldg(xg + blk[i]) : make_uint4(0u, 0u, 0u, 0u);
+        if (base + i * CT < n_blocks) v[i] = 8 * blk[i] < K ? ld_pinned_u4(xg + blk[i]) : make_uint4(0u, 0u, 0u, 0u);
       }
       if (OCC == 1 && base == 0) fill_ring(1, S);        // x is on its way: now the rest of the ring
 #pragma unroll
@@ -1414,7 +1414,7 @@ x_convert_kernel(const __half* __restrict__ x, unsigned char* __restrict__ xq, u
   if (idx >= MR * n_blocks) return;
   const int m = idx / n_blocks, blk = idx - m * n_blocks;
   const bool live = m < M && 8 * blk < K;
-  const uint4 v = live ? __ldg(reinterpret_cast<const uint4*>(x + (size_t)m * K) + blk) : make_uint4(0u, 0u, 0u, 0u);
+  const uint4 v = live ? ld_pinned_u4(reinterpret_cast<const uint4*>(x + (size_t)m * K) + blk) : make_uint4(0u, 0u, 0u, 0u);
   const __half2 h01 = as_h2(v.x), h23 = as_h2(v.y), h45 = as_h2(v.z), h67 = as_h2(v.w);
   __half2 m2 = __hmax2(__hmax2(__habs2(h01), __habs2(h23)), __hmax2(__habs2(h45), __habs2(h67)));
 #pragma unroll

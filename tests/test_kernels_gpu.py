@@ -508,3 +508,31 @@ def test_act_order_decode_waits_for_what_it_reads(M):
         want = orc.matmul4bit_ref(x.cpu(), src.qweight.cpu(), src.scales.cpu(), src.qzeros.cpu(), src.g_idx.cpu())
         assert rel_fro(warm, want) <= REL_TOL
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("g,M", [(128, 1), (128, 2), (128, 7), (128, 16), (64, 1), (64, 12), (32, 3), (-1, 1), (-1, 5), (-1, 16)])
+def test_decode_chains_see_the_product_before(g, M):
+    """Every form of the sequential decode kernels (group sizes, rows) in a chain where a product's x is the output of
+    the one before, launched without waiting, against the same chain with a synchronise behind every product."""
+    K = 2048
+    layers = [synth.make_layer(K, K, g, act_order=False, seed=i).to(DEV) for i in range(3)]
+    x0 = torch.randn(M, K, generator=torch.Generator(device=DEV).manual_seed(M), device=DEV).half()
+
+    def chain(wait):
+        x, outs = x0, []
+        for i in range(18):
+            L = layers[i % 3]
+            y = torch.empty_like(x)
+            quant_cuda.gemv(x, L.qweight, y, L.scales, L.qzeros, None, K // L.scales.shape[0], 0)
+            x = (y * (1.0 / 32)).half() if i % 3 == 2 else y
+            outs.append(x)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    want = chain(True)
+    for _ in range(4):
+        for a, b in zip(chain(False), want):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert quant_cuda.device_status() == 0
