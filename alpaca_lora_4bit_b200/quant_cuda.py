@@ -283,11 +283,30 @@ promise_sequential_groups = True     # forward: tell the kernel that group = row
 _zero_term_tables: dict = {}
 
 
+def _is_layer_table(scales, zeros, G, N) -> bool:
+    """``scales`` fp16 ``[G, N]`` and ``zeros`` packed ``[G, N / 8]`` lie contiguous on one GPU, the current one."""
+    return (scales.dtype is _F16 and zeros.dtype is torch.int32 and scales.is_cuda and scales.device == zeros.device
+            and scales.device.index == _current_device() and tuple(scales.shape) == (G, N) and N % 8 == 0
+            and tuple(zeros.shape) == (G, N // 8) and scales.is_contiguous() and zeros.is_contiguous())
+
+
+def _check_layer(qweight, scales, zeros, g_idx) -> None:
+    """Raises where the packed tensors do not describe one layer: the kernels read them by the sizes of ``qweight`` and
+    by the number of groups."""
+    K, N, G = qweight.shape[0] * 8, qweight.shape[1], scales.shape[0]
+    _check_int32(qweight, "qweight"); _check_int32(zeros, "zeros"); _check_int32(g_idx, "g_idx")
+    if tuple(scales.shape) != (G, N) or N % 8 or tuple(zeros.shape) != (G, N // 8) or g_idx.numel() < K:
+        raise RuntimeError(f"quant_cuda: scales{tuple(scales.shape)} zeros{tuple(zeros.shape)} g_idx{tuple(g_idx.shape)} "
+                           f"do not belong to a layer [{K},{N}]")
+
+
 def _zero_terms(scales, zeros, G, N, st):
     key = id(zeros)
     hit = _zero_term_tables.get(key)
     if hit is not None and hit[1] == (zeros.data_ptr(), scales.data_ptr(), zeros._version, scales._version):
         return hit[0]
+    if not _is_layer_table(scales, zeros, G, N):
+        return None                                    # nothing is launched on operands that do not describe a layer
     if torch.cuda.is_current_stream_capturing():
         return None                                    # no allocation inside a capture: this call derives the table itself
     import weakref
@@ -314,7 +333,7 @@ def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, 
     if ws is None or ws.numel() < need:
         ws = _lib.gemm_workspace_for(dev, st, need)
     zt, seq_gs = None, 0
-    if cache_zero_terms and scales.dtype is _F16 and scales.is_cuda and scales.is_contiguous() and zeros.is_contiguous():
+    if cache_zero_terms and g_idx is not None and G > 0:
         # forward: see the comment in gemm()
         if transpose or (N % 256 == 0 and K % G == 0 and groups_are_sequential(g_idx, G)):
             zt = _zero_terms(scales, zeros, G, N, st)
@@ -354,6 +373,7 @@ def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora
             return
     # operands the native call does not take: say what is wrong, or run them from another current device
     dev = _lib.require_cuda(x, qweight, out, scales, zeros, g_idx, bias, lora_u, lora_w, residual)
+    _check_layer(qweight, scales, zeros, g_idx)
     R, N = qweight.shape
     K = R * 8
     M = x.shape[0]
@@ -412,6 +432,7 @@ def gemm_swiglu(x, qweight, out, scales, zeros, g_idx, bias=None) -> None:
     kernel (the SwiGLU product in the GEMM epilogue): what ``gemm`` followed by the element-wise kernel computes,
     without the ``[M, 2 I]`` tensor.  Raises for layers the CTA-pair kernel does not take (``gemm_swiglu_supported``)."""
     dev = _lib.require_cuda(x, qweight, out, scales, zeros, g_idx, bias)
+    _check_layer(qweight, scales, zeros, g_idx)
     R, N = qweight.shape
     K, M, G = R * 8, x.shape[0], scales.shape[0]
     if x.shape != (M, K) or out.shape != (M, N // 2):

@@ -1,0 +1,85 @@
+"""What the host side of the native products checks before anything is launched; no GPU: operands are stand-ins with the
+attributes of tensors, the native module is a stub."""
+import pytest
+import torch
+
+from alpaca_lora_4bit_b200 import _lib, quant_cuda
+
+K, N, G = 512, 256, 4
+
+
+class Operand:
+    """A tensor's attributes, as far as the host code looks."""
+
+    def __init__(self, shape, dtype, device="cuda:0", contiguous=True):
+        self.shape, self.dtype, self.device, self._contiguous = torch.Size(shape), dtype, torch.device(device), contiguous
+        self.is_cuda = self.device.type == "cuda"
+        self._version = 0
+
+    def dim(self):
+        return len(self.shape)
+
+    def numel(self):
+        return self.shape.numel()
+
+    def is_contiguous(self):
+        return self._contiguous
+
+    def data_ptr(self):
+        return 4096
+
+
+class NativeStub:
+    def __init__(self):
+        self.calls = []
+
+    def gemm(self, *args):
+        self.calls.append(args)
+        return None
+
+
+@pytest.fixture
+def native(monkeypatch):
+    stub = NativeStub()
+    monkeypatch.setattr(quant_cuda, "_current_device", lambda: 0)
+    monkeypatch.setattr(quant_cuda, "_raw_stream", lambda idx: 0)
+    monkeypatch.setattr(quant_cuda, "groups_are_sequential", lambda g_idx, groups: True)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(_lib, "_gemm_workspaces", {(0, 0): Operand((1 << 30,), torch.uint8)})
+    monkeypatch.setattr(_lib, "_torch_call", stub)
+    monkeypatch.setattr(quant_cuda, "_zero_term_tables", {})
+    return stub
+
+
+def operands(**kw):
+    o = dict(x=Operand((32, K), torch.float16), qweight=Operand((K // 8, N), torch.int32), out=Operand((32, N), torch.float16),
+             scales=Operand((G, N), torch.float16), zeros=Operand((G, N // 8), torch.int32), g_idx=Operand((K,), torch.int32))
+    o.update(kw)
+    return o
+
+
+BAD = {
+    "zeros on the CPU": dict(zeros=Operand((G, N // 8), torch.int32, "cpu")),
+    "zeros on another GPU": dict(zeros=Operand((G, N // 8), torch.int32, "cuda:1")),
+    "scales on another GPU": dict(scales=Operand((G, N), torch.float16, "cuda:1")),
+    "scales too narrow": dict(scales=Operand((G, N // 2), torch.float16)),
+    "zeros too narrow": dict(zeros=Operand((G, N // 16), torch.int32)),
+    "zeros of fewer groups": dict(zeros=Operand((G - 1, N // 8), torch.int32)),
+    "zeros not packed": dict(zeros=Operand((G, N // 8), torch.float16)),
+    "scales not contiguous": dict(scales=Operand((G, N), torch.float16, contiguous=False)),
+}
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("what", sorted(BAD))
+def test_zero_term_table_is_not_made_from_operands_that_are_no_layer(native, monkeypatch, what, transpose):
+    def launched(*args):
+        raise AssertionError("the table kernel must not be launched")
+    monkeypatch.setattr(_lib, "lib", lambda: type("Lib", (), {"q4_gemm_workspace_bytes": staticmethod(lambda *a: 0),
+                                                              "q4_zero_term_table": staticmethod(launched)}))
+    o = operands(**BAD[what])
+    assert quant_cuda.gemm_new(o["x"], o["qweight"], o["out"], o["scales"], o["zeros"], o["g_idx"], transpose) is None
+    assert quant_cuda._zero_terms(o["scales"], o["zeros"], G, N, 0) is None
+    with pytest.raises(RuntimeError):                       # and the general path says what is wrong
+        quant_cuda.gemm(o["x"], o["qweight"], o["out"], o["scales"], o["zeros"], o["g_idx"], transpose)
+    assert quant_cuda._zero_term_tables == {}
