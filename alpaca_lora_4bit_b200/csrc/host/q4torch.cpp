@@ -36,6 +36,13 @@ const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariab
 bool plain(const at::Tensor& t, at::ScalarType dt, int dev) {
   return t.is_cuda() && t.scalar_type() == dt && t.get_device() == dev && t.is_contiguous();
 }
+// `t` has the leading dimensions of `x` and `cols` columns (not merely as many elements: the same numbers in another
+// shape are another matrix).
+bool rows_like(const at::Tensor& t, const at::Tensor& x, int64_t cols) {
+  return t.dim() == x.dim() && t.size(-1) == cols && t.sizes().slice(0, t.dim() - 1) == x.sizes().slice(0, x.dim() - 1);
+}
+bool vector_of(const at::Tensor& t, int64_t n) { return t.dim() == 1 && t.size(0) == n; }
+bool aligned(const at::Tensor& t) { return (uintptr_t)t.data_ptr() % 16 == 0; }
 void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 
 PyObject* failed(const char* what, int rc) {
@@ -75,7 +82,7 @@ PyObject* py_gemv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int64_t K, N, G;
   if (!plain(*x, at::kHalf, dev) || x->dim() < 1 || !layer_ok(*qw, *sc, *zr, flags & Q4_GEMV_V1, dev, &K, &N, &G) || x->size(-1) != K) Py_RETURN_NONE;
   if (gi && (!plain(*gi, at::kInt, dev) || gi->numel() < K)) Py_RETURN_NONE;
-  if (bi && (!plain(*bi, at::kHalf, dev) || bi->numel() != N)) Py_RETURN_NONE;
+  if (bi && (!plain(*bi, at::kHalf, dev) || !vector_of(*bi, N))) Py_RETURN_NONE;
   const int64_t M = K ? x->numel() / K : 0;
   if (M < 1 || M > 16 || !ws->is_cuda() || ws->get_device() != dev) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(dev);
@@ -106,15 +113,15 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t inner = transpose ? N : K, outer = transpose ? K : N;
   if (inner == 0 || x->size(-1) != inner || !plain(*gi, at::kInt, dev) || gi->numel() < K) Py_RETURN_NONE;
   const int64_t M = x->numel() / inner;
-  if (M < 1) Py_RETURN_NONE;
-  if (given && (!plain(*given, at::kHalf, dev) || given->numel() != M * outer)) Py_RETURN_NONE;
-  if (bi && (transpose || !plain(*bi, at::kHalf, dev) || bi->numel() != N)) Py_RETURN_NONE;
-  if (res && (transpose || !plain(*res, at::kHalf, dev) || res->numel() != M * N)) Py_RETURN_NONE;
+  if (M < 1 || M > INT32_MAX) Py_RETURN_NONE;
+  if (given && (!plain(*given, at::kHalf, dev) || !rows_like(*given, *x, outer))) Py_RETURN_NONE;
+  if (bi && (transpose || !plain(*bi, at::kHalf, dev) || !vector_of(*bi, N))) Py_RETURN_NONE;
+  if (res && (transpose || !plain(*res, at::kHalf, dev) || !rows_like(*res, *x, N) || !aligned(*res))) Py_RETURN_NONE;
   int64_t r = 0;
   if (lu) {
     if (!lw || lw->dim() != 2) Py_RETURN_NONE;
     r = lw->size(transpose ? 0 : 1);
-    if (!plain(*lu, at::kHalf, dev) || lu->numel() != M * 64 || !plain(*lw, at::kHalf, dev) || lw->size(transpose ? 1 : 0) != outer) Py_RETURN_NONE;
+    if (!plain(*lu, at::kHalf, dev) || lu->dim() != 2 || lu->size(0) != M || lu->size(1) != 64 || !plain(*lw, at::kHalf, dev) || lw->size(transpose ? 1 : 0) != outer) Py_RETURN_NONE;
   }
   if (zt && (!plain(*zt, at::kHalf, dev) || zt->numel() != G * N)) Py_RETURN_NONE;
   if (!ws->is_cuda() || ws->get_device() != dev) Py_RETURN_NONE;
@@ -151,10 +158,10 @@ PyObject* py_gemm_v1(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (K == 0 || N == 0 || K % 128 || N % 256 || x->size(-1) != K) Py_RETURN_NONE;
   const int64_t M = x->numel() / K;
   if (M < 1 || M > INT32_MAX) Py_RETURN_NONE;
-  if (bi && (!plain(*bi, at::kHalf, dev) || bi->numel() != N)) Py_RETURN_NONE;
-  if (res && (!plain(*res, at::kHalf, dev) || res->numel() != M * N)) Py_RETURN_NONE;
+  if (bi && (!plain(*bi, at::kHalf, dev) || !vector_of(*bi, N))) Py_RETURN_NONE;
+  if (res && (!plain(*res, at::kHalf, dev) || !rows_like(*res, *x, N))) Py_RETURN_NONE;
   for (const at::Tensor* t : {x, qw, sc, zr, res})                 // (the bias is read by the element)
-    if (t && (uintptr_t)t->data_ptr() % 16) Py_RETURN_NONE;
+    if (t && !aligned(*t)) Py_RETURN_NONE;
   if (!ws->is_cuda() || ws->get_device() != dev) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(dev);
   at::Tensor out = new_rows(*x, N);

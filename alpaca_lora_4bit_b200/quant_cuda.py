@@ -385,6 +385,8 @@ def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora
         raise RuntimeError(f"quant_cuda: gemm shapes x{tuple(x.shape)} out{tuple(out.shape)} do not match the layer [{K},{N}]")
     if x.dtype != torch.float16 or out.dtype != torch.float16 or scales.dtype != torch.float16:
         raise RuntimeError("quant_cuda: gemm takes fp16 x, out and scales")
+    if bias is not None and not transpose and (bias.dtype != torch.float16 or bias.numel() != N):
+        raise RuntimeError(f"quant_cuda: gemm takes an fp16 bias of {N} values")
     r = 0
     if lora_u is not None:
         r = lora_w.shape[0] if transpose else lora_w.shape[1]

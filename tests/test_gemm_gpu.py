@@ -663,3 +663,23 @@ def test_first_product_of_a_layer_waits_for_its_tables(rows):
         want = x.double() @ w.double() + bias.double()
         assert float((warm.double() - want).norm() / want.norm()) <= 1e-3      # fp32 sums rounded to fp16 once
     assert quant_cuda.device_status() == 0
+
+
+def test_gemm_refuses_operands_of_another_shape():
+    """As many elements in another shape are another matrix: refused with a message, forward and backward."""
+    M, K, N, r = 32, 256, 512, 8
+    L = synth.make_layer(K, N, 128, False, seed=1).to(DEV)
+    half = dict(dtype=torch.float16, device=DEV)
+    x, y = torch.zeros(M, K, **half), torch.zeros(M, N, **half)
+    u, b, a = torch.zeros(M, 64, **half), torch.zeros(N, r, **half), torch.zeros(r, K, **half)
+    for kw in (dict(residual=torch.zeros(N, M, **half)), dict(residual=torch.zeros(M * N, **half)), dict(residual=torch.zeros(1, M, N, **half)),
+               dict(lora_u=torch.zeros(2 * M, 32, **half), lora_w=b), dict(lora_u=torch.zeros(M * 64, **half), lora_w=b),
+               dict(lora_u=u, lora_w=b.t().contiguous()), dict(bias=torch.zeros(N // 2, **half)), dict(bias=torch.zeros(N, device=DEV))):
+        with pytest.raises(RuntimeError, match="quant_cuda"):
+            quant_cuda.gemm(x, L.qweight, y, L.scales, L.qzeros, L.g_idx, **kw)
+    for kw in (dict(lora_u=torch.zeros(64, M, **half), lora_w=a), dict(lora_u=u, lora_w=b), dict(residual=torch.zeros(M, K, **half))):
+        with pytest.raises(RuntimeError, match="quant_cuda"):
+            quant_cuda.gemm(y, L.qweight, x, L.scales, L.qzeros, L.g_idx, transpose=True, **kw)
+    quant_cuda.gemm(x, L.qweight, y, L.scales, L.qzeros, L.g_idx, residual=torch.ones(M, N, **half), lora_u=u, lora_w=b)
+    assert bool((y == 1.0).all())
+    assert quant_cuda.device_status() == 0
