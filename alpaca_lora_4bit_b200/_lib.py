@@ -141,6 +141,19 @@ def torch_call():
     return _torch_call
 
 
+def nobody_watches() -> bool:
+    """No function transform (vmap, grad), forward-mode level or tracer is active that would have to see the operations of
+    this call."""
+    return (torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0
+            and torch._C._get_tracing_state() is None)
+
+
+def opaque_call_ok(x) -> bool:
+    """A call that torch does not see into may stand for operations on ``x``: a plain GPU tensor that nothing
+    differentiates, batches or traces through this call."""
+    return x.is_cuda and type(x) is torch.Tensor and not (torch.is_grad_enabled() and x.requires_grad) and nobody_watches()
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         msg = lib().q4_last_error_string().decode("utf-8", "replace")

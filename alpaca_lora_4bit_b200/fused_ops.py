@@ -123,7 +123,7 @@ class _SwiGLUFused(torch.autograd.Function):
 def swiglu_fused(gu: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for ``gu = [gate | up]`` along the last dimension (the output of a fused gate_up
     projection); falls back to ``swiglu`` on the two halves where the kernel does not apply."""
-    if gu.is_cuda and not (torch.is_grad_enabled() and gu.requires_grad):      # nothing to differentiate: one native call
+    if _lib.opaque_call_ok(gu):                    # nothing to differentiate, nobody who would have to see it: one native call
         out = _lib.torch_call().swiglu(gu)
         if out is not None:
             return out

@@ -83,3 +83,25 @@ def test_zero_term_table_is_not_made_from_operands_that_are_no_layer(native, mon
     with pytest.raises(RuntimeError):                       # and the general path says what is wrong
         quant_cuda.gemm(o["x"], o["qweight"], o["out"], o["scales"], o["zeros"], o["g_idx"], transpose)
     assert quant_cuda._zero_term_tables == {}
+
+
+def test_native_calls_stand_back_where_torch_watches():
+    """Under a forward-mode level, a function transform or a tracer the opaque calls are not taken (the operators then go
+    through their autograd functions, which those modes record, refuse or batch)."""
+    x = torch.randn(3, 4)
+    assert _lib.nobody_watches()
+    seen = []
+
+    def look(t):
+        seen.append(_lib.nobody_watches())
+        return t * 2
+
+    with torch.autograd.forward_ad.dual_level():
+        look(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)))
+    torch.func.vmap(look)(x)
+    torch.func.grad(lambda t: look(t).sum())(x)
+    torch.func.jvp(look, (x,), (x,))
+    torch.jit.trace(look, (x,), check_trace=False)
+    assert seen == [False] * 5
+    assert _lib.nobody_watches()
+    assert not _lib.opaque_call_ok(x)                       # and never for tensors that are not on a GPU
