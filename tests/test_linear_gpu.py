@@ -98,3 +98,26 @@ def test_first_format_large_products_both_ways(K2, N2, rows):
     assert float((y2.double() - want).norm() / want.norm()) <= 1e-3
     assert float((yt[1].double() - (want - bias.double() - res.double())[0]).norm() / want.norm()) <= 1e-3
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("fmt", ["seq", "v1"])
+@pytest.mark.parametrize("rows", [4, 40])
+def test_skip_path_is_added_as_torch_adds_it(fmt, rows):
+    """A skip path of another shape than the product's broadcasts (a row, more leading dimensions), one that is not
+    contiguous or off a 16-byte boundary is added all the same, and a forward-mode tangent that it carries is kept."""
+    mod, w, bias = build(fmt, 128 if fmt == "seq" else K)
+    gen = torch.Generator().manual_seed(rows)
+    x, full = torch.randn(rows, K, generator=gen).half().to(DEV), torch.randn(rows, N, generator=gen).half().to(DEV)
+    off = torch.zeros(rows * N + 1, dtype=torch.float16, device=DEV)[1:].view(rows, N)
+    off.copy_(full)
+    with torch.no_grad():
+        plain = mod(x)
+        for res in (full[:1], full[0], full[None], full.t().contiguous().t(), off, full.float()):
+            mod.offer_residual(res)
+            y = mod(x)
+            want = plain + res.half()
+            assert y.shape == want.shape and torch.equal(y, want)
+        with torch.autograd.forward_ad.dual_level():
+            mod.offer_residual(torch.autograd.forward_ad.make_dual(full, full))
+            assert torch.equal(torch.autograd.forward_ad.unpack_dual(mod(x)).tangent, full)
+    assert quant_cuda.device_status() == 0
