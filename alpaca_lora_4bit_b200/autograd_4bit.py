@@ -161,11 +161,16 @@ class Autograd4bitQuantLinear(nn.Module):
         if self.bits == 4 and not torch.is_grad_enabled():
             if backend != 'cuda':
                 raise ValueError('Backend not supported.')
-            b, v1 = self._buffers, self.is_v1_model            # (a buffer looked up as an attribute costs the host a microsecond a call)
-            if 'qweight' not in b or 'bias' not in b:          # registered as something else by whoever wrapped the module
-                b = {n: getattr(self, n, None) for n in ('qweight', 'scales', 'zeros', 'qzeros', 'g_idx', 'bias')}
-            return mm4b.linear(x, b['qweight'], b['scales'], b['zeros' if v1 else 'qzeros'], None if v1 else b['g_idx'],
-                               self.groupsize, None if self.disable_bias else b['bias'], residual)
+            b, v1, bias = self._buffers, self.is_v1_model, None
+            try:                                               # (a buffer looked up as an attribute costs the host a microsecond a call)
+                packed = b['qweight'], b['scales'], b['zeros' if v1 else 'qzeros'], None if v1 else b['g_idx']
+                if not self.disable_bias:
+                    bias = b['bias']
+            except KeyError:                                   # a parameter, a plain attribute, a parametrization
+                packed = self.qweight, self.scales, self.zeros if v1 else self.qzeros, None if v1 else self.g_idx
+                if not self.disable_bias:
+                    bias = self.bias
+            return mm4b.linear(x, *packed, self.groupsize, bias, residual)
         zeros = self.zeros if self.is_v1_model else self.qzeros
         if self.bits == 4:
             if AutogradMatmul4bit is AutogradMatmul4bitCuda:

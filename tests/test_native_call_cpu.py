@@ -3,7 +3,8 @@ attributes of tensors, the native module is a stub."""
 import pytest
 import torch
 
-from alpaca_lora_4bit_b200 import _lib, quant_cuda
+from alpaca_lora_4bit_b200 import _lib, autograd_4bit as a4, matmul_utils_4bit as mm4b, quant_cuda, synth
+from tests import fake_backend
 
 K, N, G = 512, 256, 4
 
@@ -105,3 +106,29 @@ def test_native_calls_stand_back_where_torch_watches():
     assert seen == [False] * 5
     assert _lib.nobody_watches()
     assert not _lib.opaque_call_ok(x)                       # and never for tensors that are not on a GPU
+
+
+def small_module(**kw):
+    layer = synth.make_layer(256, 64, 64, False, 1)
+    mod = a4.Autograd4bitQuantLinear(256, 64, groupsize=64, **kw)
+    mod.qweight, mod.qzeros, mod.scales, mod.g_idx = layer.qweight, layer.qzeros, layer.scales, layer.g_idx
+    mod.bias = torch.randn(64, generator=torch.Generator().manual_seed(2)).half()
+    return mod, synth.make_acts(3, 256, 5)
+
+
+@pytest.mark.parametrize("how", ["parameter", "attribute", "parametrization"])
+@pytest.mark.parametrize("name", ["scales", "qzeros", "g_idx", "qweight", "bias"])
+def test_no_grad_forward_finds_operands_registered_as_something_else(name, how):
+    with fake_backend.installed(), torch.no_grad():
+        mod, x = small_module()
+        want, value = mod(x), getattr(mod, name)
+        if how == "parametrization":
+            class Same(torch.nn.Module):
+                def forward(self, t):
+                    return t.clone()
+            torch.nn.utils.parametrize.register_parametrization(mod, name, Same(), unsafe=True)
+        else:
+            delattr(mod, name)
+            setattr(mod, name, torch.nn.Parameter(value, requires_grad=False) if how == "parameter" else value)
+        assert name not in mod._buffers
+        assert torch.equal(mod(x), want)
