@@ -5,7 +5,8 @@
 (``qweight``, ``qzeros``/``zeros``, ``scales``, ``g_idx``, ``bias``) and routes like the reference
 (autograd_4bit.py:192-208): with grad enabled through ``AutogradMatmul4bit`` (forward ``x @ W``,
 backward ``dy @ W.T``, nothing but the four packed tensors saved), otherwise through
-``matmul4bit_with_backend``.  There is one backend, the sm_100a library: ``switch_backend_to('cuda')``
+``matmul4bit_with_backend`` or, as long as nobody has replaced that, the same product as one native call
+(``matmul_utils_4bit.linear``).  There is one backend, the sm_100a library: ``switch_backend_to('cuda')``
 is accepted, ``'triton'`` is refused.
 """
 from __future__ import annotations
@@ -118,6 +119,9 @@ def matmul4bit_with_backend(x, qweight, scales, qzeros, g_idx, bits, maxq, group
     raise ValueError('Backend not supported.')
 
 
+_own_matmul4bit_with_backend = matmul4bit_with_backend
+
+
 # Assumes layer is perfectly divisible into 256 * 256 blocks
 class Autograd4bitQuantLinear(nn.Module):
 
@@ -155,10 +159,10 @@ class Autograd4bitQuantLinear(nn.Module):
         self.__dict__["_q4_residual"] = residual
 
     def forward(self, x):
-        return self._forward(x, self.__dict__.pop("_q4_residual", None))
+        return self._forward(x, self.take_residual())
 
     def _forward(self, x, residual=None):
-        if self.bits == 4 and not torch.is_grad_enabled():
+        if self.bits == 4 and not torch.is_grad_enabled() and matmul4bit_with_backend is _own_matmul4bit_with_backend:
             if backend != 'cuda':
                 raise ValueError('Backend not supported.')
             b, v1, bias = self._buffers, self.is_v1_model, None
@@ -172,7 +176,9 @@ class Autograd4bitQuantLinear(nn.Module):
                     bias = self.bias
             return mm4b.linear(x, *packed, self.groupsize, bias, residual)
         zeros = self.zeros if self.is_v1_model else self.qzeros
-        if self.bits == 4:
+        if self.bits == 4 and not torch.is_grad_enabled():     # the program's own product
+            out = matmul4bit_with_backend(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, self.groupsize)
+        elif self.bits == 4:
             if AutogradMatmul4bit is AutogradMatmul4bitCuda:
                 # bias and residual ride in the product's epilogue instead of further passes over the output
                 bias = None if (self.disable_bias or self.bias is None) else self.bias

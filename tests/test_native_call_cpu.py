@@ -132,3 +132,36 @@ def test_no_grad_forward_finds_operands_registered_as_something_else(name, how):
             setattr(mod, name, torch.nn.Parameter(value, requires_grad=False) if how == "parameter" else value)
         assert name not in mod._buffers
         assert torch.equal(mod(x), want)
+
+
+def test_no_grad_forward_calls_a_product_that_was_put_in_place(monkeypatch):
+    mod, x = small_module()
+    res = torch.randn(3, 64).half()
+    seen = []
+
+    def ones(x, *args):
+        seen.append(args)
+        return torch.ones(x.shape[:-1] + (64,), dtype=torch.float16)
+
+    with torch.no_grad():
+        for target, name in ((a4, "matmul4bit_with_backend"), (mm4b, "matmul4bit")):
+            with monkeypatch.context() as m:
+                m.setattr(target, name, ones)
+                assert torch.equal(mod(x), 1 + mod.bias.expand(3, 64))
+                mod.offer_residual(res)
+                assert torch.equal(mod(x), (1 + mod.bias.expand(3, 64)) + res)
+    assert len(seen) == 4 and all(a[0] is mod.qweight and a[2] is mod.qzeros for a in seen)
+
+
+def test_skip_path_is_taken_through_the_method():
+    class Sub(a4.Autograd4bitQuantLinear):
+        def take_residual(self):
+            super().take_residual()
+            return None
+
+    mod, x = small_module()
+    with fake_backend.installed(), torch.no_grad():
+        want = mod(x)
+        mod.__class__ = Sub
+        mod.offer_residual(torch.ones(3, 64).half())
+        assert torch.equal(mod(x), want)
