@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import warnings
 from ctypes import c_char_p, c_int, c_size_t, c_uint, c_void_p
 
 import torch
@@ -119,25 +120,40 @@ def layer_gemv_call():
     return _layer_gemv_call
 
 
+class _NoTorchCall:
+    """In the place of ``_q4torch`` where it cannot be built or loaded: takes no operands, so that every product goes through
+    the ctypes binding, to the same kernels."""
+    @staticmethod
+    def gemv(*_):
+        return None
+
+    gemm = gemm_v1 = swiglu = gemv
+
+
 _torch_call = None
 
 
 def torch_call():
-    """The ``_q4torch`` module (built in-tree on first use), bound to the loaded library: products on torch tensors as
-    one native call each.  Its functions return ``None`` for operands they do not take."""
+    """The ``_q4torch`` module (built in-tree on first use, and again when its sources or torch have changed), bound to the
+    loaded library: products on torch tensors as one native call each.  Its functions return ``None`` for operands they do
+    not take.  Without a C++ compiler or torch's headers, say, the reason is given once and the stand-in above serves."""
     global _torch_call
     if _torch_call is not None:
         return _torch_call
     handle = lib()
     with _lock:
         if _torch_call is None:
-            if not os.path.exists(os.path.join(_PKG, "_q4torch.so")):
+            try:
                 from . import build as _build
                 _build.build_torch_call()
-            from . import _q4torch
-            _q4torch.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
-                "q4_gemv", "q4_gemm_fwd_residual", "q4_gemm_bwd_table", "q4_gemm_bwd", "q4_swiglu_fwd", "q4_last_error_string", "q4_gemm_fwd_v1")))
-            _torch_call = _q4torch
+                from . import _q4torch
+                _q4torch.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
+                    "q4_gemv", "q4_gemm_fwd_residual", "q4_gemm_bwd_table", "q4_gemm_bwd", "q4_swiglu_fwd", "q4_last_error_string", "q4_gemm_fwd_v1")))
+                _torch_call = _q4torch
+            except Exception as e:
+                warnings.warn(f"q4b200: the native module for torch tensors is not available ({type(e).__name__}: {e}); "
+                              "products go through the ctypes binding, at a higher cost per call")
+                _torch_call = _NoTorchCall
     return _torch_call
 
 

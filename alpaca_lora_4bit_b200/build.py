@@ -88,13 +88,34 @@ def build_call(force: bool = False) -> str:
 
 TORCH_SRC = os.path.join(CSRC, "host", "q4torch.cpp")
 TORCH_LIB = os.path.join(PKG, "_q4torch.so")
+TORCH_KEY = os.path.join(PKG, "_q4torch.key")          # what the module beside it was built from
+
+
+def _torch_call_key() -> str:
+    """The sources, and the torch and Python whose binary interface the module is compiled against."""
+    import hashlib
+    import torch
+    h = hashlib.sha256()
+    for path in (TORCH_SRC, os.path.join(ROOT, "include", "q4b200.h")):
+        with open(path, "rb") as f:
+            h.update(f.read())
+    return f"{h.hexdigest()} torch {torch.__version__} python {sys.version.split()[0]}\n"
+
+
+def _torch_call_current(key: str) -> bool:
+    try:
+        with open(TORCH_KEY) as f:
+            return f.read() == key and os.path.exists(TORCH_LIB)
+    except OSError:
+        return False
 
 
 def build_torch_call(force: bool = False) -> str:
     """Builds ``_q4torch.so`` (the CPython module that takes torch tensors through the library) with the C++ compiler,
-    against the headers and libraries of the installed torch."""
-    deps = [TORCH_SRC, os.path.join(ROOT, "include", "q4b200.h")]
-    if not force and os.path.exists(TORCH_LIB) and all(os.path.getmtime(TORCH_LIB) >= os.path.getmtime(d) for d in deps):
+    against the headers and libraries of the installed torch; a module built from other sources or against another torch
+    is built again."""
+    key = _torch_call_key()
+    if not force and _torch_call_current(key):
         return TORCH_LIB
     import sysconfig
     import torch
@@ -103,12 +124,15 @@ def build_torch_call(force: bool = False) -> str:
         raise RuntimeError("no C++ compiler; _q4torch.so cannot be built")
     base = os.path.dirname(torch.__file__)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    tmp = TORCH_LIB + ".tmp"
+    tmp = f"{TORCH_LIB}.{os.getpid()}.tmp"             # (several ranks may find it missing at once)
     subprocess.check_call([cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                            "-I", os.path.join(base, "include"), "-I", os.path.join(base, "include", "torch", "csrc", "api", "include"),
                            "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], TORCH_SRC, "-o", tmp,
                            "-L", os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
     os.replace(tmp, TORCH_LIB)
+    with open(tmp, "w") as f:
+        f.write(key)
+    os.replace(tmp, TORCH_KEY)
     return TORCH_LIB
 
 

@@ -1,5 +1,8 @@
 """What the host side of the native products checks before anything is launched; no GPU: operands are stand-ins with the
 attributes of tensors, the native module is a stub."""
+import os
+import warnings
+
 import pytest
 import torch
 
@@ -165,3 +168,56 @@ def test_skip_path_is_taken_through_the_method():
         mod.__class__ = Sub
         mod.offer_residual(torch.ones(3, 64).half())
         assert torch.equal(mod(x), want)
+
+
+@pytest.fixture
+def build_in(tmp_path, monkeypatch):
+    """The build of the native module with its products in a folder of the test's own and the compiler a stub."""
+    from alpaca_lora_4bit_b200 import build
+    src = tmp_path / "q4torch.cpp"
+    src.write_text("int one;")
+    runs = []
+
+    def compile_(cmd):
+        runs.append(cmd)
+        with open(cmd[cmd.index("-o") + 1], "w") as f:
+            f.write("module")
+    monkeypatch.setattr(build, "TORCH_SRC", str(src))
+    monkeypatch.setattr(build, "TORCH_LIB", str(tmp_path / "_q4torch.so"))
+    monkeypatch.setattr(build, "TORCH_KEY", str(tmp_path / "_q4torch.key"))
+    monkeypatch.setattr(build.subprocess, "check_call", compile_)
+    return build, src, runs
+
+
+def test_native_module_is_built_again_when_its_sources_or_torch_change(build_in, monkeypatch):
+    build, src, runs = build_in
+    for _ in range(3):
+        assert build.build_torch_call() == build.TORCH_LIB
+    assert len(runs) == 1
+    src.write_text("int two;")
+    os.utime(src, (0, 0))                                   # an older file with other contents
+    build.build_torch_call()
+    build.build_torch_call()
+    assert len(runs) == 2
+    monkeypatch.setattr(torch, "__version__", "9.9.9")
+    build.build_torch_call()
+    build.build_torch_call()
+    assert len(runs) == 3
+    os.remove(build.TORCH_LIB)
+    build.build_torch_call()
+    assert len(runs) == 4 and sorted(os.listdir(src.parent)) == ["_q4torch.key", "_q4torch.so", "q4torch.cpp"]
+
+
+def test_without_the_native_module_the_ctypes_binding_serves(monkeypatch):
+    from alpaca_lora_4bit_b200 import build
+
+    def fails():
+        raise RuntimeError("no C++ compiler")
+    monkeypatch.setattr(build, "build_torch_call", fails)
+    monkeypatch.setattr(_lib, "_torch_call", None)
+    with pytest.warns(UserWarning, match="no C\\+\\+ compiler"):
+        native = _lib.torch_call()
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")                      # said once
+        assert _lib.torch_call() is native
+    assert native.gemm() is None and native.swiglu(1) is None and native.gemv(1, 2) is None and native.gemm_v1(1) is None
