@@ -249,7 +249,7 @@ def gemv_new(x, qweight, scales, zeros, g_idx, bias, groupsize, flags):
 _gemm_ws_bytes: dict = {}
 
 
-_seq_cache: dict = {}        # id(g_idx) -> (weak reference, storage address, version counter, answer)
+_seq_cache: dict = {}        # id(g_idx) -> (weak reference, storage address, version counter, {group count: answer})
 
 
 def groups_are_sequential(g_idx, groups: int) -> bool:
@@ -260,8 +260,12 @@ def groups_are_sequential(g_idx, groups: int) -> bool:
     import weakref
     key = id(g_idx)
     hit = _seq_cache.get(key)
-    if hit is not None and hit[0]() is g_idx and hit[1] == g_idx.data_ptr() and hit[2] == g_idx._version:
-        return hit[3]
+    if hit is not None and (hit[0]() is not g_idx or hit[1] != g_idx.data_ptr() or hit[2] != g_idx._version):
+        hit = None
+    if hit is not None:
+        ok = hit[3].get(groups)
+        if ok is not None:
+            return ok
     if g_idx.is_cuda and torch.cuda.is_current_stream_capturing():
         return False
     K = g_idx.numel()
@@ -269,7 +273,9 @@ def groups_are_sequential(g_idx, groups: int) -> bool:
     if ok:
         want = torch.arange(K, device=g_idx.device, dtype=torch.int64) // (K // groups)
         ok = bool(torch.equal(g_idx.reshape(-1).to(torch.int64), want))
-    _seq_cache[key] = (weakref.ref(g_idx, lambda _r, key=key: _seq_cache.pop(key, None)), g_idx.data_ptr(), g_idx._version, ok)
+    if hit is None:
+        hit = _seq_cache[key] = (weakref.ref(g_idx, lambda _r, key=key: _seq_cache.pop(key, None)), g_idx.data_ptr(), g_idx._version, {})
+    hit[3][groups] = ok
     return ok
 
 

@@ -221,3 +221,16 @@ def test_without_the_native_module_the_ctypes_binding_serves(monkeypatch):
         warnings.simplefilter("error")                      # said once
         assert _lib.torch_call() is native
     assert native.gemm() is None and native.swiglu(1) is None and native.gemv(1, 2) is None and native.gemm_v1(1) is None
+
+
+def test_order_of_groups_is_answered_per_group_count():
+    """One g_idx asked with several group counts: each gets its own answer, also after it is written to."""
+    g_idx = torch.zeros(256, dtype=torch.int32)
+    for _ in range(2):
+        assert quant_cuda.groups_are_sequential(g_idx, 1)
+        assert not quant_cuda.groups_are_sequential(g_idx, 4)
+        assert not quant_cuda.groups_are_sequential(g_idx, 3) and not quant_cuda.groups_are_sequential(g_idx, 0)
+    g_idx.copy_(torch.arange(256) // 64)
+    for _ in range(2):
+        assert quant_cuda.groups_are_sequential(g_idx, 4)
+        assert not quant_cuda.groups_are_sequential(g_idx, 1)
