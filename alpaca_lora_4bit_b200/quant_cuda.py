@@ -309,7 +309,8 @@ def _check_layer(qweight, scales, zeros, g_idx) -> None:
 def _zero_terms(scales, zeros, G, N, st):
     key = id(zeros)
     hit = _zero_term_tables.get(key)
-    if hit is not None and hit[1] == (zeros.data_ptr(), scales.data_ptr(), zeros._version, scales._version):
+    # (the scales' object too: another tensor may have come to lie at the address of one that was freed)
+    if hit is not None and hit[1] == (zeros.data_ptr(), scales.data_ptr(), zeros._version, scales._version) and hit[3]() is scales:
         return hit[0]
     if not _is_layer_table(scales, zeros, G, N):
         return None                                    # nothing is launched on operands that do not describe a layer
@@ -319,7 +320,8 @@ def _zero_terms(scales, zeros, G, N, st):
     table = torch.empty((G, N), dtype=torch.float16, device=scales.device)
     _lib.check(_lib.lib().q4_zero_term_table(scales.data_ptr(), zeros.data_ptr(), table.data_ptr(), G, N, st), "zero_term_table")
     ref = weakref.ref(zeros, lambda _r, key=key: _zero_term_tables.pop(key, None))
-    _zero_term_tables[key] = (table, (zeros.data_ptr(), scales.data_ptr(), zeros._version, scales._version), ref)
+    _zero_term_tables[key] = (table, (zeros.data_ptr(), scales.data_ptr(), zeros._version, scales._version), ref,
+                              weakref.ref(scales))
     return table
 
 

@@ -234,3 +234,14 @@ def test_order_of_groups_is_answered_per_group_count():
     for _ in range(2):
         assert quant_cuda.groups_are_sequential(g_idx, 4)
         assert not quant_cuda.groups_are_sequential(g_idx, 1)
+
+
+def test_zero_term_table_follows_the_scales_object(native, monkeypatch):
+    """New scales at the address of freed ones, no writes counted on either: the table is made again."""
+    made = []
+    monkeypatch.setattr(_lib, "lib", lambda: type("Lib", (), {"q4_zero_term_table": staticmethod(lambda *a: made.append(a) or 0)}))
+    monkeypatch.setattr(torch, "empty", lambda shape, dtype, device: Operand(shape, dtype, str(device)))
+    zeros, first, second = operands()["zeros"], operands()["scales"], operands()["scales"]
+    a = quant_cuda._zero_terms(first, zeros, G, N, 0)
+    assert quant_cuda._zero_terms(first, zeros, G, N, 0) is a and len(made) == 1
+    assert quant_cuda._zero_terms(second, zeros, G, N, 0) is not a and len(made) == 2
