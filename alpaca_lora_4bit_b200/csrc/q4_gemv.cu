@@ -1840,20 +1840,31 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
 // Splits of the contraction for the act-order kernel: CTAs per SM times what one of them costs in steps (its own and
 // about ten for its tables, its reduction and the exchange), with no fewer than three CTAs' worth on an SM counted: fewer
 // leave it waiting for latency.  A CTA keeps the table offsets of its rows, so a split has at most ACT_MAX_STEPS steps -
-// as long as the partial sums of 16 rows stay within ACT_PART_BYTES.
-static void gemv_plan(int K, int N, int& S, int& steps_per_split) {
+// as long as the partial sums of 16 rows stay within ACT_PART_BYTES and within what the caller's workspace holds.
+static void gemv_plan(int K, int N, size_t part_bytes, int& S, int& steps_per_split) {
   const int tiles = N / GEMV_TN, steps = K / 32, sms = 148;      // (a constant: the workspace is sized without a device)
   long long best = -1;
   S = 1; steps_per_split = (steps + GEMV_WARPS - 1) / GEMV_WARPS * GEMV_WARPS;
   for (int want = 1; want <= 64; ++want) {
     const int per = ((steps + want - 1) / want + GEMV_WARPS - 1) / GEMV_WARPS * GEMV_WARPS;
     const int s = (steps + per - 1) / per;
-    if (s > 1 && (size_t)s * 16 * N * sizeof(float) > ACT_PART_BYTES) break;
+    if (s > 1 && (size_t)s * 16 * N * sizeof(float) > part_bytes) break;
     const long long ctas = ((long long)tiles * s + sms - 1) / sms;
     long long cost = (ctas < 3 ? 3 : ctas) * (per + 10);
     if (per > ACT_MAX_STEPS) cost *= 4;
     if (best < 0 || cost < best) { best = cost; S = s; steps_per_split = per; }
   }
+}
+
+// The splits a workspace has room for by its documented size: four CTAs per SM, splits of at least 1024 rows.  (The size
+// is part of the interface - callers and the built-in scratch go by it - and does not follow the plan above, which takes
+// more splits where it is given more memory.)
+static int gemv_sized_splits(int K, int N) {
+  const int tiles = N / GEMV_TN, steps = K / 32;
+  const int want = (592 + tiles - 1) / tiles, cap = steps < 32 ? 1 : steps / 32;
+  const int s = want < cap ? want : cap;
+  const int per = ((steps + s - 1) / s + 3) / 4 * 4;
+  return (steps + per - 1) / per;
 }
 
 // What q4_layer_gemv knows about the layer that follows (set around its call of q4_gemv, on the calling thread)
@@ -2051,8 +2062,7 @@ extern "C" int q4_gemv_set_variant(int variant) {
 
 extern "C" size_t q4_gemv_workspace_bytes(int M, int K, int N) {
   if (M <= 0 || K <= 0 || N <= 0 || K % 32 || N % 32) return 0;
-  int S, sps;
-  gemv_plan(K, N, S, sps);
+  const int S = gemv_sized_splits(K, N);
   const size_t split = S > 1 ? (size_t)S * M * N * sizeof(float) : 0;           // act-order kernel
   const size_t stream = (size_t)(GEMV_MAX_CTAS + 4) * 2 * 16 * GEMV_TN * sizeof(float); // streaming kernels
   return GEMV_WS_HEAD + (split > stream ? split : stream);
@@ -2162,7 +2172,8 @@ extern "C" int q4_gemv(const void* x, const int32_t* qweight, void* y, const voi
   p.qzeros = (const uint32_t*)qzeros; p.g_idx = g_idx; p.bias = (const __half*)bias;
   p.M = M; p.K = K; p.N = N; p.groupsize = groupsize;
   p.steps_total = K / 32;
-  gemv_plan(K, N, p.S, p.steps_per_split);
+  const size_t part_room = workspace_bytes - GEMV_WS_HEAD;
+  gemv_plan(K, N, part_room < ACT_PART_BYTES ? part_room : ACT_PART_BYTES, p.S, p.steps_per_split);
   p.y_f32 = (y_dtype == Q4_F32); p.accumulate = (flags & Q4_GEMV_ACCUMULATE) ? 1 : 0; p.v1 = v1 ? 1 : 0;
   p.counters = (unsigned*)workspace;
   p.part = (float*)((char*)workspace + GEMV_WS_HEAD);

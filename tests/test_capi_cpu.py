@@ -99,3 +99,14 @@ def test_call_module_makes_the_same_foreign_call():
         call(0, 0, 0)
     with pytest.raises(ValueError):
         call(0, 0, 0, -5, 0, 0, 0)
+
+
+def test_decode_workspace_sizes_are_those_callers_go_by():
+    """The size of a decode workspace does not grow with what a kernel could use: shapes that the built-in scratch serves
+    stay served (16 rows of wide layers among them), those it refuses by size stay refused."""
+    L = _lib.lib()
+    served = [(16, 4096, 8224), (16, 4096, 16384), (16, 8192, 8192), (16, 8192, 28672), (12, 8192, 12640), (16, 13824, 5472),
+              (16, 16384, 4128), (12, 28672, 8192), (1, 28672, 32768)]
+    for M, K, N in served:
+        assert L.q4_gemv_workspace_bytes(M, K, N) <= L.q4_gemv_static_max_bytes(), (M, K, N)
+    assert L.q4_gemv_workspace_bytes(16, 8192, 18432) > L.q4_gemv_static_max_bytes()

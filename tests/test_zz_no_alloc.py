@@ -72,3 +72,27 @@ def test_static_scratch_refuses_oversized_shapes():
         rc = lib.q4_gemv_static(x.data_ptr(), L.qweight.data_ptr(), y.data_ptr(), L.scales.data_ptr(), L.qzeros.data_ptr(),
                                 None, None, 16, 8192, 18432, 64, 128, _lib.Q4_F32, 0, torch.cuda.current_stream().cuda_stream)
     assert rc == -4 and b"built-in scratch" in lib.q4_last_error_string()
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 4096, 8448), (12, 8192, 12672), (16, 16384, 4224), (1, 13824, 5120), (16, 4096, 16384)])
+def test_static_scratch_serves_act_order_products_that_could_use_more(M, K, N):
+    """Act-order products whose plan takes more partial sums than the built-in scratch holds where it is given more memory:
+    within the scratch they are cut less often, same product."""
+    lib = _lib.lib()
+    layer = synth.make_layer(K, N, 128, True, seed=K + N)
+    L = layer.to(DEV)
+    x = synth.make_acts(M, K, seed=M).to(DEV)
+    w = torch.empty((K, N), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v2(L.qweight, w, L.scales, L.qzeros, L.g_idx)
+    want = x.double() @ w.double()
+    ws = torch.zeros(4 << 20, dtype=torch.uint8, device=DEV)
+    big, small = (torch.full((M, N), float("nan"), dtype=torch.float32, device=DEV) for _ in range(2))
+    with torch.cuda.device(torch.device(DEV)):
+        _call(lib.q4_gemv, x, L, big, M, K, N, _lib.GEMV_ACT_ORDER, (ws.data_ptr(), ws.numel()))
+        _call(lib.q4_gemv_static, x, L, small, M, K, N, _lib.GEMV_ACT_ORDER, ())
+    torch.cuda.synchronize()
+    for y in (big, small):                             # weights rounded to fp16 on either side: 2 * 2^-11
+        assert _rel(y, want) <= 1e-3
+    status = ctypes.c_uint(1)
+    _lib.check(lib.q4_gemv_static_status(ctypes.byref(status)), "static status")
+    assert status.value == 0
