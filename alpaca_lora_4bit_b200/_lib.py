@@ -18,7 +18,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libq4b200.so")
 
 Q4_F16, Q4_F32 = 0, 1
-GEMV_ACCUMULATE, GEMV_ACT_ORDER, GEMV_V1 = 1, 2, 4
+GEMV_ACCUMULATE, GEMV_ACT_ORDER, GEMV_V1, GEMV_WRITTEN = 1, 2, 4, 8
 
 _lib = None
 _lock = threading.Lock()

@@ -19,7 +19,7 @@
 // 32-column tile) that arrive by TMA on mbarriers; W is the A operand of mma.sync (rows = output columns),
 // x the B operand (columns = batch rows); sums are kept in fp32 (or exact integers) and added in a fixed
 // order, so results are reproducible; launches carry the programmatic-dependent-launch attribute and wait
-// for the earlier kernel only before they first touch x, y or the workspace (weights never depend on an
+// for the earlier kernel only before they first touch x, y or the workspace (weights do not depend on an
 // earlier kernel); every wait on a barrier or a flag is bounded - on expiry the kernel records a status word
 // in the workspace (q4_gemv_status), stops waiting and runs to its end.
 #include "q4_async.cuh"
@@ -50,6 +50,7 @@ struct GemvParams {
   int M, K, N, groupsize;
   int steps_total, steps_per_split, S;
   int y_f32, accumulate;
+  int overlap;                        // host: the launch may begin before the kernel ahead has ended
   int v1;                             // v1 layer: scales fp16 [N], qzeros reinterpreted as fp16 zeros [N]
 };
 
@@ -274,7 +275,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     }
   };
   issue(0);
-  issue(1);                                              // weights never depend on an earlier kernel
+  issue(1);                                              // weights do not depend on an earlier kernel (Q4_GEMV_WRITTEN)
 
   const int g = lane >> 2, t = lane & 3;
   const int K = p.K;
@@ -705,7 +706,7 @@ gemv_fast_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   };
   if (threadIdx.x == 0) trace_mark_ns(trc, 48);
   issue_w(0);
-  issue_w(1);                                            // weights never depend on an earlier kernel
+  issue_w(1);                                            // weights do not depend on an earlier kernel (Q4_GEMV_WRITTEN)
   if (threadIdx.x == 0) trace_mark_ns(trc, 41);
   pdl_wait();                                            // x, y and the workspace belong to the stream order
   if (threadIdx.x == 0) trace_mark_ns(trc, 42);
@@ -1174,7 +1175,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     trc[(size_t)blockIdx.x * 64 + 47] = smid + 1;
   }
-  // own barriers, then the copies that fill the own ring: weights never depend on an earlier kernel
+  // own barriers, then the copies that fill the own ring: weights do not depend on an earlier kernel (Q4_GEMV_WRITTEN)
   if (lane < S) { mbar_init(&full[warp * S + lane], 1); mbar_init(&empty[warp * S + lane], 1); }
   if (lane < S) mbar_fence_init();
   if (warp == 0 && lane == 0) tma_prefetch_desc(&wmap);
@@ -1540,7 +1541,7 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       }
       for (int r = 0; r < rounds; ++r, ++rc) {
         const int ux = r * W + lane;
-        if (lane < W && ux < upt) {              // weights never depend on an earlier kernel: they go first
+        if (lane < W && ux < upt) {              // weights do not depend on an earlier kernel (Q4_GEMV_WRITTEN): they go first
           const int st = n % S;
           if (n >= S && !mbar_wait_sleep_bounded(&empty[lane * S + st], ((n / S) & 1) ^ 1, flags[0] ? 4u : 200000u)) expired();
           mbar_arrive_expect_tx(&full[lane * S + st], GEMV_UNIT_BYTES);
@@ -1896,7 +1897,7 @@ static int launch_act(const GemvParams& p, int G, int copies, int staged, size_t
   cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = p.overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
   return check_cuda(cudaLaunchKernelEx(&cfg, gemv_act_kernel<MT>, p, G, copies, staged), "gemv launch");
 }
@@ -1920,7 +1921,7 @@ static int launch_stream(const CUtensorMap& map, const CUtensorMap& smap, const 
   cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = sp.g.overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
   return check_cuda(cudaLaunchKernelEx(&cfg, gemv_stream_kernel<MT, FAST, XS>, map, smap, zmap, sp), "gemv launch");
 }
@@ -1950,7 +1951,7 @@ static int launch_fast_xc(const CUtensorMap& map, const GemvStreamParams& sp, in
   cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = sp.g.overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
   return check_cuda(cudaLaunchKernelEx(&cfg, gemv_fast_kernel<MR, TRACE, XC, V1, W, OCC>, map, map, map, sp), "gemv launch");
 }
@@ -1975,7 +1976,7 @@ static int launch_ws(const CUtensorMap& wmap, const CUtensorMap& smap, const CUt
   cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = sp.g.overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
   return check_cuda(cudaLaunchKernelEx(&cfg, gemv_ws_kernel<W, S, OCC, TRACE>, wmap, smap, zmap, pmap, nmap, sp), "gemv launch");
 }
@@ -2079,6 +2080,7 @@ extern "C" int q4_gemv(const void* x, const int32_t* qweight, void* y, const voi
   if (y_dtype != Q4_F16 && y_dtype != Q4_F32) return fail(Q4_E_BADARG, "gemv: unknown y_dtype %d", y_dtype);
   const bool act = flags & Q4_GEMV_ACT_ORDER;
   const bool v1 = flags & Q4_GEMV_V1;
+  const int overlap = flags & Q4_GEMV_WRITTEN ? 0 : 1;
   if (v1) {
     if (act) return fail(Q4_E_BADARG, "gemv: v1 layers have no g_idx");
     // v1 layers are served by the lean kernel (K in whole 256-row units) and by the streaming instance for
@@ -2142,12 +2144,13 @@ extern "C" int q4_gemv(const void* x, const int32_t* qweight, void* y, const voi
       }
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      at[0].val.programmaticStreamSerializationAllowed = 1;
+      at[0].val.programmaticStreamSerializationAllowed = overlap;
       cudaLaunchConfig_t c1 = {};
       c1.gridDim = dim3((MR * n_blocks + 255) / 256); c1.blockDim = dim3(256); c1.stream = st; c1.attrs = at; c1.numAttrs = 1;
       if (int e = check_cuda(wide ? cudaLaunchKernelEx(&c1, x_convert_kernel<16>, (const __half*)x, xq, xinfo, M, K, n_blocks)
                                   : cudaLaunchKernelEx(&c1, x_convert_kernel<8>, (const __half*)x, xq, xinfo, M, K, n_blocks),
                              "gemv conversion launch")) return e;
+      at[0].val.programmaticStreamSerializationAllowed = 1;       // (what was written ahead was there before the conversion began)
       int grid = sm_count();
       if (grid > rp.tiles) grid = rp.tiles;
       cudaLaunchConfig_t c2 = {};
@@ -2174,7 +2177,7 @@ extern "C" int q4_gemv(const void* x, const int32_t* qweight, void* y, const voi
   p.steps_total = K / 32;
   const size_t part_room = workspace_bytes - GEMV_WS_HEAD;
   gemv_plan(K, N, part_room < ACT_PART_BYTES ? part_room : ACT_PART_BYTES, p.S, p.steps_per_split);
-  p.y_f32 = (y_dtype == Q4_F32); p.accumulate = (flags & Q4_GEMV_ACCUMULATE) ? 1 : 0; p.v1 = v1 ? 1 : 0;
+  p.y_f32 = (y_dtype == Q4_F32); p.accumulate = (flags & Q4_GEMV_ACCUMULATE) ? 1 : 0; p.v1 = v1 ? 1 : 0; p.overlap = overlap;
   p.counters = (unsigned*)workspace;
   p.part = (float*)((char*)workspace + GEMV_WS_HEAD);
   cudaStream_t st = (cudaStream_t)stream;

@@ -217,7 +217,7 @@ def decode_v2(x, qweight, scales, zeros, groupsize, plan_key=None):
     idx = dev.index
     if idx != torch.cuda.current_device() or not (qweight.is_contiguous() and scales.is_contiguous() and zeros.is_contiguous()):
         y = torch.empty((M, N), dtype=torch.float16, device=dev)
-        gemv(x, qweight.contiguous(), y, scales.contiguous(), zeros.contiguous(), None, groupsize, 0)
+        gemv(x, qweight.contiguous(), y, scales.contiguous(), zeros.contiguous(), None, groupsize, _lib.GEMV_WRITTEN)
         return y
     y = torch.empty((M, N), dtype=torch.float16, device=dev)
     st = _raw_stream(idx)
@@ -521,6 +521,11 @@ def _half(t):
     return t if t.dtype == torch.float16 else t.half()
 
 
+def _made(*pairs) -> int:
+    """The flag of a product whose operands (given tensor, tensor for the kernel) a cast or a copy made just ahead of it."""
+    return 0 if all(a.data_ptr() == b.data_ptr() for a, b in pairs) else _lib.GEMV_WRITTEN
+
+
 def vecquant4matmul(vec, mat, mul, scales, zeros, g_idx) -> None:
     """``mul += vec @ W`` with the group of every row taken from ``g_idx`` (quant_cuda.cpp:41-48).
 
@@ -532,8 +537,9 @@ def vecquant4matmul(vec, mat, mul, scales, zeros, g_idx) -> None:
         raise RuntimeError("quant_cuda: vec and mul must share a dtype")
     K = vec.shape[-1]
     G = scales.shape[0]
-    gemv(_half(vec).contiguous(), mat, mul, _half(scales), zeros, g_idx, max(K // G, 1),
-         _lib.GEMV_ACCUMULATE | _lib.GEMV_ACT_ORDER)
+    sh = _half(scales)
+    gemv(_half(vec).contiguous(), mat, mul, sh, zeros, g_idx, max(K // G, 1),
+         _lib.GEMV_ACCUMULATE | _lib.GEMV_ACT_ORDER | _made((scales, sh)))
 
 
 def vecquant4matmul_g(vec, mat, mul, scales, zeros, g_idx, vec_height=None) -> None:
@@ -553,7 +559,8 @@ def vecquant4matmul_old_faster(vec, mat, mul, scales, zeros, groupsize, vec_heig
     _check_int32(mat, "mat"); _check_int32(zeros, "zeros")
     if vec.dtype != torch.float16 or mul.dtype != torch.float32:
         raise RuntimeError("quant_cuda: vecquant4matmul_old_faster takes half vec and float mul")
-    gemv(vec.contiguous(), mat, mul, _half(scales), zeros, None, int(groupsize), _lib.GEMV_ACCUMULATE)
+    sh = _half(scales)
+    gemv(vec.contiguous(), mat, mul, sh, zeros, None, int(groupsize), _lib.GEMV_ACCUMULATE | _made((scales, sh)))
 
 
 def vecquant4matmul_v1_faster(vec, mat, mul, scales, zeros) -> None:
@@ -562,8 +569,8 @@ def vecquant4matmul_v1_faster(vec, mat, mul, scales, zeros) -> None:
     if vec.dtype != torch.float16 or mul.dtype != torch.float16:
         raise RuntimeError("quant_cuda: vecquant4matmul_v1_faster takes half vec and mul")
     K = vec.shape[-1]
-    gemv(vec.contiguous(), mat, mul, _half(scales).reshape(-1).contiguous(), _half(zeros).reshape(-1).contiguous(),
-         None, K, _lib.GEMV_ACCUMULATE | _lib.GEMV_V1)
+    sh, zh = _half(scales).reshape(-1).contiguous(), _half(zeros).reshape(-1).contiguous()
+    gemv(vec.contiguous(), mat, mul, sh, zh, None, K, _lib.GEMV_ACCUMULATE | _lib.GEMV_V1 | _made((scales, sh), (zeros, zh)))
 
 
 def _dead(name):

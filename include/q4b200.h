@@ -52,6 +52,9 @@ extern "C" {
                                   W = scales[n]*q - zeros[n]; G, groupsize and g_idx are ignored;
                                   K must be a multiple of 128 (Q4_E_SHAPE otherwise), as for the
                                   reference's v1 kernel */
+#define Q4_GEMV_WRITTEN    8u  /* the work just ahead on the stream wrote some of the layer's tensors (a cast of the
+                                  scales, say): nothing is read before it has ended.  Without this flag the kernels
+                                  may fetch qweight, scales and qzeros while the kernel ahead is still running */
 
 typedef void* q4_stream_t;     /* a cudaStream_t */
 

@@ -536,3 +536,28 @@ def test_decode_chains_see_the_product_before(g, M):
         for a, b in zip(chain(False), want):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("g,M", [(128, 1), (128, 7), (128, 16), (64, 1), (32, 3), (-1, 2)])
+def test_sequential_decode_behind_the_kernels_that_write_the_layer(g, M):
+    """A sequential decode product told that the layer has just been written (GEMV_WRITTEN): the same bits as later."""
+    K, N = 4096, 1024
+    for seed in range(4):
+        src = synth.make_layer(K, N, g, act_order=False, seed=seed).to(DEV)
+        x = torch.randn(M, K, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV).half()
+        scales32 = src.scales.float()
+        qweight, qzeros = torch.zeros_like(src.qweight), torch.zeros_like(src.qzeros)
+        cold, warm = (torch.empty(M, N, dtype=torch.float32, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        torch.full(scales32.shape, float("nan"), dtype=torch.float16, device=DEV)
+        qweight.copy_(src.qweight)
+        qzeros.copy_(src.qzeros)
+        scales = scales32.half()
+        quant_cuda.gemv(x, qweight, cold, scales, qzeros, None, K // src.scales.shape[0], _lib.GEMV_WRITTEN)
+        torch.cuda.synchronize()
+        quant_cuda.gemv(x, qweight, warm, scales, qzeros, None, K // src.scales.shape[0], 0)
+        torch.cuda.synchronize()
+        assert torch.equal(cold.view(torch.int32), warm.view(torch.int32))
+        want = orc.matmul4bit_ref(x.cpu(), src.qweight.cpu(), src.scales.cpu(), src.qzeros.cpu(), src.g_idx.cpu())
+        assert rel_fro(warm, want) <= REL_TOL
+    assert quant_cuda.device_status() == 0

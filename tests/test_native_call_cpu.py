@@ -245,3 +245,24 @@ def test_zero_term_table_follows_the_scales_object(native, monkeypatch):
     a = quant_cuda._zero_terms(first, zeros, G, N, 0)
     assert quant_cuda._zero_terms(first, zeros, G, N, 0) is a and len(made) == 1
     assert quant_cuda._zero_terms(second, zeros, G, N, 0) is not a and len(made) == 2
+
+
+def test_decode_products_behind_a_cast_say_so(monkeypatch):
+    """Scales (or first-format zeros) cast or copied for the call were written by the kernel just ahead: the product is
+    told, so that it starts behind it."""
+    flags = []
+    monkeypatch.setattr(quant_cuda, "gemv", lambda x, qw, y, sc, zr, gi, gs, fl, bias=None: flags.append(bool(fl & _lib.GEMV_WRITTEN)) or y.zero_())
+    layer = synth.make_layer(256, 64, 64, False, 1)
+    x, y = synth.make_acts(3, 256, 5), torch.zeros(3, 64, dtype=torch.float16)
+    for scales, said in ((layer.scales, False), (layer.scales.float(), True)):
+        mm4b._matmul4bit_v2(x, layer.qweight, scales, layer.qzeros, layer.g_idx, 64)
+        quant_cuda.vecquant4matmul_faster(x, layer.qweight, y, scales, layer.qzeros, layer.g_idx)
+        quant_cuda.vecquant4matmul_old_faster(x, layer.qweight, y.float(), scales, layer.qzeros, 64)
+        assert flags == [said] * 3
+        flags.clear()
+    one = layer.scales[:1].reshape(-1, 1).contiguous()
+    for scales, zeros, said in ((one, one, False), (one.float(), one, True), (one, one.float(), True)):
+        mm4b._matmul4bit_v1(x, layer.qweight, scales, zeros)
+        quant_cuda.vecquant4matmul_v1_faster(x, layer.qweight, y, scales, zeros)
+        assert flags == [said] * 2
+        flags.clear()
