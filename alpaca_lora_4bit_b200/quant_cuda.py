@@ -325,6 +325,19 @@ def _zero_terms(scales, zeros, G, N, st):
     return table
 
 
+def _forward_table(scales, zeros, g_idx, K, N, G, st):
+    """Kept table of zero terms and the group size promised to a forward product, or ``(None, 0)``.
+
+    Sequential groups (checked once per layer): the kernel is given the kept table of zero terms and the word that
+    group = row / groupsize, so that it fetches a task's scales and zero terms ahead with its packed words instead of
+    building shared-memory tables of all groups per tile.  (With act-order every row of a task would need its own pair of
+    loads: measured slower, so the table is not offered.)"""
+    if not (cache_zero_terms and N % 256 == 0 and K % G == 0 and groups_are_sequential(g_idx, G)):
+        return None, 0
+    zt = _zero_terms(scales, zeros, G, N, st)
+    return zt, K // G if (zt is not None and promise_sequential_groups) else 0
+
+
 def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, residual=None, lora_u=None, lora_w=None):
     """The product of ``gemm`` for ``x [..., K]`` (transpose: ``[..., N]``) through one native call (``_q4torch.gemm``),
     into ``out`` or, with ``out=None``, a new tensor; ``None`` - and nothing done - for operands it does not take."""
@@ -341,11 +354,11 @@ def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, 
     if ws is None or ws.numel() < need:
         ws = _lib.gemm_workspace_for(dev, st, need)
     zt, seq_gs = None, 0
-    if cache_zero_terms and g_idx is not None and G > 0:
-        # forward: see the comment in gemm()
-        if transpose or (N % 256 == 0 and K % G == 0 and groups_are_sequential(g_idx, G)):
+    if g_idx is not None and G > 0:
+        if not transpose:
+            zt, seq_gs = _forward_table(scales, zeros, g_idx, K, N, G, st)
+        elif cache_zero_terms:
             zt = _zero_terms(scales, zeros, G, N, st)
-            seq_gs = K // G if (zt is not None and not transpose and promise_sequential_groups) else 0
     return (_lib._torch_call or _lib.torch_call()).gemm(x, qweight, out, scales, zeros, g_idx, bias, residual, lora_u, lora_w, transpose, zt, seq_gs, ws)
 
 
@@ -418,14 +431,7 @@ def gemm(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, lora
                 rc = L.q4_gemm_bwd(x.data_ptr(), qweight.data_ptr(), out.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                                    g_idx.data_ptr(), _lib.ptr(lora_u), _lib.ptr(lora_w), r, M, K, N, G, ws.data_ptr(), ws.numel(), st)
         else:
-            # Sequential groups (checked once per layer): the kernel is given the kept table of zero terms and the word
-            # that group = row / groupsize, so that it fetches a task's scales and zero terms ahead with its packed
-            # words instead of building shared-memory tables of all groups per tile.  (With act-order every row of a
-            # task would need its own pair of loads: measured slower, so the table is not offered.)
-            zt, seq_gs = None, 0
-            if cache_zero_terms and N % 256 == 0 and K % G == 0 and groups_are_sequential(g_idx, G):
-                zt = _zero_terms(scales, zeros, G, N, st)
-                seq_gs = K // G if (zt is not None and promise_sequential_groups) else 0
+            zt, seq_gs = _forward_table(scales, zeros, g_idx, K, N, G, st)
             if zt is not None or residual is not None:
                 rc = L.q4_gemm_fwd_residual(x.data_ptr(), qweight.data_ptr(), out.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                                             _lib.ptr(zt), g_idx.data_ptr(), _lib.ptr(bias), _lib.ptr(residual), _lib.ptr(lora_u),
@@ -456,10 +462,7 @@ def gemm_swiglu(x, qweight, out, scales, zeros, g_idx, bias=None) -> None:
         if need is None:
             need = _gemm_ws_bytes[(K, N, G)] = int(L.q4_gemm_workspace_bytes(K, N, G))
         ws = _lib.gemm_workspace_for(dev, st, need)
-        zt, seq_gs = None, 0                    # sequential groups: kept zero-term table and the promise, as in gemm()
-        if cache_zero_terms and K % G == 0 and groups_are_sequential(g_idx, G):
-            zt = _zero_terms(scales, zeros, G, N, st)
-            seq_gs = K // G if (zt is not None and promise_sequential_groups) else 0
+        zt, seq_gs = _forward_table(scales, zeros, g_idx, K, N, G, st)
         rc = L.q4_gemm_fwd_swiglu(x.data_ptr(), qweight.data_ptr(), out.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                                   _lib.ptr(zt), g_idx.data_ptr(), _lib.ptr(bias), M, K, N, G, seq_gs, ws.data_ptr(), ws.numel(), st)
     _lib.check(rc, "gemm_swiglu")
