@@ -121,23 +121,3 @@ def test_skip_path_is_added_as_torch_adds_it(fmt, rows):
             mod.offer_residual(torch.autograd.forward_ad.make_dual(full, full))
             assert torch.equal(torch.autograd.forward_ad.unpack_dual(mod(x)).tangent, full)
     assert quant_cuda.device_status() == 0
-
-
-@pytest.mark.parametrize("fmt,rows", [("seq", 1), ("act", 12), ("seq", 40), ("v1", 3), ("v1", 40)])
-def test_no_grad_forward_is_no_opaque_call_where_torch_watches(fmt, rows):
-    """A tracer, which sees the sizes as tensors, is refused by the library call it comes to; it gets no trace that replays
-    uninitialised memory.  A tensor subclass goes the general way."""
-    mod, w, bias = build(fmt, 128 if fmt != "v1" else K)
-    x = torch.randn(rows, K, generator=torch.Generator().manual_seed(1)).half().to(DEV)
-    mm4b.act_order = fmt == "act"
-    try:
-        with torch.no_grad():
-            with pytest.raises(Exception):
-                torch.jit.trace(mod, (x,), check_trace=False)
-            y, yp = mod(x), mod(torch.nn.Parameter(x))
-    finally:
-        mm4b.act_order = False
-    want = x.float().cpu() @ w + bias
-    for got in (y, yp):
-        assert float((got.float().cpu() - want).norm() / want.norm()) <= 2e-3
-    assert quant_cuda.device_status() == 0
