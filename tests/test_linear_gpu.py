@@ -121,3 +121,29 @@ def test_skip_path_is_added_as_torch_adds_it(fmt, rows):
             mod.offer_residual(torch.autograd.forward_ad.make_dual(full, full))
             assert torch.equal(torch.autograd.forward_ad.unpack_dual(mod(x)).tangent, full)
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+def test_first_format_on_the_pair_kernel(variant):
+    """Above 1024 rows, and wherever the pair kernel is asked for, a first-format layer runs on it with neither packed zero
+    points nor g_idx: same product, scales of either sign and above 2 among them."""
+    rows, K2, N2 = 1100, 1280, 768
+    gen = torch.Generator().manual_seed(variant)
+    qweight = torch.randint(-2 ** 31, 2 ** 31 - 1, (K2 // 8, N2), generator=gen).to(torch.int32).to(DEV)
+    scales = (torch.rand(N2, 1, generator=gen) * 0.018 + 0.002).half()
+    scales[::7] = -3.25 * scales[::7]
+    scales[3::31] = 2.5
+    zeros = (scales.float() * torch.randint(1, 16, (N2, 1), generator=gen)).half().to(DEV)
+    scales, bias = scales.to(DEV), torch.randn(N2, generator=gen).half().to(DEV)
+    x, res = torch.randn(rows, K2, generator=gen).half().to(DEV), torch.randn(rows, N2, generator=gen).half().to(DEV)
+    w = torch.empty((K2, N2), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v1(qweight, w, scales.reshape(-1), zeros.reshape(-1))
+    want = x.double() @ w.double() + bias.double() + res.double()
+    quant_cuda.gemm_set_variant(variant)
+    try:
+        with torch.no_grad():
+            y = quant_cuda.gemm_v1_new(x, qweight, scales, zeros, bias, res)
+    finally:
+        quant_cuda.gemm_set_variant(0)
+    assert float((y.double() - want).norm() / want.norm()) <= 1e-3          # fp32 sums rounded to fp16 twice: 2 * 2^-11
+    assert quant_cuda.device_status() == 0
