@@ -530,23 +530,27 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       // least two pairs per tile every tile is cut between a whole number `n` of them.  In stages of the contraction (a
       // quarter of a microsecond), nb = blocks of 32 rows a tile really has: T / n for the pair's own run, about 9 + 1.2 nb
       // for writing and announcing the sums and 0.5 + 0.45 nb for every further contributor's sums that are added.  (8192 x
-      // 1024 at 256 rows, n = 2, 4, 6, 8, 16: 33.4, 26.4, 25.4, 25.8, 32.0 us, uncut 46.4; 4096 x 4096 at 32 / 256 rows:
-      // uncut 25.8 / 27.8, n = 4 16.7 / 22.8; 2048 x 2048 at 192 rows is better left uncut: 16.9, n = 2 18.3.  Contractions of
-      // up to 2048 are cut for one block of rows only: 77 rows would gain a microsecond (16.0 / 14.9), and whole tiles add
-      // up in the pair kernel's order.  All of these before the launch became programmatic, which takes another two to
-      // three microseconds off every one of them.)
+      // 1024 at 256 rows, uncut and n = 2, 4, 6, 8, 16: 45.2, 31.1, 24.2, 23.1, 23.5, 29.6 us; 4096 x 4096 at 32 / 256 rows:
+      // uncut 23.8 / 25.9, n = 4 15.0 / 20.7.  With the launch programmatic the stages are a third of a microsecond and the
+      // exchange weighs half as much again; the n of the estimate is still within 2 % of the best one, 4 % at 2048.)
+      // Contractions of up to 2048 are cut in three or more (uncut / cut): one block of rows from 1536 on (32 rows: 2048 x
+      // 2048 14.0 / 12.1 us, 1536 x 1536 11.5 / 11.2, 1280 x 1024 10.3 / 10.5), two at 2048 (64 rows: 2048 x 2048 14.1 / 12.2,
+      // 2048 x 4096 14.3 / 13.0; in two, 2048 x 8192, 14.5 / 14.9; 1536 x 1536 11.6 / 11.5).  More rows stay whole: up to 128 a
+      // cut would gain another microsecond (14.2 / 13.0 at 77; it loses from 192 on), but whole tiles add up in the pair
+      // kernel's order, so that up to 2048 the two kernels give the same bits - a test holds them to that.
       const int nb = ((M < 256 ? M : 256) + 31) / 32;
       const bool cut_ok = !stream3 && ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 16;
       if (cut_ok && tiles3 * 2 <= P) {
         double best = T;
-        for (int n = 2; n <= P / tiles3 && n <= T / 4; ++n) {
+        const int n_max = T > 32 || (nb <= 2 && T >= 16 + 8 * nb) ? T / 4 : 1;
+        for (int n = T > 32 ? 2 : 3; n <= P / tiles3 && n <= n_max; ++n) {
           const double cost = (double)((T + n - 1) / n) + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
-          if (T <= 32 && T * (n - 1) / n <= 12 + 7 * nb) continue;
           if (cost < best) { best = cost; stream3 = true; pairs3 = tiles3 * n; }
         }
       } else if (cut_ok && tiles3 < P && total3 * P < (1ll << 32)) {
         // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
-        // exchange (4096 x 11008, 43 tiles, uncut / dealt: 26.5 / 23.8 us at 32 rows, 28.1 / 26.8 at 128, 28.7 / 29.1 at 192).
+        // exchange (4096 x 11008, 43 tiles, uncut / dealt: 25.4 / 22.2 us at 32 rows, 26.5 / 24.4 at 128, 27.3 / 26.6 at 192;
+        // 5120 x 13824, 54 tiles: 30.1 / 28.6 at 32, 31.6 / 31.3 at 128).
         const double dealt = (double)total3 / P + 14 + 3 * nb;
         if (dealt < T) { stream3 = true; pairs3 = P; }
       }

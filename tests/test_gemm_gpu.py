@@ -683,3 +683,9 @@ def test_gemm_refuses_operands_of_another_shape():
     quant_cuda.gemm(x, L.qweight, y, L.scales, L.qzeros, L.g_idx, residual=torch.ones(M, N, **half), lora_u=u, lora_w=b)
     assert bool((y == 1.0).all())
     assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,M", [(2048, 2048, 20), (2048, 2048, 40), (2048, 1024, 64), (2048, 4096, 50), (1536, 1536, 32), (1536, 512, 17)])
+def test_short_prompts_cut_at_short_contractions(K, N, M):
+    """Contractions from 1536 to 2048 and at most 64 rows, whose tiles are cut too."""
+    test_short_prompts_cut_between_pairs(K, N, M)
