@@ -1756,19 +1756,44 @@ gemv_act_kernel(const GemvParams p, int G, int copies, int staged) {
   uint4 xv[ACT_AHEAD][MT];
 #pragma unroll
   for (int i = 0; i < ACT_AHEAD; ++i) load_x(sb + warp + i * GEMV_WARPS, xv[i]);
-  for (int i = threadIdx.x; i < G * 8; i += GEMV_THREADS) {
-    const int grp = i >> 3, quad = i & 7;
-    const uint2 s4 = *reinterpret_cast<const uint2*>(p.scales + (size_t)grp * N + c0 + 4 * quad);
-    const uint32_t zw = p.qzeros[(size_t)grp * (N >> 3) + ((c0 + 4 * quad) >> 3)] >> (16 * (quad & 1));
-    // 1024 + z + 1: the mantissa of 0x6400 plus one
-    const uint32_t z01 = ((zw & 0xFu) | ((zw & 0xF0u) << 12)) + 0x64016401u, z23 = (((zw >> 8) & 0xFu) | ((zw & 0xF000u) << 4)) + 0x64016401u;
-    const uint4 e = make_uint4(s4.x, s4.y, z01, z23);
-    unsigned char* at = tab + (size_t)grp * pitch + (quad >> 1) * copies * 32 + (quad & 1) * 16;
-    // (copies in turn from quad >> 1 on: the stores of a quarter-warp fall on different banks)
-    for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + ((c + (quad >> 1)) & (copies - 1)) * 32) = e;
+  // (several loads of a thread in flight at once: nothing else covers their trips to L2)
+  for (int i0 = threadIdx.x; i0 < G * 8; i0 += 2 * GEMV_THREADS) {
+    uint2 s4[2];
+    uint32_t zw[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = i0 + j * GEMV_THREADS, grp = i >> 3, quad = i & 7;
+      if (i < G * 8) {
+        s4[j] = *reinterpret_cast<const uint2*>(p.scales + (size_t)grp * N + c0 + 4 * quad);
+        zw[j] = p.qzeros[(size_t)grp * (N >> 3) + ((c0 + 4 * quad) >> 3)] >> (16 * (quad & 1));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = i0 + j * GEMV_THREADS, grp = i >> 3, quad = i & 7;
+      if (i >= G * 8) break;
+      // 1024 + z + 1: the mantissa of 0x6400 plus one
+      const uint32_t z = zw[j], z01 = ((z & 0xFu) | ((z & 0xF0u) << 12)) + 0x64016401u, z23 = (((z >> 8) & 0xFu) | ((z & 0xF000u) << 4)) + 0x64016401u;
+      const uint4 e = make_uint4(s4[j].x, s4[j].y, z01, z23);
+      unsigned char* at = tab + (size_t)grp * pitch + (quad >> 1) * copies * 32 + (quad & 1) * 16;
+      // (copies in turn from quad >> 1 on: the stores of a quarter-warp fall on different banks)
+      for (int c = 0; c < copies; ++c) *reinterpret_cast<uint4*>(at + ((c + (quad >> 1)) & (copies - 1)) * 32) = e;
+    }
   }
-  if (staged)
-    for (int i = threadIdx.x; i < (se - sb) * 32; i += GEMV_THREADS) offs[i] = offset_of(p.g_idx[sb * 32 + i]);
+  if (staged) {
+    const int4* gi = reinterpret_cast<const int4*>(p.g_idx + sb * 32);
+    const int n4 = (se - sb) * 8;
+    for (int i0 = threadIdx.x; i0 < n4; i0 += 4 * GEMV_THREADS) {
+      int4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * GEMV_THREADS < n4) v[j] = gi[i0 + j * GEMV_THREADS];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * GEMV_THREADS < n4)
+          reinterpret_cast<int4*>(offs)[i0 + j * GEMV_THREADS] = make_int4(offset_of(v[j].x), offset_of(v[j].y), offset_of(v[j].z), offset_of(v[j].w));
+    }
+  }
 
   float yacc[MT][2][4];
 #pragma unroll
