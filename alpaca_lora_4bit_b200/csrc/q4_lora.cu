@@ -38,8 +38,9 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local, uint32_t rank)
 // A lane takes 16 contiguous bytes of its row of X and of its row of W per block: which four of the MMA's
 // sixteen k-slots those eight elements occupy is the same for both operands, so the order of the sum is the
 // only thing the re-mapping changes.  Rows 8..15 of the MMA tile stay zero, or (RT = 2) hold eight more rows of X: a
-// CTA fills an SM, so from one CTA per SM on sixteen rows each take one round instead of two and read W half as often
-// (2048 rows, r = 16, on average over the projections of a 13B block: 14.0 -> 12.5 us).
+// CTA fills an SM, and sixteen rows each can take fewer rounds of CTAs and read W half as often (2048 rows of 5120, eight /
+// sixteen rows a CTA: 8.3 / 8.0 us at r = 8, 11.0 / 9.8 at 16, 19.2 / 15.6 at 32, 35.1 / 20.1 at 64; where they take as
+// many rounds for twice the work they lose: 3000 rows of 5120 at r = 16 16.2 / 18.0).  The rule: q4_lora_project.
 constexpr int LP_WARPS = 8, LP_THREADS = LP_WARPS * 32;
 // chunk length and ring depth per output width: as much of the contraction in flight at once as shared memory holds
 // (a CTA's time is the number of round trips to L2 it has to wait for, one after the other)
@@ -296,7 +297,13 @@ extern "C" int q4_lora_project(const void* x, const void* w, void* out, int M, i
   const cudaStream_t st = (cudaStream_t)stream;
   const __half *xh = (const __half*)x, *wh = (const __half*)w;
   __half* oh = (__half*)out;
-  const bool tall = (M + 7) / 8 > sm_count();    // eight rows each would take more than one round of CTAs
+  // Eight or sixteen rows of x per CTA: whichever takes less time in rounds of CTAs.  A CTA of sixteen rows takes `ratio`
+  // hundredths of the time of one of eight (1185 to 4096 rows, contractions of 4096 to 13824): what is copied grows by 8 of
+  // 8 + r rows, and the ring holds less of the contraction - which with r <= 8 costs more than it saves from 6656 on (8192:
+  // 10.3 / 11.4 us, 13824: 16.3 / 18.2 at 1185 rows; 5120: 8.1 / 7.9).
+  const int sms = sm_count(), rounds8 = ((M + 7) / 8 + sms - 1) / sms, rounds16 = ((M + 15) / 16 + sms - 1) / sms;
+  const int ratio = r <= 8 ? (C <= 5120 ? 190 : 205) : r <= 16 ? 190 : r <= 32 ? 164 : 113;
+  const bool tall = (long long)rounds16 * ratio < (long long)rounds8 * 100;
 #define Q4_LP(NT) return tall ? launch_lora_project<NT, 2>(xh, wh, oh, M, C, r, scale, st) : launch_lora_project<NT, 1>(xh, wh, oh, M, C, r, scale, st)
   switch ((r + 7) / 8) {
     case 1: Q4_LP(1);

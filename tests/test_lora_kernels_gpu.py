@@ -83,3 +83,14 @@ def test_cast16_rounds_as_torch_does(n):
         nan = torch.isnan(want)
         assert torch.equal(torch.isnan(out[:n]), nan) and torch.equal(out[:n][~nan].view(torch.int16), want[~nan].view(torch.int16))
         assert bool((out[n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,C,r", [(1300, 2048, 5), (2048, 5120, 16), (2048, 1056, 24), (1201, 4096, 64), (2368, 8192, 8), (3000, 4096, 16)])
+def test_project_gives_a_row_the_same_bits_in_either_form(M, C, r):
+    """Eight or sixteen rows per CTA, as the rounds of CTAs have it: a row's sums are added in the same order, so that it
+    does not matter among how many others it is projected."""
+    g = torch.Generator(device=DEV).manual_seed(M + C)
+    x = torch.randn(M, C, generator=g, device=DEV).half()
+    w = (torch.randn(r, C, generator=g, device=DEV) * 0.05).half()
+    whole, parts = project(x, w, 1.5), torch.cat([project(x[i:i + 1000], w, 1.5) for i in range(0, M, 1000)])
+    assert torch.equal(whole.view(torch.int16), parts.view(torch.int16))
