@@ -157,11 +157,13 @@ def torch_call():
     return _torch_call
 
 
+_transforms, _tracing, _forward_ad = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state, torch.autograd.forward_ad
+
+
 def nobody_watches() -> bool:
     """No function transform (vmap, grad), forward-mode level or tracer is active that would have to see the operations of
     this call."""
-    return (torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0
-            and torch._C._get_tracing_state() is None)
+    return _transforms() is None and _forward_ad._current_level < 0 and _tracing() is None
 
 
 def opaque_call_ok(x) -> bool:

@@ -165,16 +165,16 @@ class Autograd4bitQuantLinear(nn.Module):
         if self.bits == 4 and not torch.is_grad_enabled() and matmul4bit_with_backend is _own_matmul4bit_with_backend:
             if backend != 'cuda':
                 raise ValueError('Backend not supported.')
-            b, v1, bias = self._buffers, self.is_v1_model, None
+            b, v1 = self._buffers, self.is_v1_model
             try:                                               # (a buffer looked up as an attribute costs the host a microsecond a call)
-                packed = b['qweight'], b['scales'], b['zeros' if v1 else 'qzeros'], None if v1 else b['g_idx']
-                if not self.disable_bias:
-                    bias = b['bias']
+                qweight, scales = b['qweight'], b['scales']
+                zeros, g_idx = (b['zeros'], None) if v1 else (b['qzeros'], b['g_idx'])
+                bias = None if self.disable_bias else b['bias']
             except KeyError:                                   # a parameter, a plain attribute, a parametrization
-                packed = self.qweight, self.scales, self.zeros if v1 else self.qzeros, None if v1 else self.g_idx
-                if not self.disable_bias:
-                    bias = self.bias
-            return mm4b.linear(x, *packed, self.groupsize, bias, residual)
+                qweight, scales = self.qweight, self.scales
+                zeros, g_idx = (self.zeros, None) if v1 else (self.qzeros, self.g_idx)
+                bias = None if self.disable_bias else self.bias
+            return mm4b.linear(x, qweight, scales, zeros, g_idx, self.groupsize, bias, residual)
         zeros = self.zeros if self.is_v1_model else self.qzeros
         if self.bits == 4 and not torch.is_grad_enabled():     # the program's own product
             out = matmul4bit_with_backend(x, self.qweight, self.scales, zeros, self.g_idx, self.bits, self.maxq, self.groupsize)

@@ -195,8 +195,8 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   // The pair's last item: nothing follows it, so the dequant warps (three per TMEM lane quarter) share its epilogue
   // with the epilogue warp of their quarter, blocks of 32 rows dealt round robin - the output of a whole tile, and the
   // writing or the adding up of the partial sums of a shared one.  (On short prompts, where every item is a piece of a
-  // tile, one warp per quarter did the exchange block by block, a trip to L2 each: 128 rows of 4096 x 4096 23.2 us, now
-  // 18.9, of 11008 x 4096 32.5, now 28.2.)
+  // tile, one warp per quarter did the exchange block by block, a trip to L2 each: 128 rows of 4096 x 4096 took 23.2 us
+  // and 18.9 shared, of 11008 x 4096 32.5 and 28.2; since the launch is programmatic 16.9 and 25.6.)
   const WorkItem w_last = work_item<SPLIT>(p, wr, n_items > 0 ? n_items - 1 : 0, n_pairs, T);
   const bool share_last = n_items > 0;
 

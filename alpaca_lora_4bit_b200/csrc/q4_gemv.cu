@@ -1691,7 +1691,7 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 // Every element is dequantised as s*(q - (z+1)) in fp16 pairs before the MMA, with scale and zero point of its own
 // row's group from a shared-memory table of the CTA's 32 columns.  What bounds it: with a 4-byte entry looked up
 // per weight, unpacked pair by pair, the launch waited for shared memory and for the integer pipe (27.7 us on
-// average over the seven projections of a 13B block, where HBM needs 3.5; now 19.6, the table's 4 bytes per weight
+// average over the seven projections of a 13B block, where HBM needs 3.5; now 19.5, the table's 4 bytes per weight
 // through the shared-memory pipe the largest part).  Here
 //   * a table entry is the four scales and the four 1024 + z + 1 of a quad of columns, 16 bytes: one LDS.128 serves
 //     the four weights a lane has of a row, and a subtraction from the raw 1024 + q leaves q - (z+1) exactly;
