@@ -10,7 +10,7 @@ import ctypes
 import os
 import threading
 import warnings
-from ctypes import c_char_p, c_int, c_size_t, c_uint, c_void_p
+from ctypes import c_char_p, c_int, c_size_t, c_uint, c_ulonglong, c_void_p
 
 import torch
 
@@ -46,6 +46,7 @@ _SIGNATURES = {
                             c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "q4_gemm_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                             c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "q4_capture_id": (c_int, [c_void_p, ctypes.POINTER(c_ulonglong)]),
     "q4_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "q4_zero_term_table": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "q4_gemm_fwd_residual": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -247,17 +248,39 @@ def workspace_for(device: torch.device, stream_handle: int) -> torch.Tensor:
 
 
 _gemm_workspaces: dict = {}
+_GEMM_WS_HEAD = 65536                      # arrival counters: zero before the first call, left zero by every kernel
+_capture_workspaces: dict = {}             # (device index, stream handle) -> (id of the capture, its workspaces, the newest last)
 
 
 def gemm_workspace_for(device: torch.device, stream_handle: int, nbytes: int) -> torch.Tensor:
     """Scratch of the fused GEMM for one (device, stream): zeroed when (re)allocated, only ever grows.
-    The kernels leave its counter head zero, so calls ordered on the stream can share it."""
+    The kernels leave its counter head zero, so calls ordered on the stream can share it.
+
+    A stream capture has workspaces of its own, from the memory of its graph and cleared by it: the graph holds their
+    addresses for as long as it lives, when the stream's own one may long have made way for a larger one."""
     key = (device.index, stream_handle)
+    if torch.cuda.is_current_stream_capturing():
+        capture = capture_id(stream_handle)
+        held = _capture_workspaces.get(key)
+        if held is None or held[0] != capture:
+            held = _capture_workspaces[key] = (capture, [])
+        if not held[1] or held[1][-1].numel() < nbytes:
+            ws = torch.empty(max(nbytes, 24 << 20), dtype=torch.uint8, device=device)
+            ws[:_GEMM_WS_HEAD].zero_()
+            held[1].append(ws)             # (the earlier ones stay until the capture is over: nothing else of it takes their place)
+        return held[1][-1]
     ws = _gemm_workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 24 << 20), dtype=torch.uint8, device=device)
         _gemm_workspaces[key] = ws
     return ws
+
+
+def capture_id(stream_handle: int) -> int:
+    """The number of the capture that ``stream_handle`` is part of (no two captures of a process share one)."""
+    out = ctypes.c_ulonglong(0)
+    check(lib().q4_capture_id(stream_handle, ctypes.byref(out)), "capture_id")
+    return out.value
 
 
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:

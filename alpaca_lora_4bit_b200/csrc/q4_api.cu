@@ -110,3 +110,14 @@ int sm_count() {
 }
 
 }  // namespace q4
+
+extern "C" int q4_capture_id(q4_stream_t stream, unsigned long long* out) {
+  using namespace q4;
+  if (!out) return fail(Q4_E_BADARG, "capture_id: null pointer");
+  cudaStreamCaptureStatus status;
+  unsigned long long id = 0;
+  if (int e = check_cuda(cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id), "capture_id")) return e;
+  *out = status == cudaStreamCaptureStatusActive ? id : 0;
+  return Q4_OK;
+}
+

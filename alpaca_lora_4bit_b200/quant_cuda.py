@@ -351,7 +351,7 @@ def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, 
     if need is None:
         need = _gemm_ws_bytes[(K, N, G)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, G))
     ws = _lib._gemm_workspaces.get((idx, st))
-    if ws is None or ws.numel() < need:
+    if ws is None or ws.numel() < need or torch.cuda.is_current_stream_capturing():
         ws = _lib.gemm_workspace_for(dev, st, need)
     zt, seq_gs = None, 0
     if g_idx is not None and G > 0:
@@ -376,7 +376,7 @@ def gemm_v1_new(x, qweight, scales, zeros, bias=None, residual=None):
     if need is None:
         need = _gemm_ws_bytes[(K, N, 1)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, 1))
     ws = _lib._gemm_workspaces.get((dev.index, st))
-    if ws is None or ws.numel() < need:
+    if ws is None or ws.numel() < need or torch.cuda.is_current_stream_capturing():
         ws = _lib.gemm_workspace_for(dev, st, need)
     return (_lib._torch_call or _lib.torch_call()).gemm_v1(x, qweight, scales, zeros, bias, residual, ws)
 

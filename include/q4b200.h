@@ -221,6 +221,10 @@ int q4_gemm_fwd_v1(const void* x, const int32_t* qweight, void* y, const void* s
  *   - in the backward reads rn(s*(z+1)) from a [G, N] table a small kernel fills first.
  * One workspace serves calls that are ordered on one stream; calls that may overlap need one each. */
 size_t q4_gemm_workspace_bytes(int K, int N, int G);
+/* The number of the capture that `stream` is part of (no two captures of a process share one), 0 outside a capture: a
+ * host that gives every captured graph a workspace of its own - the graph holds the address for as long as it lives -
+ * tells captures apart by it. */
+int q4_capture_id(q4_stream_t stream, unsigned long long* out);
 
 /* The element-wise work of a decoder layer around the quantised linears, one kernel each way (fp16 in and
  * out, fp32 inside).  The reference leaves these to the stock modules (a handful of framework kernels each:
