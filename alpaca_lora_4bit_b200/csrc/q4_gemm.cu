@@ -27,6 +27,8 @@
 // columns, built once) or, in the backward, from global memory per row with reuse while the group
 // stays the same.  Act-order is free in this scheme: the group of every row is read from g_idx.
 // Every mbarrier wait is bounded: on expiry the kernel records a status word and stops waiting.
+#include <atomic>
+
 #include "q4_umma.cuh"
 
 namespace q4 {
@@ -71,6 +73,8 @@ struct GemmParams {
   float* ws_partials;
   unsigned* ws_counters;
   const __half* zp_table;   // rn(s * (z+1)) for every [group, column], or null
+  int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32
+  int cluster_pairs;        // weights-in-TMEM kernel: pairs of a cluster; more than one: they share a tile
   int seq_shift;            // > 0: the caller promises g_idx[k] == k >> seq_shift (sequential groups of 2^seq_shift rows)
 };
 
@@ -440,7 +444,11 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
   p.lora_r = lora_r;
   p.ws_partials = nullptr; p.ws_counters = nullptr; p.zp_table = nullptr;
   p.seq_shift = (!transpose && no_tables) ? seq_shift : 0;
-  const int box_rows = use_pair ? 128 * mh : GM_TILE_M;    // activation rows one TMA copy brings
+  // The weights-in-TMEM kernel's rows are the N side of its MMAs: as many tiles as of 256 rows, of the same height
+  const int tiles_m = (M + 255) / 256;
+  p.cluster_pairs = 1;
+  p.tile_rows = use_tm ? ((M + tiles_m - 1) / tiles_m + 31) / 32 * 32 : 256;
+  const int box_rows = use_tm ? p.tile_rows / 2 : use_pair ? 128 * mh : GM_TILE_M;    // activation rows one TMA copy brings
   CUtensorMap amap;
   if (int e = make_tmap_2d(&amap, act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)contract, (uint64_t)M,
                            (uint64_t)contract * 2, GM_TILE_C, box_rows, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -538,14 +546,20 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       // 2048 x 4096 14.3 / 13.0; in two, 2048 x 8192, 14.5 / 14.9; 1536 x 1536 11.6 / 11.5).  More rows stay whole: up to 128 a
       // cut would gain another microsecond (14.2 / 13.0 at 77; it loses from 192 on), but whole tiles add up in the pair
       // kernel's order, so that up to 2048 the two kernels give the same bits - a test holds them to that.
-      const int nb = ((M < 256 ? M : 256) + 31) / 32;
+      const int nb = p.tile_rows / 32;
       const bool cut_ok = !stream3 && ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 16;
       if (cut_ok && tiles3 * 2 <= P) {
+        // The pairs of a tile in one cluster (n = 2..4) hand their sums over through shared memory instead of the workspace:
+        // 2 + (n - 1)(1.5 + 0.3 nb) stages instead of 9 + 1.2 nb and more (77 rows, workspace / cluster: 5120 x 5120, n = 3,
+        // 18.6 / 15.8 us; 13824 x 5120 32.5 / 30.0; 4096 x 1024 13.9, n = 8, / 10.6, n = 4).  Of clusters of four pairs only
+        // 15 fit the GPU at once - the sixteen tiles of a 4096-wide layer take n = 3 (13.5 us; n = 4 by the workspace 15.7).
         double best = T;
         const int n_max = T > 32 || (nb <= 2 && T >= 16 + 8 * nb) ? T / 4 : 1;
         for (int n = T > 32 ? 2 : 3; n <= P / tiles3 && n <= n_max; ++n) {
-          const double cost = (double)((T + n - 1) / n) + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
-          if (cost < best) { best = cost; stream3 = true; pairs3 = tiles3 * n; }
+          const bool cluster = n <= G3_MAX_CLUSTER && gemm3_clusters(dev, n) >= tiles3;
+          const double run = (double)((T + n - 1) / n);
+          const double cost = cluster ? run + 2 + (n - 1) * (1.5 + 0.3 * nb) : run + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
+          if (cost < best) { best = cost; stream3 = true; pairs3 = tiles3 * n; p.cluster_pairs = cluster ? n : 1; }
         }
       } else if (cut_ok && tiles3 < P && total3 * P < (1ll << 32)) {
         // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
@@ -558,10 +572,12 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       p.ws_counters = (unsigned*)ws;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(2 * pairs3); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = gemm3_smem_bytes(); cfg.stream = st;
-      cudaLaunchAttribute at[1];
+      cudaLaunchAttribute at[2];
       at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       at[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = at; cfg.numAttrs = 1;
+      at[1].id = cudaLaunchAttributeClusterDimension;
+      at[1].val.clusterDim.x = 2 * p.cluster_pairs; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+      cfg.attrs = at; cfg.numAttrs = 2;
       if (int e = check_cuda(stream3 ? cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<true>, amap, umap, p)
                                      : cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<false>, amap, umap, p), "gemm launch")) return e;
       return check_cuda(cudaGetLastError(), "gemm launch");

@@ -6,8 +6,9 @@
 // contraction elements an SM takes 16 KiB of dequant stores on top of 16 KiB of TMA writes and 32 KiB of tensor-core
 // reads.  Here the product is transposed,
 // y^T = W^T x^T: the weights are the A operand (M side: 256 output columns per pair, 128 per CTA = one TMEM lane
-// each), the activations the B operand (N side: 256 rows of x per tile, 128 per CTA, K-major by TMA exactly as
-// before).  A dequant thread owns one output column: the eight packed words of its column and a stage are eight
+// each), the activations the B operand (N side: a tile of up to 256 rows of x, half per CTA, K-major by TMA exactly as
+// before; all tiles of a product have the same height, a multiple of 32, so that 333 rows are two tiles of 192 and 77 one
+// of 96: the MMAs of 64 contraction elements take 540 cycles at 256 rows, and 333 rows of 13824 x 5120 took 54.9 us, now 52.7).  A dequant thread owns one output column: the eight packed words of its column and a stage are eight
 // coalesced 4-byte loads, one word is eight consecutive k of that column = four half2 in contraction order, scale
 // and zero term are scalars of the thread, and the stage's 64 halves leave as one `tcgen05.st` of 32 columns.
 // Nothing of W touches shared memory; an SM moves 16 KiB of TMA writes and 16 KiB of operand reads per stage.
@@ -23,6 +24,9 @@
 // first moves its 32 columns x 256 rows into shared memory as fp16 (and hands the accumulator back: the MMAs of the
 // pair's next item start while the stores run), then stores rows of 64 bytes, four lanes each.
 // Every wait is bounded as in the pair kernel.
+// Where the pairs that share a tile form a cluster (p.cluster_pairs, few tiles), each adds up a part of the tile's rows from
+// the others' shared memory: through the workspace the exchange took 5-7 us (write, fence, count, wait, and the
+// contributors' sums one after the other from L2), in the cluster 1-2.
 // Launched with the programmatic-dependent-launch attribute: the set-up runs before the wait for the earlier kernel, and
 // every warp waits before its first read or write of global memory.  That holds for the layer's own tensors too: the
 // kernel just ahead may be the one that fills the zero-term table of a layer's first call, or casts its scales or bias.
@@ -36,6 +40,7 @@ static_assert(G3_STAGES == 8, "a stage use u lies in slot u & 7, use u >> 3");
 constexpr int G3_X_BYTES = 128 * GM_TILE_C * 2;           // 16 KiB: this CTA's 128 activation rows of a stage
 constexpr int G3_TMEM_A0 = 256;               // first TMEM column of the operand stages
 constexpr int G3_BAR_BYTES = 512;
+constexpr int G3_MAX_CLUSTER = 4;             // pairs: eight CTAs, the portable size
 constexpr int G3_GROUPS = 3;                  // dequant groups of four warps
 constexpr int G3_THREADS = 32 * (4 + 4 * G3_GROUPS + 4);
 constexpr int G3_TURN_BYTES = 4 * 256 * 64;    // per epilogue warp its 32 columns of all 256 rows of a tile, fp16
@@ -57,6 +62,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         "r"(v[30]), "r"(v[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  return v;
+}
 
 // Loads that the compiler may neither move nor take for loads of memory that nobody writes while the kernel lives (an
 // earlier kernel of the stream may still be writing it when this one is launched).
@@ -88,8 +99,9 @@ __device__ __forceinline__ void deq_word_k(uint32_t w, uint32_t s2, uint32_t c2,
 
 // SPLIT as in the pair kernel: whole tiles per pair, or equal runs of the sequence of all tiles x stages with the
 // partial sums of a shared tile meeting in the workspace (added in pair order by the pair whose run starts the tile).
+// The launch gives the cluster's size: one pair or, with p.cluster_pairs = n > 1 (SPLIT only), the n pairs that share a tile.
 template <bool SPLIT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G3_THREADS, 1)
+__global__ void __launch_bounds__(G3_THREADS, 1)
 q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap umap, const GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
   pdl_launch_dependents();
@@ -106,12 +118,13 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   unsigned char* turn = smem + S * G3_X_BYTES + G3_BAR_BYTES;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t cluster_rank = cluster_ctarank(), rank = cluster_rank & 1, even_cta = cluster_rank & ~1u;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int T = p.n_contract_tiles;
   const int lora_ks = (p.lora_r + 15) >> 4;
   const int N = p.N;
-  const int m_tiles = (p.M + 255) / 256;
+  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32
+  const int m_tiles = (p.M + TR - 1) / TR;
   const int n_tiles = m_tiles * (N / G2_TILE_N);
   const WorkRange wr = work_range<SPLIT>(pair, n_pairs, n_tiles, T);
   const int n_items = wr.n_items;
@@ -258,20 +271,70 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     block_to_smem(buf, v, bv);
   };
 
+  // The exchange inside a cluster (every pair has one item, a piece of the cluster's tile): a pair adds up the blocks of
+  // 32 rows b % n == its own number and leaves its sums of the others in its shared memory, in the place of the activation
+  // stages, which the last MMAs have read.  `w4` is the warp's number among the four of its lane quarter.
+  const int n_cl = SPLIT ? p.cluster_pairs : 1;
+  auto exchange_in_cluster = [&](int quarter, int w4) __attribute__((always_inline)) {
+    const int me = (int)(cluster_rank >> 1);
+    const int n0 = (w_last.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter, m_base = (w_last.tile % m_tiles) * TR;
+    const int nb = (min(TR, p.M - m_base) + 31) >> 5;
+    const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
+    unsigned char* sums = stages + quarter * (8 * 4096) + lane * 16;               // [quarter][block][q][lane][4 floats]
+    const uint32_t tsrc = tmem_base + ((uint32_t)(32 * quarter) << 16);
+    if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 40);
+    __syncwarp();
+    tc_fence_after();
+#pragma unroll 1
+    for (int cb = w4; cb < nb; cb += 4) {
+      if (cb % n_cl == me) continue;
+      uint32_t v[32];
+      tmem_ld32(tsrc + cb * 32, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<uint4*>(sums + cb * 4096 + q * 512) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    }
+    cluster_sync_all();
+#pragma unroll 1
+    for (int cb = me + n_cl * w4; cb < nb; cb += 4 * n_cl) {
+      uint32_t v[32];
+      tmem_ld32(tsrc + cb * 32, v);
+      tmem_ld_wait();
+#pragma unroll 1
+      for (int c = 1; c < n_cl; ++c) {
+        const int from = me + c < n_cl ? me + c : me + c - n_cl;
+        const uint32_t src = mapa_u32(smem_u32(sums + cb * 4096), 2 * from + rank);
+        float4 t[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t[q] = ld_cluster_f4(src + q * 512);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + t[q].x); v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + t[q].y);
+          v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + t[q].z); v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + t[q].w);
+        }
+      }
+      unsigned char* mine = turn + quarter * 16384 + cb * 2048;
+      block_to_smem(mine, v, bv);
+      __syncwarp();
+      block_to_global(mine, m_base + cb * 32, n0);
+    }
+  };
+
   if (warp == 0) {
     // ---------------- TMA producer: this CTA's 128 rows of x (or of lora_u) of every stage ----------------
     if (lane == 0) {
       int st = 0, use = 0;
-      const uint32_t full0 = mapa_u32(smem_u32(full), 0);
+      const uint32_t full0 = mapa_u32(smem_u32(full), even_cta);
       pdl_wait();
       for (int item = 0; item < n_items; ++item) {
         const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
-        const int m0 = (wi.tile % m_tiles) * 256 + 128 * (int)rank;
+        const int m0 = (wi.tile % m_tiles) * TR + (TR >> 1) * (int)rank;
         const int nst = wi.ke - wi.kb + (wi.lora ? 1 : 0);
         for (int j = 0; j < nst; ++j) {
           const int it = wi.kb + j;
           if (use > 0) wait_bar_idle(&empty[st], (use - 1) & 1, abort_flag, 40);
-          if (rank == 0) mbar_arrive_expect_tx(&full[st], 2 * G3_X_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(&full[st], TR * GM_TILE_C * 2);
           unsigned char* dst = stages + (size_t)st * G3_X_BYTES;
           if (it < wi.ke) tma_load_2d_pair(dst, &amap, it * GM_TILE_C, m0, full0 + 8 * st);
           else tma_load_2d_pair(dst, &umap, 0, m0, full0 + 8 * st);
@@ -286,7 +349,8 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     if (rank == 0) {
       uint32_t leader;
       asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(leader));
-      constexpr uint32_t idesc = idesc_f16(256, 256, false);
+      const uint32_t idesc = idesc_f16(256, TR, false);
+      const uint16_t both = (uint16_t)(3u << even_cta);
       // B: this CTA's 128 rows of x, K-major, 128-byte rows, 8-row groups 1024 B apart, 16 contraction elements = 32 B
       const uint64_t bd0 = smem_desc_sw128(smem_u32(stages), 16, 1024);
       constexpr uint64_t B_STEP = 32 >> 4, ST_STEP = G3_X_BYTES >> 4;
@@ -306,13 +370,13 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
           if (leader) {
             for (int ks = 0; ks < nks; ++ks)
               umma_f16_pair_ts(tmem_base, a_tmem + 8 * ks, bd + ks * B_STEP, idesc, (it > 0 || ks > 0) ? 1u : 0u);
-            umma_commit_pair(&empty[st]);
+            umma_commit_pair(&empty[st], both);
           }
           __syncwarp();
           bd += ST_STEP;
           if (++st == S) { st = 0; ++use; bd = bd0; }
         }
-        if (leader) { umma_commit_pair(acc_full); if (item == n_items - 1) umma_commit_pair(last_full); }
+        if (leader) { umma_commit_pair(acc_full, both); if (item == n_items - 1) umma_commit_pair(last_full, both); }
         __syncwarp();
         if (lane == 0 && item == 0) gm_mark_ns(p.trace, 102);
         if (lane == 0 && item == n_items - 1) gm_mark_ns(p.trace, 103);
@@ -322,7 +386,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     // ---------------- dequantisers: one output column per thread, 64 contraction elements per task ----------------
     const int grp = (warp - 4) >> 2;                               // takes the stage uses u with u % G3_GROUPS == grp
     const int quarter = warp & 3;
-    const uint32_t full0 = mapa_u32(smem_u32(full), 0);
+    const uint32_t full0 = mapa_u32(smem_u32(full), even_cta);
     const uint32_t tdst0 = tmem_base + ((uint32_t)(32 * quarter) << 16) + G3_TMEM_A0;
     int gbase = 0;                                                 // stage uses of all earlier tiles
     TaskRegs R0, R1;
@@ -377,10 +441,12 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       }
       gbase += nst;
     }
-    if (share_last) {
+    if (n_cl > 1) {
+      exchange_in_cluster(quarter, grp);
+    } else if (share_last) {
       const int n0 = (w_last.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter;
-      const int m_base = (w_last.tile % m_tiles) * 256;
-      const int nb = (min(256, p.M - m_base) + 31) >> 5;
+      const int m_base = (w_last.tile % m_tiles) * TR;
+      const int nb = (min(TR, p.M - m_base) + 31) >> 5;
       const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
       // the quarter's shared-memory rows are free once its epilogue warp has stored the item before (a meeting of
       // the quarter's four warps: named barrier 1 + quarter)
@@ -408,14 +474,15 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   } else if (warp >= 4 + 4 * G3_GROUPS) {
     // ---------------- epilogue: TMEM -> registers -> (+bias) -> fp16 -> turned over in shared memory -> (+residual) -> global ----------------
     const int quarter = warp & 3;
-    const uint32_t acc_empty0 = mapa_u32(smem_u32(acc_empty), 0);
+    const uint32_t acc_empty0 = mapa_u32(smem_u32(acc_empty), even_cta);
     unsigned char* mine = turn + quarter * 16384;                  // [256 rows][32 columns] fp16
     pdl_wait();
-    for (int item = 0; item < n_items; ++item) {
+    if (n_cl > 1) exchange_in_cluster(quarter, 3);
+    for (int item = 0; item < (n_cl > 1 ? 0 : n_items); ++item) {
       const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
       const int n0 = (wi.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter;     // this warp's 32 output columns
-      const int m_base = (wi.tile % m_tiles) * 256;
-      const int rows = min(256, p.M - m_base);                     // rows of x the tile really has
+      const int m_base = (wi.tile % m_tiles) * TR;
+      const int rows = min(TR, p.M - m_base);                     // rows of x the tile really has
       const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
       if (share_last && item == n_items - 1) named_bar_sync(1 + quarter, 128);     // the helpers may use this quarter's rows from here
       if (lane == 0) wait_bar_idle(acc_full, item & 1, abort_flag, 100);
@@ -450,6 +517,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       if (sh.reducer && lane == 0) *sh.cnt = 0;            // every contributor has been counted: ready for the next launch
     }
   }
+  if (n_cl > 1 && warp < 4) cluster_sync_all();        // the meeting of the exchange
   if (threadIdx.x == G3_THREADS - 128) gm_mark_ns(p.trace, 106);
   tc_fence_before();
   __syncthreads();
@@ -459,5 +527,22 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
 }
 
 static size_t gemm3_smem_bytes() { return 1024 + (size_t)G3_STAGES * G3_X_BYTES + G3_BAR_BYTES + G3_TURN_BYTES; }
+
+// How many clusters of `n` pairs can be resident at once on this device (asked once).
+static int gemm3_clusters(int dev, int n) {
+  static std::atomic<int> known[64][G3_MAX_CLUSTER + 1];           // the answer and one
+  const int v = known[dev][n].load(std::memory_order_relaxed);
+  if (v) return v - 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * n * 64); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = gemm3_smem_bytes();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2 * n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  int nc = 0;
+  if (cudaOccupancyMaxActiveClusters(&nc, (const void*)q4_gemm3_kernel<true>, &cfg) != cudaSuccess || nc < 0) { cudaGetLastError(); nc = 0; }
+  known[dev][n].store(nc + 1, std::memory_order_relaxed);
+  return nc;
+}
 
 }  // namespace q4

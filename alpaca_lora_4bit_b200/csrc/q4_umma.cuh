@@ -50,9 +50,8 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, u
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Arrives on the mbarrier at this shared-memory offset in BOTH CTAs of the pair when all
-// tcgen05.mma issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint16_t both = 3;
+// tcgen05.mma issued so far by this thread have completed.  `both`: the pair's CTAs, by their ranks in the cluster.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t both = 3) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_u32(bar)), "h"(both) : "memory");
 }

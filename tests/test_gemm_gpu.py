@@ -689,3 +689,17 @@ def test_gemm_refuses_operands_of_another_shape():
 def test_short_prompts_cut_at_short_contractions(K, N, M):
     """Contractions from 1536 to 2048 and at most 64 rows, whose tiles are cut too."""
     test_short_prompts_cut_between_pairs(K, N, M)
+
+
+@pytest.mark.parametrize("K,N,M", [(512, 512, 17), (512, 256, 31), (256, 512, 33), (512, 512, 97), (512, 256, 160), (512, 512, 257),
+                                   (512, 256, 289), (512, 512, 333), (256, 256, 513), (512, 512, 801)])     # heights of 32 .. 256
+def test_tiles_of_every_height(K, N, M):
+    """Rows that make tiles of other heights than 256, whole along K."""
+    test_short_prompts_cut_between_pairs(K, N, M)
+
+
+@pytest.mark.parametrize("K,N,M", [(2176, 4096, 17), (2176, 4096, 225), (4096, 7168, 40), (4096, 4096, 300),   # three and two pairs a tile
+                                   (4096, 1024, 20), (4096, 1024, 129), (2176, 256, 256), (2304, 512, 63)])      # four
+def test_pairs_of_a_tile_add_up_in_their_cluster(K, N, M):
+    """Two to four pairs a tile, in clusters of up to eight CTAs; contractions whose parts are not equal."""
+    test_short_prompts_cut_between_pairs(K, N, M)
