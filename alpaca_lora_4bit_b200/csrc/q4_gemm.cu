@@ -75,6 +75,7 @@ struct GemmParams {
   const __half* zp_table;   // rn(s * (z+1)) for every [group, column], or null
   int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32
   int cluster_pairs;        // weights-in-TMEM kernel: pairs of a cluster; more than one: they share a tile
+  int area, turn_blocks;    // weights-in-TMEM kernel: layout of its shared memory
   int seq_shift;            // > 0: the caller promises g_idx[k] == k >> seq_shift (sequential groups of 2^seq_shift rows)
 };
 
@@ -348,13 +349,17 @@ using namespace q4;
 
 // Estimated duration (SM cycles) of the pair kernel with tiles of 256 * mh rows, and whether that
 // assumes whole tiles per pair (round after round) or all tiles x stages dealt as one sequence.
-// Per contraction stage a pair takes about 700 cycles with 256-row tiles (bounded by the dequant
+// Per contraction stage a pair takes about 780 cycles with 256-row tiles (bounded by the dequant
 // warps) and 1100 with 512-row tiles (bounded by the MMAs: twice the flops per stage); exchanging
-// the partial sums of a shared tile costs about as much as 12 resp. 16 stages.
+// the partial sums of a shared tile costs about as much as 18 resp. 24 stages.  (With 700 / 12 / 16, guessed from single
+// launches, 1536 rows of 4096 x 4096 took 59 us dealt in 256-row tiles, whole 512-row tiles 50; the backward of 1024 rows of
+// 8192 x 8192 106 and 94, act-order 133 and 116; 2048 rows of 11008 x 4096 141 and 130, the backward of 4096 x 11008, act-order,
+// 169 and 150.)
+constexpr int G2_STAGE_CYCLES_256 = 780, G2_STAGE_CYCLES_512 = 1100;
 static long long gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_ok, bool* stream) {
   const int tile_m = 256 * mh;
   const long long n_tiles = (long long)(nout / G2_TILE_N) * ((M + tile_m - 1) / tile_m);
-  const long long per_stage = mh == 2 ? 1100 : 700, exchange = mh == 2 ? 16 : 12;
+  const long long per_stage = mh == 2 ? G2_STAGE_CYCLES_512 : G2_STAGE_CYCLES_256, exchange = mh == 2 ? 24 : 18;
   long long best = (n_tiles + P - 1) / P * T;
   *stream = false;
   if (ws_ok && T >= 8 && n_tiles % P != 0) {
@@ -362,6 +367,69 @@ static long long gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_o
     if (dealt < best && total >= (long long)P * 4 && total * P < (1ll << 32)) { best = dealt; *stream = true; }
   }
   return best * per_stage;
+}
+
+// Tiles and pairs of the weights-in-TMEM kernel, by what a pair's work takes in stages of the contraction (256 rows, about
+// 0.28 us).  `room`: bytes of the workspace for partial sums.  tile_rows = 0: the act-order table does not fit.
+struct Gemm3Plan { int tile_rows, pairs, cluster; bool stream, act; double cost; Gemm3Layout layout; };
+static Gemm3Plan gemm3_plan(int M, int nout, int T, int P, int dev, int G, bool act, size_t room) {
+  Gemm3Plan best = {};
+  for (int m_tiles = (M + G3_MAX_ROWS - 1) / G3_MAX_ROWS; m_tiles <= (M + 255) / 256; ++m_tiles) {
+    Gemm3Plan c = {};
+    c.tile_rows = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+    c.cluster = 1;
+    c.layout = gemm3_layout(c.tile_rows, G, act, 1);
+    if (!c.layout.bytes) continue;
+    const int tiles = nout / G2_TILE_N * m_tiles, nb = c.tile_rows / 32;
+    const long long total = (long long)tiles * T;
+    // a stage is bound by the MMAs from 256 rows on, below - act-order: below 435 - by the dequant warps
+    const double least = act ? 1.7 : 1.0, unit = c.tile_rows > 256 * least ? c.tile_rows / 256.0 : least;
+    const bool parts = room >= (size_t)P * c.tile_rows * G2_TILE_N * sizeof(float) && total * P < (1ll << 32);
+    // whole tiles, round after round
+    c.pairs = tiles < P ? tiles : P;
+    double cost = (double)((tiles + P - 1) / P) * T * unit;
+    if (tiles > P) {
+      // or, where the last round would leave pairs idle for longer than the exchange of partial sums costs, all tiles x
+      // stages as one sequence in equal runs (measured: every further item of a run and the exchange about 30 stages)
+      const double dealt = (double)((total + P - 1) / P) * unit + 30;
+      if (parts && T >= 8 && tiles % P != 0 && dealt < cost) { cost = dealt; c.stream = true; }
+    } else if (tiles * 2 <= P && T >= 16) {
+      // Fewer tiles than half the pairs (short prompts: one row tile, 16 column tiles of a 4096-wide layer on 74 pairs):
+      // every tile is cut between a whole number n of pairs.  By the workspace that costs about 9 + 1.2 nb stages for
+      // writing and announcing the sums of nb blocks of 32 rows and 0.5 + 0.45 nb for every further contributor's that are
+      // added (8192 x 1024 at 256 rows, uncut and n = 2, 4, 6, 8, 16: 45.2, 31.1, 24.2, 23.1, 23.5, 29.6 us).
+      // The pairs of a tile in one cluster (n = 2..4) hand their sums over through shared memory: 2 + (n - 1)(1.5 + 0.3 nb)
+      // (77 rows, workspace / cluster: 5120 x 5120, n = 3, 18.6 / 15.8 us; 13824 x 5120 32.5 / 30.0; 4096 x 1024 13.9, n = 8,
+      // / 10.6, n = 4).  Of clusters of four pairs only 15 fit the GPU at once - the sixteen tiles of a 4096-wide layer
+      // take n = 3 (13.5 us; n = 4 by the workspace 15.7).
+      // Contractions of up to 2048 are cut in three or more (uncut / cut): one block of rows from 1536 on (32 rows: 2048 x
+      // 2048 14.0 / 12.1 us, 1536 x 1536 11.5 / 11.2, 1280 x 1024 10.3 / 10.5), two at 2048 (64 rows: 2048 x 2048 14.1 / 12.2,
+      // 2048 x 4096 14.3 / 13.0; in two, 2048 x 8192, 14.5 / 14.9; 1536 x 1536 11.6 / 11.5).  More rows stay whole: whole
+      // tiles add up in the pair kernel's order, so that up to 2048 the two kernels give the same bits - a test holds them
+      // to that.
+      const int n_max = T > 32 || (nb <= 2 && T >= 16 + 8 * nb) ? T / 4 : 1;
+      for (int n = T > 32 ? 2 : 3; n <= P / tiles && n <= n_max; ++n) {
+        const Gemm3Layout l = n <= G3_MAX_CLUSTER ? gemm3_layout(c.tile_rows, G, act, n) : c.layout;
+        const bool cluster = n <= G3_MAX_CLUSTER && l.bytes && gemm3_clusters(dev, n) >= tiles;
+        if (!cluster && !parts) continue;
+        const double run = (double)((T + n - 1) / n) * unit;
+        const double cut = cluster ? run + 2 + (n - 1) * (1.5 + 0.3 * nb) : run + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
+        if (cut < cost) {
+          cost = cut; c.stream = true; c.pairs = tiles * n; c.cluster = cluster ? n : 1;
+          c.layout = cluster ? l : gemm3_layout(c.tile_rows, G, act, 1);
+        }
+      }
+    } else if (parts && T >= 16 && tiles < P) {
+      // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
+      // exchange (4096 x 11008, 43 tiles, uncut / dealt: 25.4 / 22.2 us at 32 rows, 26.5 / 24.4 at 128, 27.3 / 26.6 at 192;
+      // 5120 x 13824, 54 tiles: 30.1 / 28.6 at 32, 31.6 / 31.3 at 128).
+      const double dealt = (double)total / P * unit + 14 + 3 * nb;
+      if (dealt < cost) { cost = dealt; c.stream = true; c.pairs = P; }
+    }
+    c.cost = cost;
+    if (!best.tile_rows || cost < best.cost) best = c;
+  }
+  return best;
 }
 
 static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, void* out, const void* scales,
@@ -421,11 +489,46 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     const long long e2 = gemm2_estimate(M, nout, contract / GM_TILE_C, P_est, 2, ws_ok_for(2), &s2);
     if (e2 < e1) mh = 2;
   }
-  // taken where the pair kernel would run 256-row tiles, where all its tiles fit one round, and up to 1024 rows (beyond,
-  // 512-row tiles of the pair kernel - half the dequant work per flop - measured faster on the wide layers)
-  const bool use_tm = tm_ok && use_pair &&
-                      (gv == 4 || (gv == 0 && g_gemm_variant != 5 && (mh == 1 || M <= 1024 || (long long)(nout / G2_TILE_N) * ((M + 255) / 256) <= P_est)));
-  if (use_tm) mh = 1;                          // its TMA boxes are 128 activation rows, as for 256-row tiles
+  // The weights-in-TMEM kernel: sequential layers whose groups are promised (tm_ok), and any other by its act-order form
+  const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && gv == 0 && g_gemm_variant != 5 && !one_group;
+  bool use_tm = tm_ok && use_pair && (gv == 4 || (gv == 0 && g_gemm_variant != 5));
+  Gemm3Plan plan3 = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (use_tm || tm_act) {
+    static std::atomic<bool> tm_attr_done[64];
+    if (!tm_attr_done[dev].load(std::memory_order_acquire)) {
+      for (const void* f3 : {(const void*)q4_gemm3_kernel<false, false, false>, (const void*)q4_gemm3_kernel<true, false, false>,
+                             (const void*)q4_gemm3_kernel<false, true, false>, (const void*)q4_gemm3_kernel<true, true, false>,
+                             (const void*)q4_gemm3_kernel<false, false, true>, (const void*)q4_gemm3_kernel<true, false, true>,
+                             (const void*)q4_gemm3_kernel<false, true, true>, (const void*)q4_gemm3_kernel<true, true, true>})
+        if (int e = check_cuda(cudaFuncSetAttribute(f3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "gemm smem attribute")) return e;
+      tm_attr_done[dev].store(true, std::memory_order_release);
+    }
+    const size_t room = workspace && workspace_bytes > Q4_GEMM_WS_COUNTER_BYTES ? workspace_bytes - Q4_GEMM_WS_COUNTER_BYTES : 0;
+    plan3 = gemm3_plan(M, nout, contract / GM_TILE_C, P_est, dev, G, !use_tm, room);
+    plan3.act = !use_tm;
+    use_tm = plan3.tile_rows > 0;
+    if (use_tm && gv == 0 && !(tm_ok && M <= 1024)) {
+      // Which of the two kernels, by rows of the activations times stages of 256 columns that a pair multiplies (sequential
+      // layers up to 1024 rows: always this one).  The 512-row tiles of the pair kernel run as fast as the power limit lets
+      // the tensor cores; here a row costs some 10 % more when launches are that long (W is dequantised for every 384 rows
+      // instead of every 512), but tiles follow the rows: 1100 rows of 5120 x 13824 take 116 us here and 157 there, 1536 rows
+      // 145 and 171, 2048 rows 209 and 200.  An act-order stage costs no less than 435 rows (gemm3_plan) where the pair
+      // kernel, whose dequant is as slow, does 512: 333 rows of 13824 x 5120 53 and 89 us, 500 rows of 5120 x 15360 86 and 68,
+      // 700 rows 100 and 128, 2048 rows of 8192 x 28672 827 and 709.
+      const int T = contract / GM_TILE_C;
+      const long long tiles = (long long)(nout / G2_TILE_N) * ((M + 256 * mh - 1) / (256 * mh));
+      bool dealt;
+      double stages2 = (double)gemm2_estimate(M, nout, T, P_est, mh, ws_ok_for(mh), &dealt) / (mh == 2 ? G2_STAGE_CYCLES_512 : G2_STAGE_CYCLES_256);
+      // an item's epilogue, which 512-row tiles overlap with nothing, and what an exchange costs them beyond the estimate
+      stages2 += 5.0 * ((tiles + P_est - 1) / P_est + (dealt ? 1 : 0)) + (dealt && mh == 2 ? 6 : 0);
+      const double pair = stages2 * (mh == 2 ? 512 : !plan3.act ? 288 : wide_ok ? 400 : 480);
+      use_tm = plan3.cost * 256 * (!plan3.act ? 1.13 : M <= 1024 ? 1.0 : 1.1) < pair;
+    }
+  }
+  if (use_tm) mh = 1;
   int stages = GM_MAX_STAGES;
   while (stages > 2 && gemm_smem_bytes(transpose, G, stages) > 227 * 1024) --stages;
   if (use_pair) stages = mh == 2 ? stages2w : stages2;
@@ -444,11 +547,9 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
   p.lora_r = lora_r;
   p.ws_partials = nullptr; p.ws_counters = nullptr; p.zp_table = nullptr;
   p.seq_shift = (!transpose && no_tables) ? seq_shift : 0;
-  // The weights-in-TMEM kernel's rows are the N side of its MMAs: as many tiles as of 256 rows, of the same height
-  const int tiles_m = (M + 255) / 256;
-  p.cluster_pairs = 1;
-  p.tile_rows = use_tm ? ((M + tiles_m - 1) / tiles_m + 31) / 32 * 32 : 256;
-  const int box_rows = use_tm ? p.tile_rows / 2 : use_pair ? 128 * mh : GM_TILE_M;    // activation rows one TMA copy brings
+  p.tile_rows = 256; p.cluster_pairs = 1; p.area = p.turn_blocks = 0;
+  // activation rows one TMA copy brings
+  const int box_rows = use_tm ? plan3.tile_rows / (plan3.tile_rows > 256 ? 4 : 2) : use_pair ? 128 * mh : GM_TILE_M;
   CUtensorMap amap;
   if (int e = make_tmap_2d(&amap, act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)contract, (uint64_t)M,
                            (uint64_t)contract * 2, GM_TILE_C, box_rows, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -461,9 +562,6 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
   // kernel can ask for and, for the pair kernel, ask how many pairs can be resident at once
   static bool attr_done[2][2][64] = {{{false}}};
   static int max_pairs[2][64] = {{0}};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
   const int tr = transpose ? 1 : 0;
   if (!attr_done[use_pair ? 1 : 0][tr][dev]) {
     const int cap = 227 * 1024;
@@ -516,70 +614,26 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       ws_off += zp_bytes;
     }
     if (use_tm) {
-      static bool tm_attr_done[64] = {false};
-      if (!tm_attr_done[dev]) {
-        for (const void* f3 : {(const void*)q4_gemm3_kernel<false>, (const void*)q4_gemm3_kernel<true>})
-          if (int e = check_cuda(cudaFuncSetAttribute(f3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm3_smem_bytes()), "gemm smem attribute")) return e;
-        tm_attr_done[dev] = true;
-      }
-      // whole tiles round after round, or - where the last round would leave pairs idle for longer than the exchange
-      // of partial sums costs - all tiles x stages as one sequence in equal runs (as for the pair kernel below)
-      const int tiles3 = (nout / G2_TILE_N) * ((M + 255) / 256);
-      int pairs3 = tiles3 < P ? tiles3 : P;
-      bool stream3 = false;
-      const long long total3 = (long long)tiles3 * T;
-      // (measured: every further item of a pair's run and the exchange cost about 30 stages together)
-      if (ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 8 && tiles3 > P && tiles3 % P != 0 &&
-          total3 * P < (1ll << 32)) {
-        const long long whole = (long long)((tiles3 + P - 1) / P) * T, dealt = (total3 + P - 1) / P + 30;
-        stream3 = dealt < whole;
-      }
-      // Fewer tiles than pairs (short prompts: one row tile, 16 column tiles of a 4096-wide layer on 74 pairs).  With at
-      // least two pairs per tile every tile is cut between a whole number `n` of them.  In stages of the contraction (a
-      // quarter of a microsecond), nb = blocks of 32 rows a tile really has: T / n for the pair's own run, about 9 + 1.2 nb
-      // for writing and announcing the sums and 0.5 + 0.45 nb for every further contributor's sums that are added.  (8192 x
-      // 1024 at 256 rows, uncut and n = 2, 4, 6, 8, 16: 45.2, 31.1, 24.2, 23.1, 23.5, 29.6 us; 4096 x 4096 at 32 / 256 rows:
-      // uncut 23.8 / 25.9, n = 4 15.0 / 20.7.  With the launch programmatic the stages are a third of a microsecond and the
-      // exchange weighs half as much again; the n of the estimate is still within 2 % of the best one, 4 % at 2048.)
-      // Contractions of up to 2048 are cut in three or more (uncut / cut): one block of rows from 1536 on (32 rows: 2048 x
-      // 2048 14.0 / 12.1 us, 1536 x 1536 11.5 / 11.2, 1280 x 1024 10.3 / 10.5), two at 2048 (64 rows: 2048 x 2048 14.1 / 12.2,
-      // 2048 x 4096 14.3 / 13.0; in two, 2048 x 8192, 14.5 / 14.9; 1536 x 1536 11.6 / 11.5).  More rows stay whole: up to 128 a
-      // cut would gain another microsecond (14.2 / 13.0 at 77; it loses from 192 on), but whole tiles add up in the pair
-      // kernel's order, so that up to 2048 the two kernels give the same bits - a test holds them to that.
-      const int nb = p.tile_rows / 32;
-      const bool cut_ok = !stream3 && ws && workspace_bytes >= ws_off + (size_t)P * Q4_GEMM_WS_SLICE_BYTES && T >= 16;
-      if (cut_ok && tiles3 * 2 <= P) {
-        // The pairs of a tile in one cluster (n = 2..4) hand their sums over through shared memory instead of the workspace:
-        // 2 + (n - 1)(1.5 + 0.3 nb) stages instead of 9 + 1.2 nb and more (77 rows, workspace / cluster: 5120 x 5120, n = 3,
-        // 18.6 / 15.8 us; 13824 x 5120 32.5 / 30.0; 4096 x 1024 13.9, n = 8, / 10.6, n = 4).  Of clusters of four pairs only
-        // 15 fit the GPU at once - the sixteen tiles of a 4096-wide layer take n = 3 (13.5 us; n = 4 by the workspace 15.7).
-        double best = T;
-        const int n_max = T > 32 || (nb <= 2 && T >= 16 + 8 * nb) ? T / 4 : 1;
-        for (int n = T > 32 ? 2 : 3; n <= P / tiles3 && n <= n_max; ++n) {
-          const bool cluster = n <= G3_MAX_CLUSTER && gemm3_clusters(dev, n) >= tiles3;
-          const double run = (double)((T + n - 1) / n);
-          const double cost = cluster ? run + 2 + (n - 1) * (1.5 + 0.3 * nb) : run + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
-          if (cost < best) { best = cost; stream3 = true; pairs3 = tiles3 * n; p.cluster_pairs = cluster ? n : 1; }
-        }
-      } else if (cut_ok && tiles3 < P && total3 * P < (1ll << 32)) {
-        // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
-        // exchange (4096 x 11008, 43 tiles, uncut / dealt: 25.4 / 22.2 us at 32 rows, 26.5 / 24.4 at 128, 27.3 / 26.6 at 192;
-        // 5120 x 13824, 54 tiles: 30.1 / 28.6 at 32, 31.6 / 31.3 at 128).
-        const double dealt = (double)total3 / P + 14 + 3 * nb;
-        if (dealt < T) { stream3 = true; pairs3 = P; }
-      }
+      p.tile_rows = plan3.tile_rows; p.cluster_pairs = plan3.cluster; p.stages = plan3.layout.stages;
+      p.area = plan3.layout.area; p.turn_blocks = plan3.layout.turn_blocks;
       p.ws_partials = (float*)(ws + ws_off);
       p.ws_counters = (unsigned*)ws;
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(2 * pairs3); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = gemm3_smem_bytes(); cfg.stream = st;
+      cfg.gridDim = dim3(2 * plan3.pairs); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = plan3.layout.bytes; cfg.stream = st;
       cudaLaunchAttribute at[2];
       at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       at[0].val.programmaticStreamSerializationAllowed = 1;
       at[1].id = cudaLaunchAttributeClusterDimension;
       at[1].val.clusterDim.x = 2 * p.cluster_pairs; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
       cfg.attrs = at; cfg.numAttrs = 2;
-      if (int e = check_cuda(stream3 ? cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<true>, amap, umap, p)
-                                     : cudaLaunchKernelEx(&cfg, q4_gemm3_kernel<false>, amap, umap, p), "gemm launch")) return e;
+      auto launch3 = [&](auto kernel) { return check_cuda(cudaLaunchKernelEx(&cfg, kernel, amap, umap, p), "gemm launch"); };
+      const bool tall = plan3.tile_rows > 256;
+      int e3;
+      if (plan3.act) e3 = plan3.stream ? (tall ? launch3(q4_gemm3_kernel<true, true, true>) : launch3(q4_gemm3_kernel<true, true, false>))
+                                       : (tall ? launch3(q4_gemm3_kernel<false, true, true>) : launch3(q4_gemm3_kernel<false, true, false>));
+      else e3 = plan3.stream ? (tall ? launch3(q4_gemm3_kernel<true, false, true>) : launch3(q4_gemm3_kernel<true, false, false>))
+                             : (tall ? launch3(q4_gemm3_kernel<false, false, true>) : launch3(q4_gemm3_kernel<false, false, false>));
+      if (e3) return e3;
       return check_cuda(cudaGetLastError(), "gemm launch");
     }
     // Whole tiles per pair, round after round - or, when the last round would leave pairs idle for

@@ -1,28 +1,34 @@
 // The fused dequant-GEMM forward with the dequantised weights in TENSOR MEMORY (tcgen05.mma with its A operand
-// in TMEM), for layers whose groups are sequential by the caller's word.  Included by q4_gemm.cu after q4_gemm2.cuh.
+// in TMEM).  Included by q4_gemm.cu after q4_gemm2.cuh.
 //
 // The pair kernel of q4_gemm2.cuh keeps both operands in shared memory: a dequant task there is eight swizzled
 // 16-byte stores behind scale and zero-term vectors of eight columns, a proxy fence and a barrier, and per 64
 // contraction elements an SM takes 16 KiB of dequant stores on top of 16 KiB of TMA writes and 32 KiB of tensor-core
 // reads.  Here the product is transposed,
 // y^T = W^T x^T: the weights are the A operand (M side: 256 output columns per pair, 128 per CTA = one TMEM lane
-// each), the activations the B operand (N side: a tile of up to 256 rows of x, half per CTA, K-major by TMA exactly as
-// before; all tiles of a product have the same height, a multiple of 32, so that 333 rows are two tiles of 192 and 77 one
-// of 96: the MMAs of 64 contraction elements take 540 cycles at 256 rows, and 333 rows of 13824 x 5120 took 54.9 us, now 52.7).  A dequant thread owns one output column: the eight packed words of its column and a stage are eight
-// coalesced 4-byte loads, one word is eight consecutive k of that column = four half2 in contraction order, scale
-// and zero term are scalars of the thread, and the stage's 64 halves leave as one `tcgen05.st` of 32 columns.
-// Nothing of W touches shared memory; an SM moves 16 KiB of TMA writes and 16 KiB of operand reads per stage.
+// each), the activations the B operand (N side: a tile of up to 384 rows of x, half per CTA, K-major by TMA exactly as
+// before).  A dequant thread owns one output column: the eight packed words of its column and a stage are eight
+// coalesced 4-byte loads, one word is eight consecutive k of that column = four half2 in contraction order, and the
+// stage's 64 halves leave as one `tcgen05.st` of 32 columns.  Nothing of W touches shared memory.
+//   Sequential groups (by the caller's word): scale and zero term are scalars of the thread.
+//   Act-order (ACT): every weight has the scale and zero term of its own row's group.  A table in shared memory holds the
+//   two as one word per group and column of this CTA; the lanes' columns lie on different banks whatever the group, and
+//   the 64 rows' offsets into it are the same for all lanes of a warp.  (The pair kernel looks whole vectors of eight
+//   columns up row by row: 333 rows of 5120 x 5120 take 43 us there and 28 here, 77 rows 32 and 22.)
 //
-// TMEM (512 columns): accumulator [128 lanes = output columns][256 columns = rows of x] fp32, and eight operand
+// Tiles follow the rows: as many as of 384 or 256 rows, whichever takes less time (gemm3_plan), all of one height, a
+// multiple of 32.  77 rows are one tile of 96 and 333 one of 352 - two MMAs of 176 on the same dequantised operand (TALL),
+// which used to be dequantised for two tiles of 256: 333 rows of 5120 x 15360 57 -> 43 us, of 5120 x 27648 93 -> 81 us.
+// TMEM (512 columns): accumulator [128 lanes = output columns][columns = rows of x] fp32, and four to eight operand
 // stages of 32 columns (lane = output column, column c of a stage = contraction elements 2c, 2c+1 as a half2).
-// Roles (640 threads per CTA): warp 0 TMA producer of this CTA's 128 activation rows; warp 1 owns TMEM, its elected
+// Roles (640 threads per CTA): warp 0 TMA producer of this CTA's half of the activation rows; warp 1 owns TMEM, its elected
 // lane in the even CTA issues the MMAs; warps 4-15 dequantise (warp & 3 = its TMEM lane quarter; three groups of
 // four warps take every third stage use: a task is a chain of loads, arithmetic, the wait for the slot, the TMEM
-// store and its completion, about 1500 cycles where the MMAs of a stage take 540, so three tasks have to be in
+// store and its completion, about 1500 cycles where the MMAs of 256 rows take 540, so three tasks have to be in
 // flight); warps 16-19 epilogue.  Whole tiles per pair round after round, or (SPLIT) equal runs of tiles x stages.
-// The accumulator's lanes are output columns, so a thread of the epilogue holds 32 rows of one column: a warp
-// first moves its 32 columns x 256 rows into shared memory as fp16 (and hands the accumulator back: the MMAs of the
-// pair's next item start while the stores run), then stores rows of 64 bytes, four lanes each.
+// The accumulator's lanes are output columns, so a thread of the epilogue holds 32 rows of one column: a warp turns blocks
+// of 32 rows x 32 columns over in shared memory as fp16 and stores rows of 64 bytes, four lanes each.  In the plain form
+// (sequential, up to 256 rows) there is room for all blocks, and the accumulator is handed back before the stores.
 // Every wait is bounded as in the pair kernel.
 // Where the pairs that share a tile form a cluster (p.cluster_pairs, few tiles), each adds up a part of the tile's rows from
 // the others' shared memory: through the workspace the exchange took 5-7 us (write, fence, count, wait, and the
@@ -35,15 +41,15 @@
 
 namespace q4 {
 
-constexpr int G3_STAGES = 8;                  // operand stages in TMEM = activation stages in shared memory
-static_assert(G3_STAGES == 8, "a stage use u lies in slot u & 7, use u >> 3");
-constexpr int G3_X_BYTES = 128 * GM_TILE_C * 2;           // 16 KiB: this CTA's 128 activation rows of a stage
-constexpr int G3_TMEM_A0 = 256;               // first TMEM column of the operand stages
+constexpr int G3_MAX_STAGES = 8;              // operand stages in TMEM = activation stages in shared memory
+constexpr int G3_MAX_ROWS = 384;              // of a tile: its accumulator and four operand stages are all of TMEM
 constexpr int G3_BAR_BYTES = 512;
 constexpr int G3_MAX_CLUSTER = 4;             // pairs: eight CTAs, the portable size
 constexpr int G3_GROUPS = 3;                  // dequant groups of four warps
 constexpr int G3_THREADS = 32 * (4 + 4 * G3_GROUPS + 4);
-constexpr int G3_TURN_BYTES = 4 * 256 * 64;    // per epilogue warp its 32 columns of all 256 rows of a tile, fp16
+constexpr int G3_OFFS_BYTES = 4 * G3_GROUPS * 256;   // act-order: per dequant warp the table offsets of a stage's 64 rows
+constexpr int G3_PLAIN_AREA = G3_MAX_STAGES * 128 * GM_TILE_C * 2;
+constexpr int G3_TURN_BLOCK = 32 * 64;         // a warp's 32 columns of 32 rows, fp16
 
 __device__ __forceinline__ void umma_f16_pair_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -100,22 +106,32 @@ __device__ __forceinline__ void deq_word_k(uint32_t w, uint32_t s2, uint32_t c2,
 // SPLIT as in the pair kernel: whole tiles per pair, or equal runs of the sequence of all tiles x stages with the
 // partial sums of a shared tile meeting in the workspace (added in pair order by the pair whose run starts the tile).
 // The launch gives the cluster's size: one pair or, with p.cluster_pairs = n > 1 (SPLIT only), the n pairs that share a tile.
-template <bool SPLIT>
+// ACT: act-order.  Every weight has the scale and zero term of its own row's group: a table in shared memory holds, per group
+// and column of this CTA, the two as one word, a lane's loads of it lie on its own bank whatever the groups are, and the
+// rows' table offsets of a stage are the same for all lanes.
+template <bool SPLIT, bool ACT, bool TALL>
 __global__ void __launch_bounds__(G3_THREADS, 1)
 q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap umap, const GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
   pdl_launch_dependents();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   unsigned char* stages = smem;
-  constexpr int S = G3_STAGES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * G3_X_BYTES);          // even CTA: activation bytes + 4 dequant warps, of both CTAs
+  const int S = ACT || TALL ? p.stages : G3_MAX_STAGES;
+  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32
+  constexpr int nh = TALL ? 2 : 1;                     // MMAs per 16 contraction elements
+  const int HR = TR / nh;                              // and rows of each
+  constexpr bool PLAIN = !ACT && !TALL;                // one layout for all: stages of 128 rows, a place to turn every block over
+  const int x_bytes = PLAIN ? 128 * GM_TILE_C * 2 : TR * GM_TILE_C;             // this CTA's half of a tile's rows of a stage
+  unsigned char* tab = smem + S * x_bytes;             // act-order: [G][128 columns] scale | zero term
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (PLAIN ? G3_PLAIN_AREA : p.area));                  // even CTA: activation bytes + 4 dequant warps, of both CTAs
   uint64_t* empty = full + 8;                                                   // both CTAs: stage read by the MMAs
   uint64_t* acc_full = empty + 8;                                               // both CTAs: accumulator complete
   uint64_t* acc_empty = acc_full + 1;                                           // even CTA: 4 epilogue warps x 2 CTAs
   uint64_t* last_full = acc_empty + 1;                                          // both CTAs: the pair's last accumulator complete (one use)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  unsigned char* turn = smem + S * G3_X_BYTES + G3_BAR_BYTES;
+  unsigned char* offs_all = reinterpret_cast<unsigned char*>(full) + G3_BAR_BYTES;
+  unsigned char* turn = offs_all + (ACT ? G3_OFFS_BYTES : 0);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cluster_rank = cluster_ctarank(), rank = cluster_rank & 1, even_cta = cluster_rank & ~1u;
@@ -123,13 +139,17 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   const int T = p.n_contract_tiles;
   const int lora_ks = (p.lora_r + 15) >> 4;
   const int N = p.N;
-  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32
   const int m_tiles = (p.M + TR - 1) / TR;
   const int n_tiles = m_tiles * (N / G2_TILE_N);
   const WorkRange wr = work_range<SPLIT>(pair, n_pairs, n_tiles, T);
   const int n_items = wr.n_items;
 
-  struct TaskRegs { uint32_t w[8]; uint32_t s, z; };
+  // where a warp turns a block of 32 rows over: a place per block (the accumulator can be handed back before the stores) or,
+  // where shared memory is short, one per warp
+  auto turn_of = [&](int quarter, int cb) __attribute__((always_inline)) {
+    return turn + (PLAIN ? quarter * 8 + cb : p.turn_blocks ? quarter * p.turn_blocks + cb : warp - 4) * G3_TURN_BLOCK;
+  };
+  struct TaskRegs { uint32_t w[8]; uint32_t s, z; };             // (act-order: s and z are the groups of rows lane and 32 + lane)
   const bool is_deq = warp >= 4 && warp < 4 + 4 * G3_GROUPS;
   auto column_of = [&](int tile) { return (tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * (warp & 3) + lane; };
   auto prefetch = [&](int n, int j, TaskRegs& R) __attribute__((always_inline)) {
@@ -138,9 +158,14 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const uint32_t* src = wcol + (size_t)(j * (GM_TILE_C >> 3)) * N;
 #pragma unroll
     for (int i = 0; i < 8; ++i) R.w[i] = ld_pinned_u32(src + (size_t)i * N);
-    const size_t at = (size_t)((j * GM_TILE_C) >> p.seq_shift) * N + n;
-    R.s = ld_pinned_u16(p.scales + at);
-    R.z = ld_pinned_u16(p.zp_table + at);
+    if (ACT) {
+      R.s = ld_pinned_u32(p.g_idx + j * GM_TILE_C + lane);
+      R.z = ld_pinned_u32(p.g_idx + j * GM_TILE_C + 32 + lane);
+    } else {
+      const size_t at = (size_t)((j * GM_TILE_C) >> p.seq_shift) * N + n;
+      R.s = ld_pinned_u16(p.scales + at);
+      R.z = ld_pinned_u16(p.zp_table + at);
+    }
     // the words of the group's task after the next, asked into L2 (eight rows of 128 bytes per warp)
     if (j + 2 * G3_GROUPS < T && lane < 8) prefetch_l2(wcol - lane + (size_t)((j + 2 * G3_GROUPS) * (GM_TILE_C >> 3) + lane) * N);
   };
@@ -155,9 +180,16 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       if (j >= w0.ke) break;
       const size_t at = (size_t)((j * GM_TILE_C) >> p.seq_shift) * N + n;
       if (lane < 8) prefetch_l2(p.qw + (size_t)(j * (GM_TILE_C >> 3) + lane) * N + n);
-      else if (lane == 8) prefetch_l2(p.scales + at);
-      else if (lane == 9) prefetch_l2(p.zp_table + at);
+      else if (ACT && lane < 10) prefetch_l2(p.g_idx + j * GM_TILE_C + 32 * (lane - 8));
+      else if (!ACT && lane == 8) prefetch_l2(p.scales + at);
+      else if (!ACT && lane == 9) prefetch_l2(p.zp_table + at);
     }
+    if (ACT)
+      for (int i = threadIdx.x - 128; i < 3 * p.G; i += 128 * G3_GROUPS) {
+        const int c0 = (w0.tile / m_tiles) * G2_TILE_N + 128 * (int)rank, g = i / 3;
+        if (i % 3 < 2) prefetch_l2(p.scales + (size_t)g * N + c0 + 64 * (i % 3));
+        else prefetch_l2(p.qzeros + (size_t)g * (N >> 3) + (c0 >> 3));
+      }
   }
 
   if (threadIdx.x == 0) {
@@ -210,11 +242,11 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   // writing or the adding up of the partial sums of a shared one.  (On short prompts, where every item is a piece of a
   // tile, one warp per quarter did the exchange block by block, a trip to L2 each: 128 rows of 4096 x 4096 took 23.2 us
   // and 18.9 shared, of 11008 x 4096 32.5 and 28.2; since the launch is programmatic 16.9 and 25.6.)
-  const WorkItem w_last = work_item<SPLIT>(p, wr, n_items > 0 ? n_items - 1 : 0, n_pairs, T);
-  const bool share_last = n_items > 0;
+  // Not the items before: the dequant warps run ahead into the next one's stages instead (tall tiles, whose blocks may have
+  // to be stored one by one, took 5 to 20 % longer with every epilogue shared).
 
   // A shared tile of this run: who contributes, its arrival counter (per CTA of the pair and lane quarter) and the
-  // place of a contributor's sums: a warp's 32 columns x 256 rows as [block][j][lane][4 floats] (512 contiguous bytes
+  // place of a contributor's sums: a warp's 32 columns x the tile's rows as [block][j][lane][4 floats] (512 contiguous bytes
   // per 16-byte access of the warp), indexed [contributing pair][CTA of the pair][lane quarter].
   struct Shared { bool shared, reducer; int c_first, c_last; unsigned* cnt; };
   auto shared_of = [&](const WorkItem& wi, int quarter) {
@@ -228,7 +260,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     }
     return s;
   };
-  auto part_of = [&](int cpair, int quarter) -> float* { return p.ws_partials + (((size_t)cpair * 2 + rank) * 4 + quarter) * (size_t)(8 * 8 * 32 * 4); };
+  auto part_of = [&](int cpair, int quarter) -> float* { return p.ws_partials + (((size_t)cpair * 2 + rank) * 4 + quarter) * (size_t)(TR * 32); };
   auto await_partials = [&](const Shared& s) {
     if (lane == 0) {
       const unsigned want = (unsigned)(s.c_last - s.c_first);
@@ -277,23 +309,27 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   const int n_cl = SPLIT ? p.cluster_pairs : 1;
   auto exchange_in_cluster = [&](int quarter, int w4) __attribute__((always_inline)) {
     const int me = (int)(cluster_rank >> 1);
+    const WorkItem w_last = work_item<SPLIT>(p, wr, 0, n_pairs, T);
     const int n0 = (w_last.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter, m_base = (w_last.tile % m_tiles) * TR;
     const int nb = (min(TR, p.M - m_base) + 31) >> 5;
     const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
-    unsigned char* sums = stages + quarter * (8 * 4096) + lane * 16;               // [quarter][block][q][lane][4 floats]
+    // [lane quarter][block that is not the pair's own][q][lane][4 floats]
+    const int slots = (TR >> 5) - (TR >> 5) / n_cl;
+    unsigned char* sums = smem + (size_t)quarter * slots * 4096 + lane * 16;
     const uint32_t tsrc = tmem_base + ((uint32_t)(32 * quarter) << 16);
     if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 40);
     __syncwarp();
     tc_fence_after();
 #pragma unroll 1
     for (int cb = w4; cb < nb; cb += 4) {
-      if (cb % n_cl == me) continue;
+      const int whose = cb % n_cl, slot = cb / n_cl * (n_cl - 1) + whose - (whose > me);
+      if (whose == me) continue;
       uint32_t v[32];
       tmem_ld32(tsrc + cb * 32, v);
       tmem_ld_wait();
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(sums + cb * 4096 + q * 512) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        *reinterpret_cast<uint4*>(sums + slot * 4096 + q * 512) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     }
     cluster_sync_all();
 #pragma unroll 1
@@ -304,7 +340,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
 #pragma unroll 1
       for (int c = 1; c < n_cl; ++c) {
         const int from = me + c < n_cl ? me + c : me + c - n_cl;
-        const uint32_t src = mapa_u32(smem_u32(sums + cb * 4096), 2 * from + rank);
+        const uint32_t src = mapa_u32(smem_u32(sums + (cb / n_cl * (n_cl - 1) + me - (me > from)) * 4096), 2 * from + rank);
         float4 t[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) t[q] = ld_cluster_f4(src + q * 512);
@@ -314,10 +350,11 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
           v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + t[q].z); v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + t[q].w);
         }
       }
-      unsigned char* mine = turn + quarter * 16384 + cb * 2048;
+      unsigned char* mine = turn_of(quarter, cb);
       block_to_smem(mine, v, bv);
       __syncwarp();
       block_to_global(mine, m_base + cb * 32, n0);
+      __syncwarp();
     }
   };
 
@@ -329,15 +366,18 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       pdl_wait();
       for (int item = 0; item < n_items; ++item) {
         const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
-        const int m0 = (wi.tile % m_tiles) * TR + (TR >> 1) * (int)rank;
+        const int m0 = (wi.tile % m_tiles) * TR + (HR >> 1) * (int)rank;
         const int nst = wi.ke - wi.kb + (wi.lora ? 1 : 0);
         for (int j = 0; j < nst; ++j) {
           const int it = wi.kb + j;
           if (use > 0) wait_bar_idle(&empty[st], (use - 1) & 1, abort_flag, 40);
           if (rank == 0) mbar_arrive_expect_tx(&full[st], TR * GM_TILE_C * 2);
-          unsigned char* dst = stages + (size_t)st * G3_X_BYTES;
-          if (it < wi.ke) tma_load_2d_pair(dst, &amap, it * GM_TILE_C, m0, full0 + 8 * st);
-          else tma_load_2d_pair(dst, &umap, 0, m0, full0 + 8 * st);
+#pragma unroll
+          for (int h = 0; h < nh; ++h) {
+            unsigned char* dst = smem + (size_t)st * x_bytes + h * HR * GM_TILE_C;
+            if (it < wi.ke) tma_load_2d_pair(dst, &amap, it * GM_TILE_C, m0 + h * HR, full0 + 8 * st);
+            else tma_load_2d_pair(dst, &umap, 0, m0 + h * HR, full0 + 8 * st);
+          }
           if (++st == S) { st = 0; ++use; }
         }
       }
@@ -349,11 +389,13 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     if (rank == 0) {
       uint32_t leader;
       asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(leader));
-      const uint32_t idesc = idesc_f16(256, TR, false);
+      const uint32_t idesc = idesc_f16(256, HR, false);
       const uint16_t both = (uint16_t)(3u << even_cta);
       // B: this CTA's 128 rows of x, K-major, 128-byte rows, 8-row groups 1024 B apart, 16 contraction elements = 32 B
-      const uint64_t bd0 = smem_desc_sw128(smem_u32(stages), 16, 1024);
-      constexpr uint64_t B_STEP = 32 >> 4, ST_STEP = G3_X_BYTES >> 4;
+      const uint64_t bd0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
+      constexpr uint64_t B_STEP = 32 >> 4;
+      const uint64_t ST_STEP = (uint64_t)(x_bytes >> 4), H_STEP = (uint64_t)((HR * GM_TILE_C) >> 4);
+      const uint32_t a0_tmem = tmem_base + G2_TMEM_COLS - 32 * S;
       int st = 0, use = 0;
       uint64_t bd = bd0;
       for (int item = 0; item < n_items; ++item) {
@@ -365,11 +407,13 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
           wait_bar_cluster(&full[st], use & 1, abort_flag);
           if (p.trace && lane == 0 && item == 0 && (it & 7) == 0 && it < 64) gm_mark_ns(p.trace, 110 + (it >> 3));
           tc_fence_after();
-          const uint32_t a_tmem = tmem_base + G3_TMEM_A0 + 32 * st;
+          const uint32_t a_tmem = a0_tmem + 32 * st;
           const int nks = it < ncon ? 4 : lora_ks;
           if (leader) {
             for (int ks = 0; ks < nks; ++ks)
-              umma_f16_pair_ts(tmem_base, a_tmem + 8 * ks, bd + ks * B_STEP, idesc, (it > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+              for (int h = 0; h < nh; ++h)
+                umma_f16_pair_ts(tmem_base + h * HR, a_tmem + 8 * ks, bd + ks * B_STEP + h * H_STEP, idesc, (it > 0 || ks > 0) ? 1u : 0u);
             umma_commit_pair(&empty[st], both);
           }
           __syncwarp();
@@ -387,8 +431,12 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const int grp = (warp - 4) >> 2;                               // takes the stage uses u with u % G3_GROUPS == grp
     const int quarter = warp & 3;
     const uint32_t full0 = mapa_u32(smem_u32(full), even_cta);
-    const uint32_t tdst0 = tmem_base + ((uint32_t)(32 * quarter) << 16) + G3_TMEM_A0;
+    const uint32_t tdst0 = tmem_base + ((uint32_t)(32 * quarter) << 16) + G2_TMEM_COLS - 32 * S;
     int gbase = 0;                                                 // stage uses of all earlier tiles
+    int next_st = grp, next_use = 0;                               // of this group's next stage use (PLAIN: u & 7, u >> 3)
+    int tab_n0 = -1;
+    uint32_t* offs = reinterpret_cast<uint32_t*>(offs_all) + 64 * (warp - 4);
+    const unsigned char* tabl = tab + 4 * (32 * quarter + lane);
     TaskRegs R0, R1;
     pdl_wait();                                                    // scales, zero terms, adapters, bias, workspace
     for (int item = 0; item < n_items; ++item) {
@@ -396,7 +444,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       const int n = column_of(wi.tile);
       const int ncon = wi.ke - wi.kb, nst = ncon + (wi.lora ? 1 : 0);       // stages of this item: j = 0 .. nst-1, contraction stage kb + j
       auto task = [&](int j, const TaskRegs& C) __attribute__((always_inline)) {
-        const int u = gbase + j, st = u & (S - 1), use = u >> 3;
+        const int st = PLAIN ? (gbase + j) & (G3_MAX_STAGES - 1) : next_st, use = PLAIN ? (gbase + j) / G3_MAX_STAGES : next_use;
         uint32_t o[32];
         if (j == ncon) {
           // low-rank stage: lane = column n holds lora_B[n][0..r), zero beyond
@@ -406,6 +454,24 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
             const __half lo = 2 * c < p.lora_r ? src[2 * c] : __float2half(0.f);
             const __half hi = 2 * c + 1 < p.lora_r ? src[2 * c + 1] : __float2half(0.f);
             o[c] = as_u32(__halves2half2(lo, hi));
+          }
+        } else if (ACT) {
+          offs[lane] = min(C.s, (uint32_t)(p.G - 1)) * 512;
+          offs[lane + 32] = min(C.z, (uint32_t)(p.G - 1)) * 512;
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 oa = *reinterpret_cast<const uint4*>(offs + 8 * i), ob = *reinterpret_cast<const uint4*>(offs + 8 * i + 4);
+            const uint32_t at[8] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
+            uint32_t e[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) e[k] = *reinterpret_cast<const uint32_t*>(tabl + at[k]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t v = and_or(prmt(C.w[i], C.w[i], k | (k << 8)), 0x00F0000Fu, 0x54006400u);
+              const uint32_t s2 = prmt(e[2 * k], e[2 * k + 1], 0x5410), z2 = prmt(e[2 * k], e[2 * k + 1], 0x7632);
+              o[4 * i + k] = as_u32(__hsub2_rn(__hmul2_rn(as_h2(s2), __hsub2(as_h2(v), as_h2(0x54006400u))), as_h2(z2)));
+            }
           }
         } else {
           const uint32_t s2 = prmt(C.s, C.s, 0x1010), z2 = prmt(C.z, C.z, 0x1010);
@@ -426,10 +492,41 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(full0 + 8 * st);
+        if (!PLAIN) {
+          next_st += G3_GROUPS;
+          if (next_st >= S) { next_st -= S; ++next_use; }
+        }
       };
       int j = (grp + G3_GROUPS - gbase % G3_GROUPS) % G3_GROUPS;   // this group's first stage of the tile
       auto ask = [&](int jj, TaskRegs& R) __attribute__((always_inline)) { if (jj < ncon) prefetch(n, wi.kb + jj, R); };
       ask(j, R0);
+      const int c0 = (wi.tile / m_tiles) * G2_TILE_N + 128 * (int)rank;
+      if (ACT && c0 != tab_n0) {
+        if (tab_n0 >= 0) named_bar_sync(5, 128 * G3_GROUPS);       // the readers of the table before are done
+#pragma unroll 1
+        for (int i0 = threadIdx.x - 128; i0 < p.G * 16; i0 += 4 * 128 * G3_GROUPS) {
+          uint4 sv[4];
+          uint32_t zw[4];
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {                            // (nothing else covers their trips to L2: all four at once)
+            const int i = i0 + b * 128 * G3_GROUPS, g = i >> 4, c8 = i & 15;
+            if (i >= p.G * 16) break;
+            sv[b] = ld_pinned_u4(p.scales + (size_t)g * N + c0 + 8 * c8);
+            zw[b] = ld_pinned_u32(p.qzeros + (size_t)g * (N >> 3) + (c0 >> 3) + c8);
+          }
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const int i = i0 + b * 128 * G3_GROUPS;
+            if (i >= p.G * 16) break;
+            const uint4 s8 = sv[b], z8 = zero_terms(s8, zw[b]);
+            uint4* to = reinterpret_cast<uint4*>(tab + 32 * i);
+            to[0] = make_uint4(prmt(s8.x, z8.x, 0x5410), prmt(s8.x, z8.x, 0x7632), prmt(s8.y, z8.y, 0x5410), prmt(s8.y, z8.y, 0x7632));
+            to[1] = make_uint4(prmt(s8.z, z8.z, 0x5410), prmt(s8.z, z8.z, 0x7632), prmt(s8.w, z8.w, 0x5410), prmt(s8.w, z8.w, 0x7632));
+          }
+        }
+        named_bar_sync(5, 128 * G3_GROUPS);
+        tab_n0 = c0;
+      }
       while (j < nst) {
         ask(j + G3_GROUPS, R1);
         task(j, R0);
@@ -441,9 +538,8 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       }
       gbase += nst;
     }
-    if (n_cl > 1) {
-      exchange_in_cluster(quarter, grp);
-    } else if (share_last) {
+    if (n_cl == 1 && n_items > 0) {                      // the last item's epilogue, with the epilogue warp of the quarter
+      const WorkItem w_last = work_item<SPLIT>(p, wr, n_items - 1, n_pairs, T);
       const int n0 = (w_last.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter;
       const int m_base = (w_last.tile % m_tiles) * TR;
       const int nb = (min(TR, p.M - m_base) + 31) >> 5;
@@ -454,44 +550,43 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 100);
       __syncwarp();
       tc_fence_after();
-      unsigned char* mine = turn + quarter * 16384;
       const Shared sh = shared_of(w_last, quarter);
       if (sh.reducer) {
         await_partials(sh);
-        named_bar_sync(1 + quarter, 128);                          // all four warps have seen the count: the epilogue warp may clear it
+        named_bar_sync(1 + quarter, 128);                        // all four warps have seen the count: the epilogue warp may clear it
       }
 #pragma unroll 1
       for (int cb = grp; cb < nb; cb += G3_GROUPS + 1) {
-        take_block(sh, quarter, cb, tmem_base + ((uint32_t)(32 * quarter) << 16), mine + cb * 2048, bv);
+        unsigned char* mine = turn_of(quarter, cb);
+        take_block(sh, quarter, cb, tmem_base + ((uint32_t)(32 * quarter) << 16), mine, bv);
         __syncwarp();
-        if (!sh.shared || sh.reducer) block_to_global(mine + cb * 2048, m_base + cb * 32, n0);
+        if (!sh.shared || sh.reducer) block_to_global(mine, m_base + cb * 32, n0);
+        __syncwarp();
       }
       if (sh.shared && !sh.reducer) {
         __threadfence();
-        named_bar_sync(1 + quarter, 128);                          // this warp's sums are out: the epilogue warp counts for all four
+        named_bar_sync(1 + quarter, 128);                        // this warp's sums are out: the epilogue warp counts for all four
       }
     }
   } else if (warp >= 4 + 4 * G3_GROUPS) {
     // ---------------- epilogue: TMEM -> registers -> (+bias) -> fp16 -> turned over in shared memory -> (+residual) -> global ----------------
     const int quarter = warp & 3;
     const uint32_t acc_empty0 = mapa_u32(smem_u32(acc_empty), even_cta);
-    unsigned char* mine = turn + quarter * 16384;                  // [256 rows][32 columns] fp16
     pdl_wait();
-    if (n_cl > 1) exchange_in_cluster(quarter, 3);
     for (int item = 0; item < (n_cl > 1 ? 0 : n_items); ++item) {
       const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
       const int n0 = (wi.tile / m_tiles) * G2_TILE_N + 128 * (int)rank + 32 * quarter;     // this warp's 32 output columns
       const int m_base = (wi.tile % m_tiles) * TR;
       const int rows = min(TR, p.M - m_base);                     // rows of x the tile really has
       const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
-      if (share_last && item == n_items - 1) named_bar_sync(1 + quarter, 128);     // the helpers may use this quarter's rows from here
+      if (item == n_items - 1) named_bar_sync(1 + quarter, 128);   // the helpers may use this quarter's rows from here
       if (lane == 0) wait_bar_idle(acc_full, item & 1, abort_flag, 100);
       __syncwarp();
       tc_fence_after();
       if (lane == 0 && item == n_items - 1) gm_mark_ns(p.trace, 105);
       const uint32_t tsrc = tmem_base + ((uint32_t)(32 * quarter) << 16);
       const int nb = (rows + 31) >> 5;                             // blocks of 32 rows that hold anything
-      const bool shared_out = share_last && item == n_items - 1;   // the dequant warps take the blocks cb % 4 = 0, 1, 2
+      const bool shared_out = item == n_items - 1;                 // the dequant warps take the blocks cb % 4 = 0, 1, 2
       const int cb0 = shared_out ? G3_GROUPS : 0, cbs = shared_out ? G3_GROUPS + 1 : 1;
       const Shared sh = shared_of(wi, quarter);
       if (sh.reducer) {
@@ -499,14 +594,22 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
         if (shared_out) named_bar_sync(1 + quarter, 128);
       }
 #pragma unroll 1
-      for (int cb = cb0; cb < nb; cb += cbs) take_block(sh, quarter, cb, tsrc, mine + cb * 2048, bv);
+      for (int cb = cb0; cb < nb; cb += cbs) {
+        unsigned char* mine = turn_of(quarter, cb);
+        take_block(sh, quarter, cb, tsrc, mine, bv);
+        if (PLAIN || p.turn_blocks || (sh.shared && !sh.reducer)) continue;
+        __syncwarp();
+        block_to_global(mine, m_base + cb * 32, n0);
+        __syncwarp();
+      }
       // this warp has read its part of the accumulator: the even CTA may start the next item
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty0);
       if (!sh.shared || sh.reducer) {
+        if (PLAIN || p.turn_blocks)
 #pragma unroll 1
-        for (int cb = cb0; cb < nb; cb += cbs) block_to_global(mine + cb * 2048, m_base + cb * 32, n0);
+          for (int cb = cb0; cb < nb; cb += cbs) block_to_global(turn_of(quarter, cb), m_base + cb * 32, n0);
         __syncwarp();                                      // the rows are read before the next item overwrites them
       } else {                                             // publish: sums, then the count
         __threadfence();
@@ -517,7 +620,10 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       if (sh.reducer && lane == 0) *sh.cnt = 0;            // every contributor has been counted: ready for the next launch
     }
   }
-  if (n_cl > 1 && warp < 4) cluster_sync_all();        // the meeting of the exchange
+  if (n_cl > 1) {
+    if (warp >= 4) exchange_in_cluster(warp & 3, (warp - 4) >> 2);
+    else cluster_sync_all();                           // the meeting of the exchange
+  }
   if (threadIdx.x == G3_THREADS - 128) gm_mark_ns(p.trace, 106);
   tc_fence_before();
   __syncthreads();
@@ -526,21 +632,47 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   if (warp == 1) tmem_dealloc_pair(tmem_base, G2_TMEM_COLS);
 }
 
-static size_t gemm3_smem_bytes() { return 1024 + (size_t)G3_STAGES * G3_X_BYTES + G3_BAR_BYTES + G3_TURN_BYTES; }
+// How a launch lays its shared memory out: the stages that TMEM leaves room for beside a tile's accumulator, fewer (no less
+// than four) where the act-order table of G groups needs the room; a place to turn over for every block of a tile where
+// that fits.  bytes = 0: no room.
+struct Gemm3Layout { int stages, area, turn_blocks; size_t bytes; };
+static Gemm3Layout gemm3_layout(int tile_rows, int G, bool act, int cluster) {
+  Gemm3Layout l = {0, 0, 0, 0};
+  if (!act && tile_rows <= 256) {
+    l.stages = G3_MAX_STAGES; l.area = G3_PLAIN_AREA; l.turn_blocks = 8;
+    l.bytes = 1024 + (size_t)G3_PLAIN_AREA + G3_BAR_BYTES + 4 * 8 * G3_TURN_BLOCK;
+    return l;
+  }
+  const int nb = tile_rows / 32, x_bytes = tile_rows * GM_TILE_C, table = act ? G * 512 : 0, limit = 227 * 1024;
+  const int sums = cluster > 1 ? 4 * (nb - nb / cluster) * 4096 : 0;
+  for (int s = (G2_TMEM_COLS - tile_rows) / 32 < G3_MAX_STAGES ? (G2_TMEM_COLS - tile_rows) / 32 : G3_MAX_STAGES; s >= 4; --s) {
+    const int used = s * x_bytes + table > sums ? s * x_bytes + table : sums;
+    l.stages = s;
+    l.area = (used + 1023) & ~1023;
+    const int rest = 1024 + G3_BAR_BYTES + (act ? G3_OFFS_BYTES : 0);
+    for (int full = 1; full >= 0; --full) {
+      l.turn_blocks = full ? nb : 0;
+      l.bytes = (size_t)rest + l.area + (size_t)(full ? 4 * nb : 4 * G3_GROUPS + 4) * G3_TURN_BLOCK;
+      if (l.bytes <= (size_t)limit) return l;
+    }
+  }
+  l.bytes = 0;
+  return l;
+}
 
-// How many clusters of `n` pairs can be resident at once on this device (asked once).
+// How many clusters of `n` pairs can be resident at once on this device (asked once, for the most shared memory there is).
 static int gemm3_clusters(int dev, int n) {
   static std::atomic<int> known[64][G3_MAX_CLUSTER + 1];           // the answer and one
   const int v = known[dev][n].load(std::memory_order_relaxed);
   if (v) return v - 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * n * 64); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = gemm3_smem_bytes();
+  cfg.gridDim = dim3(2 * n * 64); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = 227 * 1024;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2 * n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
   int nc = 0;
-  if (cudaOccupancyMaxActiveClusters(&nc, (const void*)q4_gemm3_kernel<true>, &cfg) != cudaSuccess || nc < 0) { cudaGetLastError(); nc = 0; }
+  if (cudaOccupancyMaxActiveClusters(&nc, (const void*)q4_gemm3_kernel<true, false, false>, &cfg) != cudaSuccess || nc < 0) { cudaGetLastError(); nc = 0; }
   known[dev][n].store(nc + 1, std::memory_order_relaxed);
   return nc;
 }

@@ -703,3 +703,57 @@ def test_tiles_of_every_height(K, N, M):
 def test_pairs_of_a_tile_add_up_in_their_cluster(K, N, M):
     """Two to four pairs a tile, in clusters of up to eight CTAs; contractions whose parts are not equal."""
     test_short_prompts_cut_between_pairs(K, N, M)
+
+
+def _product_with_everything(layer, M, seed):
+    """A product with bias, skip path and a rank-16 term against fp64 of the reconstructed weights (fp32 sums rounded to
+    fp16, twice with the skip path: 2 * 2^-11), three times the same bits."""
+    K, N = layer.qweight.shape[0] * 8, layer.qweight.shape[1]
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.randn(M, K, generator=gen, device=DEV).half()
+    bias = torch.randn(N, generator=gen, device=DEV).half()
+    res = torch.randn(M, N, generator=gen, device=DEV).half()
+    u = torch.zeros(M, 64, dtype=torch.float16, device=DEV)
+    u[:, :16] = torch.randn(M, 16, generator=gen, device=DEV).half()
+    b = (torch.randn(N, 16, generator=gen, device=DEV) * 0.05).half()
+    w = torch.empty((K, N), dtype=torch.float16, device=DEV)
+    quant_cuda.vecquant4recons_v2(layer.qweight, w, layer.scales, layer.qzeros, layer.g_idx)
+    want = x.double() @ w.double() + bias.double() + u[:, :16].double() @ b.double().t() + res.double()
+    runs = []
+    for _ in range(3):
+        full = torch.full((M + 2, N), -9.0, dtype=torch.float16, device=DEV)
+        quant_cuda.gemm(x, layer.qweight, full[1:M + 1], layer.scales, layer.qzeros, layer.g_idx, bias=bias, lora_u=u, lora_w=b, residual=res)
+        assert bool((full[0] == -9.0).all()) and bool((full[M + 1] == -9.0).all())
+        runs.append(full[1:M + 1])
+    assert float((runs[0].double() - want).norm() / want.norm()) <= 1e-3
+    assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+    assert quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,M", [(512, 512, 258), (512, 256, 352), (512, 512, 384), (512, 256, 385), (512, 256, 700), (512, 256, 769),
+                                   (4096, 4096, 333), (2304, 256, 300), (4096, 11008, 333), (1024, 9984, 1152)])
+def test_tall_tiles(K, N, M):
+    """Tiles of more than 256 rows: two MMAs on one dequantised operand, whole, in clusters and in runs."""
+    _product_with_everything(synth.make_layer(K, N, 128, act_order=False, seed=K + M).to(DEV), M, M)
+
+
+@pytest.mark.parametrize("K,N,g,M", [(256, 256, 128, 17), (512, 512, 64, 77), (512, 256, 32, 256), (512, 256, 128, 257), (1024, 512, 128, 333),
+                                     (512, 256, 128, 384), (512, 512, 128, 600), (2304, 512, 128, 100), (4096, 4096, 128, 333), (4096, 11008, 128, 40),
+                                     (8192, 256, 32, 350), (8192, 256, 32, 200), (4096, 4096, 64, 768)])    # 256 groups: four stages
+def test_act_order_with_weights_in_tensor_memory(K, N, g, M):
+    _product_with_everything(synth.make_layer(K, N, g, act_order=True, seed=K + M).to(DEV), M, M)
+
+
+@pytest.mark.parametrize("kind", ["one group", "few rows in some groups", "sequential in 32s"])
+def test_act_order_forward_takes_any_order_of_groups(kind):
+    K, N, G = 1024, 512, 8
+    layer = synth.make_layer(K, N, K // G, act_order=True, seed=5).to(DEV)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    if kind == "one group":
+        layer.g_idx.fill_(G - 1)
+    elif kind == "few rows in some groups":
+        layer.g_idx.copy_((torch.rand(K, generator=gen, device=DEV) ** 4 * G).to(torch.int32))
+    else:
+        layer.g_idx.copy_((torch.arange(K, device=DEV) // 32 % G).to(torch.int32))
+    for M in (40, 300):
+        _product_with_everything(layer, M, M)
