@@ -256,9 +256,54 @@ def _fuse_gate_up(model: nn.Module) -> int:
     return done
 
 
+class _CausalLoss(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, labels, seq, ignore):
+        V = logits.shape[-1]
+        rows = logits.numel() // V
+        f32 = dict(dtype=torch.float32, device=logits.device)
+        stats, row_loss = torch.empty((rows, 2), **f32), torch.empty(rows, **f32)
+        loss, count = torch.empty((), **f32), torch.empty((), **f32)
+        with _lib.on_device(logits.device):
+            _lib.check(_lib.lib().q4_causal_loss_fwd(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), row_loss.data_ptr(), loss.data_ptr(),
+                                                     count.data_ptr(), rows, V, seq, ignore, int(logits.dtype == torch.bfloat16), _lib.stream_of(logits)), "causal_loss")
+        ctx.save_for_backward(logits, labels, stats, count)
+        ctx.seq, ctx.ignore = seq, ignore
+        return loss
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_loss):
+        logits, labels, stats, count = ctx.saved_tensors
+        V = logits.shape[-1]
+        g = grad_loss.float()
+        grad = torch.empty_like(logits)
+        with _lib.on_device(logits.device):
+            _lib.check(_lib.lib().q4_causal_loss_bwd(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), g.data_ptr(), count.data_ptr(),
+                                                     grad.data_ptr(), logits.numel() // V, V, ctx.seq, ctx.ignore,
+                                                     int(logits.dtype == torch.bfloat16), _lib.stream_of(logits)), "causal_loss_bwd")
+        return grad, None, None, None
+
+
+def causal_lm_loss(stock):
+    """The loss function of a transformers causal language model (``loss(logits, labels, vocab_size, ...)``: the mean cross
+    entropy of the next tokens, in fp32) on the library's kernels for 16-bit logits on a GPU; ``stock`` for anything else."""
+    def loss(logits, labels, vocab_size, num_items_in_batch=None, ignore_index=-100, shift_labels=None, **kwargs):
+        classes = labels if shift_labels is None else shift_labels
+        if (num_items_in_batch is None and not kwargs and isinstance(logits, torch.Tensor) and isinstance(classes, torch.Tensor)
+                and type(logits) is torch.Tensor and type(classes) is torch.Tensor and logits.is_cuda and classes.device == logits.device
+                and logits.dtype in (torch.float16, torch.bfloat16) and classes.dtype is torch.int64 and logits.dim() >= 2
+                and logits.shape[-1] == vocab_size and vocab_size % 8 == 0 and classes.shape == logits.shape[:-1] and 0 < classes.numel() < 2 ** 31
+                and logits.is_contiguous() and classes.is_contiguous() and logits.data_ptr() % 16 == 0 and _lib.nobody_watches()):
+            return _CausalLoss.apply(logits, classes, classes.shape[-1] if shift_labels is None else 0, int(ignore_index))
+        return stock(logits, labels, vocab_size, num_items_in_batch=num_items_in_batch, ignore_index=ignore_index, shift_labels=shift_labels, **kwargs)
+    loss.stock = stock
+    return loss
+
+
 def patch_llama(model: nn.Module, fuse_gate_up: bool = False) -> nn.Module:
-    """Route the RMSNorms, the SwiGLU products, the rotary embedding and the skip-path adds of a transformers LLaMA
-    through the fused operators above.  The norm, MLP and decoder-layer modules are patched per instance; the rotary
+    """Route the RMSNorms, the SwiGLU products, the rotary embedding, the skip-path adds and the loss of a transformers
+    LLaMA through the fused operators above.  The norm, MLP and decoder-layer modules are patched per instance; the rotary
     function is a module-level name of ``transformers.models.llama.modeling_llama`` and is replaced there (the
     replacement computes exactly the stock expression whenever the fused path does not apply).  Call it before
     anything wraps the layers' ``forward`` (gradient checkpointing).  ``fuse_gate_up`` also concatenates the gate
@@ -276,4 +321,7 @@ def patch_llama(model: nn.Module, fuse_gate_up: bool = False) -> nn.Module:
         elif isinstance(mod, ml.LlamaMLP) and type(getattr(mod, "act_fn", None)).__name__ in ("SiLU", "SiLUActivation"):
             mod.forward = (lambda x, _m=mod: _m.down_proj(swiglu(_m.gate_proj(x), _m.up_proj(x))))
     ml.apply_rotary_pos_emb = apply_rotary_pos_emb
+    for mod in model.modules():
+        if isinstance(mod, ml.LlamaForCausalLM) and not hasattr(mod.loss_function, "stock"):
+            mod.loss_function = causal_lm_loss(mod.loss_function)
     return model

@@ -261,6 +261,19 @@ int q4_lora_project(const void* x, const void* w, void* out, int M, int C, int r
 /* dst[i] = src[i] rounded from bf16 to fp16 (to_half != 0) or from fp16 to bf16; n elements, pointers 16-byte aligned:
  * the activations of a bf16 step on their way into and out of an adapted layer. */
 int q4_cast16(const void* src, void* dst, size_t n, int to_half, q4_stream_t stream);
+
+/* The loss of a causal language model over 16-bit logits [rows, V] (fp16, or bf16 with `bf16`): the mean cross entropy of the
+ * rows that have a class, computed in fp32 as `cross_entropy(logits.float(), labels, ignore_index)` computes it (what
+ * LlamaForCausalLM returns with labels), without an fp32 copy of the logits.  labels int64 [rows]; with seq > 0 the rows are
+ * sequences of `seq` tokens and a row's class is the next token's label (the last token of a sequence has none), with
+ * seq = 0 its own.  Label `ignore`: no class; a label outside 0..V-1 makes the loss NaN.  fwd fills stats [rows][2], row_loss
+ * [rows], *loss and *count (the number of rows with a class); bwd writes grad [rows, V] in the logits' type from the
+ * gradient of the loss at *grad_loss.  V % 8 == 0, logits and grad 16-byte aligned.  No reference counterpart (its
+ * trainer runs the framework's kernels). */
+int q4_causal_loss_fwd(const void* logits, const long long* labels, float* stats, float* row_loss, float* loss, float* count, int rows,
+                       int V, int seq, long long ignore, int bf16, q4_stream_t stream);
+int q4_causal_loss_bwd(const void* logits, const long long* labels, const float* stats, const float* grad_loss, const float* count,
+                       void* grad, int rows, int V, int seq, long long ignore, int bf16, q4_stream_t stream);
 int q4_lora_grads(const void* v, const void* x, float* d_a, int K, const void* dy, const void* u, float* d_b, int N,
                   int M, int r, q4_stream_t stream);
 

@@ -218,3 +218,71 @@ def test_swiglu_fused_is_no_opaque_call_where_torch_watches():
                 with pytest.raises(Exception, match="jvp"):
                     fused_ops.swiglu_fused(torch.autograd.forward_ad.make_dual(a, b))
             assert torch.equal(fused_ops.swiglu_fused(a), fused_ops._SwiGLUFused.apply(a))
+
+
+def _stock_loss(logits, labels, vocab_size, num_items_in_batch=None, ignore_index=-100, shift_labels=None, **kwargs):
+    if shift_labels is None:
+        shift_labels = torch.nn.functional.pad(labels, (0, 1), value=ignore_index)[..., 1:]
+    return torch.nn.functional.cross_entropy(logits.float().reshape(-1, vocab_size), shift_labels.reshape(-1), ignore_index=ignore_index)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,T,V,shifted", [(1, 1, 8, True), (2, 5, 32000, False), (3, 7, 4104, False), (1, 33, 128256, True), (4, 64, 4096, False)])
+def test_causal_loss_matches_stock(B, T, V, shifted, dtype):
+    """The mean cross entropy in fp32 and its gradient rounded once to the logits' type: sums of up to V exponentials in
+    another order (V * 2^-24 at the very most, as for the framework's own), and the one rounding."""
+    gen = torch.Generator(device=DEV).manual_seed(V + T)
+    logits = (torch.randn((B, T, V), generator=gen, device=DEV) * 4).to(dtype).requires_grad_(True)
+    labels = torch.randint(0, V, (B, T), generator=gen, device=DEV)
+    if T > 2:
+        labels[0, 2] = -100
+    kw = dict(shift_labels=labels) if shifted else {}
+    fused = fused_ops.causal_lm_loss(lambda *a, **k: (_ for _ in ()).throw(AssertionError("the stock loss ran")))
+    got = fused(logits, labels, V, **kw)
+    assert got.dtype == torch.float32 and got.dim() == 0
+    (got * 1024).backward()
+    dgot, logits.grad = logits.grad, None
+    want = _stock_loss(logits, labels, V, **kw)
+    (want * 1024).backward()
+    if not shifted and T == 1:
+        return
+    assert abs(float(got.detach()) - float(want.detach())) <= 1e-6 * abs(float(want.detach())) + 1e-6
+    l64 = logits.detach().double().requires_grad_(True)
+    loss64 = torch.nn.functional.cross_entropy(l64.reshape(-1, V), (labels if shifted else torch.nn.functional.pad(labels, (0, 1), value=-100)[..., 1:]).reshape(-1))
+    (loss64 * 1024).backward()
+    assert rel(dgot, l64.grad) <= rel(logits.grad, l64.grad) * 1.02 + 1e-6
+    assert float((dgot.float() - logits.grad.float()).abs().max()) <= 2 ** (-10 if dtype == torch.float16 else -7) * float(logits.grad.float().abs().max())
+
+
+def test_causal_loss_at_the_edges():
+    """No row with a class, infinities and NaN among the logits: what the framework's loss gives; the loss may be written in
+    place before its backward; a second derivative is refused; other calls go to the stock loss."""
+    V = 64
+    fused = fused_ops.causal_lm_loss(_stock_loss)
+    none = torch.full((1, 4), -100, device=DEV)
+    x = torch.randn((1, 4, V), device=DEV).half().requires_grad_(True)
+    assert torch.isnan(fused(x, none, V))
+    for special in (float("inf"), float("-inf"), float("nan")):
+        for where in (3, slice(None)):
+            y = torch.randn((1, 4, V), device=DEV).half()
+            y[0, 1, where] = special
+            labels = torch.tensor([[1, 2, 3, 4]], device=DEV)
+            a, b = fused(y, labels, V), _stock_loss(y, labels, V)
+            assert torch.allclose(a, b, rtol=0, atol=1e-5, equal_nan=True), (special, where, a, b)
+    labels = torch.randint(0, V, (1, 4), device=DEV)
+    loss = fused(x, labels, V)
+    loss /= 2
+    loss.backward()
+    ref = x.detach().clone().requires_grad_(True)
+    (_stock_loss(ref, labels, V) / 2).backward()
+    assert rel(x.grad, ref.grad) <= 1e-3
+    loss = fused(x, labels, V)
+    (g,) = torch.autograd.grad(loss, x, create_graph=True)
+    with pytest.raises(RuntimeError):
+        g.sum().backward()
+    seen = []
+    spy = fused_ops.causal_lm_loss(lambda *a, **k: seen.append(1) or _stock_loss(*a, **k))
+    for args, kw in (((x.float(), labels, V), {}), ((x, labels, V), dict(num_items_in_batch=torch.tensor(4, device=DEV))),
+                     ((x.transpose(0, 1).contiguous().transpose(0, 1), labels, V), dict(label_smoothing=0.0)), ((x.cpu(), labels.cpu(), V), {})):
+        spy(*args, **kw)
+    assert len(seen) == 4
