@@ -133,8 +133,10 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t cta_addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
   return r;
 }
-// all threads of all CTAs of the cluster
+// all threads of all CTAs of the cluster.  (.aligned: a warp comes to it as one - a lane that ran a loop of its own meets the
+// others first, here and in named_bar_sync, instead of where the compiler happens to let it.)
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Arrive on an mbarrier of any CTA of the cluster (address from mapa_u32).  Default semantics
@@ -187,6 +189,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
