@@ -73,7 +73,7 @@ struct GemmParams {
   float* ws_partials;
   unsigned* ws_counters;
   const __half* zp_table;   // rn(s * (z+1)) for every [group, column], or null
-  int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32
+  int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32, above 256 of 64
   int cluster_pairs;        // weights-in-TMEM kernel: pairs of a cluster; more than one: they share a tile
   int area, turn_blocks;    // weights-in-TMEM kernel: layout of its shared memory
   int seq_shift;            // > 0: the caller promises g_idx[k] == k >> seq_shift (sequential groups of 2^seq_shift rows)
@@ -372,11 +372,13 @@ static long long gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_o
 // Tiles and pairs of the weights-in-TMEM kernel, by what a pair's work takes in stages of the contraction (256 rows, about
 // 0.28 us).  `room`: bytes of the workspace for partial sums.  tile_rows = 0: the act-order table does not fit.
 struct Gemm3Plan { int tile_rows, pairs, cluster; bool stream, act; double cost; Gemm3Layout layout; };
-static Gemm3Plan gemm3_plan(int M, int nout, int T, int P, int dev, int G, bool act, size_t room) {
+static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int G, bool act, size_t room) {
+  const int P = dev.sm_pairs;
   Gemm3Plan best = {};
   for (int m_tiles = (M + G3_MAX_ROWS - 1) / G3_MAX_ROWS; m_tiles <= (M + 255) / 256; ++m_tiles) {
     Gemm3Plan c = {};
     c.tile_rows = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+    if (c.tile_rows > 256) c.tile_rows = (c.tile_rows + 63) / 64 * 64;         // two MMAs of half the rows each: see idesc_f16
     c.cluster = 1;
     c.layout = gemm3_layout(c.tile_rows, G, act, 1);
     if (!c.layout.bytes) continue;
@@ -410,7 +412,7 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, int P, int dev, int G, bool 
       const int n_max = T > 32 || (nb <= 2 && T >= 16 + 8 * nb) ? T / 4 : 1;
       for (int n = T > 32 ? 2 : 3; n <= P / tiles && n <= n_max; ++n) {
         const Gemm3Layout l = n <= G3_MAX_CLUSTER ? gemm3_layout(c.tile_rows, G, act, n) : c.layout;
-        const bool cluster = n <= G3_MAX_CLUSTER && l.bytes && gemm3_clusters(dev, n) >= tiles;
+        const bool cluster = n <= G3_MAX_CLUSTER && l.bytes && dev.clusters[n] >= tiles;
         if (!cluster && !parts) continue;
         const double run = (double)((T + n - 1) / n) * unit;
         const double cut = cluster ? run + 2 + (n - 1) * (1.5 + 0.3 * nb) : run + 9 + 1.2 * nb + (n - 1) * (0.5 + 0.45 * nb);
@@ -432,43 +434,40 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, int P, int dev, int G, bool 
   return best;
 }
 
-static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, void* out, const void* scales,
-                       const int32_t* qzeros, const int32_t* g_idx, const void* bias, const void* lora_u,
-                       const void* lora_w, int lora_r, int M, int K, int N, int G, void* workspace, size_t workspace_bytes,
-                       q4_stream_t stream, bool swiglu = false, const void* zp_cached = nullptr, const void* residual = nullptr,
-                       int seq_groupsize = 0, bool one_group = false) {
-  // one_group: a layer of the first format - G = 1, the zero-term table given, neither qzeros nor g_idx
-  if (!act || !qweight || !out || !scales || (!one_group && (!qzeros || !g_idx))) return fail(Q4_E_BADARG, "gemm: null pointer");
-  const int gv = g_gemm_variant == 5 ? 0 : g_gemm_variant;
-  if (M <= 0 || K <= 0 || N <= 0 || G <= 0) return fail(Q4_E_BADARG, "gemm: M=%d K=%d N=%d G=%d", M, K, N, G);
-  if (K % 128 || N % 128) return fail(Q4_E_SHAPE, "gemm: K=%d and N=%d must be multiples of 128", K, N);
-  if (!aligned16(act) || !aligned16(qweight) || !aligned16(out) || !aligned16(scales) || !aligned16(g_idx))
-    return fail(Q4_E_ALIGN, "gemm: pointers must be 16-byte aligned");
-  if (lora_r < 0 || lora_r > 64) return fail(Q4_E_SHAPE, "gemm: low-rank width %d outside 0..64", lora_r);
-  if (lora_r > 0 && (!lora_u || !lora_w || !aligned16(lora_u) || !aligned16(lora_w)))
-    return fail(Q4_E_BADARG, "gemm: the low-rank term needs 16-byte aligned lora_u [M,64] and lora_w");
-  if (workspace && !aligned16(workspace)) return fail(Q4_E_ALIGN, "gemm: the workspace must be 16-byte aligned");
-  if (residual && (transpose || swiglu || !aligned16(residual))) return fail(Q4_E_BADARG, "gemm: a residual needs the plain forward and 16-byte alignment");
-  if (int e = check_device()) return e;
+// The sizes of a product and what its caller gives and promises: what the choice of a kernel goes by.
+struct GemmRequest {
+  bool transpose, swiglu, one_group, table;     // table: zero terms as a [G, N] table
+  int M, K, N, G, lora_r, seq_groupsize, variant;
+  size_t workspace_bytes;                       // 0: none
+};
+struct GemmChoice {
+  bool use_pair, use_tm, no_tables;
+  int mh, seq_shift, stages;                    // stages: of the pair kernel at this mh
+  Gemm3Plan plan3;
+};
+
+static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice* choice) {
+  const bool transpose = q.transpose, swiglu = q.swiglu, one_group = q.one_group;
+  const int M = q.M, K = q.K, N = q.N, G = q.G, gv = q.variant == 5 ? 0 : q.variant;
   const int contract = transpose ? N : K, nout = transpose ? K : N;
   // forward with the caller's zero-term table: scales and zero terms come from L2 as in the backward, and the
   // shared memory the tables would take goes to pipeline stages (CTA-pair kernel only)
-  const bool may_drop_tables = !transpose && zp_cached != nullptr;
+  const bool may_drop_tables = !transpose && q.table;
   int stages2 = gemm2_stages(transpose, G, 1), stages2w = gemm2_stages(transpose, G, 2);
   const int stages2_nt = may_drop_tables ? gemm2_stages(true, G, 1) : stages2, stages2w_nt = may_drop_tables ? gemm2_stages(true, G, 2) : stages2w;
   // the table is used where it buys a stage for both tile heights (or makes the pair kernel possible at all)
   // groups promised sequential (a power of two of at least 8 rows): the forward fetches a task's scales and zero terms
   // one task ahead with its packed words, so the table is taken whether or not it buys a stage
   int seq_shift = 0;
-  if (seq_groupsize >= 8 && (seq_groupsize & (seq_groupsize - 1)) == 0 && (long long)seq_groupsize * G >= K)
-    while ((1 << seq_shift) < seq_groupsize) ++seq_shift;
+  if (q.seq_groupsize >= 8 && (q.seq_groupsize & (q.seq_groupsize - 1)) == 0 && (long long)q.seq_groupsize * G >= K)
+    while ((1 << seq_shift) < q.seq_groupsize) ++seq_shift;
   const bool no_tables = transpose || (may_drop_tables && ((stages2_nt > stages2 && stages2w_nt > stages2w) || seq_shift > 0));
   if (no_tables && !transpose) { stages2 = stages2_nt; stages2w = stages2w_nt; }
   const bool pair_ok = nout % G2_TILE_N == 0 && stages2 > 0;
   const bool wide_ok = nout % G2_TILE_N == 0 && stages2w > 0;
   if ((gv == 2 && !pair_ok) || (gv == 3 && !wide_ok))
     return fail(Q4_E_SHAPE, "gemm: the CTA-pair kernel needs %d output columns to be a multiple of 256 and G=%d tables to fit", nout, G);
-  if (swiglu && (transpose || lora_r > 0 || !pair_ok || N % 256))
+  if (swiglu && (transpose || q.lora_r > 0 || !pair_ok || N % 256))
     return fail(Q4_E_SHAPE, "gemm: the fused gate_up product needs the CTA-pair kernel (N=%d a multiple of 256, G=%d tables that fit) and no low-rank term", N, G);
   if (one_group && !pair_ok) return fail(Q4_E_SHAPE, "gemm: a layer of the first format needs %d output columns to be a multiple of 256", nout);
   const bool use_pair = (pair_ok && (gv != 1 || one_group)) || gv == 3 || swiglu;
@@ -478,9 +477,9 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     return fail(Q4_E_SHAPE, "gemm: the weights-in-TMEM kernel takes the forward of a layer with N=%d a multiple of 256, its zero-term table and sequential groups of 64 rows or more", N);
   // 512-row tiles halve the dequant work per flop but leave fewer, larger tiles to deal: take the
   // form the estimate favours
-  const int P_est = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
-  const size_t zp_need = transpose && !zp_cached ? (((size_t)G * N * sizeof(__half) + 255) & ~(size_t)255) : 0;
-  auto ws_ok_for = [&](int m) { return workspace && workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + zp_need + (size_t)P_est * m * Q4_GEMM_WS_SLICE_BYTES; };
+  const int P_est = dev.sm_pairs;
+  const size_t zp_need = transpose && !q.table ? (((size_t)G * N * sizeof(__half) + 255) & ~(size_t)255) : 0;
+  auto ws_ok_for = [&](int m) { return q.workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + zp_need + (size_t)P_est * m * Q4_GEMM_WS_SLICE_BYTES; };
   int mh = 1;
   if (use_pair && gv == 3) mh = 2;
   else if (use_pair && gv == 0 && wide_ok && M > 256) {
@@ -490,24 +489,12 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     if (e2 < e1) mh = 2;
   }
   // The weights-in-TMEM kernel: sequential layers whose groups are promised (tm_ok), and any other by its act-order form
-  const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && gv == 0 && g_gemm_variant != 5 && !one_group;
-  bool use_tm = tm_ok && use_pair && (gv == 4 || (gv == 0 && g_gemm_variant != 5));
+  const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && gv == 0 && q.variant != 5 && !one_group;
+  bool use_tm = tm_ok && use_pair && (gv == 4 || (gv == 0 && q.variant != 5));
   Gemm3Plan plan3 = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
   if (use_tm || tm_act) {
-    static std::atomic<bool> tm_attr_done[64];
-    if (!tm_attr_done[dev].load(std::memory_order_acquire)) {
-      for (const void* f3 : {(const void*)q4_gemm3_kernel<false, false, false>, (const void*)q4_gemm3_kernel<true, false, false>,
-                             (const void*)q4_gemm3_kernel<false, true, false>, (const void*)q4_gemm3_kernel<true, true, false>,
-                             (const void*)q4_gemm3_kernel<false, false, true>, (const void*)q4_gemm3_kernel<true, false, true>,
-                             (const void*)q4_gemm3_kernel<false, true, true>, (const void*)q4_gemm3_kernel<true, true, true>})
-        if (int e = check_cuda(cudaFuncSetAttribute(f3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "gemm smem attribute")) return e;
-      tm_attr_done[dev].store(true, std::memory_order_release);
-    }
-    const size_t room = workspace && workspace_bytes > Q4_GEMM_WS_COUNTER_BYTES ? workspace_bytes - Q4_GEMM_WS_COUNTER_BYTES : 0;
-    plan3 = gemm3_plan(M, nout, contract / GM_TILE_C, P_est, dev, G, !use_tm, room);
+    const size_t room = q.workspace_bytes > Q4_GEMM_WS_COUNTER_BYTES ? q.workspace_bytes - Q4_GEMM_WS_COUNTER_BYTES : 0;
+    plan3 = gemm3_plan(M, nout, contract / GM_TILE_C, dev, G, !use_tm, room);
     plan3.act = !use_tm;
     use_tm = plan3.tile_rows > 0;
     if (use_tm && gv == 0 && !(tm_ok && M <= 1024)) {
@@ -529,9 +516,65 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     }
   }
   if (use_tm) mh = 1;
+  *choice = {use_pair, use_tm, no_tables, mh, seq_shift, mh == 2 ? stages2w : stages2, plan3};
+  return Q4_OK;
+}
+
+// Whole tiles per pair, round after round - or, when the last round would leave pairs idle for
+// longer than the exchange of partial sums costs (about a dozen stages), all tiles x stages as one
+// sequence cut into equal runs.
+struct Gemm2Deal { int pairs; bool stream; };
+static Gemm2Deal gemm2_deal(int M, int nout, int T, int P, int mh, bool ws_ok) {
+  const int n_tiles = (nout / G2_TILE_N) * ((M + 256 * mh - 1) / (256 * mh));
+  Gemm2Deal d = {n_tiles < P ? n_tiles : P, false};
+  gemm2_estimate(M, nout, T, P, mh, ws_ok, &d.stream);
+  if (d.stream) {
+    // Fewer tiles than half the pairs: take a whole number of pairs per tile, so that every tile is shared by the
+    // same number of pairs in equal parts and a pair has one piece of one tile.  Cut into P runs the pieces fall
+    // anywhere, a pair's run can lie inside one tile, and the tile's reducer then waits for a contributor that ends
+    // when it does (32 tiles x 172 stages at 1024 rows: 90.2 us on 74 pairs, 78.6 us on 64).
+    const int per_tile = n_tiles > 0 ? P / n_tiles : 0;
+    d.pairs = per_tile >= 2 ? n_tiles * per_tile : P;
+  }
+  return d;
+}
+
+static int sm_pairs() { return sm_count() / 2 > 0 ? sm_count() / 2 : 1; }
+
+static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, void* out, const void* scales,
+                       const int32_t* qzeros, const int32_t* g_idx, const void* bias, const void* lora_u,
+                       const void* lora_w, int lora_r, int M, int K, int N, int G, void* workspace, size_t workspace_bytes,
+                       q4_stream_t stream, bool swiglu = false, const void* zp_cached = nullptr, const void* residual = nullptr,
+                       int seq_groupsize = 0, bool one_group = false) {
+  // one_group: a layer of the first format - G = 1, the zero-term table given, neither qzeros nor g_idx
+  if (!act || !qweight || !out || !scales || (!one_group && (!qzeros || !g_idx))) return fail(Q4_E_BADARG, "gemm: null pointer");
+  if (M <= 0 || K <= 0 || N <= 0 || G <= 0) return fail(Q4_E_BADARG, "gemm: M=%d K=%d N=%d G=%d", M, K, N, G);
+  if (K % 128 || N % 128) return fail(Q4_E_SHAPE, "gemm: K=%d and N=%d must be multiples of 128", K, N);
+  if (!aligned16(act) || !aligned16(qweight) || !aligned16(out) || !aligned16(scales) || !aligned16(g_idx))
+    return fail(Q4_E_ALIGN, "gemm: pointers must be 16-byte aligned");
+  if (lora_r < 0 || lora_r > 64) return fail(Q4_E_SHAPE, "gemm: low-rank width %d outside 0..64", lora_r);
+  if (lora_r > 0 && (!lora_u || !lora_w || !aligned16(lora_u) || !aligned16(lora_w)))
+    return fail(Q4_E_BADARG, "gemm: the low-rank term needs 16-byte aligned lora_u [M,64] and lora_w");
+  if (workspace && !aligned16(workspace)) return fail(Q4_E_ALIGN, "gemm: the workspace must be 16-byte aligned");
+  if (residual && (transpose || swiglu || !aligned16(residual))) return fail(Q4_E_BADARG, "gemm: a residual needs the plain forward and 16-byte alignment");
+  if (int e = check_device()) return e;
+  const int contract = transpose ? N : K, nout = transpose ? K : N;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  GemmResident resident = {sm_pairs(), {}};
+  if (!transpose && !swiglu)
+    if (int e = gemm3_resident(dev, &resident)) return e;
+  GemmChoice choice;
+  const GemmRequest request = {transpose, swiglu, one_group, zp_cached != nullptr, M, K, N, G, lora_r, seq_groupsize, g_gemm_variant,
+                               workspace ? workspace_bytes : 0};
+  if (int e = gemm_choose(request, resident, &choice)) return e;
+  const bool use_pair = choice.use_pair, use_tm = choice.use_tm, no_tables = choice.no_tables;
+  const int mh = choice.mh, seq_shift = choice.seq_shift;
+  const Gemm3Plan& plan3 = choice.plan3;
   int stages = GM_MAX_STAGES;
   while (stages > 2 && gemm_smem_bytes(transpose, G, stages) > 227 * 1024) --stages;
-  if (use_pair) stages = mh == 2 ? stages2w : stages2;
+  if (use_pair) stages = choice.stages;
   const size_t smem = use_pair ? gemm2_smem_bytes(no_tables, G, stages, mh) : gemm_smem_bytes(transpose, G, stages);
   if (smem > 227 * 1024) return fail(Q4_E_SHAPE, "gemm: scale tables for G=%d groups do not fit shared memory", G);
 
@@ -597,8 +640,6 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
     swiglu_attr_done[dev] = true;
   }
   if (use_pair) {
-    const int tile_m = 256 * mh;
-    const int n_tiles = (nout / G2_TILE_N) * ((M + tile_m - 1) / tile_m);
     const int P = max_pairs[tr][dev], T = p.n_contract_tiles;
     unsigned char* ws = (unsigned char*)workspace;
     size_t ws_off = Q4_GEMM_WS_COUNTER_BYTES;
@@ -636,20 +677,9 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       if (e3) return e3;
       return check_cuda(cudaGetLastError(), "gemm launch");
     }
-    // Whole tiles per pair, round after round - or, when the last round would leave pairs idle for
-    // longer than the exchange of partial sums costs (about a dozen stages), all tiles x stages as one
-    // sequence cut into equal runs.
-    bool stream = false;
-    int pairs = n_tiles < P ? n_tiles : P;
-    gemm2_estimate(M, nout, T, P, mh, ws && workspace_bytes >= ws_off + (size_t)P * mh * Q4_GEMM_WS_SLICE_BYTES, &stream);
-    if (stream) {
-      // Fewer tiles than half the pairs: take a whole number of pairs per tile, so that every tile is shared by the
-      // same number of pairs in equal parts and a pair has one piece of one tile.  Cut into P runs the pieces fall
-      // anywhere, a pair's run can lie inside one tile, and the tile's reducer then waits for a contributor that ends
-      // when it does (32 tiles x 172 stages at 1024 rows: 90.2 us on 74 pairs, 78.6 us on 64).
-      const int per_tile = n_tiles > 0 ? P / n_tiles : 0;
-      pairs = per_tile >= 2 ? n_tiles * per_tile : P;
-    }
+    const Gemm2Deal deal = gemm2_deal(M, nout, T, P, mh, ws && workspace_bytes >= ws_off + (size_t)P * mh * Q4_GEMM_WS_SLICE_BYTES);
+    const bool stream = deal.stream;
+    const int pairs = deal.pairs;
     const int f = stream ? 2 : 1;
     p.ws_partials = (float*)(ws + ws_off);
     p.ws_counters = (unsigned*)ws;
@@ -746,6 +776,38 @@ extern "C" int q4_gemm_fwd_v1(const void* x, const int32_t* qweight, void* y, co
   while (group < K) group <<= 1;
   return gemm_launch(false, x, qweight, y, scales, nullptr, nullptr, bias, nullptr, nullptr, 0, M, K, N, 1, workspace, workspace_bytes, stream,
                      false, zeros, residual, group, true);
+}
+
+extern "C" int q4_gemm_plan(int transpose, int M, int K, int N, int G, int sequential_groupsize, int has_table, size_t workspace_bytes,
+                            const int* resident, int* out) {
+  if (!out) return fail(Q4_E_BADARG, "gemm_plan: null pointer");
+  if (M <= 0 || K <= 0 || N <= 0 || G <= 0) return fail(Q4_E_BADARG, "gemm_plan: M=%d K=%d N=%d G=%d", M, K, N, G);
+  if (K % 128 || N % 128) return fail(Q4_E_SHAPE, "gemm_plan: K=%d and N=%d must be multiples of 128", K, N);
+  GemmResident r = {0, {}};
+  if (resident) {
+    r.sm_pairs = resident[0];
+    for (int n = 1; n <= G3_MAX_CLUSTER; ++n) r.clusters[n] = resident[n];
+    if (r.sm_pairs <= 0) return fail(Q4_E_BADARG, "gemm_plan: %d pairs", r.sm_pairs);
+  } else {
+    if (int e = check_device()) return e;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    r.sm_pairs = sm_pairs();
+    if (int e = gemm3_resident(dev < 0 || dev >= 64 ? 0 : dev, &r)) return e;
+  }
+  GemmChoice c;
+  if (int e = gemm_choose({transpose != 0, false, false, has_table != 0, M, K, N, G, 0, has_table ? sequential_groupsize : 0, g_gemm_variant, workspace_bytes}, r, &c)) return e;
+  const int contract = transpose ? N : K, nout = transpose ? K : N;
+  out[0] = !c.use_pair ? 1 : c.use_tm ? 4 : 1 + c.mh;
+  if (c.use_tm) {
+    out[1] = c.plan3.tile_rows; out[2] = c.plan3.pairs; out[3] = c.plan3.cluster; out[4] = c.plan3.stream; out[5] = c.plan3.act;
+  } else if (c.use_pair) {
+    const Gemm2Deal d = gemm2_deal(M, nout, contract / GM_TILE_C, r.sm_pairs, c.mh, workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + (size_t)r.sm_pairs * c.mh * Q4_GEMM_WS_SLICE_BYTES);
+    out[1] = 256 * c.mh; out[2] = d.pairs; out[3] = 1; out[4] = d.stream; out[5] = 0;
+  } else {
+    out[1] = GM_TILE_M; out[2] = 0; out[3] = 1; out[4] = 0; out[5] = 0;
+  }
+  return Q4_OK;
 }
 
 extern "C" int q4_gemm_set_variant(int variant) {

@@ -17,8 +17,8 @@
 //   columns up row by row: 333 rows of 5120 x 5120 take 43 us there and 28 here, 77 rows 32 and 22.)
 //
 // Tiles follow the rows: as many as of 384 or 256 rows, whichever takes less time (gemm3_plan), all of one height, a
-// multiple of 32.  77 rows are one tile of 96 and 333 one of 352 - two MMAs of 176 on the same dequantised operand (TALL),
-// which used to be dequantised for two tiles of 256: 333 rows of 5120 x 15360 57 -> 43 us, of 5120 x 27648 93 -> 81 us.
+// multiple of 32 up to 256 and of 64 above (MMAs with A in TMEM have N in steps of 32).  77 rows are one tile of 96 and 333
+// one of 384 - two MMAs of 192 on the same dequantised operand (TALL), which used to be dequantised for two tiles of 256.
 // TMEM (512 columns): accumulator [128 lanes = output columns][columns = rows of x] fp32, and four to eight operand
 // stages of 32 columns (lane = output column, column c of a stage = contraction elements 2c, 2c+1 as a half2).
 // Roles (640 threads per CTA): warp 0 TMA producer of this CTA's half of the activation rows; warp 1 owns TMEM, its elected
@@ -115,9 +115,8 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   extern __shared__ unsigned char smem_raw[];
   pdl_launch_dependents();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  unsigned char* stages = smem;
   const int S = ACT || TALL ? p.stages : G3_MAX_STAGES;
-  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32
+  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32 (TALL: of 64)
   constexpr int nh = TALL ? 2 : 1;                     // MMAs per 16 contraction elements
   const int HR = TR / nh;                              // and rows of each
   constexpr bool PLAIN = !ACT && !TALL;                // one layout for all: stages of 128 rows, a place to turn every block over
@@ -660,21 +659,32 @@ static Gemm3Layout gemm3_layout(int tile_rows, int G, bool act, int cluster) {
   return l;
 }
 
-// How many clusters of `n` pairs can be resident at once on this device (asked once, for the most shared memory there is).
-static int gemm3_clusters(int dev, int n) {
+// How many pairs the device's SMs make, and how many clusters of 1 .. G3_MAX_CLUSTER pairs of this kernel it holds at once.
+struct GemmResident { int sm_pairs, clusters[G3_MAX_CLUSTER + 1]; };
+
+// Asked once per device, for the most shared memory there is (which the kernel's forms are allowed here).
+static int gemm3_resident(int dev, GemmResident* r) {
   static std::atomic<int> known[64][G3_MAX_CLUSTER + 1];           // the answer and one
-  const int v = known[dev][n].load(std::memory_order_relaxed);
-  if (v) return v - 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * n * 64); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = 227 * 1024;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2 * n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  int nc = 0;
-  if (cudaOccupancyMaxActiveClusters(&nc, (const void*)q4_gemm3_kernel<true, false, false>, &cfg) != cudaSuccess || nc < 0) { cudaGetLastError(); nc = 0; }
-  known[dev][n].store(nc + 1, std::memory_order_relaxed);
-  return nc;
+  if (!known[dev][G3_MAX_CLUSTER].load(std::memory_order_acquire)) {
+    for (const void* f3 : {(const void*)q4_gemm3_kernel<false, false, false>, (const void*)q4_gemm3_kernel<true, false, false>,
+                           (const void*)q4_gemm3_kernel<false, true, false>, (const void*)q4_gemm3_kernel<true, true, false>,
+                           (const void*)q4_gemm3_kernel<false, false, true>, (const void*)q4_gemm3_kernel<true, false, true>,
+                           (const void*)q4_gemm3_kernel<false, true, true>, (const void*)q4_gemm3_kernel<true, true, true>})
+      if (int e = check_cuda(cudaFuncSetAttribute(f3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "gemm smem attribute")) return e;
+    for (int n = 1; n <= G3_MAX_CLUSTER; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2 * n * 64); cfg.blockDim = dim3(G3_THREADS); cfg.dynamicSmemBytes = 227 * 1024;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 2 * n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      cfg.attrs = at; cfg.numAttrs = 1;
+      int nc = 0;
+      if (cudaOccupancyMaxActiveClusters(&nc, (const void*)q4_gemm3_kernel<true, false, false>, &cfg) != cudaSuccess || nc < 0) { cudaGetLastError(); nc = 0; }
+      known[dev][n].store(nc + 1, std::memory_order_release);
+    }
+  }
+  for (int n = 1; n <= G3_MAX_CLUSTER; ++n) r->clusters[n] = known[dev][n].load(std::memory_order_acquire) - 1;
+  return Q4_OK;
 }
 
 }  // namespace q4

@@ -81,6 +81,8 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo
   return d;
 }
 // Instruction descriptor for kind::f16: D fp32, A/B fp16, A K-major, B K-major or MN-major, M x N.
+// N of a CTA pair's MMA (cta_group::2, M = 256): 16 .. 256 in steps of 16 with A in shared memory, 32 .. 256 in steps of 32 with
+// A in tensor memory - the forms that CUTLASS's SM100_MMA_F16BF16_2x1SM_SS and _TS admit.
 __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, bool b_mn_major) {
   return (1u << 4) | (0u << 7) | (0u << 10) | (0u << 15) | ((b_mn_major ? 1u : 0u) << 16) |
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
