@@ -373,7 +373,9 @@ static long long gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_o
 // 0.28 us).  `room`: bytes of the workspace for partial sums.  tile_rows = 0: the act-order table does not fit.
 struct Gemm3Plan { int tile_rows, pairs, cluster; bool stream, act; double cost; Gemm3Layout layout; };
 static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int G, bool act, size_t room) {
-  const int P = dev.sm_pairs;
+  // Pairs that are resident at once: a pair that adds up a tile waits for others that must not be waiting for its SMs.  Where
+  // the device does not say, tiles are not cut by the workspace.
+  const int P = dev.clusters[1] > 0 && dev.clusters[1] < dev.sm_pairs ? dev.clusters[1] : dev.sm_pairs;
   Gemm3Plan best = {};
   for (int m_tiles = (M + G3_MAX_ROWS - 1) / G3_MAX_ROWS; m_tiles <= (M + 255) / 256; ++m_tiles) {
     Gemm3Plan c = {};
@@ -386,7 +388,7 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int
     const long long total = (long long)tiles * T;
     // a stage is bound by the MMAs from 256 rows on, below - act-order: below 435 - by the dequant warps
     const double least = act ? 1.7 : 1.0, unit = c.tile_rows > 256 * least ? c.tile_rows / 256.0 : least;
-    const bool parts = room >= (size_t)P * c.tile_rows * G2_TILE_N * sizeof(float) && total * P < (1ll << 32);
+    const bool parts = dev.clusters[1] > 0 && room >= (size_t)P * c.tile_rows * G2_TILE_N * sizeof(float) && total * P < (1ll << 32);
     // whole tiles, round after round
     c.pairs = tiles < P ? tiles : P;
     double cost = (double)((tiles + P - 1) / P) * T * unit;

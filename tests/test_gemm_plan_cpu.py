@@ -37,3 +37,20 @@ def test_tiles_have_heights_that_the_mma_takes(act_order):
             assert 0 < rows <= 384 and (rows // 2 if rows > 256 else rows) % 32 == 0, (M, K, N, p)
             tall += rows > 256
     assert tall > 20
+
+
+@pytest.mark.parametrize("resident", [(74, 70, 33, 20, 13), (74, 61, 30, 20, 15), (74, 0, 0, 0, 0), RESIDENT])
+def test_pairs_that_wait_for_one_another_are_resident_together(resident):
+    """A pair that adds a tile up waits for the sums of others: with more pairs in the launch than the device holds at once it
+    can keep an SM from the one it waits for.  (The number of pairs was half the number of SMs, whatever fits.)"""
+    cut = 0
+    for act_order in (False, True):
+        for K, N in SHAPES:
+            for M in ROWS:
+                p = plan(M, K, N, K // 128, act_order, resident=resident)
+                if p[KERNEL] != 4 or not p[CUT]:
+                    continue
+                cut += 1
+                held = resident[p[CLUSTER]] * p[CLUSTER]
+                assert p[PAIRS] <= held, (M, K, N, p)
+    assert (cut > 20) == (resident[1] > 0)
