@@ -73,7 +73,7 @@ struct GemmParams {
   float* ws_partials;
   unsigned* ws_counters;
   const __half* zp_table;   // rn(s * (z+1)) for every [group, column], or null
-  int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32, above 256 of 64
+  int tile_rows;            // weights-in-TMEM kernel: rows of a tile, a multiple of 32
   int cluster_pairs;        // weights-in-TMEM kernel: pairs of a cluster; more than one: they share a tile
   int area, turn_blocks;    // weights-in-TMEM kernel: layout of its shared memory
   int seq_shift;            // > 0: the caller promises g_idx[k] == k >> seq_shift (sequential groups of 2^seq_shift rows)
@@ -380,7 +380,6 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int
   for (int m_tiles = (M + G3_MAX_ROWS - 1) / G3_MAX_ROWS; m_tiles <= (M + 255) / 256; ++m_tiles) {
     Gemm3Plan c = {};
     c.tile_rows = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
-    if (c.tile_rows > 256) c.tile_rows = (c.tile_rows + 63) / 64 * 64;         // two MMAs of half the rows each: see idesc_f16
     c.cluster = 1;
     c.layout = gemm3_layout(c.tile_rows, G, act, 1);
     if (!c.layout.bytes) continue;
@@ -491,8 +490,8 @@ static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice
     if (e2 < e1) mh = 2;
   }
   // The weights-in-TMEM kernel: sequential layers whose groups are promised (tm_ok), and any other by its act-order form
-  const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && gv == 0 && q.variant != 5 && !one_group;
-  bool use_tm = tm_ok && use_pair && (gv == 4 || (gv == 0 && q.variant != 5));
+  const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && (gv == 6 || (gv == 0 && q.variant != 5)) && !one_group;
+  bool use_tm = tm_ok && use_pair && (gv == 4 || gv == 6 || (gv == 0 && q.variant != 5));
   Gemm3Plan plan3 = {};
   if (use_tm || tm_act) {
     const size_t room = q.workspace_bytes > Q4_GEMM_WS_COUNTER_BYTES ? q.workspace_bytes - Q4_GEMM_WS_COUNTER_BYTES : 0;
@@ -517,6 +516,7 @@ static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice
       use_tm = plan3.cost * 256 * (!plan3.act ? 1.13 : M <= 1024 ? 1.0 : 1.1) < pair;
     }
   }
+  if (gv == 6 && !use_tm) return fail(Q4_E_SHAPE, "gemm: the weights-in-TMEM kernel does not take this product (M=%d K=%d N=%d G=%d)", M, K, N, G);
   if (use_tm) mh = 1;
   *choice = {use_pair, use_tm, no_tables, mh, seq_shift, mh == 2 ? stages2w : stages2, plan3};
   return Q4_OK;
@@ -594,7 +594,7 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
   p.seq_shift = (!transpose && no_tables) ? seq_shift : 0;
   p.tile_rows = 256; p.cluster_pairs = 1; p.area = p.turn_blocks = 0;
   // activation rows one TMA copy brings
-  const int box_rows = use_tm ? plan3.tile_rows / (plan3.tile_rows > 256 ? 4 : 2) : use_pair ? 128 * mh : GM_TILE_M;
+  const int box_rows = use_tm ? (plan3.tile_rows > 256 ? gemm3_first_rows(plan3.tile_rows) : plan3.tile_rows) / 2 : use_pair ? 128 * mh : GM_TILE_M;
   CUtensorMap amap;
   if (int e = make_tmap_2d(&amap, act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)contract, (uint64_t)M,
                            (uint64_t)contract * 2, GM_TILE_C, box_rows, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
@@ -803,19 +803,20 @@ extern "C" int q4_gemm_plan(int transpose, int M, int K, int N, int G, int seque
   out[0] = !c.use_pair ? 1 : c.use_tm ? 4 : 1 + c.mh;
   if (c.use_tm) {
     out[1] = c.plan3.tile_rows; out[2] = c.plan3.pairs; out[3] = c.plan3.cluster; out[4] = c.plan3.stream; out[5] = c.plan3.act;
+    out[6] = c.plan3.tile_rows > 256 ? gemm3_first_rows(c.plan3.tile_rows) : c.plan3.tile_rows;
   } else if (c.use_pair) {
     const Gemm2Deal d = gemm2_deal(M, nout, contract / GM_TILE_C, r.sm_pairs, c.mh, workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + (size_t)r.sm_pairs * c.mh * Q4_GEMM_WS_SLICE_BYTES);
-    out[1] = 256 * c.mh; out[2] = d.pairs; out[3] = 1; out[4] = d.stream; out[5] = 0;
+    out[1] = 256 * c.mh; out[2] = d.pairs; out[3] = 1; out[4] = d.stream; out[5] = 0; out[6] = 256;
   } else {
-    out[1] = GM_TILE_M; out[2] = 0; out[3] = 1; out[4] = 0; out[5] = 0;
+    out[1] = GM_TILE_M; out[2] = 0; out[3] = 1; out[4] = 0; out[5] = 0; out[6] = 128;
   }
   return Q4_OK;
 }
 
 extern "C" int q4_gemm_set_variant(int variant) {
-  if (variant < 0 || variant > 5)
+  if (variant < 0 || variant > 6)
     return fail(Q4_E_BADARG, "gemm_set_variant: %d is not 0 (choose per shape), 1 (single CTA), 2 (CTA pair, 256-row tiles), 3 (CTA pair, 512-row tiles), "
-                "4 (weights in TMEM) or 5 (choose per shape among 1-3)", variant);
+                "4 (weights in TMEM, sequential form), 5 (choose per shape among 1-3) or 6 (weights in TMEM, either form)", variant);
   g_gemm_variant = variant;
   return Q4_OK;
 }

@@ -17,8 +17,10 @@
 //   columns up row by row: 333 rows of 5120 x 5120 take 43 us there and 28 here, 77 rows 32 and 22.)
 //
 // Tiles follow the rows: as many as of 384 or 256 rows, whichever takes less time (gemm3_plan), all of one height, a
-// multiple of 32 up to 256 and of 64 above (MMAs with A in TMEM have N in steps of 32).  77 rows are one tile of 96 and 333
-// one of 384 - two MMAs of 192 on the same dequantised operand (TALL), which used to be dequantised for two tiles of 256.
+// multiple of 32.  77 rows are one tile of 96 and 333 one of 352 - two MMAs, of 192 and 160 rows, on the same dequantised
+// operand (TALL), which used to be dequantised for two tiles of 256.  (Each a multiple of 32: an MMA with A in TMEM has N in
+// steps of 32.  The activation stage then holds twice the larger part, and the copies of the smaller one bring rows that
+// nothing reads.)
 // TMEM (512 columns): accumulator [128 lanes = output columns][columns = rows of x] fp32, and four to eight operand
 // stages of 32 columns (lane = output column, column c of a stage = contraction elements 2c, 2c+1 as a half2).
 // Roles (640 threads per CTA): warp 0 TMA producer of this CTA's half of the activation rows; warp 1 owns TMEM, its elected
@@ -50,6 +52,9 @@ constexpr int G3_THREADS = 32 * (4 + 4 * G3_GROUPS + 4);
 constexpr int G3_OFFS_BYTES = 4 * G3_GROUPS * 256;   // act-order: per dequant warp the table offsets of a stage's 64 rows
 constexpr int G3_PLAIN_AREA = G3_MAX_STAGES * 128 * GM_TILE_C * 2;
 constexpr int G3_TURN_BLOCK = 32 * 64;         // a warp's 32 columns of 32 rows, fp16
+
+// A tile of more than 256 rows is two MMAs: the rows of the first, a multiple of 32 and no fewer than the second's.
+__host__ __device__ constexpr int gemm3_first_rows(int tile_rows) { return (tile_rows / 2 + 31) / 32 * 32; }
 
 __device__ __forceinline__ void umma_f16_pair_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -116,11 +121,11 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   pdl_launch_dependents();
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int S = ACT || TALL ? p.stages : G3_MAX_STAGES;
-  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32 (TALL: of 64)
+  const int TR = p.tile_rows;                          // rows of x per tile, a multiple of 32
   constexpr int nh = TALL ? 2 : 1;                     // MMAs per 16 contraction elements
-  const int HR = TR / nh;                              // and rows of each
+  const int HR = TALL ? gemm3_first_rows(TR) : TR;     // rows of the first, which takes no fewer than the second
   constexpr bool PLAIN = !ACT && !TALL;                // one layout for all: stages of 128 rows, a place to turn every block over
-  const int x_bytes = PLAIN ? 128 * GM_TILE_C * 2 : TR * GM_TILE_C;             // this CTA's half of a tile's rows of a stage
+  const int x_bytes = PLAIN ? 128 * GM_TILE_C * 2 : nh * HR * GM_TILE_C;        // this CTA's half of a tile's rows of a stage
   unsigned char* tab = smem + S * x_bytes;             // act-order: [G][128 columns] scale | zero term
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (PLAIN ? G3_PLAIN_AREA : p.area));                  // even CTA: activation bytes + 4 dequant warps, of both CTAs
   uint64_t* empty = full + 8;                                                   // both CTAs: stage read by the MMAs
@@ -365,17 +370,18 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       pdl_wait();
       for (int item = 0; item < n_items; ++item) {
         const WorkItem wi = work_item<SPLIT>(p, wr, item, n_pairs, T);
-        const int m0 = (wi.tile % m_tiles) * TR + (HR >> 1) * (int)rank;
+        const int m0 = (wi.tile % m_tiles) * TR;
+        const int at[2] = {m0 + (HR >> 1) * (int)rank, m0 + HR + ((TR - HR) >> 1) * (int)rank};
         const int nst = wi.ke - wi.kb + (wi.lora ? 1 : 0);
         for (int j = 0; j < nst; ++j) {
           const int it = wi.kb + j;
           if (use > 0) wait_bar_idle(&empty[st], (use - 1) & 1, abort_flag, 40);
-          if (rank == 0) mbar_arrive_expect_tx(&full[st], TR * GM_TILE_C * 2);
+          if (rank == 0) mbar_arrive_expect_tx(&full[st], nh * HR * GM_TILE_C * 2);
 #pragma unroll
           for (int h = 0; h < nh; ++h) {
             unsigned char* dst = smem + (size_t)st * x_bytes + h * HR * GM_TILE_C;
-            if (it < wi.ke) tma_load_2d_pair(dst, &amap, it * GM_TILE_C, m0 + h * HR, full0 + 8 * st);
-            else tma_load_2d_pair(dst, &umap, 0, m0 + h * HR, full0 + 8 * st);
+            if (it < wi.ke) tma_load_2d_pair(dst, &amap, it * GM_TILE_C, at[h], full0 + 8 * st);
+            else tma_load_2d_pair(dst, &umap, 0, at[h], full0 + 8 * st);
           }
           if (++st == S) { st = 0; ++use; }
         }
@@ -388,7 +394,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     if (rank == 0) {
       uint32_t leader;
       asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(leader));
-      const uint32_t idesc = idesc_f16(256, HR, false);
+      const uint32_t idesc[2] = {idesc_f16(256, HR, false), idesc_f16(256, TR - HR, false)};
       const uint16_t both = (uint16_t)(3u << even_cta);
       // B: this CTA's 128 rows of x, K-major, 128-byte rows, 8-row groups 1024 B apart, 16 contraction elements = 32 B
       const uint64_t bd0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
@@ -412,7 +418,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
             for (int ks = 0; ks < nks; ++ks)
 #pragma unroll
               for (int h = 0; h < nh; ++h)
-                umma_f16_pair_ts(tmem_base + h * HR, a_tmem + 8 * ks, bd + ks * B_STEP + h * H_STEP, idesc, (it > 0 || ks > 0) ? 1u : 0u);
+                umma_f16_pair_ts(tmem_base + h * HR, a_tmem + 8 * ks, bd + ks * B_STEP + h * H_STEP, idesc[h], (it > 0 || ks > 0) ? 1u : 0u);
             umma_commit_pair(&empty[st], both);
           }
           __syncwarp();
@@ -642,7 +648,7 @@ static Gemm3Layout gemm3_layout(int tile_rows, int G, bool act, int cluster) {
     l.bytes = 1024 + (size_t)G3_PLAIN_AREA + G3_BAR_BYTES + 4 * 8 * G3_TURN_BLOCK;
     return l;
   }
-  const int nb = tile_rows / 32, x_bytes = tile_rows * GM_TILE_C, table = act ? G * 512 : 0, limit = 227 * 1024;
+  const int nb = tile_rows / 32, x_bytes = (tile_rows > 256 ? 2 * gemm3_first_rows(tile_rows) : tile_rows) * GM_TILE_C, table = act ? G * 512 : 0, limit = 227 * 1024;
   const int sums = cluster > 1 ? 4 * (nb - nb / cluster) * 4096 : 0;
   for (int s = (G2_TMEM_COLS - tile_rows) / 32 < G3_MAX_STAGES ? (G2_TMEM_COLS - tile_rows) / 32 : G3_MAX_STAGES; s >= 4; --s) {
     const int used = s * x_bytes + table > sums ? s * x_bytes + table : sums;

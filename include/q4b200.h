@@ -322,13 +322,15 @@ int q4_gemm_set_trace(void* device_buffer);
  * weights in tensor memory, where 256-row tiles would be chosen, where its tiles fit one round, and up to 1024
  * rows; the single-CTA kernel otherwise), 1 = always the single-CTA kernel, 2 / 3 = always the CTA-pair kernel
  * with 256- / 512-row tiles, 4 = always the weights-in-tensor-memory kernel (calls a forced kernel cannot serve
- * fail with Q4_E_SHAPE), 5 = as 0 without the weights-in-tensor-memory kernel.  For tests and measurements. */
+ * fail with Q4_E_SHAPE), 5 = as 0 without the weights-in-tensor-memory kernel, 6 = that kernel in its sequential or its
+ * act-order form.  For tests and measurements. */
 int q4_gemm_set_variant(int variant);
 /* What a product of these sizes runs, for tests and measurements; no device is touched when `resident` is given.
  * sequential_groupsize: as promised to q4_gemm_fwd_residual (0: none), with has_table = 1 where the call brings the table of
  * zero terms.  resident: five ints - pairs of SMs, then how many clusters of 1, 2, 3 and 4 pairs the device holds at once -
- * or null for the current device's.  out: six ints - the kernel (as q4_gemm_set_variant numbers them), rows of a tile, CTA
- * pairs, pairs of a cluster, whether tiles are cut between pairs, whether it is the act-order form of kernel 4. */
+ * or null for the current device's.  out: seven ints - the kernel (as q4_gemm_set_variant numbers them), rows of a tile, CTA
+ * pairs, pairs of a cluster, whether tiles are cut between pairs, whether it is the act-order form of kernel 4, rows of a
+ * tile's (first) MMA. */
 int q4_gemm_plan(int transpose, int M, int K, int N, int G, int sequential_groupsize, int has_table, size_t workspace_bytes,
                  const int* resident, int* out);
 /* Forms of the sequential-group decode kernels, for tests and measurements (process-wide; no

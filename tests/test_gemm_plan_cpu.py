@@ -9,13 +9,13 @@ RESIDENT = (74, 74, 36, 22, 15)            # a B200: pairs of SMs; clusters of o
 SHAPES = [(4096, 4096), (4096, 1024), (4096, 11008), (11008, 4096), (5120, 5120), (5120, 15360), (5120, 27648), (13824, 5120), (8192, 28672),
           (28672, 8192), (2176, 256), (512, 512)]
 ROWS = [1, 17, 32, 77, 128, 250, 256, 257, 270, 288, 289, 320, 321, 333, 352, 384, 385, 500, 512, 513, 700, 800, 1024, 1038, 1100, 1152, 1536, 2048, 4096]
-KERNEL, TILE, PAIRS, CLUSTER, CUT, ACT = range(6)
+KERNEL, TILE, PAIRS, CLUSTER, CUT, ACT, FIRST = range(7)
 
 
 def plan(M, K, N, G, act_order, transpose=False, resident=RESIDENT, workspace=None):
     """``G`` groups; a sequential layer's forward comes with its table of zero terms and the promise of its group size."""
     L = _lib.lib()
-    out = (ctypes.c_int * 6)()
+    out = (ctypes.c_int * 7)()
     dev = None if resident is None else (ctypes.c_int * 5)(*resident)
     size = int(L.q4_gemm_workspace_bytes(K, N, G)) if workspace is None else workspace
     table = not act_order and not transpose
@@ -25,16 +25,17 @@ def plan(M, K, N, G, act_order, transpose=False, resident=RESIDENT, workspace=No
 
 @pytest.mark.parametrize("act_order", [False, True])
 def test_tiles_have_heights_that_the_mma_takes(act_order):
-    """An MMA of a CTA pair with A in tensor memory takes N in steps of 32; tiles above 256 rows are two MMAs of half the rows.
-    (Tiles of 288 and 352 rows came to N = 144 and 176.)"""
+    """An MMA of a CTA pair with A in tensor memory takes N in steps of 32, up to 256; tiles above 256 rows are two MMAs.
+    (In halves, tiles of 288 and 352 rows came to N = 144 and 176.)"""
     tall = 0
     for K, N in SHAPES:
         for M in ROWS:
             p = plan(M, K, N, K // 128, act_order)
             if p[KERNEL] != 4:
                 continue
-            rows = p[TILE]
-            assert 0 < rows <= 384 and (rows // 2 if rows > 256 else rows) % 32 == 0, (M, K, N, p)
+            rows, first = p[TILE], p[FIRST]
+            assert 0 < rows <= 384 and (first == rows if rows <= 256 else first >= rows - first > 0), (M, K, N, p)
+            assert first % 32 == 0 and first <= 256 and (rows - first) % 32 == 0, (M, K, N, p)
             tall += rows > 256
     assert tall > 20
 
