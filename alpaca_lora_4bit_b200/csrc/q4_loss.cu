@@ -91,11 +91,11 @@ ce_fwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__
       m = top;
     }
     if (m == -INFINITY) continue;
-    const float ml = m * LOG2E;
 #pragma unroll
     for (int e = 0; e < 4 * CE_BATCH; ++e) {
+      // (the difference first: a product m log2(e) is rounded at the size of the logits)
       const float2 x = ce_pair<BF16>(w[e]);
-      sum += exp2f(fmaf(x.x, LOG2E, -ml)) + exp2f(fmaf(x.y, LOG2E, -ml));
+      sum += exp2f((x.x - m) * LOG2E) + exp2f((x.y - m) * LOG2E);
     }
     s += sum;
   }
@@ -156,7 +156,6 @@ ce_bwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__
   const float g = *grad_loss / *count;
   const float2 st = stats[row];
   const int at = (int)(label >> 3), which = (int)(label & 7);
-  const float shift = -(st.x + st.y) * LOG2E;
 #pragma unroll 4
   for (int i = threadIdx.x; i < V / 8; i += CE_THREADS) {
     const uint4 v = ldg_stream(src + i);
@@ -165,8 +164,12 @@ ce_bwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 x = ce_pair<BF16>(w[e]);
-      float a = exp2f(fmaf(x.x, LOG2E, shift)), b = exp2f(fmaf(x.y, LOG2E, shift));
-      if (i == at) { a -= which == 2 * e ? 1.f : 0.f; b -= which == 2 * e + 1 ? 1.f : 0.f; }
+      const float la = (x.x - st.x) - st.y, lb = (x.y - st.x) - st.y;
+      float a = exp2f(la * LOG2E), b = exp2f(lb * LOG2E);
+      if (i == at) {                                       // softmax - 1, also where it is next to nothing
+        if (which == 2 * e) a = expm1f(la);
+        if (which == 2 * e + 1) b = expm1f(lb);
+      }
       o[e] = ce_pack<BF16>(a * g, b * g);
     }
     dst[i] = make_uint4(o[0], o[1], o[2], o[3]);

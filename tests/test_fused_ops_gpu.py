@@ -254,6 +254,35 @@ def test_causal_loss_matches_stock(B, T, V, shifted, dtype):
     assert float((dgot.float() - logits.grad.float()).abs().max()) <= 2 ** (-10 if dtype == torch.float16 else -7) * float(logits.grad.float().abs().max())
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("offset", [0.0, 300.0, 1000.0, -20000.0])
+def test_causal_loss_of_confident_rows_and_of_logits_with_an_offset(offset, dtype):
+    """Against 64 bits on the same 16-bit logits.  fp32: log s of a sum s = 1 + eps carries a few 2^-24, absolute, so that
+    softmax - 1 does too, however small it is; an exponent d (the log probability) two roundings, 2^-24 |d| each, which are
+    relative errors of its exponential; the gradient is then rounded once to 16 bits.  (With the exponent formed as
+    x log2(e) - m log2(e) the errors grew with the logits.)"""
+    B, V = 16, 32000
+    gen = torch.Generator(device=DEV).manual_seed(int(abs(offset)) + 1)
+    x = torch.randn((B, V), generator=gen, device=DEV) * 2
+    labels = torch.randint(0, V, (B,), generator=gen, device=DEV)
+    x[torch.arange(B, device=DEV), labels] = 14 + 8 * torch.rand(B, generator=gen, device=DEV)      # probability 0.9 .. 0.9999
+    logits = (x + offset).to(dtype).requires_grad_(True)
+    fused = fused_ops.causal_lm_loss(lambda *a, **k: (_ for _ in ()).throw(AssertionError("the stock loss ran")))
+    loss = fused(logits, None, V, shift_labels=labels)
+    scale = 1024.0 * B
+    (loss * scale).backward()
+    l64 = logits.detach().double().requires_grad_(True)
+    loss64 = torch.nn.functional.cross_entropy(l64, labels)
+    (loss64 * scale).backward()
+    assert abs(float(loss.detach()) - float(loss64.detach())) <= 8 * 2 ** -24 * (1 + float(loss64.detach()))
+    got, want = logits.grad.double(), l64.grad
+    hot, d = torch.nn.functional.one_hot(labels, V), torch.log_softmax(l64.detach(), 1).abs()
+    tol = 2 ** (-11 if dtype == torch.float16 else -8) * want.abs() + 2 ** -24 * ((8 + 2 * d) * want.abs() + 8 * (scale / B) * hot)
+    if dtype == torch.float16:
+        tol = tol + 2 ** -25                             # half the smallest subnormal
+    assert bool(((got - want).abs() <= tol * 1.001).all()), float(((got - want).abs() / tol).max())
+
+
 def test_causal_loss_at_the_edges():
     """No row with a class, infinities and NaN among the logits: what the framework's loss gives; the loss may be written in
     place before its backward; a second derivative is refused; other calls go to the stock loss."""
