@@ -347,31 +347,50 @@ static size_t gemm_smem_bytes(bool transpose, int G, int stages) {
 
 using namespace q4;
 
-// Estimated duration (SM cycles) of the pair kernel with tiles of 256 * mh rows, and whether that
-// assumes whole tiles per pair (round after round) or all tiles x stages dealt as one sequence.
-// Per contraction stage a pair takes about 780 cycles with 256-row tiles (bounded by the dequant
-// warps) and 1100 with 512-row tiles (bounded by the MMAs: twice the flops per stage); exchanging
-// the partial sums of a shared tile costs about as much as 18 resp. 24 stages.  (With 700 / 12 / 16, guessed from single
-// launches, 1536 rows of 4096 x 4096 took 59 us dealt in 256-row tiles, whole 512-row tiles 50; the backward of 1024 rows of
-// 8192 x 8192 106 and 94, act-order 133 and 116; 2048 rows of 11008 x 4096 141 and 130, the backward of 4096 x 11008, act-order,
-// 169 and 150.)
-constexpr int G2_STAGE_CYCLES_256 = 780, G2_STAGE_CYCLES_512 = 1100;
-static long long gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_ok, bool* stream) {
+// Estimated duration (us) of the pair kernel with tiles of 256 * mh rows, and whether that assumes whole tiles per pair
+// (round after round) or tiles cut between pairs.  `stage_us`: a contraction stage (gemm2_stage_us).
+// Fitted to 6400 launches of 22 shapes (1024 x 4096 to 28672 x 8192) at 18 to 29 heights from 32 to 4096 rows, both orders of
+// groups and both directions; within 3 to 7 % of them.  A launch takes 11 us, an item 1.9 (256 rows) or 4.1 beside its stages.  All
+// tiles x stages dealt in equal runs: 22.5 and 36 us with the exchange.  Up to half as many tiles as pairs, each cut
+// in n: 16 us and 5.4 and 9.6 for every contributor after the first, whose sums are added one by one.
+static double gemm2_estimate(int M, int nout, int T, int P, int mh, bool ws_ok, double stage_us, bool* stream) {
   const int tile_m = 256 * mh;
-  const long long n_tiles = (long long)(nout / G2_TILE_N) * ((M + tile_m - 1) / tile_m);
-  const long long per_stage = mh == 2 ? G2_STAGE_CYCLES_512 : G2_STAGE_CYCLES_256, exchange = mh == 2 ? 24 : 18;
-  long long best = (n_tiles + P - 1) / P * T;
+  const long long n_tiles = (long long)(nout / G2_TILE_N) * ((M + tile_m - 1) / tile_m), total = n_tiles * T;
+  const double item = mh == 2 ? 4.1 : 1.9;
+  double best = 11 + (double)((n_tiles + P - 1) / P) * (stage_us * T + item);
   *stream = false;
-  if (ws_ok && T >= 8 && n_tiles % P != 0) {
-    const long long total = n_tiles * T, dealt = (total + P - 1) / P + exchange;
-    if (dealt < best && total >= (long long)P * 4 && total * P < (1ll << 32)) { best = dealt; *stream = true; }
+  if (ws_ok && T >= 8 && n_tiles % P != 0 && total >= (long long)P * 4 && total * P < (1ll << 32)) {
+    const int per_tile = (int)(P / n_tiles);
+    const double cut = per_tile >= 2 ? 16 + stage_us * T / per_tile + (per_tile - 1) * (mh == 2 ? 9.6 : 5.4)
+                                     : (mh == 2 ? 36 : 22.5) + 1.02 * stage_us * (double)total / P + item * (double)n_tiles / P;
+    if (cut < best) { best = cut; *stream = true; }
   }
-  return best * per_stage;
+  return best;
+}
+// A stage of the pair kernel (us).  Measured in launches of up to 150 us: forward 0.50 and 0.60 (256- and 512-row tiles) with
+// sequential groups, 0.565 and 0.68 by look-up in tables, a third more where those leave three stages of the pipeline (512 rows
+// from 76 groups on); longer launches, at the power limit, take 12 to 15 % more, dealt ones of 512 rows up to 30: the figures here
+// choose best over both.  Backward: 0.45 and 0.65 in a sequential layer, 0.73 and 0.85 with act-order, which the call does not
+// say.  (With 780 and 1100 cycles and an exchange of 18 and 24 stages for every case, 257 rows of 3584 x 9728 took 78 us in
+// one 512-row tile, 57 in two of 256; 1800 rows of 2048 x 5632, act-order, 74 and 66; the forward of 1100 rows of 11008 x 4096
+// 94 and 84.)
+static double gemm2_stage_us(bool transpose, bool sequential, int stages, int mh) {
+  if (transpose) return mh == 2 ? 0.81 : 0.60;
+  if (sequential) return mh == 2 ? 0.71 : 0.50;
+  return (mh == 2 ? 0.78 : 0.60) * (stages <= 3 ? 1.3 : 1.0);
 }
 
-// Tiles and pairs of the weights-in-TMEM kernel, by what a pair's work takes in stages of the contraction (256 rows, about
-// 0.28 us).  `room`: bytes of the workspace for partial sums.  tile_rows = 0: the act-order table does not fit.
+// Tiles and pairs of the weights-in-TMEM kernel, by what a pair's work takes in stages of the contraction (256 rows of a
+// sequential layer, G3_STAGE_US).  `room`: bytes of the workspace for partial sums.  tile_rows = 0: the act-order table does not fit.
 struct Gemm3Plan { int tile_rows, pairs, cluster; bool stream, act; double cost; Gemm3Layout layout; };
+constexpr double G3_STAGE_US = 0.41;
+// A stage of tiles of `rows` rows in those of 256.  Measured (us): sequential 0.36 at 128 rows, 0.41 at 256, then - two MMAs, four
+// to seven stages in flight instead of eight - 0.525 at 288, 0.53 at 320, 0.56 at 352, 0.59 at 384; act-order, bound by the
+// dequant warps, 0.585 up to 256, 0.62 at 288, 0.64 at 320, 0.67 at 352, 0.70 at 384.
+static double gemm3_stage(int rows, bool act) {
+  const double over = (rows - 288) / 96.0;
+  return rows <= 256 ? (act ? 1.47 : 1.0) : act ? 1.49 + 0.19 * over : 1.23 + 0.18 * over;
+}
 static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int G, bool act, size_t room) {
   // Pairs that are resident at once: a pair that adds up a tile waits for others that must not be waiting for its SMs.  Where
   // the device does not say, tiles are not cut by the workspace.
@@ -385,16 +404,15 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int
     if (!c.layout.bytes) continue;
     const int tiles = nout / G2_TILE_N * m_tiles, nb = c.tile_rows / 32;
     const long long total = (long long)tiles * T;
-    // a stage is bound by the MMAs from 256 rows on, below - act-order: below 435 - by the dequant warps
-    const double least = act ? 1.7 : 1.0, unit = c.tile_rows > 256 * least ? c.tile_rows / 256.0 : least;
+    const double unit = gemm3_stage(c.tile_rows, act);
     const bool parts = dev.clusters[1] > 0 && room >= (size_t)P * c.tile_rows * G2_TILE_N * sizeof(float) && total * P < (1ll << 32);
     // whole tiles, round after round
     c.pairs = tiles < P ? tiles : P;
     double cost = (double)((tiles + P - 1) / P) * T * unit;
     if (tiles > P) {
       // or, where the last round would leave pairs idle for longer than the exchange of partial sums costs, all tiles x
-      // stages as one sequence in equal runs (measured: every further item of a run and the exchange about 30 stages)
-      const double dealt = (double)((total + P - 1) / P) * unit + 30;
+      // stages as one sequence in equal runs (measured: every further item of a run and the exchange about 27 stages)
+      const double dealt = (double)((total + P - 1) / P) * unit + 27;
       if (parts && T >= 8 && tiles % P != 0 && dealt < cost) { cost = dealt; c.stream = true; }
     } else if (tiles * 2 <= P && T >= 16) {
       // Fewer tiles than half the pairs (short prompts: one row tile, 16 column tiles of a 4096-wide layer on 74 pairs):
@@ -426,7 +444,7 @@ static Gemm3Plan gemm3_plan(int M, int nout, int T, const GemmResident& dev, int
       // One to two pairs per tile: one sequence in equal runs over all pairs, where the shorter runs are worth the
       // exchange (4096 x 11008, 43 tiles, uncut / dealt: 25.4 / 22.2 us at 32 rows, 26.5 / 24.4 at 128, 27.3 / 26.6 at 192;
       // 5120 x 13824, 54 tiles: 30.1 / 28.6 at 32, 31.6 / 31.3 at 128).
-      const double dealt = (double)total / P * unit + 14 + 3 * nb;
+      const double dealt = (double)total / P * unit + 16 + 1.5 * nb;
       if (dealt < cost) { cost = dealt; c.stream = true; c.pairs = P; }
     }
     c.cost = cost;
@@ -444,6 +462,7 @@ struct GemmRequest {
 struct GemmChoice {
   bool use_pair, use_tm, no_tables;
   int mh, seq_shift, stages;                    // stages: of the pair kernel at this mh
+  double stage_us;                              // and what one takes
   Gemm3Plan plan3;
 };
 
@@ -481,14 +500,14 @@ static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice
   const int P_est = dev.sm_pairs;
   const size_t zp_need = transpose && !q.table ? (((size_t)G * N * sizeof(__half) + 255) & ~(size_t)255) : 0;
   auto ws_ok_for = [&](int m) { return q.workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + zp_need + (size_t)P_est * m * Q4_GEMM_WS_SLICE_BYTES; };
+  const bool sequential = no_tables && seq_shift > 0;
+  const double us1 = gemm2_stage_us(transpose, sequential, stages2, 1), us2 = gemm2_stage_us(transpose, sequential, stages2w, 2);
+  bool dealt;
+  const double pair1 = gemm2_estimate(M, nout, contract / GM_TILE_C, P_est, 1, ws_ok_for(1), us1, &dealt);
+  const double pair2 = gemm2_estimate(M, nout, contract / GM_TILE_C, P_est, 2, ws_ok_for(2), us2, &dealt);
   int mh = 1;
   if (use_pair && gv == 3) mh = 2;
-  else if (use_pair && gv == 0 && wide_ok && M > 256) {
-    bool s1, s2;
-    const long long e1 = gemm2_estimate(M, nout, contract / GM_TILE_C, P_est, 1, ws_ok_for(1), &s1);
-    const long long e2 = gemm2_estimate(M, nout, contract / GM_TILE_C, P_est, 2, ws_ok_for(2), &s2);
-    if (e2 < e1) mh = 2;
-  }
+  else if (use_pair && gv == 0 && wide_ok && M > 256 && pair2 < pair1) mh = 2;
   // The weights-in-TMEM kernel: sequential layers whose groups are promised (tm_ok), and any other by its act-order form
   const bool tm_act = !tm_ok && !transpose && !swiglu && nout % G2_TILE_N == 0 && use_pair && (gv == 6 || (gv == 0 && q.variant != 5)) && !one_group;
   bool use_tm = tm_ok && use_pair && (gv == 4 || gv == 6 || (gv == 0 && q.variant != 5));
@@ -499,26 +518,13 @@ static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice
     plan3.act = !use_tm;
     use_tm = plan3.tile_rows > 0;
     if (use_tm && gv == 0 && !(tm_ok && M <= 1024)) {
-      // Which of the two kernels, by rows of the activations times stages of 256 columns that a pair multiplies (sequential
-      // layers up to 1024 rows: always this one).  The 512-row tiles of the pair kernel run as fast as the power limit lets
-      // the tensor cores; here a row costs some 10 % more when launches are that long (W is dequantised for every 384 rows
-      // instead of every 512), but tiles follow the rows: 1100 rows of 5120 x 13824 take 116 us here and 157 there, 1536 rows
-      // 145 and 171, 2048 rows 209 and 200.  An act-order stage costs no less than 435 rows (gemm3_plan) where the pair
-      // kernel, whose dequant is as slow, does 512: 333 rows of 13824 x 5120 53 and 89 us, 500 rows of 5120 x 15360 86 and 68,
-      // 700 rows 100 and 128, 2048 rows of 8192 x 28672 827 and 709.
-      const int T = contract / GM_TILE_C;
-      const long long tiles = (long long)(nout / G2_TILE_N) * ((M + 256 * mh - 1) / (256 * mh));
-      bool dealt;
-      double stages2 = (double)gemm2_estimate(M, nout, T, P_est, mh, ws_ok_for(mh), &dealt) / (mh == 2 ? G2_STAGE_CYCLES_512 : G2_STAGE_CYCLES_256);
-      // an item's epilogue, which 512-row tiles overlap with nothing, and what an exchange costs them beyond the estimate
-      stages2 += 5.0 * ((tiles + P_est - 1) / P_est + (dealt ? 1 : 0)) + (dealt && mh == 2 ? 6 : 0);
-      const double pair = stages2 * (mh == 2 ? 512 : !plan3.act ? 288 : wide_ok ? 400 : 480);
-      use_tm = plan3.cost * 256 * (!plan3.act ? 1.13 : M <= 1024 ? 1.0 : 1.1) < pair;
+      // Which of the two kernels (sequential layers up to 1024 rows: always this one).
+      use_tm = 9 + G3_STAGE_US * plan3.cost < (mh == 2 ? pair2 : pair1);
     }
   }
   if (gv == 6 && !use_tm) return fail(Q4_E_SHAPE, "gemm: the weights-in-TMEM kernel does not take this product (M=%d K=%d N=%d G=%d)", M, K, N, G);
   if (use_tm) mh = 1;
-  *choice = {use_pair, use_tm, no_tables, mh, seq_shift, mh == 2 ? stages2w : stages2, plan3};
+  *choice = {use_pair, use_tm, no_tables, mh, seq_shift, mh == 2 ? stages2w : stages2, mh == 2 ? us2 : us1, plan3};
   return Q4_OK;
 }
 
@@ -526,10 +532,10 @@ static int gemm_choose(const GemmRequest& q, const GemmResident& dev, GemmChoice
 // longer than the exchange of partial sums costs (about a dozen stages), all tiles x stages as one
 // sequence cut into equal runs.
 struct Gemm2Deal { int pairs; bool stream; };
-static Gemm2Deal gemm2_deal(int M, int nout, int T, int P, int mh, bool ws_ok) {
+static Gemm2Deal gemm2_deal(int M, int nout, int T, int P, int mh, bool ws_ok, double stage_us) {
   const int n_tiles = (nout / G2_TILE_N) * ((M + 256 * mh - 1) / (256 * mh));
   Gemm2Deal d = {n_tiles < P ? n_tiles : P, false};
-  gemm2_estimate(M, nout, T, P, mh, ws_ok, &d.stream);
+  gemm2_estimate(M, nout, T, P, mh, ws_ok, stage_us, &d.stream);
   if (d.stream) {
     // Fewer tiles than half the pairs: take a whole number of pairs per tile, so that every tile is shared by the
     // same number of pairs in equal parts and a pair has one piece of one tile.  Cut into P runs the pieces fall
@@ -679,7 +685,7 @@ static int gemm_launch(bool transpose, const void* act, const int32_t* qweight, 
       if (e3) return e3;
       return check_cuda(cudaGetLastError(), "gemm launch");
     }
-    const Gemm2Deal deal = gemm2_deal(M, nout, T, P, mh, ws && workspace_bytes >= ws_off + (size_t)P * mh * Q4_GEMM_WS_SLICE_BYTES);
+    const Gemm2Deal deal = gemm2_deal(M, nout, T, P, mh, ws && workspace_bytes >= ws_off + (size_t)P * mh * Q4_GEMM_WS_SLICE_BYTES, choice.stage_us);
     const bool stream = deal.stream;
     const int pairs = deal.pairs;
     const int f = stream ? 2 : 1;
@@ -805,7 +811,7 @@ extern "C" int q4_gemm_plan(int transpose, int M, int K, int N, int G, int seque
     out[1] = c.plan3.tile_rows; out[2] = c.plan3.pairs; out[3] = c.plan3.cluster; out[4] = c.plan3.stream; out[5] = c.plan3.act;
     out[6] = c.plan3.tile_rows > 256 ? gemm3_first_rows(c.plan3.tile_rows) : c.plan3.tile_rows;
   } else if (c.use_pair) {
-    const Gemm2Deal d = gemm2_deal(M, nout, contract / GM_TILE_C, r.sm_pairs, c.mh, workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + (size_t)r.sm_pairs * c.mh * Q4_GEMM_WS_SLICE_BYTES);
+    const Gemm2Deal d = gemm2_deal(M, nout, contract / GM_TILE_C, r.sm_pairs, c.mh, workspace_bytes >= Q4_GEMM_WS_COUNTER_BYTES + (size_t)r.sm_pairs * c.mh * Q4_GEMM_WS_SLICE_BYTES, c.stage_us);
     out[1] = 256 * c.mh; out[2] = d.pairs; out[3] = 1; out[4] = d.stream; out[5] = 0; out[6] = 256;
   } else {
     out[1] = GM_TILE_M; out[2] = 0; out[3] = 1; out[4] = 0; out[5] = 0; out[6] = 128;

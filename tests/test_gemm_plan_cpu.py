@@ -5,7 +5,7 @@ import pytest
 
 from alpaca_lora_4bit_b200 import _lib
 
-RESIDENT = (74, 74, 36, 22, 15)            # a B200: pairs of SMs; clusters of one to four pairs at once
+RESIDENT = (74, 74, 33, 22, 15)            # a B200: pairs of SMs; clusters of one to four pairs at once
 SHAPES = [(4096, 4096), (4096, 1024), (4096, 11008), (11008, 4096), (5120, 5120), (5120, 15360), (5120, 27648), (13824, 5120), (8192, 28672),
           (28672, 8192), (2176, 256), (512, 512)]
 ROWS = [1, 17, 32, 77, 128, 250, 256, 257, 270, 288, 289, 320, 321, 333, 352, 384, 385, 500, 512, 513, 700, 800, 1024, 1038, 1100, 1152, 1536, 2048, 4096]
@@ -55,3 +55,19 @@ def test_pairs_that_wait_for_one_another_are_resident_together(resident):
                 held = resident[p[CLUSTER]] * p[CLUSTER]
                 assert p[PAIRS] <= held, (M, K, N, p)
     assert (cut > 20) == (resident[1] > 0)
+
+
+@pytest.mark.parametrize("M,K,N,act_order,transpose,want", [
+    (257, 9728, 3584, False, True, dict(KERNEL=2)),               # 49 us in two 256-row tiles, 57 in one of 512
+    (257, 3584, 9728, False, True, dict(KERNEL=2)),               # 56 and 78
+    (1800, 2048, 5632, True, True, dict(KERNEL=3)),               # 66 us in 512-row tiles, 74 in 256
+    (1600, 5120, 5120, False, True, dict(KERNEL=2)),              # 84 in 256, 93 in 512
+    (4096, 8192, 1024, True, True, dict(KERNEL=3, CUT=0)),        # whole tiles 84 us, dealt 107
+    (1100, 11008, 4096, False, False, dict(KERNEL=4, CUT=1)),     # 84 us dealt; 94 in whole tiles of 288 rows
+    (2500, 8192, 8192, False, False, dict(KERNEL=4, CUT=1)),      # 260 us dealt; 306 in whole tiles of 288 rows
+    (1200, 11008, 4096, True, False, dict(KERNEL=4, ACT=1)),      # 110 us; the pair kernel 129
+    (128, 8192, 1024, True, False, dict(KERNEL=4, ACT=1)),        # 29 us; 18 pairs a tile of the pair kernel 100
+])
+def test_choices_that_were_measured(M, K, N, act_order, transpose, want):
+    p = plan(M, K, N, K // 128, act_order, transpose)
+    assert {k: p[globals()[k]] for k in want} == want, p
