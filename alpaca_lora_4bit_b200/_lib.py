@@ -68,6 +68,8 @@ _SIGNATURES = {
     "q4_lora_project": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, ctypes.c_float, c_void_p]),
     "q4_cast16": (c_int, [c_void_p, c_void_p, c_size_t, c_int, c_void_p]),
     "q4_causal_loss_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_int, c_void_p]),
+    "q4_causal_loss_fwd_keep": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong,
+                                        c_int, c_void_p]),
     "q4_causal_loss_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_int, c_void_p]),
     "q4_lora_grads": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "q4_adamw_flat": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, ctypes.c_float, ctypes.c_float, ctypes.c_float,

@@ -51,9 +51,10 @@ __device__ __forceinline__ void ce_merge(float& m, float& s, float m2, float s2)
 template <bool BF16>
 __global__ void __launch_bounds__(CE_THREADS, 4)
 ce_fwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__ labels, float2* __restrict__ stats, float* __restrict__ row_loss,
-              int V, int seq, long long ignore) {
+              uint16_t* __restrict__ kept, long long* __restrict__ classes, int V, int seq, long long ignore) {
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint4* src = reinterpret_cast<const uint4*>(logits + (size_t)row * V);
+  uint4* copy = reinterpret_cast<uint4*>(kept + (size_t)row * V);          // (a null `kept`: never written)
   // four vectors at a time, the next four on their way meanwhile: one rescaling for 32 elements
   uint4 v[CE_BATCH];
   auto fetch = [&](int i0) __attribute__((always_inline)) {
@@ -65,8 +66,11 @@ ce_fwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__
   };
   fetch(threadIdx.x);
   const long long label = ce_label(labels, row, seq, ignore);
+  if (classes && threadIdx.x == 0) classes[row] = label;
   if (label == ignore) {
     if (threadIdx.x == 0) row_loss[row] = 0.f;
+    if (kept)
+      for (int i = threadIdx.x; i < V / 8; i += CE_THREADS) copy[i] = src[i];
     return;
   }
   const bool known = label >= 0 && label < V;
@@ -78,6 +82,11 @@ ce_fwd_kernel(const uint16_t* __restrict__ logits, const long long* __restrict__
     uint32_t w[4 * CE_BATCH];
 #pragma unroll
     for (int j = 0; j < CE_BATCH; ++j) { w[4 * j] = v[j].x; w[4 * j + 1] = v[j].y; w[4 * j + 2] = v[j].z; w[4 * j + 3] = v[j].w; }
+    if (kept) {
+#pragma unroll
+      for (int j = 0; j < CE_BATCH; ++j)
+        if (i0 + j * CE_THREADS < V / 8) copy[i0 + j * CE_THREADS] = v[j];
+    }
     fetch(i0 + CE_BATCH * CE_THREADS);
     float top = -INFINITY, sum = 0.f;
 #pragma unroll
@@ -189,11 +198,17 @@ using namespace q4;
 
 extern "C" int q4_causal_loss_fwd(const void* logits, const long long* labels, float* stats, float* row_loss, float* loss, float* count, int rows,
                                   int V, int seq, long long ignore, int bf16, q4_stream_t stream) {
+  return q4_causal_loss_fwd_keep(logits, labels, stats, row_loss, loss, count, nullptr, nullptr, rows, V, seq, ignore, bf16, stream);
+}
+
+extern "C" int q4_causal_loss_fwd_keep(const void* logits, const long long* labels, float* stats, float* row_loss, float* loss, float* count,
+                                       void* kept, long long* classes, int rows, int V, int seq, long long ignore, int bf16, q4_stream_t stream) {
   if (!logits || !labels || !stats || !row_loss || !loss || !count) return fail(Q4_E_BADARG, "causal_loss: null pointer");
   if (int e = ce_check(logits, rows, V, seq, "causal_loss")) return e;
+  if (!aligned16(kept)) return fail(Q4_E_ALIGN, "causal_loss: the copy of the logits must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
-  if (bf16) ce_fwd_kernel<true><<<rows, CE_THREADS, 0, st>>>((const uint16_t*)logits, labels, (float2*)stats, row_loss, V, seq, ignore);
-  else ce_fwd_kernel<false><<<rows, CE_THREADS, 0, st>>>((const uint16_t*)logits, labels, (float2*)stats, row_loss, V, seq, ignore);
+  if (bf16) ce_fwd_kernel<true><<<rows, CE_THREADS, 0, st>>>((const uint16_t*)logits, labels, (float2*)stats, row_loss, (uint16_t*)kept, classes, V, seq, ignore);
+  else ce_fwd_kernel<false><<<rows, CE_THREADS, 0, st>>>((const uint16_t*)logits, labels, (float2*)stats, row_loss, (uint16_t*)kept, classes, V, seq, ignore);
   ce_mean_kernel<<<1, 1024, 0, st>>>(row_loss, labels, loss, count, rows, seq, ignore);
   return check_cuda(cudaGetLastError(), "causal_loss launch");
 }

@@ -257,32 +257,46 @@ def _fuse_gate_up(model: nn.Module) -> int:
 
 
 class _CausalLoss(torch.autograd.Function):
+    """The loss and, where a gradient may be asked for, the copy of the logits that the backward reads: a program may write to
+    its logits and labels before then, as with the stock loss, whose backward reads an fp32 copy.  The copy is an output, so
+    that a second derivative finds its way through it to the logits."""
+
     @staticmethod
-    def forward(ctx, logits, labels, seq, ignore):
+    def forward(ctx, logits, labels, seq, ignore, keep):
         V = logits.shape[-1]
         rows = logits.numel() // V
         f32 = dict(dtype=torch.float32, device=logits.device)
         stats, row_loss = torch.empty((rows, 2), **f32), torch.empty(rows, **f32)
         loss, count = torch.empty((), **f32), torch.empty((), **f32)
+        kept = classes = None
+        if keep:
+            kept, classes = torch.empty_like(logits), torch.empty(rows, dtype=torch.int64, device=logits.device)
         with _lib.on_device(logits.device):
-            _lib.check(_lib.lib().q4_causal_loss_fwd(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), row_loss.data_ptr(), loss.data_ptr(),
-                                                     count.data_ptr(), rows, V, seq, ignore, int(logits.dtype == torch.bfloat16), _lib.stream_of(logits)), "causal_loss")
-        ctx.save_for_backward(logits, labels, stats, count)
-        ctx.seq, ctx.ignore = seq, ignore
-        return loss
+            _lib.check(_lib.lib().q4_causal_loss_fwd_keep(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), row_loss.data_ptr(), loss.data_ptr(),
+                                                          count.data_ptr(), _lib.ptr(kept), _lib.ptr(classes), rows, V, seq, ignore,
+                                                          int(logits.dtype == torch.bfloat16), _lib.stream_of(logits)), "causal_loss")
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(kept, classes, stats, count)
+        ctx.ignore = ignore
+        return loss, kept
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
-    def backward(ctx, grad_loss):
-        logits, labels, stats, count = ctx.saved_tensors
-        V = logits.shape[-1]
-        g = grad_loss.float()
-        grad = torch.empty_like(logits)
-        with _lib.on_device(logits.device):
-            _lib.check(_lib.lib().q4_causal_loss_bwd(logits.data_ptr(), labels.data_ptr(), stats.data_ptr(), g.data_ptr(), count.data_ptr(),
-                                                     grad.data_ptr(), logits.numel() // V, V, ctx.seq, ctx.ignore,
-                                                     int(logits.dtype == torch.bfloat16), _lib.stream_of(logits)), "causal_loss_bwd")
-        return grad, None, None, None
+    def backward(ctx, grad_loss, grad_kept):
+        if grad_loss is None:
+            return grad_kept, None, None, None, None
+        kept, classes, stats, count = ctx.saved_tensors
+        V = kept.shape[-1]
+        if torch.is_grad_enabled():                     # a derivative of this gradient may follow: the stock operations
+            loss = F.cross_entropy(kept.float().view(-1, V), classes, ignore_index=ctx.ignore)
+            (grad,) = torch.autograd.grad(loss, kept, grad_loss, create_graph=True)
+        else:
+            g = grad_loss.float()
+            grad = torch.empty_like(kept)
+            with _lib.on_device(kept.device):
+                _lib.check(_lib.lib().q4_causal_loss_bwd(kept.data_ptr(), classes.data_ptr(), stats.data_ptr(), g.data_ptr(), count.data_ptr(),
+                                                         grad.data_ptr(), kept.numel() // V, V, 0, ctx.ignore,
+                                                         int(kept.dtype == torch.bfloat16), _lib.stream_of(kept)), "causal_loss_bwd")
+        return grad if grad_kept is None else grad + grad_kept, None, None, None, None
 
 
 def causal_lm_loss(stock):
@@ -295,7 +309,8 @@ def causal_lm_loss(stock):
                 and logits.dtype in (torch.float16, torch.bfloat16) and classes.dtype is torch.int64 and logits.dim() >= 2
                 and logits.shape[-1] == vocab_size and vocab_size % 8 == 0 and classes.shape == logits.shape[:-1] and 0 < classes.numel() < 2 ** 31
                 and logits.is_contiguous() and classes.is_contiguous() and logits.data_ptr() % 16 == 0 and _lib.nobody_watches()):
-            return _CausalLoss.apply(logits, classes, classes.shape[-1] if shift_labels is None else 0, int(ignore_index))
+            return _CausalLoss.apply(logits, classes, classes.shape[-1] if shift_labels is None else 0, int(ignore_index),
+                                     torch.is_grad_enabled() and logits.requires_grad)[0]
         return stock(logits, labels, vocab_size, num_items_in_batch=num_items_in_batch, ignore_index=ignore_index, shift_labels=shift_labels, **kwargs)
     loss.stock = stock
     return loss

@@ -272,6 +272,10 @@ int q4_cast16(const void* src, void* dst, size_t n, int to_half, q4_stream_t str
  * trainer runs the framework's kernels). */
 int q4_causal_loss_fwd(const void* logits, const long long* labels, float* stats, float* row_loss, float* loss, float* count, int rows,
                        int V, int seq, long long ignore, int bf16, q4_stream_t stream);
+/* The same, and on the way copies the logits to `kept` [rows, V] (16-byte aligned) and every row's class to `classes` [rows]
+ * (either may be NULL): what a backward with seq = 0 needs when the caller's logits and labels may change before it. */
+int q4_causal_loss_fwd_keep(const void* logits, const long long* labels, float* stats, float* row_loss, float* loss, float* count,
+                            void* kept, long long* classes, int rows, int V, int seq, long long ignore, int bf16, q4_stream_t stream);
 int q4_causal_loss_bwd(const void* logits, const long long* labels, const float* stats, const float* grad_loss, const float* count,
                        void* grad, int rows, int V, int seq, long long ignore, int bf16, q4_stream_t stream);
 int q4_lora_grads(const void* v, const void* x, float* d_a, int K, const void* dy, const void* u, float* d_b, int N,

@@ -283,9 +283,51 @@ def test_causal_loss_of_confident_rows_and_of_logits_with_an_offset(offset, dtyp
     assert bool(((got - want).abs() <= tol * 1.001).all()), float(((got - want).abs() / tol).max())
 
 
+@pytest.mark.parametrize("shifted", [False, True])
+def test_causal_loss_keeps_what_its_backward_reads(shifted):
+    """Logits and labels are the program's own: written to before the backward (as a sampler or the next batch does), they
+    leave the gradient alone, once and again, as with the stock loss.  (The backward read them, and raised.)"""
+    V = 512
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    leaf = torch.randn((2, 9, V), generator=gen, device=DEV).half().requires_grad_(True)
+    labels = torch.randint(0, V, (2, 9), generator=gen, device=DEV)
+    labels[1, 4] = -100
+    kw = lambda l: dict(labels=None, shift_labels=l) if shifted else dict(labels=l)
+    (want,) = torch.autograd.grad(_stock_loss(leaf, vocab_size=V, **kw(labels)), leaf)
+    fused = fused_ops.causal_lm_loss(lambda *a, **k: (_ for _ in ()).throw(AssertionError("the stock loss ran")))
+    logits = leaf * 1
+    given = labels.clone()
+    loss = fused(logits, vocab_size=V, **kw(given))
+    with torch.no_grad():
+        logits.fill_(3.0)
+        given.fill_(1)
+    for last in (False, True):
+        (got,) = torch.autograd.grad(loss, leaf, retain_graph=not last)
+        assert rel(got, want) <= 2 ** -10
+    with torch.no_grad():
+        assert not fused(leaf, vocab_size=V, **kw(labels)).requires_grad
+
+
+def test_causal_loss_has_a_second_derivative():
+    """As the stock loss has, through the copy of the logits and through the gradient of the loss (it was refused)."""
+    V = 64
+    gen = torch.Generator(device=DEV).manual_seed(6)
+    leaf = torch.randn((1, 5, V), generator=gen, device=DEV).half().requires_grad_(True)
+    labels = torch.randint(0, V, (1, 5), generator=gen, device=DEV)
+    labels[0, 2] = -100
+    v = torch.randn(leaf.shape, generator=gen, device=DEV)
+    out = []
+    for f in (fused_ops.causal_lm_loss(_stock_loss), _stock_loss):
+        scale = torch.tensor(64.0, device=DEV, requires_grad=True)
+        (g,) = torch.autograd.grad(f(leaf, labels, V) * scale, leaf, create_graph=True)
+        out.append((g, *torch.autograd.grad((g.float() * v).sum() + 3 * f(leaf, labels, V) * scale, (leaf, scale))))
+    for a, b in zip(*out):
+        assert a.shape == b.shape and rel(a, b) <= 2 ** -9
+
+
 def test_causal_loss_at_the_edges():
     """No row with a class, infinities and NaN among the logits: what the framework's loss gives; the loss may be written in
-    place before its backward; a second derivative is refused; other calls go to the stock loss."""
+    place before its backward; other calls go to the stock loss."""
     V = 64
     fused = fused_ops.causal_lm_loss(_stock_loss)
     none = torch.full((1, 4), -100, device=DEV)
@@ -305,10 +347,6 @@ def test_causal_loss_at_the_edges():
     ref = x.detach().clone().requires_grad_(True)
     (_stock_loss(ref, labels, V) / 2).backward()
     assert rel(x.grad, ref.grad) <= 1e-3
-    loss = fused(x, labels, V)
-    (g,) = torch.autograd.grad(loss, x, create_graph=True)
-    with pytest.raises(RuntimeError):
-        g.sum().backward()
     seen = []
     spy = fused_ops.causal_lm_loss(lambda *a, **k: seen.append(1) or _stock_loss(*a, **k))
     for args, kw in (((x.float(), labels, V), {}), ((x, labels, V), dict(num_items_in_batch=torch.tensor(4, device=DEV))),

@@ -64,7 +64,7 @@ def test_pairs_that_wait_for_one_another_are_resident_together(resident):
     (1600, 5120, 5120, False, True, dict(KERNEL=2)),              # 84 in 256, 93 in 512
     (4096, 8192, 1024, True, True, dict(KERNEL=3, CUT=0)),        # whole tiles 84 us, dealt 107
     (1100, 11008, 4096, False, False, dict(KERNEL=4, CUT=1)),     # 84 us dealt; 94 in whole tiles of 288 rows
-    (2500, 8192, 8192, False, False, dict(KERNEL=4, CUT=1)),      # 260 us dealt; 306 in whole tiles of 288 rows
+    (2500, 8192, 8192, False, False, dict(KERNEL=4, CUT=1)),      # 267 us dealt; 306 in whole tiles of 288 rows
     (1200, 11008, 4096, True, False, dict(KERNEL=4, ACT=1)),      # 110 us; the pair kernel 129
     (128, 8192, 1024, True, False, dict(KERNEL=4, ACT=1)),        # 29 us; 18 pairs a tile of the pair kernel 100
 ])
