@@ -336,7 +336,8 @@ def patch_llama(model: nn.Module, fuse_gate_up: bool = False) -> nn.Module:
         elif isinstance(mod, ml.LlamaMLP) and type(getattr(mod, "act_fn", None)).__name__ in ("SiLU", "SiLUActivation"):
             mod.forward = (lambda x, _m=mod: _m.down_proj(swiglu(_m.gate_proj(x), _m.up_proj(x))))
     ml.apply_rotary_pos_emb = apply_rotary_pos_emb
+    from transformers.loss.loss_utils import ForCausalLMLoss
     for mod in model.modules():
-        if isinstance(mod, ml.LlamaForCausalLM) and not hasattr(mod.loss_function, "stock"):
+        if isinstance(mod, ml.LlamaForCausalLM) and mod.loss_function is ForCausalLMLoss:      # (a loss of the program's own stays)
             mod.loss_function = causal_lm_loss(mod.loss_function)
     return model

@@ -240,3 +240,30 @@ def test_llama_patches_on_tiny_model():
     assert isinstance(model.model.layers[0].mlp, patch.QuantLlamaMLP)
     assert model.model.layers[0].self_attn.qkv_proj.out_features == 128 + 64 + 64
     assert torch.allclose(out.float(), ref.float(), atol=5e-2, rtol=5e-2)
+
+
+@pytest.mark.parametrize("chosen", ["stock", "assigned", "type"])
+def test_patch_llama_leaves_a_loss_of_the_programs_own(chosen, monkeypatch):
+    """Only the framework's next-token cross entropy is replaced: a loss function that the program assigned, or another loss
+    type, is what runs after the patch too.  (Any loss was wrapped, and 16-bit logits on a GPU never reached it.)"""
+    from transformers import LlamaConfig, LlamaForCausalLM
+    from transformers.loss.loss_utils import LOSS_MAPPING
+    from transformers.models.llama import modeling_llama as ml
+    from alpaca_lora_4bit_b200 import fused_ops
+    monkeypatch.setattr(ml, "apply_rotary_pos_emb", ml.apply_rotary_pos_emb)
+    model = LlamaForCausalLM(LlamaConfig(hidden_size=64, intermediate_size=64, num_hidden_layers=1, num_attention_heads=2,
+                                         num_key_value_heads=2, vocab_size=32, max_position_embeddings=16))
+    if chosen == "assigned":
+        model.loss_function = lambda logits, labels, vocab_size, **kw: logits.float().square().mean()
+    elif chosen == "type":
+        model.loss_type = next(k for k, v in LOSS_MAPPING.items() if v is not LOSS_MAPPING["ForCausalLM"])
+    before = model.loss_function
+    fused_ops.patch_llama(model)
+    if chosen == "stock":
+        assert model.loss_function is not before and model.loss_function.stock is before
+        assert fused_ops.patch_llama(model).loss_function.stock is before
+        ids = torch.arange(8)[None]
+        logits = torch.randn(1, 8, 32)
+        assert torch.equal(model.loss_function(logits, ids, 32), before(logits, ids, 32))
+    else:
+        assert model.loss_function is before
