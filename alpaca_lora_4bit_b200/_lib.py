@@ -76,6 +76,7 @@ _SIGNATURES = {
                               ctypes.c_float, ctypes.c_float, ctypes.c_float, c_void_p, ctypes.c_float, ctypes.c_float, c_int, c_void_p, c_void_p]),
     "q4_device_status": (c_int, [ctypes.POINTER(c_uint)]),
     "q4_gemv_status": (c_int, [c_void_p, c_size_t, ctypes.POINTER(c_uint)]),
+    "q4_gemv_device_status": (c_int, [c_void_p]),
     "q4_gemv_static_status": (c_int, [ctypes.POINTER(c_uint)]),
     "q4_gemv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_int, c_int, c_int, c_int, c_int, c_int, c_uint, c_void_p, c_size_t, c_void_p]),
@@ -240,45 +241,31 @@ def dtype_code(dt: torch.dtype) -> int:
 
 _workspaces: dict = {}
 _WS_BYTES = 4 << 20          # covers q4_gemv_workspace_bytes() of every shape the decode kernels accept
-
-
-def workspace_for(device: torch.device, stream_handle: int) -> torch.Tensor:
-    """The decode workspace of one (device, stream): allocated zeroed on first use, then reused."""
-    key = (device.index, stream_handle)
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = torch.zeros(_WS_BYTES, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
-
-
+_DECODE_WS_HEAD = 131072     # what the decode kernels need zero before the first call and leave zero
 _gemm_workspaces: dict = {}
-_GEMM_WS_HEAD = 65536                      # arrival counters: zero before the first call, left zero by every kernel
-_capture_workspaces: dict = {}             # (device index, stream handle) -> (id of the capture, its workspaces, the newest last)
+_GEMM_WS_HEAD = 65536        # arrival counters: zero before the first call, left zero by every kernel
+
+# Workspaces of stream captures: (device index, stream handle) and, for decode, the same with "decode" -> (id of the
+# capture, its workspaces, the newest last).
+# A graph holds the addresses of its products' workspaces for as long as it lives, so every capture has its own, from the memory
+# of its graph and cleared by it.  (The stream's own one makes way for a larger one; first asked for inside a capture it was cleared
+# by that graph's replay alone; and torch captures every graph on one stream unless told otherwise, so that two graphs
+# replayed on two streams counted their arrivals in one place.)  A graph is larger by them: 4 MiB with decode products, 24 to 42
+# with fused ones.  They are only held here for the next product of the same capture, and let go by the first eager product after
+# it: an eager call of another thread in the middle of a capture costs that capture a second workspace, nothing else.
+_capture_workspaces: dict = {}
 
 
-def gemm_workspace_for(device: torch.device, stream_handle: int, nbytes: int) -> torch.Tensor:
-    """Scratch of the fused GEMM for one (device, stream): zeroed when (re)allocated, only ever grows.
-    The kernels leave its counter head zero, so calls ordered on the stream can share it.
-
-    A stream capture has workspaces of its own, from the memory of its graph and cleared by it: the graph holds their
-    addresses for as long as it lives, when the stream's own one may long have made way for a larger one."""
-    key = (device.index, stream_handle)
-    if torch.cuda.is_current_stream_capturing():
-        capture = capture_id(stream_handle)
-        held = _capture_workspaces.get(key)
-        if held is None or held[0] != capture:
-            held = _capture_workspaces[key] = (capture, [])
-        if not held[1] or held[1][-1].numel() < nbytes:
-            ws = torch.empty(max(nbytes, 24 << 20), dtype=torch.uint8, device=device)
-            ws[:_GEMM_WS_HEAD].zero_()
-            held[1].append(ws)             # (the earlier ones stay until the capture is over: nothing else of it takes their place)
-        return held[1][-1]
-    ws = _gemm_workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 24 << 20), dtype=torch.uint8, device=device)
-        _gemm_workspaces[key] = ws
-    return ws
+def _of_capture(key, capture: int, nbytes: int, head: int, device: torch.device) -> torch.Tensor:
+    held = _capture_workspaces.get(key)
+    if held is None or held[0] != capture:
+        held = _capture_workspaces[key] = (capture, [])
+    if not held[1] or held[1][-1].numel() < nbytes:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        ws[:head].zero_()
+        held[1].append(ws)
+        return ws
+    return held[1][-1]
 
 
 def capture_id(stream_handle: int) -> int:
@@ -288,15 +275,46 @@ def capture_id(stream_handle: int) -> int:
     return out.value
 
 
-def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Per-(device, stream) zero-initialised scratch that only ever grows.
+def _capture_of(stream_handle: int) -> int:
+    """0 outside a capture; the legacy default stream (handle 0) cannot be captured."""
+    return capture_id(stream_handle) if stream_handle and torch.cuda.is_current_stream_capturing() else 0
 
-    The decode kernel keeps its arrival counters zero between launches, so the buffer is
-    cleared once, when it is (re)allocated.
-    """
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+
+def workspace_for(device: torch.device, stream_handle: int) -> torch.Tensor:
+    """The decode workspace of one (device, stream): allocated zeroed on first use, then reused; a capture has its own."""
+    key = (device.index, stream_handle)
+    capture = _capture_of(stream_handle)
+    if capture:
+        return _of_capture(key + ("decode",), capture, _WS_BYTES, _DECODE_WS_HEAD, device)
+    _capture_workspaces.clear()
     ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+    if ws is None:
+        ws = torch.zeros(_WS_BYTES, dtype=torch.uint8, device=device)
         _workspaces[key] = ws
+    return ws
+
+
+def gemm_workspace_for(device: torch.device, stream_handle: int, nbytes: int) -> torch.Tensor:
+    """Scratch of the fused GEMM for one (device, stream): zeroed when (re)allocated, only ever grows; a capture has its own.
+    The kernels leave its counter head zero, so calls ordered on the stream can share it."""
+    key = (device.index, stream_handle)
+    capture = _capture_of(stream_handle)
+    if capture:
+        return _of_capture(key, capture, max(nbytes, 24 << 20), _GEMM_WS_HEAD, device)
+    _capture_workspaces.clear()
+    ws = _gemm_workspaces.get(key)
+    if ws is None or ws.numel() < nbytes:
+        ws = torch.zeros(max(nbytes, 24 << 20), dtype=torch.uint8, device=device)
+        _gemm_workspaces[key] = ws
+    return ws
+
+
+def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+    """The decode workspace of the current stream, grown to ``nbytes`` where it is smaller (and cleared then)."""
+    stream = torch.cuda.current_stream(device).cuda_stream
+    ws = workspace_for(device, stream)
+    if ws.numel() < nbytes:
+        ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
+        if not _capture_of(stream):
+            _workspaces[(device.index, stream)] = ws
     return ws

@@ -34,6 +34,14 @@ constexpr int GEMV_WARPS = 8;
 constexpr int GEMV_TN = 32;          // columns per CTA
 // Workspace layout: a fixed 64 KiB head of arrival counters (one per column tile, so the
 // counters of one shape never alias the partial sums of another), then the partial sums.
+// Beside the word in the workspace: one per device, which is still there when the workspace is out of reach - a captured
+// graph's own, in the memory of its graph.
+__device__ unsigned g_gemv_status = 0;
+__device__ __forceinline__ void wait_expired(unsigned* status) {
+  atomicExch(status, Q4_STATUS_WAIT_EXPIRED);
+  atomicExch(&g_gemv_status, Q4_STATUS_WAIT_EXPIRED);
+}
+
 constexpr size_t GEMV_WS_HEAD = 131072;           // first half: arrival counters and the status word; second half: the
                                                   // exchange slots of the warp-specialised kernel (GEMV_WS_SLOTS)
 
@@ -459,7 +467,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
       uint4 xv[MT][4];
       load_x(xv, ux, 0);
       if (!mbar_wait_warp(&my_full[st], use & 1, flags[0] ? 4u : 20000u)) {
-        flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED);
+        flags[0] = 1; wait_expired(sp.status);
       }
       if (warp == 0 && lane == 0) trace_mark(sp.trace, 3 + 2 * n);
       const unsigned char* stg = my_stages + (size_t)st * GEMV_STAGE_BYTES;
@@ -820,7 +828,7 @@ gemv_fast_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         uint32_t tries = 0;
         const uint32_t lim = flags[0] ? 64u : 20000000u;
         while (!mbar_test_wait(&my_full[st], use & 1) && ++tries < lim) {}
-        if (tries >= lim) { flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED); }
+        if (tries >= lim) { flags[0] = 1; wait_expired(sp.status); }
       }
       if (warp == 0 && lane == 0) trace_mark(trc, 3 + 2 * n);
       if (warp == 0 && lane == 0 && n == 0) trace_mark_ns(trc, 43);
@@ -1070,7 +1078,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
     auto issue_meta = [&](int tile) {
       const int seq = tile - tile_first, slot = seq & 1;
       if (seq >= 2 && !mbar_wait_sleep_bounded(&mempty[slot], ((seq >> 1) & 1) ^ 1, 200000u)) {
-        flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED);
+        flags[0] = 1; wait_expired(sp.status);
       }
       unsigned char* m = smem + L.meta + slot * L.meta_slot;
       mbar_arrive_expect_tx(&mfull[slot], meta_tx);
@@ -1137,7 +1145,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
         if (__any_sync(MASK, ready)) { idle = 0; continue; }
         __nanosleep(40);
         if (++idle > (flags[0] ? 64u : 4000000u)) {
-          if (lane == 0) { flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED); }
+          if (lane == 0) { flags[0] = 1; wait_expired(sp.status); }
           break;
         }
       }
@@ -1160,7 +1168,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
       volatile unsigned long long* slot = sp.slots + (size_t)cc * 32 + lane;
       unsigned long long v = *slot;
       for (int i = 0; (v >> 32) == 0ull && i < (flags[0] ? 8 : 100000); ++i) { __nanosleep(100); v = *slot; }
-      if ((v >> 32) == 0ull) { flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED); }
+      if ((v >> 32) == 0ull) { flags[0] = 1; wait_expired(sp.status); }
       acc += __uint_as_float((unsigned)v);       // in CTA order: the result does not depend on timing
       *slot = 0ull;
     }
@@ -1300,7 +1308,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
       return;
     }
     // the first part of a tile that later CTAs continue: their sums, collected by the helper warp
-    if (!mbar_spin_bounded(rfull, 0, flags[0] ? 64u : 20000000u)) { flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED); }
+    if (!mbar_spin_bounded(rfull, 0, flags[0] ? 64u : 20000000u)) { flags[0] = 1; wait_expired(sp.status); }
     store_y_biased(p, 0, tc0 + col, v + remote[col] + bv);
   };
 
@@ -1315,7 +1323,7 @@ gemv_ws_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
       const int st = n % S;
       const uint32_t lim = flags[0] ? 64u : 20000000u;
       if ((!meta_ready && !mbar_spin_bounded(&mfull[slot], (seq >> 1) & 1, lim)) || !mbar_spin_bounded(&full[warp * S + st], (n / S) & 1, lim)) {
-        flags[0] = 1; atomicExch(sp.status, Q4_STATUS_WAIT_EXPIRED);
+        flags[0] = 1; wait_expired(sp.status);
       }
       meta_ready = true;
       if (tile == tile_last && u + W >= seg_u1 && warp == 0 && lane == 0 && Gd < (int)gridDim.x)
@@ -1511,7 +1519,7 @@ gemv_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   if (threadIdx.x < 2 * W * S + 11) mbar_fence_init();
   __syncthreads();
   pdl_launch_dependents();
-  auto expired = [&]() { flags[0] = 1; atomicExch(rp.status, Q4_STATUS_WAIT_EXPIRED); };
+  auto expired = [&]() { flags[0] = 1; wait_expired(rp.status); };
 
   if (warp == W) {
     // ---- issuer: lane w the units of consumer w, lane W the rounds' digits, lane W + 1 the tiles' metadata ----
@@ -2356,4 +2364,11 @@ extern "C" int q4_layer_gemv(const q4_layer_t* l, const void* x, void* y, int M,
                          workspace, workspace_bytes, stream);
   t_next_layer = nullptr;
   return rc;
+}
+
+extern "C" int q4_gemv_device_status(unsigned* out) {
+  if (!out) return fail(Q4_E_BADARG, "gemv_device_status: null pointer");
+  if (int e = check_cuda(cudaMemcpyFromSymbol(out, g_gemv_status, sizeof(unsigned)), "read decode status")) return e;
+  const unsigned none = 0;
+  return *out ? check_cuda(cudaMemcpyToSymbol(g_gemv_status, &none, sizeof(unsigned)), "clear decode status") : Q4_OK;
 }

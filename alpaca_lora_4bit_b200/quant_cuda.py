@@ -113,13 +113,23 @@ def gemv(x, qweight, y, scales, zeros, g_idx, groupsize, flags, bias=None) -> No
                 _lib.check(rc, "gemv")
 
 
-_decode_ws: dict = {}          # (device index, stream handle) -> (pointer, bytes, tensor)
+_decode_ws: dict = {}          # (device index, stream handle) -> (pointer, bytes, tensor): of eager calls
 
 try:                                                      # the handle of the current stream without building a Stream object
     _raw_stream = torch._C._cuda_getCurrentRawStream
 except AttributeError:                                    # pragma: no cover - older / newer torch without the private hook
     def _raw_stream(idx):
         return torch.cuda.current_stream(idx).cuda_stream
+
+
+def _decode_workspace(device, idx, st):
+    """The workspace of a decode product on stream ``st``, as ``_decode_ws`` keeps it; a capture's is looked up every time
+    (and the eager calls that follow a capture come here once, to let go of what it held)."""
+    t = _lib.workspace_for(device, st)
+    w = (t.data_ptr(), t.numel(), t)
+    if _lib._workspaces.get((idx, st)) is t:
+        _decode_ws[(idx, st)] = w
+    return w
 
 
 class _LayerPlan:
@@ -190,9 +200,8 @@ def decode_planned(x, qweight, scales, zeros, groupsize, max_rows):
     y = x.new_empty((M, p.N))
     st = _raw_stream(p.index)
     w = _decode_ws.get((p.index, st))
-    if w is None:
-        t = _lib.workspace_for(p.device, st)
-        w = _decode_ws[(p.index, st)] = (t.data_ptr(), t.numel(), t)
+    if w is None or _lib._capture_workspaces or (st and torch.cuda.is_current_stream_capturing()):
+        w = _decode_workspace(p.device, p.index, st)
     rc = (_layer_gemv or _bind_layer_gemv())(p.handle, x.data_ptr(), y.data_ptr(), M, w[0], w[1], st)
     if rc:
         _lib.check(rc, "layer_gemv")
@@ -222,9 +231,8 @@ def decode_v2(x, qweight, scales, zeros, groupsize, plan_key=None):
     y = torch.empty((M, N), dtype=torch.float16, device=dev)
     st = _raw_stream(idx)
     w = _decode_ws.get((idx, st))
-    if w is None:
-        t = _lib.workspace_for(dev, st)
-        w = _decode_ws[(idx, st)] = (t.data_ptr(), t.numel(), t)
+    if w is None or _lib._capture_workspaces or (st and torch.cuda.is_current_stream_capturing()):
+        w = _decode_workspace(dev, idx, st)
     rc = _lib.lib().q4_gemv(x.data_ptr(), qweight.data_ptr(), y.data_ptr(), scales.data_ptr(), zeros.data_ptr(), None, None,
                             M, K, N, G, groupsize, _lib.Q4_F16, 0, w[0], w[1], st)
     if rc:
@@ -240,9 +248,8 @@ def gemv_new(x, qweight, scales, zeros, g_idx, bias, groupsize, flags):
     idx = x.device.index
     st = _raw_stream(idx)
     w = _decode_ws.get((idx, st))
-    if w is None:
-        t = _lib.workspace_for(x.device, st)
-        w = _decode_ws[(idx, st)] = (t.data_ptr(), t.numel(), t)
+    if w is None or _lib._capture_workspaces or (st and torch.cuda.is_current_stream_capturing()):
+        w = _decode_workspace(x.device, idx, st)
     return (_lib._torch_call or _lib.torch_call()).gemv(x, qweight, scales, zeros, g_idx, bias, groupsize, flags, w[2])
 
 
@@ -351,7 +358,7 @@ def gemm_new(x, qweight, out, scales, zeros, g_idx, transpose=False, bias=None, 
     if need is None:
         need = _gemm_ws_bytes[(K, N, G)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, G))
     ws = _lib._gemm_workspaces.get((idx, st))
-    if ws is None or ws.numel() < need or torch.cuda.is_current_stream_capturing():
+    if ws is None or ws.numel() < need or _lib._capture_workspaces or (st and torch.cuda.is_current_stream_capturing()):
         ws = _lib.gemm_workspace_for(dev, st, need)
     zt, seq_gs = None, 0
     if g_idx is not None and G > 0:
@@ -376,7 +383,7 @@ def gemm_v1_new(x, qweight, scales, zeros, bias=None, residual=None):
     if need is None:
         need = _gemm_ws_bytes[(K, N, 1)] = int(_lib.lib().q4_gemm_workspace_bytes(K, N, 1))
     ws = _lib._gemm_workspaces.get((dev.index, st))
-    if ws is None or ws.numel() < need or torch.cuda.is_current_stream_capturing():
+    if ws is None or ws.numel() < need or _lib._capture_workspaces or (st and torch.cuda.is_current_stream_capturing()):
         ws = _lib.gemm_workspace_for(dev, st, need)
     return (_lib._torch_call or _lib.torch_call()).gemm_v1(x, qweight, scales, zeros, bias, residual, ws)
 
@@ -501,8 +508,9 @@ def device_status() -> int:
     """Status of every kernel family on the current device (synchronises): 0 unless a bounded device-side
     wait expired in a fused GEMM kernel (one word per device) or in a decode kernel (one word per decode
     workspace, i.e. per stream that has run a decode product, plus the built-in scratch of
-    ``q4_gemv_static``).  A non-zero decode word means the workspace head must be cleared before reuse;
-    this function does that for the workspaces this module owns."""
+    ``q4_gemv_static``, and one per device for all of them, captured graphs' own workspaces included).  A
+    non-zero decode word means the workspace head must be cleared before reuse; this function does that for
+    the workspaces this module owns, and a captured graph clears its own on every replay."""
     import ctypes
     L = _lib.lib()
     v = ctypes.c_uint(0)
@@ -517,6 +525,8 @@ def device_status() -> int:
             ws[:131072].zero_()
             status = status or v.value
     _lib.check(L.q4_gemv_static_status(ctypes.byref(v)), "gemv_static_status")
+    status = status or v.value
+    _lib.check(L.q4_gemv_device_status(ctypes.byref(v)), "gemv_device_status")
     return status or v.value
 
 

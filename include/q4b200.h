@@ -308,6 +308,10 @@ int q4_device_status(unsigned* out);
  * is used again (128 KiB from the library version that exchanges shared column tiles through it).
  * No counterpart in the reference, whose kernels wait on nothing. */
 int q4_gemv_status(const void* workspace, size_t workspace_bytes, unsigned* out);
+/* One word per device for all decode products on it, whatever workspace they were given (a captured graph's own, say, that
+ * the host no longer holds): synchronises the device and copies the word to *out; a non-zero word is cleared once it has
+ * been reported.  The workspace of the call that set it still has to be cleared, where nothing clears it before every use. */
+int q4_gemv_device_status(unsigned* out);
 /* The status word of the built-in scratch of q4_gemv_static on the current device; a non-zero word
  * is cleared once it has been reported (q4_gemv_static itself re-zeroes the counters before every
  * launch but leaves the word for this call to find). */

@@ -55,7 +55,7 @@ def test_bad_arguments_are_rejected_without_a_device():
     v = ctypes.c_uint(0)
     assert L.q4_gemv_status(None, 1 << 20, ctypes.byref(v)) == -1
     assert L.q4_gemv_status(fake, 100, ctypes.byref(v)) == -4
-    assert L.q4_gemv_static_status(None) == -1
+    assert L.q4_gemv_static_status(None) == -1 and L.q4_gemv_device_status(None) == -1
     assert L.q4_gemv_set_variant(3) == -1 and L.q4_gemv_set_variant(128) == -1 and L.q4_gemv_set_variant(4 + 8 + 1) == 0
     assert L.q4_gemv_set_variant(0) == 0
     assert L.q4_gemv_workspace_bytes(1, 100, 128) == 0

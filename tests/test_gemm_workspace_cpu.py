@@ -1,4 +1,7 @@
 """Workspaces of the fused products: one per stream that grows, and one per stream capture."""
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -37,36 +40,34 @@ def test_a_capture_never_holds_a_workspace_that_growth_replaces(capture):
     assert _lib.gemm_workspace_for(CPU, STREAM, 50 * mib) is not eager
 
 
-@pytest.mark.gpu
-def test_a_captured_product_survives_growth_of_the_stream_workspace():
-    """Two captures on one stream, the second with a larger layer, the allocator's cache emptied in between: the first
-    graph still gives the eager product, on inputs it has not seen."""
-    from alpaca_lora_4bit_b200 import quant_cuda, synth
-    dev = torch.device("cuda")
-    small, large = (synth.make_layer(K, N, 32, act_order=True, seed=K).to(dev) for K, N in ((512, 512), (4096, 2048)))
-    xs = [synth.make_acts(300, L.qweight.shape[0] * 8, seed=3).to(dev) for L in (small, large)]
-    outs = [torch.empty((300, L.qweight.shape[1]), dtype=torch.float16, device=dev) for L in (small, large)]
-    stream, graphs = torch.cuda.Stream(), []
+def test_a_capture_has_a_decode_workspace_of_its_own(capture, monkeypatch):
+    """First asked for inside a capture, the decode workspace was cleared by that graph's replay alone and then kept for the
+    stream: later captures and eager calls on it counted arrivals in memory that nothing had cleared."""
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    capture["id"] = 1
+    first = _lib.workspace_for(CPU, STREAM)
+    assert first.numel() == _lib._WS_BYTES and int(first[:_lib._DECODE_WS_HEAD].sum()) == 0
+    assert _lib.workspace_for(CPU, STREAM) is first and not _lib._workspaces
+    fused = _lib.gemm_workspace_for(CPU, STREAM, 1)
+    assert fused is not first and _lib.workspace_for(CPU, STREAM) is first
+    capture["id"] = 2
+    second = _lib.workspace_for(CPU, STREAM)
+    assert second is not first and int(second[:_lib._DECODE_WS_HEAD].sum()) == 0
+    capture["id"] = 0
+    eager = _lib.workspace_for(CPU, STREAM)
+    assert eager is not first and eager is not second and int(eager.sum()) == 0 and _lib.workspace_for(CPU, STREAM) is eager
+    capture["id"] = 3
+    assert _lib.workspace_for(CPU, STREAM) is not eager
 
-    def product(i):
-        L = (small, large)[i]
-        quant_cuda.gemm(xs[i], L.qweight, outs[i], L.scales, L.qzeros, L.g_idx)
 
-    for i in (0, 1):
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=stream):
-            if i:
-                product(0)
-            product(i)
-        graphs.append(graph)
-        torch.cuda.empty_cache()
-    for x in xs:
-        x.mul_(0.5)
-    graphs[1].replay()
-    graphs[0].replay()
-    torch.cuda.synchronize()
-    got = [o.clone() for o in outs]
-    for i in (0, 1):
-        product(i)
-    torch.cuda.synchronize()
-    assert all(torch.equal(a, b) for a, b in zip(got, outs)) and quant_cuda.device_status() == 0
+@pytest.mark.parametrize("ask", [lambda: _lib.workspace_for(CPU, STREAM), lambda: _lib.gemm_workspace_for(CPU, STREAM, 1)])
+def test_what_a_capture_held_is_let_go_by_the_next_eager_call(capture, monkeypatch, ask):
+    """... so that the memory goes with its graph.  (The last capture's workspaces of every stream stayed for good.)"""
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    capture["id"] = 1
+    kept = [weakref.ref(_lib.workspace_for(CPU, STREAM)), weakref.ref(_lib.gemm_workspace_for(CPU, STREAM + 1, 1))]
+    assert all(r() is not None for r in kept)
+    capture["id"] = 0
+    ask()
+    gc.collect()
+    assert all(r() is None for r in kept)
