@@ -5,6 +5,7 @@ import torch
 
 from alpaca_lora_4bit_b200 import autograd_4bit as a4, matmul_utils_4bit as mm4b, models, quant_cuda, synth
 from oracle import q4_oracle as orc
+from tests import test_gemm_plan_cpu as gemm_plan
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -692,7 +693,7 @@ def test_short_prompts_cut_at_short_contractions(K, N, M):
 
 
 @pytest.mark.parametrize("K,N,M", [(512, 512, 17), (512, 256, 31), (256, 512, 33), (512, 512, 97), (512, 256, 160), (512, 512, 257),
-                                   (512, 256, 289), (512, 512, 333), (256, 256, 513), (512, 512, 801)])     # heights of 32 .. 256
+                                   (512, 256, 289), (512, 512, 333), (256, 256, 513), (512, 512, 801)])
 def test_tiles_of_every_height(K, N, M):
     """Rows that make tiles of other heights than 256, whole along K."""
     test_short_prompts_cut_between_pairs(K, N, M)
@@ -733,7 +734,7 @@ def _product_with_everything(layer, M, seed):
 @pytest.mark.parametrize("K,N,M", [(512, 512, 258), (512, 256, 352), (512, 512, 384), (512, 256, 385), (512, 256, 700), (512, 256, 769),
                                    (4096, 4096, 333), (2304, 256, 300), (4096, 11008, 333), (1024, 9984, 1152)])
 def test_tall_tiles(K, N, M):
-    """Tiles of more than 256 rows: two MMAs on one dequantised operand, whole, in clusters and in runs."""
+    """Rows above 256 of sequential layers, in however many tiles the plan makes of them (the forms one by one: below)."""
     _product_with_everything(synth.make_layer(K, N, 128, act_order=False, seed=K + M).to(DEV), M, M)
 
 
@@ -757,3 +758,21 @@ def test_act_order_forward_takes_any_order_of_groups(kind):
         layer.g_idx.copy_((torch.arange(K, device=DEV) // 32 % G).to(torch.int32))
     for M in (40, 300):
         _product_with_everything(layer, M, M)
+
+
+@pytest.mark.parametrize("K,N,M,act_order,form", [
+    (1024, 9984, 257, False, dict(TILE=288, CUT=0, PAIRS=39)), (1024, 9984, 352, False, dict(TILE=352, CUT=0, PAIRS=39)),    # whole, one round
+    (1024, 9984, 1400, False, dict(TILE=288, CUT=0, PAIRS=74)), (1024, 9984, 1152, False, dict(TILE=384, CUT=0, PAIRS=74)),  # whole, in rounds
+    (5120, 5120, 333, False, dict(TILE=352, CLUSTER=3)), (2304, 5120, 384, False, dict(TILE=384, CLUSTER=3)),                # in clusters
+    (4096, 6144, 333, False, dict(TILE=352, CLUSTER=2)),
+    (4096, 11008, 333, False, dict(TILE=352, CUT=1, CLUSTER=1)), (11008, 4096, 1038, False, dict(TILE=352, CUT=1, CLUSTER=1)),     # in runs
+    (4096, 4096, 1600, False, dict(TILE=320, CUT=1, CLUSTER=1)),
+    (1024, 9984, 333, True, dict(TILE=352, CUT=0, PAIRS=39)), (1024, 20480, 800, True, dict(TILE=288, CUT=0, PAIRS=74)),
+    (4096, 4096, 768, True, dict(TILE=384, CLUSTER=2)), (2304, 4096, 333, True, dict(TILE=352, CLUSTER=3)), (11008, 3584, 270, True, dict(TILE=288, CLUSTER=4)),
+    (4096, 11008, 257, True, dict(TILE=288, CUT=1, CLUSTER=1)), (11008, 4096, 1100, True, dict(TILE=384, CUT=1, CLUSTER=1)),
+    (4096, 4096, 77, True, dict(TILE=96, CLUSTER=3)), (8192, 1024, 128, True, dict(TILE=128, CUT=1, CLUSTER=1))])
+def test_forms_of_the_tensor_memory_kernel(K, N, M, act_order, form):
+    """Every form of the kernel that a cut, a cluster, a tall tile or an act-order layer makes, by the plan of this device."""
+    p = gemm_plan.plan(M, K, N, K // 128, act_order, resident=None)
+    assert p[gemm_plan.KERNEL] == 4 and p[gemm_plan.ACT] == act_order and {k: p[getattr(gemm_plan, k)] for k in form} == form, p
+    _product_with_everything(synth.make_layer(K, N, 128, act_order=act_order, seed=K + M).to(DEV), M, M)
