@@ -134,7 +134,7 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t cta_addr, uint32_t rank) {
   return r;
 }
 // all threads of all CTAs of the cluster.  (.aligned: a warp comes to it as one - a lane that ran a loop of its own meets the
-// others first, here and in named_bar_sync, instead of where the compiler happens to let it.)
+// others first, here and in named_bar_sync_warps, instead of where the compiler happens to let it.)
 __device__ __forceinline__ void cluster_sync_all() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -189,8 +189,13 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
-  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// ... by warps whose lanes may have come apart.  (Not in the decode kernels, whose lanes part for single instructions only: four
+// 7B layers of one token took 152 us with the plain form and 154 with this one.)
+__device__ __forceinline__ void named_bar_sync_warps(int id, int threads) {
+  __syncwarp();
+  named_bar_sync(id, threads);
 }
 
 #endif  // __CUDACC__

@@ -192,7 +192,7 @@ q4_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__
         *reinterpret_cast<uint4*>(tab + g * 512 + 16 * c8) = s;
         *reinterpret_cast<uint4*>(tab + g * 512 + 256 + 16 * c8) = z;
       }
-      named_bar_sync(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);
+      named_bar_sync_warps(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);
     }
     // packed words of the stage: rows (k0/8 + r), columns ncol0 .. ncol0+7
     auto word_ptr = [&](int it) -> const uint32_t* {

@@ -397,7 +397,7 @@ q4_gemm2_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       prefetch(j0, R0);                              // in flight while the tables below are built
       if (!TRANSPOSE && !p.zp_table && out0 != tab_out0) {
         // tables for the CTA's 128 columns: scale and rn(s*(z+1)) of every group
-        if (tab_out0 >= 0) named_bar_sync(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);      // all readers of the old tables are done
+        if (tab_out0 >= 0) named_bar_sync_warps(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);      // all readers of the old tables are done
         for (int i = (dw << 5) | lane; i < p.G * 16; i += GM_DEQ_THREADS * GM_DEQ_GROUPS) {
           const int g = i >> 4, c8 = i & 15;
           const uint4 s = __ldg(reinterpret_cast<const uint4*>(p.scales + (size_t)g * N + out0 + 8 * c8));
@@ -406,7 +406,7 @@ q4_gemm2_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
           *reinterpret_cast<uint4*>(tab + g * 512 + 16 * c8) = s;
           *reinterpret_cast<uint4*>(tab + g * 512 + 256 + 16 * c8) = z;
         }
-        named_bar_sync(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);
+        named_bar_sync_warps(1, GM_DEQ_THREADS * GM_DEQ_GROUPS);
         if (tl == 0 && dw == 0 && lane == 0) gm_mark_ns(p.trace, 104);
         tab_out0 = out0;
       }

@@ -507,7 +507,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       ask(j, R0);
       const int c0 = (wi.tile / m_tiles) * G2_TILE_N + 128 * (int)rank;
       if (ACT && c0 != tab_n0) {
-        if (tab_n0 >= 0) named_bar_sync(5, 128 * G3_GROUPS);       // the readers of the table before are done
+        if (tab_n0 >= 0) named_bar_sync_warps(5, 128 * G3_GROUPS);       // the readers of the table before are done
 #pragma unroll 1
         for (int i0 = threadIdx.x - 128; i0 < p.G * 16; i0 += 4 * 128 * G3_GROUPS) {
           uint4 sv[4];
@@ -529,7 +529,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
             to[1] = make_uint4(prmt(s8.z, z8.z, 0x5410), prmt(s8.z, z8.z, 0x7632), prmt(s8.w, z8.w, 0x5410), prmt(s8.w, z8.w, 0x7632));
           }
         }
-        named_bar_sync(5, 128 * G3_GROUPS);
+        named_bar_sync_warps(5, 128 * G3_GROUPS);
         tab_n0 = c0;
       }
       while (j < nst) {
@@ -551,14 +551,14 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
       // the quarter's shared-memory rows are free once its epilogue warp has stored the item before (a meeting of
       // the quarter's four warps: named barrier 1 + quarter)
-      named_bar_sync(1 + quarter, 128);
+      named_bar_sync_warps(1 + quarter, 128);
       if (lane == 0) wait_bar_idle(last_full, 0, abort_flag, 100);
       __syncwarp();
       tc_fence_after();
       const Shared sh = shared_of(w_last, quarter);
       if (sh.reducer) {
         await_partials(sh);
-        named_bar_sync(1 + quarter, 128);                        // all four warps have seen the count: the epilogue warp may clear it
+        named_bar_sync_warps(1 + quarter, 128);                        // all four warps have seen the count: the epilogue warp may clear it
       }
 #pragma unroll 1
       for (int cb = grp; cb < nb; cb += G3_GROUPS + 1) {
@@ -570,7 +570,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       }
       if (sh.shared && !sh.reducer) {
         __threadfence();
-        named_bar_sync(1 + quarter, 128);                        // this warp's sums are out: the epilogue warp counts for all four
+        named_bar_sync_warps(1 + quarter, 128);                        // this warp's sums are out: the epilogue warp counts for all four
       }
     }
   } else if (warp >= 4 + 4 * G3_GROUPS) {
@@ -584,7 +584,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       const int m_base = (wi.tile % m_tiles) * TR;
       const int rows = min(TR, p.M - m_base);                     // rows of x the tile really has
       const float bv = p.bias ? __half2float(p.bias[n0 + lane]) : 0.f;
-      if (item == n_items - 1) named_bar_sync(1 + quarter, 128);   // the helpers may use this quarter's rows from here
+      if (item == n_items - 1) named_bar_sync_warps(1 + quarter, 128);   // the helpers may use this quarter's rows from here
       if (lane == 0) wait_bar_idle(acc_full, item & 1, abort_flag, 100);
       __syncwarp();
       tc_fence_after();
@@ -596,7 +596,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       const Shared sh = shared_of(wi, quarter);
       if (sh.reducer) {
         await_partials(sh);
-        if (shared_out) named_bar_sync(1 + quarter, 128);
+        if (shared_out) named_bar_sync_warps(1 + quarter, 128);
       }
 #pragma unroll 1
       for (int cb = cb0; cb < nb; cb += cbs) {
@@ -619,7 +619,7 @@ q4_gemm3_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       } else {                                             // publish: sums, then the count
         __threadfence();
         __syncwarp();
-        if (shared_out) named_bar_sync(1 + quarter, 128);
+        if (shared_out) named_bar_sync_warps(1 + quarter, 128);
         if (lane == 0) atomicAdd(sh.cnt, 1u);
       }
       if (sh.reducer && lane == 0) *sh.cnt = 0;            // every contributor has been counted: ready for the next launch
