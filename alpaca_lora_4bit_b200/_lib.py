@@ -46,6 +46,7 @@ _SIGNATURES = {
                             c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "q4_gemm_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                             c_int, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "q4_clear": (c_int, [c_void_p, c_size_t, c_void_p]),
     "q4_capture_id": (c_int, [c_void_p, ctypes.POINTER(c_ulonglong)]),
     "q4_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_size_t, c_void_p, c_void_p]),
     "q4_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
@@ -256,13 +257,16 @@ _GEMM_WS_HEAD = 65536        # arrival counters: zero before the first call, lef
 _capture_workspaces: dict = {}
 
 
-def _of_capture(key, capture: int, nbytes: int, head: int, device: torch.device) -> torch.Tensor:
+def _of_capture(key, capture: int, nbytes: int, head: int, device: torch.device, stream_handle: int) -> torch.Tensor:
     held = _capture_workspaces.get(key)
     if held is None or held[0] != capture:
         held = _capture_workspaces[key] = (capture, [])
     if not held[1] or held[1][-1].numel() < nbytes:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        ws[:head].zero_()
+        if device.type == "cuda":
+            check(lib().q4_clear(ws.data_ptr(), head, stream_handle), "clear")
+        else:
+            ws[:head].zero_()
         held[1].append(ws)
         return ws
     return held[1][-1]
@@ -285,7 +289,7 @@ def workspace_for(device: torch.device, stream_handle: int) -> torch.Tensor:
     key = (device.index, stream_handle)
     capture = _capture_of(stream_handle)
     if capture:
-        return _of_capture(key + ("decode",), capture, _WS_BYTES, _DECODE_WS_HEAD, device)
+        return _of_capture(key + ("decode",), capture, _WS_BYTES, _DECODE_WS_HEAD, device, stream_handle)
     _capture_workspaces.clear()
     ws = _workspaces.get(key)
     if ws is None:
@@ -300,7 +304,7 @@ def gemm_workspace_for(device: torch.device, stream_handle: int, nbytes: int) ->
     key = (device.index, stream_handle)
     capture = _capture_of(stream_handle)
     if capture:
-        return _of_capture(key, capture, max(nbytes, 24 << 20), _GEMM_WS_HEAD, device)
+        return _of_capture(key, capture, max(nbytes, 24 << 20), _GEMM_WS_HEAD, device, stream_handle)
     _capture_workspaces.clear()
     ws = _gemm_workspaces.get(key)
     if ws is None or ws.numel() < nbytes:

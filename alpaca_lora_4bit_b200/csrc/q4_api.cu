@@ -111,6 +111,31 @@ int sm_count() {
 
 }  // namespace q4
 
+namespace q4 {
+// The head of a workspace as a node of a captured graph.  Programmatic on both sides, so that the product behind it is launched
+// meanwhile: every kernel that takes a workspace waits for the earlier kernel before it touches it.
+__global__ void __launch_bounds__(256) clear_kernel(uint4* p, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) p[i] = make_uint4(0, 0, 0, 0);
+}
+}  // namespace q4
+
+extern "C" int q4_clear(void* p, size_t bytes, q4_stream_t stream) {
+  using namespace q4;
+  if (!p) return fail(Q4_E_BADARG, "clear: null pointer");
+  if (!aligned16(p) || bytes % 16 || bytes > (1u << 30)) return fail(Q4_E_ALIGN, "clear: %zu bytes, a multiple of 16 on a 16-byte boundary", bytes);
+  if (bytes == 0) return Q4_OK;
+  if (int e = check_device()) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(bytes < (32u << 12) ? (unsigned)((bytes + 4095) >> 12) : 32); cfg.blockDim = dim3(256); cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, clear_kernel, (uint4*)p, (int)(bytes / 16)), "clear launch");
+}
+
 extern "C" int q4_capture_id(q4_stream_t stream, unsigned long long* out) {
   using namespace q4;
   if (!out) return fail(Q4_E_BADARG, "capture_id: null pointer");

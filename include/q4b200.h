@@ -225,6 +225,9 @@ size_t q4_gemm_workspace_bytes(int K, int N, int G);
  * host that gives every captured graph a workspace of its own - the graph holds the address for as long as it lives -
  * tells captures apart by it. */
 int q4_capture_id(q4_stream_t stream, unsigned long long* out);
+/* Zeroes `bytes` (a multiple of 16) at p (16-byte aligned): the head of a workspace ahead of the first product that takes it,
+ * whose launch it does not hold up as a memset would. */
+int q4_clear(void* p, size_t bytes, q4_stream_t stream);
 
 /* The element-wise work of a decoder layer around the quantised linears, one kernel each way (fp16 in and
  * out, fp32 inside).  The reference leaves these to the stock modules (a handful of framework kernels each:
@@ -325,10 +328,9 @@ int q4_gemv_set_trace(void* device_buffer);
 int q4_gemm_set_trace(void* device_buffer);
 /* Which fused GEMM kernel q4_gemm_fwd / q4_gemm_bwd launch (process-wide; no reference counterpart):
  * 0 = choose per shape (the default: with the number of output columns a multiple of 256, the CTA-pair kernel
- * with 256- or 512-row tiles, whichever its estimate favours, or - forward only, when the caller keeps the
- * zero-term table and promises sequential groups of 64 rows or more - the kernel that holds the dequantised
- * weights in tensor memory, where 256-row tiles would be chosen, where its tiles fit one round, and up to 1024
- * rows; the single-CTA kernel otherwise), 1 = always the single-CTA kernel, 2 / 3 = always the CTA-pair kernel
+ * with 256- or 512-row tiles or - forward only - the kernel that holds the dequantised weights in tensor memory,
+ * whichever is estimated to take less time, and up to 1024 rows always the latter when the caller keeps the zero-term
+ * table and promises sequential groups of 64 rows or more; the single-CTA kernel otherwise), 1 = always the single-CTA kernel, 2 / 3 = always the CTA-pair kernel
  * with 256- / 512-row tiles, 4 = always the weights-in-tensor-memory kernel (calls a forced kernel cannot serve
  * fail with Q4_E_SHAPE), 5 = as 0 without the weights-in-tensor-memory kernel, 6 = that kernel in its sequential or its
  * act-order form.  For tests and measurements. */

@@ -60,6 +60,9 @@ def test_bad_arguments_are_rejected_without_a_device():
     assert L.q4_gemv_set_variant(0) == 0
     assert L.q4_gemv_workspace_bytes(1, 100, 128) == 0
     assert L.q4_gemv_workspace_bytes(16, 11008, 4096) > 0
+    # clear: whole 16-byte words on 16-byte boundaries; nothing to do is done without a device
+    assert L.q4_clear(None, 64, None) == -1 and L.q4_clear(fake, 60, None) == -3 and L.q4_clear(ctypes.c_void_p(0x1004), 64, None) == -3
+    assert L.q4_clear(fake, 0, None) == 0
     # layer handle: made and destroyed on the host; bad geometry and null pointers give no handle
     h = ctypes.c_void_p()
     assert L.q4_layer_create(ctypes.byref(h), fake, fake, None, 128, 128, 1, 128) == -1 and not h.value

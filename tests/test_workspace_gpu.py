@@ -87,3 +87,10 @@ def test_captured_decode_has_a_workspace_of_its_own(M, act_order):
     torch.cuda.synchronize()
     assert not _lib._capture_workspaces
     assert all(torch.equal(a, b) for a, b in zip(eager, want)) and quant_cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("nbytes", [16, 4096, 65536, 131072, (1 << 20) + 16])
+def test_clear(nbytes):
+    buf = torch.full((nbytes + 64,), 7, dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.lib().q4_clear(buf.data_ptr() + 32, nbytes, torch.cuda.current_stream().cuda_stream), "clear")
+    assert int(buf[32:32 + nbytes].sum()) == 0 and bool((buf[:32] == 7).all()) and bool((buf[32 + nbytes:] == 7).all())
