@@ -1,10 +1,11 @@
 // The loss of a causal language model over 16-bit logits: cross entropy in fp32, forward and backward, without the fp32
 // copy of the logits that the framework makes (`logits.float()`, log-softmax, negative log-likelihood).
 //
-// Bound by HBM and the exponentials: the forward reads the logits once, the backward reads them and writes their gradient.
-// The framework's kernels move 24 bytes an element instead of 6: at 1024 x 32000 fp16 the casts took 93 us, log-softmax 71
-// and its backward 110, the two kernels of the likelihood 31; here 22 and 22 us and 2 for the mean (10 and 20 at the rate of a
-// copy).  A CTA of 256 threads per row, so that four rows on an SM cover each other's loads and reductions (512 threads:
+// Bound by HBM and the exponentials: the forward reads the logits once and, where a gradient may be asked for, writes the copy
+// that the backward reads (the caller may write to its own before then); the backward reads that and writes the gradient.
+// The framework's kernels move 24 bytes an element instead of 8: at 1024 x 32000 fp16 the casts took 93 us, log-softmax 71
+// and its backward 110, the two kernels of the likelihood 31; here 24 and 20 us and 2 for the mean (20 and 20 at the rate of a
+// copy; 22 and 22 when the forward wrote nothing and the backward read the caller's logits).  A CTA of 256 threads per row, so that four rows on an SM cover each other's loads and reductions (512 threads:
 // 30 us); a thread keeps a running maximum and the sum of exponentials relative to it, so a row of any length is read once,
 // and all sums are added in a fixed order.
 #include <cuda_bf16.h>

@@ -2,12 +2,13 @@
 the SwiGLU product and the rotary embedding, each one kernel forward and one backward instead of the
 half-dozen framework kernels of the stock modules (``LlamaRMSNorm.forward``, ``LlamaMLP.forward``,
 ``apply_rotary_pos_emb`` of transformers, which the reference's finetune step runs unchanged around its
-quant linears, finetune.py:150-175).
+quant linears, finetune.py:150-175), and the loss of a causal language model over its 16-bit logits.
 
-``patch_llama(model)`` re-routes the three in a transformers LLaMA.  Every operator takes the fused path
-only for fp16 CUDA tensors of a supported shape and otherwise falls back to the stock computation, so a
-patched model still runs (and is tested) on the CPU.  The norm weight and the rotary tables are treated as
-constants in the backward: in a LoRA finetune only the LoRA factors train.
+``patch_llama(model)`` re-routes them, and the skip-path adds, in a transformers LLaMA.  The three
+element-wise operators take the fused path only for fp16 CUDA tensors of a supported shape, the loss for
+fp16 or bf16 CUDA logits, and otherwise fall back to the stock computation, so a patched model still runs
+(and is tested) on the CPU.  The norm weight and the rotary tables are treated as constants in the
+backward: in a LoRA finetune only the LoRA factors train.
 """
 from __future__ import annotations
 
