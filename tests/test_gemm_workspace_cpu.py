@@ -1,4 +1,4 @@
-"""Workspaces of the fused products: one per stream that grows, and one per stream capture."""
+"""Workspaces of decode and fused products: one per stream (the fused one grows), and a capture's own."""
 import gc
 import weakref
 
