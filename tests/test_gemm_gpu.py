@@ -772,7 +772,10 @@ def test_act_order_forward_takes_any_order_of_groups(kind):
     (4096, 11008, 257, True, dict(TILE=288, CUT=1, CLUSTER=1)), (11008, 4096, 1100, True, dict(TILE=384, CUT=1, CLUSTER=1)),
     (4096, 4096, 77, True, dict(TILE=96, CLUSTER=3)), (8192, 1024, 128, True, dict(TILE=128, CUT=1, CLUSTER=1))])
 def test_forms_of_the_tensor_memory_kernel(K, N, M, act_order, form):
-    """Every form of the kernel that a cut, a cluster, a tall tile or an act-order layer makes, by the plan of this device."""
-    p = gemm_plan.plan(M, K, N, K // 128, act_order, resident=None)
+    """Every form of the kernel that a cut, a cluster, a tall tile or an act-order layer makes, by the plan for a B200 that holds
+    33 / 22 / 15 clusters of two to four pairs at once (another one's products are right too, in other forms)."""
+    p = gemm_plan.plan(M, K, N, K // 128, act_order)
     assert p[gemm_plan.KERNEL] == 4 and p[gemm_plan.ACT] == act_order and {k: p[getattr(gemm_plan, k)] for k in form} == form, p
     _product_with_everything(synth.make_layer(K, N, 128, act_order=act_order, seed=K + M).to(DEV), M, M)
+    if gemm_plan.plan(M, K, N, K // 128, act_order, resident=None) != p:
+        pytest.skip("this device holds other numbers of clusters at once")
